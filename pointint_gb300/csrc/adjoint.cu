@@ -351,6 +351,7 @@ struct ChainObj {
   int64_t n_elems, pool_off, grad_off;   // grad_off: offset (doubles) of this object's DoF gradient
   const unsigned char* src;             // reference-layout packed source
   const double* dofs;
+  const int32_t* perm;                  // pool entry -> element, or nullptr
 };
 
 struct TriSrcC { double a[3], e1[3], e2[3], S[3]; int32_t vid0, vid1, vid2, pad; };
@@ -367,10 +368,11 @@ __global__ void chain_affine_kernel(const ChainObj* objs, const float* __restric
   double acc[18];
 #pragma unroll
   for (int a = 0; a < 18; ++a) acc[a] = 0.0;
-  for (int64_t e = threadIdx.x; e < o.n_elems; e += blockDim.x) {
+  for (int64_t p = threadIdx.x; p < o.n_elems; p += blockDim.x) {
+    const int64_t e = o.perm ? o.perm[p] : p;
     if (o.geom_type == PI_GEOM_TRIANGLE) {
       const TriSrcC& t = reinterpret_cast<const TriSrcC*>(o.src)[e];
-      const float* g = tri_g + 9 * (o.pool_off + e);
+      const float* g = tri_g + 9 * (o.pool_off + p);
       const double v[3][3] = {{t.a[0], t.a[1], t.a[2]},
                               {t.a[0] + t.e1[0], t.a[1] + t.e1[1], t.a[2] + t.e1[2]},
                               {t.a[0] + t.e2[0], t.a[1] + t.e2[1], t.a[2] + t.e2[2]}};
@@ -382,7 +384,7 @@ __global__ void chain_affine_kernel(const ChainObj* objs, const float* __restric
         }
     } else {
       const SurfSrcC& s = reinterpret_cast<const SurfSrcC*>(o.src)[e];
-      const float* g = surf_g + 12 * (o.pool_off + e);
+      const float* g = surf_g + 12 * (o.pool_off + p);
       for (int r = 0; r < 3; ++r) {
         acc[r] += g[r];
         for (int c = 0; c < 3; ++c) acc[3 + 3 * r + c] += (double)g[r] * s.c[c] + (double)g[3 + r] * s.n[c];
@@ -506,7 +508,8 @@ int launch_dof_gradients(const pi_kgrid_impl* kg, pi_batch_impl* b, const float2
   for (int i = 0; i < n; ++i) {
     const HostObjInfo& in = b->info[i];
     co[i] = ChainObj{in.geom_type, in.dof_type, in.n_elems, in.pool_off, goff,
-                     static_cast<const unsigned char*>(b->d_src) + in.src_off, b->d_dofs + in.dof_off};
+                     static_cast<const unsigned char*>(b->d_src) + in.src_off, b->d_dofs + in.dof_off,
+                     in.perm_off >= 0 ? b->d_perm + in.perm_off : nullptr};
     goff += in.n_dofs;
     any_mesh |= in.dof_type == PI_DOF_TRIANGLE_MESH;
   }

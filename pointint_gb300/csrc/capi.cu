@@ -14,6 +14,7 @@
 #include <vector>
 #include "pi_internal.h"
 #include "group.h"
+#include "moments.h"
 
 using namespace pi;
 
@@ -84,7 +85,8 @@ __global__ void jacobian_to_qd_kernel(const float2* __restrict__ G, int64_t Q, i
 // Vertex -> (triangle, slot) adjacency of every TriangleMeshDoF object, for
 // the deterministic per-vertex gather of the adjoint.  Device-resident
 // elements are read back once.
-int build_vertex_csr(pi_batch_impl* b, const pi_object* objs, int on_device, cudaStream_t s) {
+int build_vertex_csr(pi_batch_impl* b, const pi_object* objs, const std::vector<int32_t>& perm, int on_device,
+                     cudaStream_t s) {
   int64_t nv = 0, goff = 0;
   std::vector<int64_t> voff(b->n_obj, -1), gofs(b->n_obj);
   for (int i = 0; i < b->n_obj; ++i) {
@@ -107,10 +109,12 @@ int build_vertex_csr(pi_batch_impl* b, const pi_object* objs, int on_device, cud
       T = tmp.data();
     }
     const int64_t nvi = in.n_dofs / 3;
+    std::vector<int32_t> pos(in.perm_off >= 0 ? in.n_elems : 0);  // pool entry of each element
+    for (int64_t p = 0; p < (int64_t)pos.size(); ++p) pos[perm[in.perm_off + p]] = (int32_t)p;
     for (int64_t f = 0; f < in.n_elems; ++f) {
       const int32_t v[3] = {T[f].vid0, T[f].vid1, T[f].vid2};
       if (v[0] < 0 || v[1] < 0 || v[2] < 0 || v[0] >= nvi || v[1] >= nvi || v[2] >= nvi) continue;
-      for (int sl = 0; sl < 3; ++sl) adj[voff[i] + v[sl]].push_back((in.pool_off + f) * 3 + sl);
+      for (int sl = 0; sl < 3; ++sl) adj[voff[i] + v[sl]].push_back((in.pool_off + (pos.empty() ? f : pos[f])) * 3 + sl);
     }
   }
   std::vector<int64_t> row(nv + 1, 0), ent, vmap(nv);
@@ -251,6 +255,77 @@ std::vector<double> direction_vectors(const double* dirs, const double* kmag, in
   return dv;
 }
 
+// Whether the cluster expansions apply (KGridDev::moments): unit directions,
+// ascending radii, at least MOMENT_MIN_L of them (their set-up is shared by
+// the radii) and no more than their running sums in shared memory allow.
+bool moment_grid(const std::vector<double>& dv, const std::vector<float2>& km, int64_t M, int64_t L, bool tensor) {
+  if (!tensor || L < MOMENT_MIN_L || L > MOMENT_MAX_L) return false;
+  for (int64_t r = 1; r < L; ++r)
+    if (!(km[r].x >= km[r - 1].x)) return false;
+  for (int64_t j = 0; j < M; ++j) {
+    const double n2 = dv[3 * j] * dv[3 * j] + dv[3 * j + 1] * dv[3 * j + 1] + dv[3 * j + 2] * dv[3 * j + 2];
+    if (!(std::fabs(n2 - 1.0) < 1e-6)) return false;
+  }
+  return km[0].x >= 0.f;
+}
+
+// Order of an object's elements in which every PI_CLUSTER consecutive entries
+// are compact in space: recursive bisection of the anchors (centroids of
+// triangles, centres of surfels) at the widest coordinate, the lower part
+// taking whole clusters.  Coordinates that are not finite count as 0.
+struct OrderPoint { float x[3]; int32_t id; };
+
+void bisect_order(OrderPoint* p, int64_t n) {
+  while (n > PI_CLUSTER) {
+    float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int64_t t = 0; t < n; ++t)
+      for (int c = 0; c < 3; ++c) { mn[c] = std::min(mn[c], p[t].x[c]); mx[c] = std::max(mx[c], p[t].x[c]); }
+    int ax = 0;
+    for (int c = 1; c < 3; ++c) if (mx[c] - mn[c] > mx[ax] - mn[ax]) ax = c;
+    const int64_t mid = ((n + PI_CLUSTER - 1) / PI_CLUSTER / 2) * PI_CLUSTER;
+    std::nth_element(p, p + mid, p + n, [ax](const OrderPoint& a, const OrderPoint& b) {
+      return a.x[ax] < b.x[ax] || (a.x[ax] == b.x[ax] && a.id < b.id);
+    });
+    bisect_order(p, mid);
+    p += mid;
+    n -= mid;
+  }
+}
+
+// Appends the order of `o`'s elements to perm (host elements).
+void append_order(const pi_object& o, std::vector<int32_t>& perm) {
+  std::vector<OrderPoint> pts(o.n_elems);
+  for (int64_t e = 0; e < o.n_elems; ++e) {
+    double x[3];
+    if (o.geom_type == PI_GEOM_TRIANGLE) {
+      const pi_tri_packed& t = static_cast<const pi_tri_packed*>(o.elems)[e];
+      for (int c = 0; c < 3; ++c) x[c] = t.a[c] + (t.e1[c] + t.e2[c]) / 3.0;
+      if (o.dof_type == PI_DOF_TRIANGLE_MESH && t.vid0 >= 0 && t.vid1 >= 0 && t.vid2 >= 0)
+        for (int c = 0; c < 3; ++c)
+          x[c] = (o.dofs[3 * (int64_t)t.vid0 + c] + o.dofs[3 * (int64_t)t.vid1 + c] + o.dofs[3 * (int64_t)t.vid2 + c]) / 3.0;
+    } else {
+      const pi_disk_packed& d = static_cast<const pi_disk_packed*>(o.elems)[e];
+      for (int c = 0; c < 3; ++c) x[c] = d.c[c];
+    }
+    for (int c = 0; c < 3; ++c) pts[e].x[c] = std::isfinite((float)x[c]) ? (float)x[c] : 0.f;
+    pts[e].id = (int32_t)e;
+  }
+  bisect_order(pts.data(), o.n_elems);
+  for (const OrderPoint& p : pts) perm.push_back(p.id);
+}
+
+// Element gradients from pool order (width floats per element) to element order.
+__global__ void unpermute_kernel(BatchDev b, int tri, int width, const float* __restrict__ in, float* __restrict__ out) {
+  const ObjDev od = b.objs[blockIdx.y];
+  if ((od.type == PI_GEOM_TRIANGLE) != (tri != 0)) return;
+  const int64_t n = (int64_t)od.n_elems * width;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t p = t / width, c = t - p * width;
+    const int64_t e = od.perm_off >= 0 ? b.perm[od.perm_off + p] : p;
+    out[(od.elem_off + e) * width + c] = in[od.elem_off * width + t];
+  }
+}
+
 }  // namespace
 
 extern "C" {
@@ -346,6 +421,7 @@ int pi_kgrid_create(const double* dirs, const double* kmag, const double* w, int
   kg->dev.dpair = reinterpret_cast<const int2*>(base + o_pair);
   kg->dev.Me = (int)Me;
   kg->Me = (int)Me;
+  kg->dev.moments = moment_grid(dv, km, M, L, tensor) ? 1 : 0;
   *out = kg.release();
   return PI_OK;
 }
@@ -399,6 +475,9 @@ int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t 
   int64_t dof_count = 0;
   std::vector<char> owns_src(n, 1);  // whether object i's source is copied (first of its array)
   std::unordered_map<const void*, int> first_of;  // element array -> first object naming it
+  std::vector<int32_t> perm;  // element orders of the objects, one per distinct element array and DoF kind
+  std::unordered_map<const void*, int> order_of;  // element array -> first object ordered by it
+  int64_t n_clusters = 0;
   for (int i = 0; i < n; ++i) {
     int rc = validate_object(objs[i], i);
     if (rc) return rc;
@@ -423,12 +502,27 @@ int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t 
     dof_count += in.n_dofs;
     if (in.geom_type == PI_GEOM_TRIANGLE) { in.pool_off = b->n_tri; b->n_tri += in.n_elems; }
     else { in.pool_off = b->n_surf; b->n_surf += in.n_elems; }
+    in.cl_off = n_clusters;
+    n_clusters += (in.n_elems + PI_CLUSTER - 1) / PI_CLUSTER;
+    in.perm_off = -1;
     if (!on_device && in.dof_type == PI_DOF_TRIANGLE_MESH) {
       const pi_tri_packed* T = static_cast<const pi_tri_packed*>(objs[i].elems);
       const int64_t nv = in.n_dofs / 3;
       for (int64_t f = 0; f < in.n_elems; ++f)
         if (T[f].vid0 >= nv || T[f].vid1 >= nv || T[f].vid2 >= nv)
           return fail(PI_ERR_INVALID_ARGUMENT, "TriangleMeshDoF vertex index beyond the DoF vector");
+    }
+    // one cluster needs no order; elements that live on the device keep theirs
+    if (!on_device && in.n_elems > PI_CLUSTER) {
+      auto it = order_of.find(objs[i].elems);
+      if (in.dof_type == PI_DOF_AFFINE && it != order_of.end() && b->info[it->second].n_elems == in.n_elems &&
+          b->info[it->second].geom_type == in.geom_type) {
+        in.perm_off = b->info[it->second].perm_off;
+      } else {
+        in.perm_off = (int64_t)perm.size();
+        append_order(objs[i], perm);
+        if (in.dof_type == PI_DOF_AFFINE) order_of.emplace(objs[i].elems, i);
+      }
     }
   }
   b->order.resize(n);
@@ -439,7 +533,7 @@ int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t 
     cudaFree(b->d_block); cudaFree(b->d_vrow); cudaFree(b->d_vent); cudaFree(b->d_vmap);
   };
   // one device allocation carved into the batch's buffers (256-byte aligned)
-  const size_t sizes[9] = {std::max<size_t>(src_bytes, 16),
+  const size_t sizes[12] = {std::max<size_t>(src_bytes, 16),
                            std::max<size_t>(dof_count * sizeof(double), 16),
                            std::max<size_t>(b->n_tri * 3 * sizeof(float4), 16),
                            std::max<size_t>(b->n_surf * 2 * sizeof(float4), 16),
@@ -447,9 +541,12 @@ int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t 
                            std::max<size_t>(b->n_surf * sizeof(float4), 16),
                            std::max<size_t>(b->n_surf * sizeof(float4), 16),
                            std::max<size_t>(n * sizeof(ObjDev), 16),
-                           std::max<size_t>(n * sizeof(int32_t), 16)};
-  size_t offs[9], total = 0;
-  for (int i = 0; i < 9; ++i) {
+                           std::max<size_t>(n * sizeof(int32_t), 16),
+                           std::max<size_t>(perm.size() * sizeof(int32_t), 16),
+                           std::max<size_t>(n_clusters * sizeof(float4), 16),
+                           std::max<size_t>(n * sizeof(unsigned), 16)};
+  size_t offs[12], total = 0;
+  for (int i = 0; i < 12; ++i) {
     offs[i] = total;
     total += (sizes[i] + 255) & ~(size_t)255;
   }
@@ -465,6 +562,9 @@ int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t 
   b->d_surf_nref = reinterpret_cast<float4*>(blk + offs[6]);
   b->d_objs = reinterpret_cast<ObjDev*>(blk + offs[7]);
   b->d_order = reinterpret_cast<int32_t*>(blk + offs[8]);
+  b->d_perm = reinterpret_cast<int32_t*>(blk + offs[9]);
+  b->d_clusters = reinterpret_cast<float4*>(blk + offs[10]);
+  b->d_cl_rho = reinterpret_cast<unsigned*>(blk + offs[11]);
   if (on_device) {
     for (int i = 0; i < n && e == cudaSuccess; ++i) {
       const HostObjInfo& in = b->info[i];
@@ -490,8 +590,10 @@ int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t 
   }
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(b->d_order, b->order.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess && !perm.empty())
+    e = cudaMemcpyAsync(b->d_perm, perm.data(), perm.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) { cleanup(); return cuda_fail(e, "pi_batch_create upload"); }
-  int rc0 = build_vertex_csr(b.get(), objs, on_device, s);
+  int rc0 = build_vertex_csr(b.get(), objs, perm, on_device, s);
   if (rc0) { cleanup(); return rc0; }
   int rc = launch_prepare(b.get(), -1, s);
   if (rc) { cleanup(); return rc; }
@@ -648,10 +750,18 @@ int pi_element_gradients(pi_kgrid kg, pi_batch b, const void* d_Jw, const double
   float *tg = nullptr, *sg = nullptr;
   int rc = launch_adjoint_elements(kg, b, static_cast<const float2*>(d_Jw), W, &tg, &sg, d_ws, ws_bytes, s);
   if (rc) return rc;
-  if (d_tri_grad && b->n_tri)
-    PI_CUDA(cudaMemcpyAsync(d_tri_grad, tg, b->n_tri * 9 * sizeof(float), cudaMemcpyDeviceToDevice, s));
-  if (d_surf_grad && b->n_surf)
-    PI_CUDA(cudaMemcpyAsync(d_surf_grad, sg, b->n_surf * 12 * sizeof(float), cudaMemcpyDeviceToDevice, s));
+  if ((d_tri_grad && b->n_tri) || (d_surf_grad && b->n_surf)) {
+    if (b->n_obj > 65535) return fail(PI_ERR_UNSUPPORTED, "more than 65535 objects in one batch");
+    const dim3 grid((unsigned)std::max(1, std::min(64, 1024 / b->n_obj)), (unsigned)b->n_obj);
+    if (d_tri_grad && b->n_tri) {
+      unpermute_kernel<<<grid, 256, 0, s>>>(b->dev(), 1, 9, tg, d_tri_grad);
+      PI_LAUNCHED("unpermute_kernel");
+    }
+    if (d_surf_grad && b->n_surf) {
+      unpermute_kernel<<<grid, 256, 0, s>>>(b->dev(), 0, 12, sg, d_surf_grad);
+      PI_LAUNCHED("unpermute_kernel");
+    }
+  }
   return PI_OK;
 }
 

@@ -28,6 +28,7 @@
 #include "pi_internal.h"
 #include "dfmath.cuh"
 #include "bessel.cuh"
+#include "moments.h"
 
 namespace pi {
 
@@ -41,7 +42,7 @@ struct PrepObj {
   int64_t n_elems, n_dofs;
   const unsigned char* src;
   const double* dofs;
-  int64_t pool_off;
+  int64_t pool_off, perm_off, cl_off;
 };
 
 __device__ __forceinline__ void affine_apply(const double* d, const double* x, double* y, bool translate) {
@@ -70,7 +71,7 @@ __device__ __forceinline__ void anchor(const PrepObj& o, int64_t e, double* y) {
 
 // One CTA per object: fixed-order mean of the anchors (deterministic), plus
 // the object's A for the surfel k' = A^T k rule.
-__global__ void prepare_origin_kernel(const PrepObj* objs, ObjDev* out, int only) {
+__global__ void prepare_origin_kernel(const PrepObj* objs, ObjDev* out, unsigned* cl_rho, int only) {
   const int oi = only >= 0 ? only : blockIdx.x;
   const PrepObj o = objs[oi];
   __shared__ double red[3][256];
@@ -102,22 +103,37 @@ __global__ void prepare_origin_kernel(const PrepObj* objs, ObjDev* out, int only
     d.type = o.geom_type;
     d.n_elems = (int32_t)o.n_elems;
     d.elem_off = o.pool_off;
+    d.perm_off = o.perm_off;
+    d.cl_off = o.cl_off;
     out[oi] = d;
+    cl_rho[oi] = 0u;  // prepare_elems_kernel takes the maximum
   }
 }
 
-// grid (x: element blocks, y: object).  Writes the FP32 local-frame pools.
-__global__ void prepare_elems_kernel(const PrepObj* objs, const ObjDev* od, float4* tri_pool, float4* surf_pool,
-                                     float4* tri_lo, float4* surf_lo, float4* surf_nref, int only) {
+constexpr int PREP_THREADS = 256;
+static_assert(PREP_THREADS % PI_CLUSTER == 0 && PI_CLUSTER == 64, "a cluster is two warps of the preparing CTA");
+
+// grid (x: blocks of pool entries, y: object).  Writes the FP32 local-frame
+// pools and the bounding sphere of every cluster: its centre (that of the
+// bounding box, an FP32 point) and its radius, which for a surfel includes the
+// reach of its own expansion, rho |A| for a disk and 2.5 sigma |A| for a
+// Gaussian (the n-th root of E|Z|^n at n = 16 is 2.48).
+__global__ void __launch_bounds__(PREP_THREADS)
+prepare_elems_kernel(const PrepObj* objs, const ObjDev* od, float4* tri_pool, float4* surf_pool, float4* tri_lo,
+                     float4* surf_lo, float4* surf_nref, const int32_t* perm, float4* clusters, unsigned* cl_rho,
+                     int only) {
   const int oi = only >= 0 ? only : blockIdx.y;
   const PrepObj o = objs[oi];
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= o.n_elems) return;
+  if ((int64_t)blockIdx.x * blockDim.x >= o.n_elems) return;
+  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const double* org = od[oi].origin;
-  if (o.geom_type == PI_GEOM_TRIANGLE) {
+  float v[3][3];        // points that bound the entry (triangles: vertices), object frame
+  float reach = 0.f;    // added to their distance from the centre
+  bool ok = p < o.n_elems;
+  const int64_t e = !ok ? 0 : o.perm_off >= 0 ? perm[o.perm_off + p] : p;
+  if (ok && o.geom_type == PI_GEOM_TRIANGLE) {
     const TriSrc& t = reinterpret_cast<const TriSrc*>(o.src)[e];
     double a[3], e1[3], e2[3];
-    bool ok = true;
     if (o.dof_type == PI_DOF_TRIANGLE_MESH) {
       int64_t nv = o.n_dofs / 3;
       ok = t.vid0 >= 0 && t.vid1 >= 0 && t.vid2 >= 0 && t.vid0 < nv && t.vid1 < nv && t.vid2 < nv;
@@ -132,50 +148,99 @@ __global__ void prepare_elems_kernel(const PrepObj* objs, const ObjDev* od, floa
       affine_apply(o.dofs, t.e1, e1, false);
       affine_apply(o.dofs, t.e2, e2, false);
     }
-    float4* dst = tri_pool + 3 * (o.pool_off + e);
+    float4* dst = tri_pool + 3 * (o.pool_off + p);
     if (!ok) {  // unset vertex ids contribute nothing (triangle_mesh_dof.cpp:44-45)
       dst[0] = make_float4(0.f, 0.f, 0.f, 0.f); dst[1] = dst[0]; dst[2] = dst[0];
-      tri_lo[o.pool_off + e] = dst[0];
-      return;
+      tri_lo[o.pool_off + p] = dst[0];
+    } else {
+      double S[3] = {0.5 * (e1[1] * e2[2] - e1[2] * e2[1]), 0.5 * (e1[2] * e2[0] - e1[0] * e2[2]),
+                     0.5 * (e1[0] * e2[1] - e1[1] * e2[0])};
+      // centroid m = a + (e1 + e2)/3 relative to the object origin, FP32 hi + lo;
+      // beside its low word the longest edge (the series-length bound k |e|max)
+      const double l1 = e1[0] * e1[0] + e1[1] * e1[1] + e1[2] * e1[2];
+      const double l2 = e2[0] * e2[0] + e2[1] * e2[1] + e2[2] * e2[2];
+      const double l3 = (e2[0] - e1[0]) * (e2[0] - e1[0]) + (e2[1] - e1[1]) * (e2[1] - e1[1]) +
+                        (e2[2] - e1[2]) * (e2[2] - e1[2]);
+      const float lmax = (float)sqrt(fmax(fmax(l1, l2), l3));
+      float mh[3], ml[3];
+      for (int c = 0; c < 3; ++c) {
+        const double m = a[c] + (e1[c] + e2[c]) / 3.0 - org[c];
+        mh[c] = (float)m;
+        ml[c] = (float)(m - (double)mh[c]);
+        const double r = a[c] - org[c];
+        v[0][c] = (float)r; v[1][c] = (float)(r + e1[c]); v[2][c] = (float)(r + e2[c]);
+      }
+      dst[0] = make_float4(mh[0], mh[1], mh[2], (float)S[0]);
+      tri_lo[o.pool_off + p] = make_float4(ml[0], ml[1], ml[2], lmax);
+      dst[1] = make_float4((float)e1[0], (float)e1[1], (float)e1[2], (float)S[1]);
+      dst[2] = make_float4((float)e2[0], (float)e2[1], (float)e2[2], (float)S[2]);
     }
-    double S[3] = {0.5 * (e1[1] * e2[2] - e1[2] * e2[1]), 0.5 * (e1[2] * e2[0] - e1[0] * e2[2]),
-                   0.5 * (e1[0] * e2[1] - e1[1] * e2[0])};
-    // centroid m = a + (e1 + e2)/3 relative to the object origin, FP32 hi + lo;
-    // beside its low word the longest edge (the series-length bound k |e|max)
-    const double l1 = e1[0] * e1[0] + e1[1] * e1[1] + e1[2] * e1[2];
-    const double l2 = e2[0] * e2[0] + e2[1] * e2[1] + e2[2] * e2[2];
-    const double l3 = (e2[0] - e1[0]) * (e2[0] - e1[0]) + (e2[1] - e1[1]) * (e2[1] - e1[1]) +
-                      (e2[2] - e1[2]) * (e2[2] - e1[2]);
-    const float lmax = (float)sqrt(fmax(fmax(l1, l2), l3));
-    float mh[3], ml[3];
-    for (int c = 0; c < 3; ++c) {
-      const double m = a[c] + (e1[c] + e2[c]) / 3.0 - org[c];
-      mh[c] = (float)m;
-      ml[c] = (float)(m - (double)mh[c]);
-    }
-    dst[0] = make_float4(mh[0], mh[1], mh[2], (float)S[0]);
-    tri_lo[o.pool_off + e] = make_float4(ml[0], ml[1], ml[2], lmax);
-    dst[1] = make_float4((float)e1[0], (float)e1[1], (float)e1[2], (float)S[1]);
-    dst[2] = make_float4((float)e2[0], (float)e2[1], (float)e2[2], (float)S[2]);
-  } else {
+  } else if (ok) {
     const SurfSrc& s = reinterpret_cast<const SurfSrc*>(o.src)[e];
     double c[3], n[3];
     affine_apply(o.dofs, s.c, c, true);
     affine_apply(o.dofs, s.n, n, false);  // n' = A n so that k'.n = k.(A n) with k' = A^T k
-    float4* dst = surf_pool + 2 * (o.pool_off + e);
+    float4* dst = surf_pool + 2 * (o.pool_off + p);
     float ch[3], cl[3];
     for (int a = 0; a < 3; ++a) {
       const double r = c[a] - org[a];
       ch[a] = (float)r;
       cl[a] = (float)(r - (double)ch[a]);
+      v[0][a] = v[1][a] = v[2][a] = ch[a];
     }
     dst[0] = make_float4(ch[0], ch[1], ch[2], (float)s.p0);
-    surf_lo[o.pool_off + e] = make_float4(cl[0], cl[1], cl[2], 0.f);
+    surf_lo[o.pool_off + p] = make_float4(cl[0], cl[1], cl[2], 0.f);
     const double nn = s.n[0] * s.n[0] + s.n[1] * s.n[1] + s.n[2] * s.n[2];
     const double in = nn > 0.0 ? 1.0 / sqrt(nn) : 0.0;
-    surf_nref[o.pool_off + e] =
+    surf_nref[o.pool_off + p] =
         make_float4((float)(s.n[0] * in), (float)(s.n[1] * in), (float)(s.n[2] * in), (float)(1.0 - nn));
     dst[1] = make_float4((float)n[0], (float)n[1], (float)n[2], (float)s.p1);
+    // |k'_perp|^2 <= |k'|^2 max(1, |1 - |n|^2| + |n|^2) with |k'| <= |A| |k|
+    double A2 = 0.0;
+    for (int a = 3; a < 12; ++a) A2 += o.dofs[a] * o.dofs[a];
+    reach = (float)((o.geom_type == PI_GEOM_DISK ? 1.0 : 2.5) * fabs(s.p0) *
+                    sqrt(A2 * fmax(1.0, fabs(1.0 - nn) + nn)));
+  }
+  // the cluster's bounding box: within each warp, then over its two warps
+  float lo[3], hi[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    lo[c] = ok ? fminf(fminf(v[0][c], v[1][c]), v[2][c]) : INFINITY;
+    hi[c] = ok ? fmaxf(fmaxf(v[0][c], v[1][c]), v[2][c]) : -INFINITY;
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+      lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], w));
+      hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], w));
+    }
+  }
+  __shared__ float box[PREP_THREADS / 32][6];
+  __shared__ float rad[PREP_THREADS / 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0)
+    for (int c = 0; c < 3; ++c) { box[warp][c] = lo[c]; box[warp][3 + c] = hi[c]; }
+  __syncthreads();
+  float ctr[3], rho = 0.f;
+  bool any = true;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const float l = fminf(box[warp][c], box[warp ^ 1][c]), h = fmaxf(box[warp][3 + c], box[warp ^ 1][3 + c]);
+    any = any && l <= h;
+    ctr[c] = l <= h ? 0.5f * l + 0.5f * h : 0.f;
+  }
+  if (ok)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const float dx = v[i][0] - ctr[0], dy = v[i][1] - ctr[1], dz = v[i][2] - ctr[2];
+      rho = fmaxf(rho, sqrtf(dx * dx + dy * dy + dz * dz) + reach);
+    }
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1) rho = fmaxf(rho, __shfl_xor_sync(0xffffffffu, rho, w));
+  if (lane == 0) rad[warp] = rho;
+  __syncthreads();
+  if ((threadIdx.x & (PI_CLUSTER - 1)) == 0 && p < o.n_elems) {
+    rho = any ? fmaxf(rad[warp], rad[warp + 1]) : 0.f;
+    clusters[o.cl_off + p / PI_CLUSTER] = make_float4(ctr[0], ctr[1], ctr[2], rho);
+    atomicMax(cl_rho + oi, __float_as_uint(rho));  // non-negative floats order like their bits
   }
 }
 
@@ -258,8 +323,11 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
   const int slot = (int)(lin % gridDim.y), cta = (int)(lin / gridDim.y);
   const int oi = SERVE ? evals[slot].obj : b.order[slot];
   const ObjDev od = b.objs[oi];
-  const int nrb = (kg.L + R - 1) / R;
+  // the radii [0, r_first) are moments.cu's
+  const int r_first = moment_radii(kg, od.type, __uint_as_float(b.cl_rho[oi]));
+  const int nrb = (kg.L - r_first + R - 1) / R;
   const int ndt = (kg.Me + 31) / 32;
+  if (cta * FF_WARPS >= ndt * nrb) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Warps of a CTA take neighbouring direction blocks at the same radial
   // block: they see the same radii, so they take the large-spread branch at
@@ -273,7 +341,8 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
   // jm = dpair[.].y (A(-k) = -conj A(k)), when the grid has one.
   const int item = cta * FF_WARPS + warp;
   const int ib = item / ndt, dt = item - ib * ndt;
-  const int rb = ib < nrb ? nrb - 1 - ib : 0;
+  const int rlo = kg.L - (ib + 1) * R;         // the block's radii are rlo .. rlo + R - 1,
+  const int skip = max(0, r_first - rlo);      // of which the first `skip` are not its own
   const int ei = dt * 32 + lane;
   const bool active = item < ndt * nrb && ei < kg.Me;
   int j = 0, jm = -1;
@@ -297,7 +366,7 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
       dl = make_float3((float)(e[0] - (double)dh.x), (float)(e[1] - (double)dh.y), (float)(e[2] - (double)dh.z));
     }
   }
-  // radii r = rb R + i: a warp's radii are neighbours, so warps at small k
+  // radii r = rlo + i: a warp's radii are neighbours, so warps at small k
   // take the short series for every radius of most elements (the lean loop
   // below, chosen once per element for the whole warp), and the branches of
   // the others are taken together more often.
@@ -309,8 +378,8 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
   __shared__ float2 ctab[256];
   for (int t = threadIdx.x; t < 256; t += FF_THREADS) ctab[t] = kg.cis_tab[t];
   if (lane < R) {
-    const int r = rb * R + lane;
-    const bool ok = item < ndt * nrb && r < kg.L;
+    const int r = rlo + lane;
+    const bool ok = item < ndt * nrb && lane >= skip;
     const float2 k = ok ? kg.kmag[r] : make_float2(0.f, 0.f);
     const float2 k2 = ok ? kg.kt256[r] : make_float2(0.f, 0.f);
     krad[warp][lane] = make_float4(k2.x, k2.y, k.x * k.x, k.x * k.x * k.x);
@@ -322,8 +391,8 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
     float v[2][4];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int r = rb * R + 2 * lane + h;
-      const bool ok = item < ndt * nrb && r < kg.L;
+      const int r = rlo + 2 * lane + h;
+      const bool ok = item < ndt * nrb && 2 * lane + h >= skip;
       const float2 k = ok ? kg.kmag[r] : make_float2(0.f, 0.f);
       const float2 k2 = ok ? kg.kt256[r] : make_float2(0.f, 0.f);
       v[h][0] = k2.x; v[h][1] = k2.y; v[h][2] = k.x * k.x; v[h][3] = k.x * k.x * k.x;
@@ -382,6 +451,7 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
             const float2 smh = make_float2(sm.hi, sm.hi), sml = make_float2(sm.lo, sm.lo);
 #pragma unroll
             for (int p = 0; p < R / 2; ++p) {
+              if (2 * p + 1 < skip) continue;
               const float4 kx = ld_shared_f4(kp + 2 * p), ku = ld_shared_f4(kp + 2 * p + 1);
               const cf2 P = cis_tab_df2(ctab, make_float2(kx.x, kx.y), make_float2(kx.z, kx.w), smh, sml);
               const cf2 T = tri_series_eval_short2(tp, make_float2(ku.x, ku.y), make_float2(ku.z, ku.w));
@@ -397,6 +467,7 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
           const float da = -(s1 + s2) * (1.0f / 3.0f), db = da + s1, dc = da + s2;
 #pragma unroll
           for (int i = 0; i < R; ++i) {
+            if (i < skip) continue;
             const float4 kr = ld_shared_f4(kw + i);
             const float2 kt = make_float2(kr.x, kr.y);
             const cf P = cis_tab_df(ctab, kt, sm);  // centroid phase
@@ -463,6 +534,7 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
             const float rr = q0.w * sqrt_fast(fmaxf(perp, 0.f)) * PI_TURN256;  // rho |k'_perp| / kmag, per 1/256 turn
 #pragma unroll
             for (int p = 0; p < R / 2; ++p) {
+              if (2 * p + 1 < skip) continue;
               const float4 kx = ld_shared_f4(kp + 2 * p);
               const float xa = kx.x * rr, xb = kx.y * rr;
               const float Sa = (xa < 1e-10f) ? 1.0f : 2.0f * j1x(xa);
@@ -476,6 +548,7 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
             const float hs = -0.5f * q0.w * q0.w * perp;
 #pragma unroll
             for (int p = 0; p < R / 2; ++p) {
+              if (2 * p + 1 < skip) continue;
               const float4 kx = ld_shared_f4(kp + 2 * p), ku = ld_shared_f4(kp + 2 * p + 1);
               const float2 m = make_float2(__expf(hs * ku.x) * amp, __expf(hs * ku.y) * amp);
               const cf2 P = cis_tab_df2(ctab, make_float2(kx.x, kx.y), make_float2(kx.z, kx.w), sch, scl);
@@ -497,8 +570,8 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
     float m = 0.f;
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-      const int r = rb * R + i;
-      if (r < kg.L) {
+      const int r = rlo + i;
+      if (i >= skip) {
         const int64_t q = (int64_t)r * kg.M + j;
         cf v{acc.sre(i), acc.sim(i)};
         if (kw[i].x * PI_TURN256 * dnorm < 1e-10f) v = cf{0.f, 0.f};  // A(0) = 0 (affine_dof.cpp:64-65)
@@ -524,8 +597,8 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
   float m = 0.f;
 #pragma unroll
   for (int i = 0; i < R; ++i) {
-    const int r = rb * R + i;
-    if (r < kg.L) {
+    const int r = rlo + i;
+    if (i >= skip) {
       const int64_t q = (int64_t)r * kg.M + j;
       const double kd = ((double)kw[i].x + (double)kw[i].y) * (6.283185307179586476925 / 256.0);
       cf v = cmul(cis_f64(kd * so_d), cf{acc.sre(i), acc.sim(i)});
@@ -568,6 +641,8 @@ int launch_prepare(pi_batch_impl* b, int only_index, cudaStream_t s) {
     p.src = static_cast<const unsigned char*>(b->d_src) + in.src_off;
     p.dofs = b->d_dofs + in.dof_off;
     p.pool_off = in.pool_off;
+    p.perm_off = in.perm_off;
+    p.cl_off = in.cl_off;
     if (only_index < 0 || only_index == i) max_elems = std::max(max_elems, in.n_elems);
   }
   if (b->n_obj == 0) return PI_OK;
@@ -575,12 +650,13 @@ int launch_prepare(pi_batch_impl* b, int only_index, cudaStream_t s) {
   PI_CUDA(cudaMallocAsync((void**)&d, sizeof(PrepObj) * h.size(), s));
   PI_CUDA(cudaMemcpyAsync(d, h.data(), sizeof(PrepObj) * h.size(), cudaMemcpyHostToDevice, s));
   const int nobj_launch = only_index >= 0 ? 1 : b->n_obj;
-  prepare_origin_kernel<<<nobj_launch, 256, 0, s>>>(d, b->d_objs, only_index);
+  prepare_origin_kernel<<<nobj_launch, 256, 0, s>>>(d, b->d_objs, b->d_cl_rho, only_index);
   PI_LAUNCHED("prepare_origin_kernel");
   if (max_elems > 0) {
-    dim3 grid((unsigned)((max_elems + 255) / 256), (unsigned)nobj_launch);
-    prepare_elems_kernel<<<grid, 256, 0, s>>>(d, b->d_objs, b->d_tri_pool, b->d_surf_pool, b->d_tri_lo,
-                                              b->d_surf_lo, b->d_surf_nref, only_index);
+    dim3 grid((unsigned)((max_elems + PREP_THREADS - 1) / PREP_THREADS), (unsigned)nobj_launch);
+    prepare_elems_kernel<<<grid, PREP_THREADS, 0, s>>>(d, b->d_objs, b->d_tri_pool, b->d_surf_pool, b->d_tri_lo,
+                                                       b->d_surf_lo, b->d_surf_nref, b->d_perm, b->d_clusters,
+                                                       b->d_cl_rho, only_index);
     PI_LAUNCHED("prepare_elems_kernel");
   }
   // The host staging array `h` has been consumed by the copy above once the
@@ -614,7 +690,7 @@ int launch_form_factors(const pi_kgrid_impl* kg, const pi_batch_impl* b, int sca
     default: ff_kernel<2, false><<<grid, FF_THREADS, 0, s>>>(K, B, J, scale_sqrt_w, nullptr, ra); break;
   }
   PI_LAUNCHED("ff_kernel");
-  return PI_OK;
+  return launch_moments(kg, b, scale_sqrt_w, J, s, row_amax);
 }
 
 int ff_serve_threads() { return FF_THREADS; }
@@ -645,6 +721,12 @@ int launch_form_factors_serve(const pi_kgrid_impl* kg, const pi_batch_impl* lib,
   void* args[6] = {&K, &B, &none, &scale, const_cast<EvalDev**>(&evals), &no_amax};
   PI_CUDA(cudaLaunchKernel(ff_serve_fn(kg), dim3((unsigned)ff_serve_grid_x(kg), (unsigned)n_evals), dim3(FF_THREADS),
                            args, 0, s));
+  count_launch();
+  if (!K.moments) return PI_OK;
+  int rc = moment_setup();
+  if (rc) return rc;
+  PI_CUDA(cudaLaunchKernel(moment_serve_fn(), dim3((unsigned)moment_serve_grid_x(kg), (unsigned)n_evals),
+                           dim3((unsigned)moment_threads()), args, (size_t)moment_smem_bytes(K.L), s));
   count_launch();
   return PI_OK;
 }

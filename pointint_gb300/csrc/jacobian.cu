@@ -279,7 +279,7 @@ jac_affine_tri_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, 
       tile[6 * e + 2] = pool[3 * (int64_t)(base + e) + 2];
       // the reference vertex a0 and edges E1, E2; in .w the reference
       // doubled area vector N0 = E1 x E2
-      const TriSrcJ& s = src[base + e];
+      const TriSrcJ& s = src[od.perm_off >= 0 ? b.perm[od.perm_off + base + e] : base + e];
       const double n0x = s.e1[1] * s.e2[2] - s.e1[2] * s.e2[1], n0y = s.e1[2] * s.e2[0] - s.e1[0] * s.e2[2],
                    n0z = s.e1[0] * s.e2[1] - s.e1[1] * s.e2[0];
       tile[6 * e + 3] = make_float4((float)s.a[0], (float)s.a[1], (float)s.a[2], (float)n0x);
@@ -437,7 +437,7 @@ jac_affine_surf_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs,
     for (int e = threadIdx.x; e < cnt; e += JAC_THREADS) {
       tile[4 * e] = pool[2 * (int64_t)(base + e)];
       tile[4 * e + 1] = pool[2 * (int64_t)(base + e) + 1];
-      const SurfSrcJ& s = src[base + e];  // reference centre c0 and normal n0
+      const SurfSrcJ& s = src[od.perm_off >= 0 ? b.perm[od.perm_off + base + e] : base + e];  // reference centre c0 and normal n0
       tile[4 * e + 2] = make_float4((float)s.c[0], (float)s.c[1], (float)s.c[2], 0.f);
       tile[4 * e + 3] = make_float4((float)s.n[0], (float)s.n[1], (float)s.n[2], 0.f);
       tile[4 * JAC_TILE + e] = pool_lo[base + e];  // centre low word

@@ -1,0 +1,50 @@
+// Cluster expansions of the form factors at small k (moments.cu): which radii
+// of an object they cover.
+#pragma once
+#include <cuda_runtime.h>
+#include "pi_internal.h"
+
+namespace pi {
+
+// An element of a cluster lies within the cluster's bounding radius rho of its
+// centre, so its form factor is e^{i k.c} times a power series in k whose
+// n-th term is at most (k rho)^n / n! of the element's amplitude, and for a
+// triangle 2 / ((n + 1)(n + 2)) of that.  With the MOMENT_TERMS = 16 terms
+// kept, the first dropped one is below 1.4e-8 (triangles, k rho <= 3) and
+// 2.1e-8 (surfels, k rho <= 2.25) for an element on the rim seen edge-on, and
+// orders of magnitude below that for the others of its cluster.
+constexpr int MOMENT_TERMS = 16;
+constexpr float MOMENT_X_TRI = 3.0f, MOMENT_X_SURF = 2.25f;
+
+// Radii a grid needs for the expansions to pay (an element's moments cost
+// about as much as two radii of the direct sum), and at most as many as the
+// running sums of moments.cu fit in shared memory.
+constexpr int MOMENT_MIN_L = 8, MOMENT_MAX_L = 288;
+
+#ifdef __CUDACC__
+// The radii [0, n) that the expansions of an object cover (radii ascend on a
+// grid with kg.moments); every lane of a warp calls this together.
+__device__ __forceinline__ int moment_radii(const KGridDev& kg, int type, float rho) {
+  if (!kg.moments) return 0;
+  const float bound = type == PI_GEOM_TRIANGLE ? MOMENT_X_TRI : MOMENT_X_SURF;
+  int n = 0;
+  for (int r0 = 0; r0 < kg.L; r0 += 32) {
+    const int r = r0 + (int)(threadIdx.x & 31);
+    n += __popc(__ballot_sync(0xffffffffu, r < kg.L && kg.kmag[r].x * rho <= bound));
+  }
+  return n;
+}
+#endif
+
+// Form factors of the radii below moment_radii; ff_kernel evaluates the others.
+int launch_moments(const pi_kgrid_impl* kg, const pi_batch_impl* b, int scale_sqrt_w, float2* J, cudaStream_t s,
+                   float* row_amax);
+// Serving evaluations: a node with this function, block and shared memory, the
+// arguments of ff_serve_fn's, grid (moment_serve_grid_x, n_evals).
+const void* moment_serve_fn();
+int moment_threads();
+int moment_serve_grid_x(const pi_kgrid_impl* kg);
+int moment_smem_bytes(int L);
+int moment_setup();
+
+}  // namespace pi

@@ -59,6 +59,10 @@ struct KGridDev {
   // a time into compact clusters of directions; otherwise (j, -1) in order.
   const int2* dpair;
   int Me;
+  // Whether the cluster expansions of moments.cu apply: a tensor grid of unit
+  // directions whose radii ascend, so that "k rho <= bound" selects the first
+  // radii (moment_radii).
+  int moments;
 };
 
 struct pi_kgrid_impl {
@@ -79,7 +83,12 @@ struct ObjDev {
   int32_t type;           // PI_GEOM_*
   int32_t n_elems;
   int64_t elem_off;       // offset (in elements) into the pool of its type
+  int64_t perm_off;       // its slice of BatchDev::perm, or -1: pool order is element order
+  int64_t cl_off;         // its first cluster in BatchDev::clusters
 };
+
+// Elements per cluster: PI_CLUSTER consecutive pool entries of one object.
+constexpr int PI_CLUSTER = 64;
 
 // Pools in the kernels' layout, object-local frame, FP32:
 //   triangles: 3 x float4 per element  (m.xyz, S.x) (e1.xyz, S.y) (e2.xyz, S.z), m the centroid
@@ -90,6 +99,8 @@ struct ObjDev {
 // surf_nref: (n / |n|, 1 - |n|^2) of the reference-frame normal n, for
 // |k'_perp|^2 = |k'|^2 - (k'.n)^2 = |k'|^2 (1 - |n|^2) + |n|^2 |k' x n/|n||^2
 // without the cancellation of the difference form near the normal.
+// Pool entry p of an object holds its element perm[perm_off + p]: the host
+// orders elements so that PI_CLUSTER consecutive entries are compact in space.
 struct BatchDev {
   int n_obj;
   const ObjDev* objs;
@@ -99,6 +110,9 @@ struct BatchDev {
   const float4* tri_lo;
   const float4* surf_lo;
   const float4* surf_nref;
+  const int32_t* perm;
+  const float4* clusters;    // (centre, bounding radius) of each cluster, object frame
+  const unsigned* cl_rho;    // per object: FP32 bits of its largest cluster radius
 };
 
 // One form-factor evaluation of the serving path: library object `obj`,
@@ -121,6 +135,8 @@ struct HostObjInfo {
   int64_t src_off;           // byte offset of its packed source in the source arena
   int64_t dof_off;           // offset (doubles) into the dof arena
   int64_t pool_off;          // element offset in its pool
+  int64_t perm_off;          // its slice of the element permutation, or -1 (identity)
+  int64_t cl_off;            // its first cluster
 };
 
 struct pi_batch_impl {
@@ -137,6 +153,9 @@ struct pi_batch_impl {
   float4* d_tri_lo = nullptr;
   float4* d_surf_lo = nullptr;
   float4* d_surf_nref = nullptr;
+  int32_t* d_perm = nullptr;
+  float4* d_clusters = nullptr;
+  unsigned* d_cl_rho = nullptr;
   ObjDev* d_objs = nullptr;
   int32_t* d_order = nullptr;
   // TriangleMeshDoF vertex adjacency (CSR over every mesh object's vertices):
@@ -150,6 +169,7 @@ struct pi_batch_impl {
     BatchDev b;
     b.n_obj = n_obj; b.objs = d_objs; b.order = d_order; b.tri_pool = d_tri_pool; b.surf_pool = d_surf_pool;
     b.tri_lo = d_tri_lo; b.surf_lo = d_surf_lo; b.surf_nref = d_surf_nref;
+    b.perm = d_perm; b.clusters = d_clusters; b.cl_rho = d_cl_rho;
     return b;
   }
 };

@@ -43,6 +43,7 @@
 #include <vector>
 #include "pi_internal.h"
 #include "group.h"
+#include "moments.h"
 
 using namespace pi;
 
@@ -97,7 +98,7 @@ struct Slot {
   GroupDev g{};
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  cudaGraphNode_t n_h2d = nullptr, n_ff = nullptr, n_d2h_out = nullptr;
+  cudaGraphNode_t n_h2d = nullptr, n_ff = nullptr, n_fm = nullptr, n_d2h_out = nullptr;
   bool ff_enabled = true;
   // current batch
   bool busy = false;
@@ -241,6 +242,18 @@ int build_graph(Server& S, Slot& sl) {
   kp.sharedMemBytes = 0;
   kp.kernelParams = ff_args;
   PI_CUDA(cudaGraphAddKernelNode(&sl.n_ff, sl.graph, &n_err, 1, &kp));
+  // beside it (other radii of the same rows) the cluster expansions
+  cudaGraphNode_t evaluated[2] = {sl.n_ff, nullptr};
+  if (K.moments) {
+    int rc = moment_setup();
+    if (rc) return rc;
+    kp.func = const_cast<void*>(moment_serve_fn());
+    kp.gridDim = dim3((unsigned)moment_serve_grid_x(S.kg), 1);
+    kp.blockDim = dim3((unsigned)moment_threads());
+    kp.sharedMemBytes = (unsigned)moment_smem_bytes(K.L);
+    PI_CUDA(cudaGraphAddKernelNode(&sl.n_fm, sl.graph, &n_err, 1, &kp));
+    evaluated[1] = sl.n_fm;
+  }
   // row maxima of the new rows into the pool
   const int32_t* n_evals = &reinterpret_cast<const GHeader*>(sl.d_io + S.lay.hdr)->n_evals;
   void* cm_args[2] = {&evals, const_cast<int32_t**>(&n_evals)};
@@ -250,7 +263,7 @@ int build_graph(Server& S, Slot& sl) {
   cmp.blockDim = dim3((unsigned)amax_commit_threads());
   cmp.kernelParams = cm_args;
   cudaGraphNode_t n_commit = nullptr;
-  PI_CUDA(cudaGraphAddKernelNode(&n_commit, sl.graph, &sl.n_ff, 1, &cmp));
+  PI_CUDA(cudaGraphAddKernelNode(&n_commit, sl.graph, evaluated, K.moments ? 2 : 1, &cmp));
   // contraction
   void* con_args[2] = {&sl.g, &S.pool_map};
   cudaKernelNodeParams cpar{};
@@ -544,9 +557,17 @@ int launch_batch(Server& S, Slot& sl, const std::vector<cudaEvent_t>& waits) {
       kp.blockDim = dim3((unsigned)ff_serve_threads());
       kp.kernelParams = ff_args;
       PI_CUDA(cudaGraphExecKernelNodeSetParams(sl.exec, sl.n_ff, &kp));
+      if (K.moments) {
+        kp.func = const_cast<void*>(moment_serve_fn());
+        kp.gridDim = dim3((unsigned)moment_serve_grid_x(S.kg), (unsigned)sl.n_evals);
+        kp.blockDim = dim3((unsigned)moment_threads());
+        kp.sharedMemBytes = (unsigned)moment_smem_bytes(K.L);
+        PI_CUDA(cudaGraphExecKernelNodeSetParams(sl.exec, sl.n_fm, &kp));
+      }
     }
     if (ff != sl.ff_enabled) {
       PI_CUDA(cudaGraphNodeSetEnabled(sl.exec, sl.n_ff, ff ? 1u : 0u));
+      if (sl.n_fm) PI_CUDA(cudaGraphNodeSetEnabled(sl.exec, sl.n_fm, ff ? 1u : 0u));
       sl.ff_enabled = ff;
     }
     PI_CUDA(cudaGraphExecMemcpyNodeSetParams1D(sl.exec, sl.n_d2h_out, sl.h_io + S.lay.err, sl.d_io + S.lay.err,
