@@ -22,6 +22,7 @@
 //    its own outputs (no reduction across threads), 32-element partials in
 //    registers and compensated running sums in shared memory; each output
 //    element is written once, in the contraction's operand layout.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <algorithm>
@@ -302,8 +303,8 @@ struct Acc {
       im(i) = 0.f;
     }
   }
-  __device__ __forceinline__ float sre(int i) const { return run[4 * i * FF_THREADS]; }
-  __device__ __forceinline__ float sim(int i) const { return run[(4 * i + 1) * FF_THREADS]; }
+  __device__ __forceinline__ float& sre(int i) const { return run[4 * i * FF_THREADS]; }
+  __device__ __forceinline__ float& sim(int i) const { return run[(4 * i + 1) * FF_THREADS]; }
 };
 
 // The grid is (CTAs per object) x (objects or evaluations); the CTAs are
@@ -315,11 +316,16 @@ struct Acc {
 // the k directions, local-frame direction-major output, row maximum);
 // otherwise it indexes the batch's objects (largest first) and J is written
 // q-major with the origin phase.
+// The CTAs of a thread-block cluster (S along x) take the same object,
+// directions and radii and split the elements; their running sums meet
+// through distributed shared memory, each CTA writing every S-th radius.
 template <int R, bool SERVE>
-__global__ void __launch_bounds__(FF_THREADS, 5)
-ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, const EvalDev* __restrict__ evals,
-          unsigned* __restrict__ row_amax) {
-  const unsigned lin = blockIdx.y * gridDim.x + blockIdx.x;
+__device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, float2* __restrict__ J,
+                                        int scale_sqrt_w, const EvalDev* __restrict__ evals,
+                                        unsigned* __restrict__ row_amax) {
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const unsigned lin = (blockIdx.y * gridDim.x + blockIdx.x) / (unsigned)S;
   const int slot = (int)(lin % gridDim.y), cta = (int)(lin / gridDim.y);
   const int oi = SERVE ? evals[slot].obj : b.order[slot];
   const ObjDev od = b.objs[oi];
@@ -409,17 +415,20 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
   __shared__ float run_sm[4 * R * FF_THREADS];
   Acc<R> acc;
   acc.init(run_sm);
+  float2 total[R];
 
   // tile[0, 3 FF_TILE): the elements' pool entries (surfels use the first
   // 2 FF_TILE and put their unit normals at tile[2 FF_TILE + e]);
   // tile[3 FF_TILE + e]: the low word of element e's centroid (centre).
   __shared__ float4 tile[4 * FF_TILE];
-  const int n = od.n_elems;
+  // this CTA's elements [n0, n), whole chunks
+  const int per = (od.n_elems + S * FF_CHUNK - 1) / (S * FF_CHUNK) * FF_CHUNK;
+  const int n0 = min(od.n_elems, rank * per), n = min(od.n_elems, n0 + per);
 
   if (od.type == PI_GEOM_TRIANGLE) {
     const float4* src = b.tri_pool + 3 * od.elem_off;
     const float4* lo = b.tri_lo + od.elem_off;
-    for (int base = 0; base < n; base += FF_TILE) {
+    for (int base = n0; base < n; base += FF_TILE) {
       const int cnt = min(FF_TILE, n - base);
       __syncthreads();
       for (int t = threadIdx.x; t < 3 * cnt; t += FF_THREADS) tile[t] = src[3 * (int64_t)base + t];
@@ -504,7 +513,7 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
                                  Am[2] * dh.x + Am[5] * dh.y + Am[8] * dh.z);
     const float qd = fmaf(v.x, v.x, fmaf(v.y, v.y, v.z * v.z));
     const float4* nref = b.surf_nref + od.elem_off;
-    for (int base = 0; base < n; base += FF_TILE) {
+    for (int base = n0; base < n; base += FF_TILE) {
       const int cnt = min(FF_TILE, n - base);
       __syncthreads();
       for (int t = threadIdx.x; t < 2 * cnt; t += FF_THREADS) tile[t] = src[2 * (int64_t)base + t];
@@ -563,15 +572,36 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
     }
   }
 
-  if (!active) return;
   acc.flush();
+  const auto mine = [&](int i) { return (i & (S - 1)) == rank; };  // S is a power of two
+  if (S > 1) {
+    cluster.sync();
+    // the sums of this CTA's radii over the cluster; compensated, in the
+    // order of the ranks
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      if (!mine(i)) continue;
+      kbsum re{0.f, 0.f}, im{0.f, 0.f};
+      for (int q = 0; q < S; ++q) {
+        const float* o = cluster.map_shared_rank(run_sm, q) + 4 * i * FF_THREADS + threadIdx.x;
+        re.add(o[0]); im.add(o[FF_THREADS]);
+        re.lo -= o[2 * FF_THREADS]; im.lo -= o[3 * FF_THREADS];
+      }
+      total[i] = make_float2(re.hi + re.lo, im.hi + im.lo);
+    }
+    cluster.sync();  // no CTA leaves while its sums are read
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+      if (mine(i)) { acc.sre(i) = total[i].x; acc.sim(i) = total[i].y; }
+  }
+  if (!active) return;
   if (SERVE) {
     const EvalDev& ev = evals[slot];
     float m = 0.f;
 #pragma unroll
     for (int i = 0; i < R; ++i) {
       const int r = rlo + i;
-      if (i >= skip) {
+      if (i >= skip && mine(i)) {
         const int64_t q = (int64_t)r * kg.M + j;
         cf v{acc.sre(i), acc.sim(i)};
         if (kw[i].x * PI_TURN256 * dnorm < 1e-10f) v = cf{0.f, 0.f};  // A(0) = 0 (affine_dof.cpp:64-65)
@@ -598,7 +628,7 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const int r = rlo + i;
-    if (i >= skip) {
+    if (i >= skip && mine(i)) {
       const int64_t q = (int64_t)r * kg.M + j;
       const double kd = ((double)kw[i].x + (double)kw[i].y) * (6.283185307179586476925 / 256.0);
       cf v = cmul(cis_f64(kd * so_d), cf{acc.sre(i), acc.sim(i)});
@@ -625,6 +655,28 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
 __global__ void to_double2_kernel(const float2* __restrict__ J, int64_t n, double2* __restrict__ out) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) { float2 v = J[i]; out[i] = make_double2(v.x, v.y); }
+}
+
+}  // namespace
+
+namespace {
+
+template <int R>
+__global__ void __launch_bounds__(FF_THREADS, 5)
+ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, const EvalDev* __restrict__ evals,
+          unsigned* __restrict__ row_amax) {
+  ff_body<R, false>(kg, b, J, scale_sqrt_w, evals, row_amax);
+}
+
+// Serving evaluations always split their elements over FF_SERVE_SPLIT CTAs: a
+// row's value must not depend on the batch it is evaluated in.
+constexpr int FF_SERVE_SPLIT = 4;
+
+template <int R>
+__global__ void __cluster_dims__(FF_SERVE_SPLIT, 1, 1) __launch_bounds__(FF_THREADS, 5)
+ff_serve_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, const EvalDev* __restrict__ evals,
+                unsigned* __restrict__ row_amax) {
+  ff_body<R, true>(kg, b, J, scale_sqrt_w, evals, row_amax);
 }
 
 }  // namespace
@@ -673,22 +725,27 @@ int launch_form_factors(const pi_kgrid_impl* kg, const pi_batch_impl* b, int sca
   unsigned* ra = reinterpret_cast<unsigned*>(row_amax);
   const KGridDev K = kg->dev;
   const BatchDev B = b->dev();
+  if (b->n_obj > 65535) return fail(PI_ERR_UNSUPPORTED, "more than 65535 objects in one batch");
   int R = radii_per_thread(K.L);
   const int ndt = (K.Me + 31) / 32;
   auto ctas = [&](int r) { return ((int64_t)((K.L + r - 1) / r) * ndt + FF_WARPS - 1) / FF_WARPS; };
-  // a launch of fewer than two CTAs per SM at 8 radii per thread, such as
-  // one moving mesh of the alignment caller (76 CTAs), takes 4, which fills
-  // twice the SMs; above that 8 radii share the per-element work better
-  // (the 8-object surfel sample, 608 CTAs: 64.1 ms at 8, 68.6 ms at 4)
-  const int n_sm = current_sm_count();
-  if (R == 8 && ctas(8) * b->n_obj < 2 * (int64_t)n_sm) R = 4;
-  dim3 grid((unsigned)ctas(R), (unsigned)b->n_obj);
-  if (grid.y > 65535) return fail(PI_ERR_UNSUPPORTED, "more than 65535 objects in one batch");
-  switch (R) {
-    case 8: ff_kernel<8, false><<<grid, FF_THREADS, 0, s>>>(K, B, J, scale_sqrt_w, nullptr, ra); break;
-    case 4: ff_kernel<4, false><<<grid, FF_THREADS, 0, s>>>(K, B, J, scale_sqrt_w, nullptr, ra); break;
-    default: ff_kernel<2, false><<<grid, FF_THREADS, 0, s>>>(K, B, J, scale_sqrt_w, nullptr, ra); break;
-  }
+  // CTAs that carry the launch: those of the objects of at least a quarter of
+  // the largest one's elements, for the fifth of the radii that the cluster
+  // expansions usually leave
+  const int64_t n_max = b->info[b->order[0]].n_elems;
+  int64_t heavy = 0;
+  for (int i = 0; i < b->n_obj; ++i) heavy += 4 * b->info[i].n_elems >= n_max;
+  auto busy = [&](int r) { return (K.moments ? (ctas(r) + 4) / 5 : ctas(r)) * heavy; };
+  const int64_t full = 10 * (int64_t)current_sm_count();  // two waves of five CTAs per SM
+  if (R == 8 && 16 * busy(8) < full) R = 4;
+  int S = 1;
+  while (S < 16 && S * busy(R) < full && n_max > 2 * S * FF_CHUNK) S *= 2;
+  const void* fn = R == 8   ? reinterpret_cast<const void*>(ff_kernel<8>)
+                   : R == 4 ? reinterpret_cast<const void*>(ff_kernel<4>)
+                            : reinterpret_cast<const void*>(ff_kernel<2>);
+  const EvalDev* no_evals = nullptr;
+  void* args[6] = {const_cast<KGridDev*>(&K), const_cast<BatchDev*>(&B), &J, &scale_sqrt_w, &no_evals, &ra};
+  if (int rc = launch_split(fn, dim3((unsigned)(ctas(R) * S), (unsigned)b->n_obj), FF_THREADS, 0, S, args, s)) return rc;
   PI_LAUNCHED("ff_kernel");
   return launch_moments(kg, b, scale_sqrt_w, J, s, row_amax);
 }
@@ -698,14 +755,14 @@ int ff_serve_threads() { return FF_THREADS; }
 int ff_serve_grid_x(const pi_kgrid_impl* kg) {
   const int R = radii_per_thread(kg->dev.L);
   const int64_t items = (int64_t)((kg->dev.L + R - 1) / R) * ((kg->dev.Me + 31) / 32);
-  return (int)((items + FF_WARPS - 1) / FF_WARPS);
+  return (int)((items + FF_WARPS - 1) / FF_WARPS) * FF_SERVE_SPLIT;
 }
 
 const void* ff_serve_fn(const pi_kgrid_impl* kg) {
   switch (radii_per_thread(kg->dev.L)) {
-    case 8: return reinterpret_cast<const void*>(ff_kernel<8, true>);
-    case 4: return reinterpret_cast<const void*>(ff_kernel<4, true>);
-    default: return reinterpret_cast<const void*>(ff_kernel<2, true>);
+    case 8: return reinterpret_cast<const void*>(ff_serve_kernel<8>);
+    case 4: return reinterpret_cast<const void*>(ff_serve_kernel<4>);
+    default: return reinterpret_cast<const void*>(ff_serve_kernel<2>);
   }
 }
 

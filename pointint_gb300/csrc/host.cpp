@@ -10,6 +10,7 @@
 #include <vector>
 #include <atomic>
 #include <map>
+#include <set>
 #include <mutex>
 #include <utility>
 #include "pi_internal.h"
@@ -52,6 +53,35 @@ int ensure_smem_limit(const void* fn, int bytes, const char* what) {
     it = done.emplace(std::make_pair(fn, dev), cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes))
              .first;
   return it->second == cudaSuccess ? PI_OK : cuda_fail(it->second, what);
+}
+
+int launch_split(const void* fn, dim3 grid, int threads, size_t smem, int split, void** args, cudaStream_t s) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  if (split > 1) {
+    if (split > 8) {
+      static std::mutex mu;
+      static std::set<std::pair<const void*, int>> done;  // (function, device)
+      int dev = 0;
+      PI_CUDA(cudaGetDevice(&dev));
+      std::lock_guard<std::mutex> lock(mu);
+      if (!done.count({fn, dev})) {
+        PI_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        done.insert({fn, dev});
+      }
+    }
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)split;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+  }
+  PI_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
+  return PI_OK;
 }
 
 }  // namespace pi

@@ -36,6 +36,7 @@
 //   2. each warp sums the tile's clusters over its own radii, 8 at a time in
 //      registers (two per packed instruction), and adds them to compensated
 //      running sums in shared memory.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
@@ -211,14 +212,18 @@ __device__ __forceinline__ float2 horner8(const float (&c)[8], float2 u) {
   return r;
 }
 
-// SERVE as in ff_kernel.  The grid is (direction groups) x (objects or
-// evaluations), re-mapped so that the objects (largest first) vary fastest.
+// SERVE and the S CTAs of a thread-block cluster as in ff_kernel: they take
+// every S-th tile, and their running sums meet at the end.  The grid is
+// (direction groups x S) x (objects or evaluations), re-mapped so that the
+// objects (largest first) vary fastest.
 template <bool SERVE>
-__global__ void __launch_bounds__(FM_THREADS, 2)
-moment_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, const EvalDev* __restrict__ evals,
-              unsigned* __restrict__ row_amax) {
+__device__ __forceinline__ void moment_body(const KGridDev& kg, const BatchDev& b, float2* __restrict__ J,
+                                            int scale_sqrt_w, const EvalDev* __restrict__ evals,
+                                            unsigned* __restrict__ row_amax) {
   extern __shared__ float4 sm[];
-  const unsigned lin = blockIdx.y * gridDim.x + blockIdx.x;
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const unsigned lin = (blockIdx.y * gridDim.x + blockIdx.x) / (unsigned)S;
   const int slot = (int)(lin % gridDim.y), dt = (int)(lin / gridDim.y);
   const int oi = SERVE ? evals[slot].obj : b.order[slot];
   const ObjDev od = b.objs[oi];
@@ -281,7 +286,7 @@ moment_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w,
   for (int t = threadIdx.x; t < nb * FM_R * 32; t += FM_THREADS) run[t] = make_float4(0.f, 0.f, 0.f, 0.f);
 
   const int ncl = (od.n_elems + PI_CLUSTER - 1) / PI_CLUSTER;
-  for (int t0 = 0; t0 < ncl; t0 += FM_WARPS) {
+  for (int t0 = rank * FM_WARPS; t0 < ncl; t0 += S * FM_WARPS) {
     __syncthreads();  // the last tile's coefficients have been read (and the tables written, before the first)
     const int cl = t0 + warp;
     if (cl < ncl) {
@@ -350,14 +355,19 @@ moment_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w,
       }
     }
   }
-  __syncthreads();
-  if (!active) return;
+  if (S > 1) cluster.sync();
+  else __syncthreads();
   float m = 0.f;
   const double so = ((double)D.dh.x + (double)D.dl.x) * od.origin[0] + ((double)D.dh.y + (double)D.dl.y) * od.origin[1] +
                     ((double)D.dh.z + (double)D.dl.z) * od.origin[2];
-  for (int r = warp; r < nr; r += FM_WARPS) {
-    const float4 v4 = run[r * 32 + lane];
-    cf v{v4.x, v4.y};
+  for (int r = warp * S + rank; r < nr && active; r += FM_WARPS * S) {
+    kbsum re{0.f, 0.f}, im{0.f, 0.f};  // over the cluster, in the order of the ranks
+    for (int q = 0; q < S; ++q) {
+      const float4 v4 = (S > 1 ? cluster.map_shared_rank(run, q) : run)[r * 32 + lane];
+      re.add(v4.x); im.add(v4.y);
+      re.lo -= v4.z; im.lo -= v4.w;
+    }
+    cf v{re.hi + re.lo, im.hi + im.lo};
     const float2 km = kg.kmag[r];
     if (!SERVE) {
       const float2 kt = kg.kt256[r];
@@ -379,6 +389,8 @@ moment_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w,
       if (jm >= 0) J[(int64_t)oi * kg.Q + qm] = om;
     }
   }
+  if (S > 1) cluster.sync();  // no CTA leaves while its sums are read
+  if (!active) return;
   unsigned* amax = SERVE ? reinterpret_cast<unsigned*>(evals[slot].amax) : row_amax ? row_amax + oi : nullptr;
   if (amax) {  // FP32 bits order like the non-negative floats
     const unsigned mask = __activemask();
@@ -387,15 +399,30 @@ moment_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w,
   }
 }
 
+__global__ void __launch_bounds__(FM_THREADS, 2)
+moment_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, const EvalDev* __restrict__ evals,
+              unsigned* __restrict__ row_amax) {
+  moment_body<false>(kg, b, J, scale_sqrt_w, evals, row_amax);
+}
+
+// The split of a serving evaluation does not depend on its batch.
+constexpr int FM_SERVE_SPLIT = 2;
+
+__global__ void __cluster_dims__(FM_SERVE_SPLIT, 1, 1) __launch_bounds__(FM_THREADS, 2)
+moment_serve_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w,
+                    const EvalDev* __restrict__ evals, unsigned* __restrict__ row_amax) {
+  moment_body<true>(kg, b, J, scale_sqrt_w, evals, row_amax);
+}
+
 }  // namespace
 
 int moment_threads() { return FM_THREADS; }
 int moment_smem_bytes(int L) { return fm_smem_f4(L) * (int)sizeof(float4); }
-int moment_serve_grid_x(const pi_kgrid_impl* kg) { return (kg->dev.Me + 31) / 32; }
-const void* moment_serve_fn() { return reinterpret_cast<const void*>(moment_kernel<true>); }
+int moment_serve_grid_x(const pi_kgrid_impl* kg) { return (kg->dev.Me + 31) / 32 * FM_SERVE_SPLIT; }
+const void* moment_serve_fn() { return reinterpret_cast<const void*>(moment_serve_kernel); }
 
 int moment_setup() {
-  int rc = ensure_smem_limit(reinterpret_cast<const void*>(moment_kernel<false>), moment_smem_bytes(MOMENT_MAX_L),
+  int rc = ensure_smem_limit(reinterpret_cast<const void*>(moment_kernel), moment_smem_bytes(MOMENT_MAX_L),
                              "moment_kernel");
   if (rc == PI_OK)
     rc = ensure_smem_limit(moment_serve_fn(), moment_smem_bytes(MOMENT_MAX_L), "moment_kernel");
@@ -407,9 +434,20 @@ int launch_moments(const pi_kgrid_impl* kg, const pi_batch_impl* b, int scale_sq
   if (!kg->dev.moments || b->n_obj == 0) return PI_OK;
   int rc = moment_setup();
   if (rc) return rc;
-  const dim3 grid((unsigned)((kg->dev.Me + 31) / 32), (unsigned)b->n_obj);
-  moment_kernel<false><<<grid, FM_THREADS, moment_smem_bytes(kg->dev.L), s>>>(
-      kg->dev, b->dev(), J, scale_sqrt_w, nullptr, reinterpret_cast<unsigned*>(row_amax));
+  // as in launch_form_factors: CTAs of the objects that carry the launch, and
+  // a split of their tiles that gives two waves of two CTAs per SM
+  const int64_t n_max = b->info[b->order[0]].n_elems, ndt = (kg->dev.Me + 31) / 32;
+  int64_t heavy = 0;
+  for (int i = 0; i < b->n_obj; ++i) heavy += 4 * b->info[i].n_elems >= n_max;
+  int S = 1;
+  while (S < 8 && S * ndt * heavy < 4 * (int64_t)current_sm_count() && n_max > S * FM_WARPS * PI_CLUSTER) S *= 2;
+  const KGridDev K = kg->dev;
+  const BatchDev B = b->dev();
+  const EvalDev* no_evals = nullptr;
+  void* args[6] = {const_cast<KGridDev*>(&K), const_cast<BatchDev*>(&B), &J, &scale_sqrt_w, &no_evals, &row_amax};
+  rc = launch_split(reinterpret_cast<const void*>(moment_kernel), dim3((unsigned)(ndt * S), (unsigned)b->n_obj),
+                    FM_THREADS, (size_t)moment_smem_bytes(K.L), S, args, s);
+  if (rc) return rc;
   PI_LAUNCHED("moment_kernel");
   return PI_OK;
 }

@@ -21,6 +21,9 @@ int current_sm_count();
 // once per (function, device): the attribute belongs to the device's context.
 // Returns PI_OK or the first attempt's error status.
 int ensure_smem_limit(const void* fn, int bytes, const char* what);
+// Launches fn with thread-block clusters of `split` CTAs along x (1: none;
+// above 8 the function's non-portable cluster size is allowed first).
+int launch_split(const void* fn, dim3 grid, int threads, size_t smem, int split, void** args, cudaStream_t s);
 
 #define PI_CUDA(call)                                        \
   do {                                                       \
