@@ -43,6 +43,9 @@ namespace {
 constexpr int ADJ_THREADS = 128;
 constexpr int ADJ_DT = 8;        // directions staged per shared-memory tile
 constexpr int ADJ_LMAX = 256;    // radii per direction held in shared memory
+// one copy of the phasor table: the lanes of a warp hold neighbouring elements
+// at one direction and radius, whose phases mostly share an entry (a broadcast)
+constexpr int ADJ_COPIES = 1;
 constexpr double INV8PI3 = 1.0 / (8.0 * 3.14159265358979323846 * 3.14159265358979323846 * 3.14159265358979323846);
 
 // Kahan-compensated FP32 accumulator.
@@ -103,15 +106,15 @@ struct AdjStage {
   int2 jp[ADJ_DT];    // (direction, its antipode or -1); -1, -1 past the last direction
 };
 
-// Per-CTA copies of the radii (double-float |k|, and |k| in 1/256 turns per
+// Per-CTA copies of the radii (double-float |k|, and |k| in 1/64 turns per
 // unit length for the table phasors) and of the phasor table; the first
 // __syncthreads of the direction loop publishes them.
 __device__ __forceinline__ void stage_radii(const KGridDev& kg, float2* km, float2* kt, float2* ctab) {
   for (int r = threadIdx.x; r < kg.L; r += blockDim.x) {
     km[r] = kg.kmag[r];
-    kt[r] = kg.kt256[r];
+    kt[r] = kg.kt64[r];
   }
-  for (int t = threadIdx.x; t < 256; t += blockDim.x) ctab[t] = kg.cis_tab[t];
+  stage_phasors<ADJ_COPIES>(kg.cis_tab, ctab);
 }
 
 // The tile holds evaluated directions e0 .. e0 + ADJ_DT - 1 (KGridDev::dpair).
@@ -178,13 +181,14 @@ __global__ void __launch_bounds__(ADJ_THREADS)
 adj_surf_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const float2* __restrict__ Bw,
                 float* __restrict__ out) {
   __shared__ AdjStage st;
-  __shared__ float2 km[ADJ_LMAX], kt[ADJ_LMAX], ctab[256];
+  __shared__ float2 km[ADJ_LMAX], kt[ADJ_LMAX], ctab_sm[PHASOR_ENTRIES * ADJ_COPIES];
   const AdjWork wk = work[blockIdx.x];
   const ObjDev od = b.objs[wk.obj];
   const int e = wk.first + threadIdx.x;
   const bool valid = e < od.n_elems;
   const bool disk = od.type == PI_GEOM_DISK;
-  stage_radii(kg, km, kt, ctab);
+  stage_radii(kg, km, kt, ctab_sm);
+  const float2* ctab = ctab_sm + (threadIdx.x % ADJ_COPIES);
   float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0, ql = q0, nr = q0;
   if (valid) {
     q0 = b.surf_pool[2 * (od.elem_off + e)];
@@ -221,7 +225,7 @@ adj_surf_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const
       for (int r = 0; r < kg.L; ++r) {
         const float2 Bv = Bj[r];
         const df k = df{km[r].x, km[r].y};
-        const cf P = cis_tab_df(ctab, kt[r], sc);
+        const cf P = cis_tab_df<ADJ_COPIES>(ctab, kt[r], sc);
         const float ure = Bv.x * P.re + Bv.y * P.im;  // Re(conj(B) P)
         const float uim = Bv.x * P.im - Bv.y * P.re;  // Im(conj(B) P)
         const float k2 = k.hi * k.hi;
@@ -257,12 +261,13 @@ __global__ void __launch_bounds__(ADJ_THREADS, 4)
 adj_tri_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const float2* __restrict__ Bw,
                float* __restrict__ out) {
   __shared__ AdjStage st;
-  __shared__ float2 km[ADJ_LMAX], kt[ADJ_LMAX], ctab[256];
+  __shared__ float2 km[ADJ_LMAX], kt[ADJ_LMAX], ctab_sm[PHASOR_ENTRIES * ADJ_COPIES];
   const AdjWork wk = work[blockIdx.x];
   const ObjDev od = b.objs[wk.obj];
   const int e = wk.first + threadIdx.x;
   const bool valid = e < od.n_elems;
-  stage_radii(kg, km, kt, ctab);
+  stage_radii(kg, km, kt, ctab_sm);
+  const float2* ctab = ctab_sm + (threadIdx.x % ADJ_COPIES);
   float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0, q2 = q0, ql = q0;
   if (valid) {
     q0 = b.tri_pool[3 * (od.elem_off + e)];
@@ -299,7 +304,7 @@ adj_tri_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const 
         if (k.hi < kthr) {
           // F = P SF, D_v = P SV with the series as polynomials in k; with
           // BP = conj(B) P, Re(conj(B) X) = Re(BP SX) and D_a = i F - D_b - D_c
-          const cf P = cis_tab_df(ctab, kt[r], sm);
+          const cf P = cis_tab_df<ADJ_COPIES>(ctab, kt[r], sm);
           const float u = k.hi * k.hi, k3 = u * k.hi;
           const float fre = poly_u(cp.fa, u), fim = k3 * poly_u(cp.fb, u);
           const float bim = poly_u(cp.ba, u), bre = k.hi * poly_u(cp.bb, u);
@@ -312,7 +317,7 @@ adj_tri_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const 
           tb = fmaf(k.hi, b_re, tb);
           tc = fmaf(k.hi, c_re, tc);
         } else {
-          const TriDer d = tri_generic_der_at(ctab, kt[r], sa, sb, sc, k.hi * d1.hi, k.hi * d2.hi);
+          const TriDer d = tri_generic_der_at<ADJ_COPIES>(ctab, kt[r], sa, sb, sc, k.hi * d1.hi, k.hi * d2.hi);
           // Re(conj(B) X) = B.re X.re + B.im X.im
           t0 = fmaf(Bv.x, d.F.re, fmaf(Bv.y, d.F.im, t0));
           ta = fmaf(k.hi, fmaf(Bv.x, d.Da.re, Bv.y * d.Da.im), ta);

@@ -16,6 +16,7 @@
 #include <vector>
 #include "pi_internal.h"
 #include "group.h"
+#include "dfmath.cuh"
 #include "moments.h"
 
 using namespace pi;
@@ -272,21 +273,22 @@ bool moment_grid(const std::vector<double>& dv, const std::vector<float2>& km, i
 }
 
 // Order of an object's elements in which every PI_CLUSTER consecutive entries
-// are compact in space: recursive bisection of the anchors (centroids of
-// triangles, centres of surfels) at the widest coordinate, the lower part
-// taking whole clusters.  Coordinates that are not finite count as 0.
+// are compact in space, and every PI_LEAF within them: recursive bisection of
+// the anchors (centroids of triangles, centres of surfels) at the widest
+// coordinate, the lower part taking whole clusters (leaves).  Coordinates that are not finite count as 0.
 struct OrderPoint { float x[3]; int32_t id; };
 
 // Large parts are handed to threads (200,000 elements: 17 -> 4 ms on 16 cores).
 void bisect_order(OrderPoint* p, int64_t n) {
   std::vector<std::future<void>> parts;
-  while (n > PI_CLUSTER) {
+  while (n > PI_LEAF) {
+    const int64_t unit = n > PI_CLUSTER ? PI_CLUSTER : PI_LEAF;
     float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
     for (int64_t t = 0; t < n; ++t)
       for (int c = 0; c < 3; ++c) { mn[c] = std::min(mn[c], p[t].x[c]); mx[c] = std::max(mx[c], p[t].x[c]); }
     int ax = 0;
     for (int c = 1; c < 3; ++c) if (mx[c] - mn[c] > mx[ax] - mn[ax]) ax = c;
-    const int64_t mid = ((n + PI_CLUSTER - 1) / PI_CLUSTER / 2) * PI_CLUSTER;
+    const int64_t mid = ((n + unit - 1) / unit / 2) * unit;
     std::nth_element(p, p + mid, p + n, [ax](const OrderPoint& a, const OrderPoint& b) {
       return a.x[ax] < b.x[ax] || (a.x[ax] == b.x[ax] && a.id < b.id);
     });
@@ -304,6 +306,12 @@ void bisect_order(OrderPoint* p, int64_t n) {
   }
   for (std::future<void>& f : parts) f.get();
 }
+
+// Element x node values from which a one-shot call orders an object's elements:
+// ordering takes ~0.1 us per element on the host, the direct sum of this many
+// values ~0.2 ms on the device.  (In the caller's order the cluster expansions
+// still apply where that order is compact.)
+constexpr double ORDER_MIN_VALUES = 2e8;
 
 // Appends the order of `o`'s elements to perm (host elements).
 void append_order(const pi_object& o, std::vector<int32_t>& perm) {
@@ -355,7 +363,7 @@ int pi_kgrid_create(const double* dirs, const double* kmag, const double* w, int
   const bool tensor = grid_layout(dirs, kmag, Q, &M);
   const int64_t L = tensor ? Q / M : 1;
   std::vector<float4> dh(M), dl(M);
-  std::vector<float2> km(L), kt(L), k256(L), tab(256);
+  std::vector<float2> km(L), kt(L), k256(L), tab(2 * PHASOR_ENTRIES);
   const std::vector<double> dv = direction_vectors(dirs, kmag, M, tensor);
   for (int64_t j = 0; j < M; ++j) {
     double d[3];
@@ -373,13 +381,14 @@ int pi_kgrid_create(const double* dirs, const double* kmag, const double* w, int
     const double u = k / (2.0 * 3.14159265358979323846);
     const float uh = (float)u;
     kt[r] = make_float2(uh, (float)(u - (double)uh));
-    const double v = u * 256.0;
+    const double v = u * 64.0;
     const float vh = (float)v;
     k256[r] = make_float2(vh, (float)(v - (double)vh));
   }
-  for (int j = 0; j < 256; ++j) {
-    const double a = 2.0 * 3.14159265358979323846 * j / 256.0;
+  for (int j = 0; j < PHASOR_ENTRIES; ++j) {
+    const double a = 2.0 * 3.14159265358979323846 * j / PHASOR_ENTRIES;
     tab[j] = make_float2((float)std::cos(a), (float)std::sin(a));
+    tab[PHASOR_ENTRIES + j] = make_float2((float)(-2.0 * std::sin(0.5 * a) * std::sin(0.5 * a)), (float)std::sin(a));
   }
   std::vector<float> sw(Q), sg(Q);
   kg->w.resize(Q);
@@ -394,7 +403,7 @@ int pi_kgrid_create(const double* dirs, const double* kmag, const double* w, int
   const size_t o_dh = 0, o_dl = align16(o_dh + M * sizeof(float4)), o_km = align16(o_dl + M * sizeof(float4)),
                o_sw = align16(o_km + L * sizeof(float2)), o_sg = align16(o_sw + Q * sizeof(float)),
                o_kt = align16(o_sg + Q * sizeof(float)), o_k256 = align16(o_kt + L * sizeof(float2)),
-               o_tab = align16(o_k256 + L * sizeof(float2)), o_pair = align16(o_tab + 256 * sizeof(float2));
+               o_tab = align16(o_k256 + L * sizeof(float2)), o_pair = align16(o_tab + 2 * PHASOR_ENTRIES * sizeof(float2));
   const std::vector<int2> pairs = direction_pairs(dv, M, tensor);
   const int64_t Me = (int64_t)pairs.size();
   {  // every direction is written exactly once, as evaluated or as a mirror
@@ -417,7 +426,7 @@ int pi_kgrid_create(const double* dirs, const double* kmag, const double* w, int
   std::memcpy(host.data() + o_sg, sg.data(), Q * sizeof(float));
   std::memcpy(host.data() + o_kt, kt.data(), L * sizeof(float2));
   std::memcpy(host.data() + o_k256, k256.data(), L * sizeof(float2));
-  std::memcpy(host.data() + o_tab, tab.data(), 256 * sizeof(float2));
+  std::memcpy(host.data() + o_tab, tab.data(), tab.size() * sizeof(float2));
   std::memcpy(host.data() + o_pair, pairs.data(), Me * sizeof(int2));
   PI_CUDA(cudaMalloc(&kg->d_mem, total));
   cudaError_t e = cudaMemcpy(kg->d_mem, host.data(), total, cudaMemcpyHostToDevice);
@@ -431,8 +440,9 @@ int pi_kgrid_create(const double* dirs, const double* kmag, const double* w, int
   kg->dev.sqrtw = reinterpret_cast<const float*>(base + o_sw);
   kg->dev.sign = reinterpret_cast<const float*>(base + o_sg);
   kg->dev.kturn = reinterpret_cast<const float2*>(base + o_kt);
-  kg->dev.kt256 = reinterpret_cast<const float2*>(base + o_k256);
+  kg->dev.kt64 = reinterpret_cast<const float2*>(base + o_k256);
   kg->dev.cis_tab = reinterpret_cast<const float2*>(base + o_tab);
+  kg->dev.cis_tabm = kg->dev.cis_tab + PHASOR_ENTRIES;
   kg->dev.dpair = reinterpret_cast<const int2*>(base + o_pair);
   kg->dev.Me = (int)Me;
   kg->Me = (int)Me;
@@ -478,7 +488,8 @@ namespace {
 // source on the device (instances of one mesh under different DoFs upload
 // it once).  Only batches whose sources are never replaced share them: the
 // host entry points' temporary batches.
-int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t s, bool share_sources,
+// Q: the nodes of the one k-grid the batch is for, or 0 for a batch that is kept.
+int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t s, bool share_sources, int64_t Q,
                       pi_batch* out) {
   if (!out) return fail(PI_ERR_INVALID_ARGUMENT, "pi_batch_create: null output");
   *out = nullptr;
@@ -528,7 +539,7 @@ int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t 
           return fail(PI_ERR_INVALID_ARGUMENT, "TriangleMeshDoF vertex index beyond the DoF vector");
     }
     // one cluster needs no order; elements that live on the device keep theirs
-    if (!on_device && in.n_elems > PI_CLUSTER) {
+    if (!on_device && in.n_elems > PI_CLUSTER && (Q == 0 || (double)in.n_elems * (double)Q >= ORDER_MIN_VALUES)) {
       auto it = order_of.find(objs[i].elems);
       if (in.dof_type == PI_DOF_AFFINE && it != order_of.end() && b->info[it->second].n_elems == in.n_elems &&
           b->info[it->second].geom_type == in.geom_type) {
@@ -548,7 +559,7 @@ int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t 
     cudaFree(b->d_block); cudaFree(b->d_vrow); cudaFree(b->d_vent); cudaFree(b->d_vmap);
   };
   // one device allocation carved into the batch's buffers (256-byte aligned)
-  const size_t sizes[12] = {std::max<size_t>(src_bytes, 16),
+  const size_t sizes[13] = {std::max<size_t>(src_bytes, 16),
                            std::max<size_t>(dof_count * sizeof(double), 16),
                            std::max<size_t>(b->n_tri * 3 * sizeof(float4), 16),
                            std::max<size_t>(b->n_surf * 2 * sizeof(float4), 16),
@@ -559,9 +570,10 @@ int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t 
                            std::max<size_t>(n * sizeof(int32_t), 16),
                            std::max<size_t>(perm.size() * sizeof(int32_t), 16),
                            std::max<size_t>(n_clusters * sizeof(float4), 16),
-                           std::max<size_t>(n * sizeof(unsigned), 16)};
-  size_t offs[12], total = 0;
-  for (int i = 0; i < 12; ++i) {
+                           std::max<size_t>(n * sizeof(unsigned), 16),
+                           std::max<size_t>(n_clusters * (PI_CLUSTER / PI_LEAF) * sizeof(float4), 16)};
+  size_t offs[13], total = 0;
+  for (int i = 0; i < 13; ++i) {
     offs[i] = total;
     total += (sizes[i] + 255) & ~(size_t)255;
   }
@@ -580,6 +592,7 @@ int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t 
   b->d_perm = reinterpret_cast<int32_t*>(blk + offs[9]);
   b->d_clusters = reinterpret_cast<float4*>(blk + offs[10]);
   b->d_cl_rho = reinterpret_cast<unsigned*>(blk + offs[11]);
+  b->d_leaves = reinterpret_cast<float4*>(blk + offs[12]);
   if (on_device) {
     for (int i = 0; i < n && e == cudaSuccess; ++i) {
       const HostObjInfo& in = b->info[i];
@@ -621,7 +634,7 @@ int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t 
 extern "C" {
 
 int pi_batch_create(const pi_object* objs, int n, int on_device, pi_stream stream, pi_batch* out) {
-  return batch_create_impl(objs, n, on_device, reinterpret_cast<cudaStream_t>(stream), false, out);
+  return batch_create_impl(objs, n, on_device, reinterpret_cast<cudaStream_t>(stream), false, 0, out);
 }
 
 int pi_batch_set_dofs(pi_batch b, int index, const double* d_dofs, pi_stream stream) {
@@ -801,7 +814,7 @@ int pi_volume_matrix_host(const pi_object* objs, int n, const double* dirs, cons
   int rc = pi_kgrid_create(dirs, kmag, w, Q, &kg.k);
   if (rc) return rc;
   BatchGuard b;
-  rc = batch_create_impl(objs, n, 0, s, true, &b.b);
+  rc = batch_create_impl(objs, n, 0, s, true, Q, &b.b);
   if (rc) return rc;
   size_t ws_bytes = 0;
   rc = pi_contract_workspace_size(kg.k, n, precision, &ws_bytes);
@@ -843,7 +856,7 @@ static int volume_and_grads_host(const pi_object* objs, int n, const double* dir
   int rc = pi_kgrid_create(dirs, kmag, w, Q, &kg.k);
   if (rc) return rc;
   BatchGuard b;
-  rc = batch_create_impl(objs, n, 0, s, true, &b.b);
+  rc = batch_create_impl(objs, n, 0, s, true, Q, &b.b);
   if (rc) return rc;
   size_t ws_c = 0, ws_a = 0;
   if ((rc = pi_contract_workspace_size(kg.k, n, PI_CONTRACT_FP32, &ws_c)) || (rc = pi_adjoint_workspace_size(kg.k, b.b, &ws_a)))
@@ -923,7 +936,7 @@ static int stacked_gram_host(const pi_object* objs, int n, const double* dirs, c
   int rc = pi_kgrid_create(dirs, kmag, w, Q, &kg.k);
   if (rc) return rc;
   BatchGuard b;
-  rc = batch_create_impl(objs, n, 0, s, true, &b.b);
+  rc = batch_create_impl(objs, n, 0, s, true, Q, &b.b);
   if (rc) return rc;
   const int64_t D = dof_gradient_size(b.b), m = n + D;
   if (m > INT32_MAX) return fail(PI_ERR_UNSUPPORTED, "too many DoFs for the Hessian");
@@ -1007,7 +1020,7 @@ int pi_compute_Ak(const pi_object* obj, const double* dirs, const double* kmag, 
   int rc = pi_kgrid_create(dirs, kmag, nullptr, Q, &kg.k);
   if (rc) return rc;
   BatchGuard b;
-  rc = pi_batch_create(obj, 1, 0, reinterpret_cast<pi_stream>(s), &b.b);
+  rc = batch_create_impl(obj, 1, 0, s, false, Q, &b.b);
   if (rc) return rc;
   DevBuf J;
   if ((rc = J.alloc((size_t)Q * sizeof(float2), s))) return rc;
@@ -1043,7 +1056,7 @@ int pi_compute_Ak_gradient(const pi_object* obj, const double* dirs, const doubl
   int rc = pi_kgrid_create(dirs, kmag, nullptr, Q, &kg.k);  // unit weights: G = dA/dtheta
   if (rc) return rc;
   BatchGuard b;
-  rc = pi_batch_create(obj, 1, 0, reinterpret_cast<pi_stream>(s), &b.b);
+  rc = batch_create_impl(obj, 1, 0, s, false, Q, &b.b);
   if (rc) return rc;
   const int64_t D = obj->n_dofs;
   DevBuf G;

@@ -185,52 +185,77 @@ __device__ __forceinline__ cf cis_f64(double x) {
 }
 
 // ---------------------------------------------------------------------------
-// Table phasors.  A phase given in units of 1/256 turn, y = 256 x / (2 pi),
-// is split as y = n + f with n = round(y) (the 1.5 * 2^23 shift: |y| < 2^22,
-// so |x| < 1.0e5 rad) and |f| <= 1/2; then
-//   e^{i x} = tab[n mod 256] e^{i c f},  c = 2 pi / 256,
-// with tab[j] = e^{2 pi i j / 256} rounded once from FP64 (per component
-// error <= 2^-25) and, on |c f| <= pi / 256 = 0.0123, cos(c f) = 1 - (c f)^2 / 2
-// and sin(c f) = c f - (c f)^3 / 6 (truncation 9.4e-10 and 2.4e-12; Taylor
-// series, whose next terms bound the error on so short an interval).  About
+// Table phasors.  A phase given in units of 1/64 turn, y = 64 x / (2 pi), is
+// split as y = n + f with n = round(y) (the 1.5 * 2^23 shift: |y| < 2^22, so
+// |x| < 4.1e5 rad) and |f| <= 1/2; then
+//   e^{i x} = tab[n mod 64] e^{i c f},  c = 2 pi / 64,
+// with tab[j] = e^{2 pi i j / 64} rounded once from FP64 (per component error
+// <= 2^-25) and, on |c f| <= pi / 64 = 0.049, cos(c f) = 1 - (c f)^2 / 2 +
+// (c f)^4 / 24 and sin(c f) = c f - (c f)^3 / 6 (Taylor series, whose next
+// terms, 1.9e-11 and 2.4e-9, bound the error on so short an interval).  About
 // 7e-8 per component overall, the same order as FP32 rounding of the phasor.
-#define PI_TURN256 0.024543692606170259f  // 2 pi / 256
-#define PI_TURN256_C2 0.00030119642337308832f  // c^2 / 2
-#define PI_TURN256_C3 2.4641574764489986e-06f  // c^3 / 6
+//
+// The table sits in shared memory in C copies, entry j of copy c at
+// [j C + c], and a lane reads copy (lane mod C) (`tab` points to its first
+// entry): with C = 16 the lanes of a half-warp, whose 8-byte reads share the
+// 16 bank pairs, never collide.  One copy of 256 entries, which saves the
+// fourth-power term, costs about 6 shared-memory cycles per lookup at random
+// phases instead of 2: at large k, where an element takes three phasors, the
+// lookups and not the FP32 pipe were the limit.
+#define PI_TURN64 0.098174770424681035f      // 2 pi / 64
+#define PI_TURN64_C2 0.0048191427739694131f  // c^2 / 2
+#define PI_TURN64_C3 0.00015770607849273588f // c^3 / 6
+#define PI_TURN64_C4 3.870689512650268e-06f    // c^4 / 24
+constexpr int PHASOR_ENTRIES = 64, PHASOR_COPIES = 16;
 
-// e^{i c f} times tab[idx] (idx already reduced mod 256).
-// cos = 1 + cm with cm = -(c f)^2 / 2 tiny: tab (cos + i sin) is formed as
+// Copies the grid's table into PHASOR_ENTRIES * C entries of shared memory;
+// every thread of the CTA takes part, a __syncthreads publishes it.
+template <int C>
+__device__ __forceinline__ void stage_phasors(const float2* __restrict__ src, float2* tab) {
+  for (int t = threadIdx.x; t < PHASOR_ENTRIES * C; t += blockDim.x) tab[t] = src[t / C];
+}
+
+// e^{i c f} times entry idx mod 64.
+// cos = 1 + cm with cm tiny: tab (cos + i sin) is formed as
 // tab + tab cm + i tab sin, so both roundings happen at the phasor's scale.
+template <int C>
 __device__ __forceinline__ cf cis_tab_frac(const float2* tab, int idx, float f) {
   const float f2 = f * f;
-  const float cm = f2 * -PI_TURN256_C2;
-  const float sn = f * fmaf(f2, -PI_TURN256_C3, PI_TURN256);
-  const float2 t = tab[idx];
+  const float cm = f2 * fmaf(f2, PI_TURN64_C4, -PI_TURN64_C2);
+  const float sn = f * fmaf(f2, -PI_TURN64_C3, PI_TURN64);
+  const float2 t = tab[(idx & (PHASOR_ENTRIES - 1)) * C];
   return {fmaf(t.x, cm, fmaf(-t.y, sn, t.x)), fmaf(t.y, cm, fmaf(t.x, sn, t.y))};
 }
 
-// e^{i x} with x = 2 pi (kt.hi + kt.lo) (sm.hi + sm.lo) / 256: kt is a radius
-// in units of 1/256 turn per unit length (double-float), sm a direction dot
+// e^{i x} with x = 2 pi (kt.hi + kt.lo) (sm.hi + sm.lo) / 64: kt is a radius
+// in units of 1/64 turn per unit length (double-float), sm a direction dot
 // product (double-float, unnormalised).  The leading product's rounding is
 // recovered by an FMA against the rounded integer, so f carries the full
 // product to ~2^-25 of a unit; the cross terms are added to it (the lo.lo
 // term, ~2^-48 relative, is dropped).
+template <int C = PHASOR_COPIES>
 __device__ __forceinline__ cf cis_tab_df(const float2* tab, float2 kt, df sm) {
   const float t = fmaf(kt.x, sm.hi, PI_ROUND_SHIFT);  // rounds the exact product to an integer
   const float n = t - PI_ROUND_SHIFT;
   float f = fmaf(kt.x, sm.hi, -n);
   f = fmaf(kt.x, sm.lo, f);
   f = fmaf(kt.y, sm.hi, f);
-  return cis_tab_frac(tab, __float_as_int(t) & 255, f);
+  return cis_tab_frac<C>(tab, __float_as_int(t), f);
 }
 
-// The same for an FP32 dot product d (kt still double-float).
-__device__ __forceinline__ cf cis_tab_f(const float2* tab, float2 kt, float d) {
-  const float t = fmaf(kt.x, d, PI_ROUND_SHIFT);
-  const float n = t - PI_ROUND_SHIFT;
-  float f = fmaf(kt.x, d, -n);
-  f = fmaf(kt.y, d, f);
-  return cis_tab_frac(tab, __float_as_int(t) & 255, f);
+// e^{2 pi i kt d / 64} - 1 for FP32 kt and d, to a relative 1e-7 or so however
+// small the phase: tabm holds (cos - 1, sin), rounded once from FP64, and
+//   e^{i(a+b)} - 1 = ta + cm + i sn + ta (cm + i sn),  ta = e^{ia} - 1,
+// b = c f.  (Entry 0 is zero, so short phases come from cm and sn alone.)
+constexpr int PHASOR_M1_COPIES = 8;
+__device__ __forceinline__ cf cis_tab_m1(const float2* tabm, float kt, float d) {
+  const float t = fmaf(kt, d, PI_ROUND_SHIFT);
+  const float f = fmaf(kt, d, PI_ROUND_SHIFT - t);
+  const float f2 = f * f;
+  const float cm = f2 * fmaf(f2, PI_TURN64_C4, -PI_TURN64_C2);
+  const float sn = f * fmaf(f2, -PI_TURN64_C3, PI_TURN64);
+  const float2 a = tabm[(__float_as_int(t) & (PHASOR_ENTRIES - 1)) * PHASOR_M1_COPIES];
+  return {a.x + fmaf(a.x, cm, fmaf(-a.y, sn, cm)), a.y + fmaf(a.y, cm, fmaf(a.x, sn, sn))};
 }
 
 // Two phasors at once with packed FP32 (sm_100 family): radii a, b in the
@@ -242,19 +267,25 @@ struct cf2 { float2 re, im; };
 __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
 __device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
 
+// cis_tab_frac on both halves, the indices in the low bits of t.
+template <int C>
+__device__ __forceinline__ cf2 cis_tab_frac2(const float2* tab, float2 t, float2 f) {
+  const float2 f2 = __fmul2_rn(f, f);
+  const float2 cm = __fmul2_rn(f2, __ffma2_rn(f2, dup2(PI_TURN64_C4), dup2(-PI_TURN64_C2)));
+  const float2 sn = __fmul2_rn(f, __ffma2_rn(f2, dup2(-PI_TURN64_C3), dup2(PI_TURN64)));
+  const float2* ta = tab + (__float_as_int(t.x) & (PHASOR_ENTRIES - 1)) * C;
+  const float2* tb = tab + (__float_as_int(t.y) & (PHASOR_ENTRIES - 1)) * C;
+  const float2 tx = make_float2(ta->x, tb->x), ty = make_float2(ta->y, tb->y);
+  return {__ffma2_rn(tx, cm, __ffma2_rn(neg2(ty), sn, tx)), __ffma2_rn(ty, cm, __ffma2_rn(tx, sn, ty))};
+}
+
+template <int C = PHASOR_COPIES>
 __device__ __forceinline__ cf2 cis_tab_df2(const float2* tab, float2 kth, float2 ktl, float2 smh, float2 sml) {
   const float2 t = __ffma2_rn(kth, smh, dup2(PI_ROUND_SHIFT));
   const float2 mn = __ffma2_rn(t, dup2(-1.0f), dup2(PI_ROUND_SHIFT));  // -n, exact
   float2 f = __ffma2_rn(kth, smh, mn);
   f = __ffma2_rn(kth, sml, f);
-  f = __ffma2_rn(ktl, smh, f);
-  const float2 f2 = __fmul2_rn(f, f);
-  const float2 cm = __fmul2_rn(f2, dup2(-PI_TURN256_C2));
-  const float2 sn = __fmul2_rn(f, __ffma2_rn(f2, dup2(-PI_TURN256_C3), dup2(PI_TURN256)));
-  const float2* ta = tab + (__float_as_int(t.x) & 255);
-  const float2* tb = tab + (__float_as_int(t.y) & 255);
-  const float2 tx = make_float2(ta->x, tb->x), ty = make_float2(ta->y, tb->y);
-  return {__ffma2_rn(tx, cm, __ffma2_rn(neg2(ty), sn, tx)), __ffma2_rn(ty, cm, __ffma2_rn(tx, sn, ty))};
+  return cis_tab_frac2<C>(tab, t, __ffma2_rn(ktl, smh, f));
 }
 
 __device__ __forceinline__ cf cmul(cf a, cf b) { return {a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re}; }
@@ -330,12 +361,25 @@ __device__ __forceinline__ TriPoly tri_series_coeffs(float s1, float s2, float g
   return t;
 }
 
-// u = k^2, k3 = k^3.
-__device__ __forceinline__ cf tri_series_eval(const TriPoly& t, float u, float k3) {
-  const float re = fmaf(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, t.a[6], t.a[5]), t.a[4]), t.a[3]), t.a[2]), t.a[1]), t.a[0]);
-  const float im =
-      k3 * fmaf(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, t.b[5], t.b[4]), t.b[3]), t.b[2]), t.b[1]), t.b[0]);
-  return {re, im};
+// The same coefficients paired for packed FP32: one Horner chain carries the
+// real part in its first half and the imaginary one in its second, so no
+// coefficient is duplicated into both halves of a register pair.
+struct TriPoly2 { float2 c[7]; };
+
+__device__ __forceinline__ TriPoly2 tri_series_coeffs2(float s1, float s2, float g) {
+  const TriPoly t = tri_series_coeffs(s1, s2, g);
+  TriPoly2 r;
+#pragma unroll
+  for (int j = 0; j < 7; ++j) r.c[j] = make_float2(t.a[j], j < 6 ? t.b[j] : 0.f);
+  return r;
+}
+
+__device__ __forceinline__ cf tri_series_eval(const TriPoly2& t, float u, float k3) {
+  const float2 uu = dup2(u);
+  float2 a = t.c[6];
+#pragma unroll
+  for (int j = 5; j >= 0; --j) a = __ffma2_rn(a, uu, t.c[j]);
+  return {a.x, k3 * a.y};
 }
 
 // The coefficients that tri_series_eval_short reads (a[0..3], b[0..2]) alone.
@@ -392,6 +436,50 @@ __device__ __forceinline__ cf dd1(cf Pu, cf Pv, float g) {
   const cf m = cmul(Pu, cf{c, x * sc});
   const bool b = fabsf(g) >= 0.5f;
   return {b ? big.re : -m.im * sc, b ? big.im : m.re * sc};
+}
+
+// Wide spread with the vertices sorted along the direction, u <= v <= w (gaps
+// G2 = v - u, G1 = w - v, D = G1 + G2), k-independent parts formed once per
+// element and direction:
+//   e[u, v, w] = (f[v, w] - f[u, v]) / (k D),
+//   f[v, w] = e^{iv} (e^{ikG1} - 1) / (k G1),
+//   f[u, v] = e^{iv} (1 - e^{-ikG2}) / (k G2),
+// so with M = e^{ikG} - 1 formed without cancellation (cis_tab_m1),
+//   g e = e^{iv} g/(D k^2) ( M1 / G1 + conj(M2) / G2 ).
+// Three phasors, no roles, selects or reciprocals per radius (tri_generic
+// takes four phasors with the centroid's, and at every radius selects its
+// near pair and one of two forms of its divided difference).  The triangle is
+// consistent by construction (the outer vertices are v plus the gaps), so
+// the rounding of the FP32 gaps, and of the FP32 radius in their phases,
+// changes its size by 6e-8.
+struct TriGaps {
+  df sv;           // middle vertex
+  float G1, G2;    // at least 1e-20, so that M / G has its limit i k at a closed gap
+  float i1, i2;    // 1 / G1, 1 / G2
+  float D;
+};
+
+__device__ __forceinline__ TriGaps tri_gaps(float s1, float s2, df sm) {
+  const float lo12 = fminf(s1, s2), hi12 = fmaxf(s1, s2);
+  const float lo = fminf(lo12, 0.f), hi = fmaxf(hi12, 0.f), mid = fmaxf(lo12, fminf(hi12, 0.f));
+  TriGaps t;
+  t.G1 = fmaxf(hi - mid, 1e-20f);
+  t.G2 = fmaxf(mid - lo, 1e-20f);
+  t.D = t.G1 + t.G2;
+  t.i1 = rcp_fast(t.G1);
+  t.i2 = rcp_fast(t.G2);
+  // the middle vertex relative to the centroid, mid - (s1 + s2)/3, hi + lo
+  const float s12 = s1 + s2, off = fmaf(s12, -1.0f / 3.0f, mid), offl = fmaf(s12, -1.0f / 3.0f, mid - off);
+  const df v = two_sum(sm.hi, off);
+  t.sv = df{v.hi, v.lo + (sm.lo + offl)};
+  return t;
+}
+
+// g e[u, v, w] without the factor e^{iv}; tabm: the table of cis_tab_m1, kt
+// the radius in 1/64 turns, gik = g/(D k^2).
+__device__ __forceinline__ cf tri_wide(const float2* tabm, float kt, const TriGaps& t, float gik) {
+  const cf M1 = cis_tab_m1(tabm, kt, t.G1), M2 = cis_tab_m1(tabm, kt, t.G2);
+  return {gik * fmaf(M1.re, t.i1, M2.re * t.i2), gik * fmaf(M1.im, t.i1, -M2.im * t.i2)};
 }
 
 // tri_generic: spread D >= 2 (the form-factor kernel takes it for D >= 3,

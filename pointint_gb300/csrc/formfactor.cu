@@ -115,14 +115,14 @@ constexpr int PREP_THREADS = 256;
 static_assert(PREP_THREADS % PI_CLUSTER == 0 && PI_CLUSTER == 64, "a cluster is two warps of the preparing CTA");
 
 // grid (x: blocks of pool entries, y: object).  Writes the FP32 local-frame
-// pools and the bounding sphere of every cluster: its centre (that of the
+// pools and the bounding sphere of every cluster and leaf: its centre (that of the
 // bounding box, an FP32 point) and its radius, which for a surfel includes the
 // reach of its own expansion, rho |A| for a disk and 2.5 sigma |A| for a
 // Gaussian (the n-th root of E|Z|^n at n = 16 is 2.48).
 __global__ void __launch_bounds__(PREP_THREADS)
 prepare_elems_kernel(const PrepObj* objs, const ObjDev* od, float4* tri_pool, float4* surf_pool, float4* tri_lo,
-                     float4* surf_lo, float4* surf_nref, const int32_t* perm, float4* clusters, unsigned* cl_rho,
-                     int only) {
+                     float4* surf_lo, float4* surf_nref, const int32_t* perm, float4* clusters, float4* leaves,
+                     unsigned* cl_rho, int only) {
   const int oi = only >= 0 ? only : blockIdx.y;
   const PrepObj o = objs[oi];
   if ((int64_t)blockIdx.x * blockDim.x >= o.n_elems) return;
@@ -202,18 +202,30 @@ prepare_elems_kernel(const PrepObj* objs, const ObjDev* od, float4* tri_pool, fl
     reach = (float)((o.geom_type == PI_GEOM_DISK ? 1.0 : 2.5) * fabs(s.p0) *
                     sqrt(A2 * fmax(1.0, fabs(1.0 - nn) + nn)));
   }
-  // the cluster's bounding box: within each warp, then over its two warps
-  float lo[3], hi[3];
+  // the bounding box: of the leaf, within the warp, then over the cluster's two warps
+  float lo[3], hi[3], lctr[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     lo[c] = ok ? fminf(fminf(v[0][c], v[1][c]), v[2][c]) : INFINITY;
     hi[c] = ok ? fmaxf(fmaxf(v[0][c], v[1][c]), v[2][c]) : -INFINITY;
 #pragma unroll
-    for (int w = 16; w > 0; w >>= 1) {
+    for (int w = 1; w < 32; w <<= 1) {
+      if (w == PI_LEAF) lctr[c] = lo[c] <= hi[c] ? 0.5f * lo[c] + 0.5f * hi[c] : 0.f;
       lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], w));
       hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], w));
     }
   }
+  float lrho = 0.f;
+  if (ok)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const float dx = v[i][0] - lctr[0], dy = v[i][1] - lctr[1], dz = v[i][2] - lctr[2];
+      lrho = fmaxf(lrho, sqrtf(dx * dx + dy * dy + dz * dz) + reach);
+    }
+#pragma unroll
+  for (int w = 1; w < PI_LEAF; w <<= 1) lrho = fmaxf(lrho, __shfl_xor_sync(0xffffffffu, lrho, w));
+  if (threadIdx.x % PI_LEAF == 0 && p < o.n_elems)
+    leaves[o.cl_off * (PI_CLUSTER / PI_LEAF) + p / PI_LEAF] = make_float4(lctr[0], lctr[1], lctr[2], lrho);
   __shared__ float box[PREP_THREADS / 32][6];
   __shared__ float rad[PREP_THREADS / 32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -247,6 +259,9 @@ prepare_elems_kernel(const PrepObj* objs, const ObjDev* od, float4* tri_pool, fl
 
 constexpr int FF_THREADS = 128;
 constexpr int FF_WARPS = FF_THREADS / 32;
+#ifndef FF_CTAS
+#define FF_CTAS 4
+#endif
 constexpr int FF_TILE = 256;  // elements staged per shared-memory tile (a multiple of FF_CHUNK)
 constexpr int FF_CHUNK = 32;  // elements summed in FP32 before the compensated outer sum
 static_assert(FF_TILE % FF_CHUNK == 0, "element chunks must not straddle tiles");
@@ -307,6 +322,66 @@ struct Acc {
   __device__ __forceinline__ float& sim(int i) const { return run[(4 * i + 1) * FF_THREADS]; }
 };
 
+// Adds the triangles [l0, l1) of a leaf to the radii of pairs [p0, np) by the
+// leaf's expansion about its centre lf (moments.cu has the formulas), in units
+// of a power of two above its radius.
+template <int R>
+__device__ __forceinline__ void leaf_sum(const float4* tile, int l0, int l1, float4 lf, float3 dh, float3 dl,
+                                         float inv_norm, const float2* ctab, const float4* kp, int p0, int np,
+                                         Acc<R>& acc) {
+  const int ex = lf.w > 0.f ? min(120, max(-100, ilogbf(lf.w) + 1)) : 0;
+  const float s = __int_as_float((127 + ex) << 23), inv_s = __int_as_float((127 - ex) << 23);
+  const float3 d = make_float3(dh.x * inv_s, dh.y * inv_s, dh.z * inv_s);
+  float2 mu[MOMENT_TERMS];
+#pragma unroll
+  for (int n = 0; n < MOMENT_TERMS; ++n) mu[n] = make_float2(0.f, 0.f);
+#pragma unroll 1
+  for (int e = l0; e < l1; e += 2) {  // two triangles per packed instruction
+    float a[2], bv[2], c[2], g[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int t = min(e + h, l1 - 1);
+      const float4 q0 = tile[3 * t], q1 = tile[3 * t + 1], q2 = tile[3 * t + 2], ml = tile[3 * FF_TILE + t];
+      const float mx = (q0.x - lf.x) + ml.x, my = (q0.y - lf.y) + ml.y, mz = (q0.z - lf.z) + ml.z;
+      const float sm = fmaf(d.x, mx, fmaf(d.y, my, d.z * mz));
+      const float s1 = fmaf(d.x, q1.x, fmaf(d.y, q1.y, d.z * q1.z));
+      const float s2 = fmaf(d.x, q2.x, fmaf(d.y, q2.y, d.z * q2.z));
+      g[h] = e + h < l1 ? dh.x * q0.w + dh.y * q1.w + dh.z * q2.w : 0.f;
+      a[h] = fmaf(s1 + s2, -1.0f / 3.0f, sm);
+      bv[h] = a[h] + s1;
+      c[h] = a[h] + s2;
+    }
+    tri_moments(make_float2(a[0], a[1]), make_float2(bv[0], bv[1]), make_float2(c[0], c[1]), make_float2(g[0], g[1]), mu);
+  }
+  constexpr FmConst<PI_GEOM_TRIANGLE> C{};
+  float2 cf8[MOMENT_TERMS / 2];  // (real, imaginary) coefficients of u^j
+#pragma unroll
+  for (int j = 0; j < MOMENT_TERMS / 2; ++j) {
+    const float f0 = (j & 1) ? -C.f[2 * j] : C.f[2 * j], f1 = (j & 1) ? -C.f[2 * j + 1] : C.f[2 * j + 1];
+    cf8[j] = make_float2((mu[2 * j].x + mu[2 * j].y) * (f0 * inv_norm), (mu[2 * j + 1].x + mu[2 * j + 1].y) * (f1 * inv_norm));
+  }
+  const df sc = cdot(dh, dl, make_float3(lf.x, lf.y, lf.z));
+  const float2 sh = dup2(sc.hi), sl = dup2(sc.lo);
+#pragma unroll
+  for (int p = 0; p < R / 2; ++p) {
+    if (p < p0 || p >= np) continue;
+    const float4 kx = ld_shared_f4(kp + 2 * p);
+    const float2 kth = make_float2(kx.x, kx.y);
+    const cf2 P = cis_tab_df2(ctab, kth, make_float2(kx.z, kx.w), sh, sl);
+    const float2 k = __fmul2_rn(kth, dup2(PI_TURN64 * s)), u = __fmul2_rn(k, k);
+    const float2 ua = dup2(u.x), ub = dup2(u.y);
+    float2 x = cf8[7], y = cf8[7];
+#pragma unroll
+    for (int j = 6; j >= 0; --j) {
+      x = __ffma2_rn(x, ua, cf8[j]);
+      y = __ffma2_rn(y, ub, cf8[j]);
+    }
+    const float2 tr = make_float2(x.x, y.x), ti = __fmul2_rn(k, make_float2(x.y, y.y));
+    acc.re2[p] = __ffma2_rn(P.re, tr, __ffma2_rn(neg2(P.im), ti, acc.re2[p]));
+    acc.im2[p] = __ffma2_rn(P.re, ti, __ffma2_rn(P.im, tr, acc.im2[p]));
+  }
+}
+
 // The grid is (CTAs per object) x (objects or evaluations); the CTAs are
 // taken in the order the hardware dispatches them (x fastest, then y) and
 // re-mapped so that the object slot varies fastest and the CTA index within
@@ -350,7 +425,7 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
   const int rlo = kg.L - (ib + 1) * R;         // the block's radii are rlo .. rlo + R - 1,
   const int skip = max(0, r_first - rlo);      // of which the first `skip` are not its own
   const int ei = dt * 32 + lane;
-  const bool active = item < ndt * nrb && ei < kg.Me;
+  const bool busy = item < ndt * nrb, active = busy && ei < kg.Me;
   int j = 0, jm = -1;
   if (active) { const int2 pr = kg.dpair[ei]; j = pr.x; jm = pr.y; }
 
@@ -376,18 +451,22 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
   // take the short series for every radius of most elements (the lean loop
   // below, chosen once per element for the whole warp), and the branches of
   // the others are taken together more often.
-  // The warp's radii as (k 256 / 2 pi hi, lo, k^2, k^3), in shared memory:
+  // The warp's radii as (k 64 / 2 pi hi, lo, k^2, k^3), in shared memory:
   // every lane reads the same entry (a broadcast), once per element and
   // radius, which keeps them out of the registers the element loop needs.
   __shared__ float4 krad[FF_WARPS][R];
-  // e^{2 pi i j / 256}, j = 0..255: the phasor table of cis_tab_*
-  __shared__ float2 ctab[256];
-  for (int t = threadIdx.x; t < 256; t += FF_THREADS) ctab[t] = kg.cis_tab[t];
+  // the phasor table of cis_tab_*
+  __shared__ float2 ctab_sm[PHASOR_ENTRIES * PHASOR_COPIES];
+  stage_phasors<PHASOR_COPIES>(kg.cis_tab, ctab_sm);
+  const float2* ctab = ctab_sm + (threadIdx.x % PHASOR_COPIES);
+  __shared__ float2 ctabm_sm[PHASOR_ENTRIES * PHASOR_M1_COPIES];
+  stage_phasors<PHASOR_M1_COPIES>(kg.cis_tabm, ctabm_sm);
+  const float2* ctabm = ctabm_sm + (threadIdx.x % PHASOR_M1_COPIES);
   if (lane < R) {
     const int r = rlo + lane;
     const bool ok = item < ndt * nrb && lane >= skip;
     const float2 k = ok ? kg.kmag[r] : make_float2(0.f, 0.f);
-    const float2 k2 = ok ? kg.kt256[r] : make_float2(0.f, 0.f);
+    const float2 k2 = ok ? kg.kt64[r] : make_float2(0.f, 0.f);
     krad[warp][lane] = make_float4(k2.x, k2.y, k.x * k.x, k.x * k.x * k.x);
   }
   // the same constants paired for packed FP32: radii (2p, 2p + 1) as
@@ -400,7 +479,7 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
       const int r = rlo + 2 * lane + h;
       const bool ok = item < ndt * nrb && 2 * lane + h >= skip;
       const float2 k = ok ? kg.kmag[r] : make_float2(0.f, 0.f);
-      const float2 k2 = ok ? kg.kt256[r] : make_float2(0.f, 0.f);
+      const float2 k2 = ok ? kg.kt64[r] : make_float2(0.f, 0.f);
       v[h][0] = k2.x; v[h][1] = k2.y; v[h][2] = k.x * k.x; v[h][3] = k.x * k.x * k.x;
     }
     kpair[warp][2 * lane] = make_float4(v[0][0], v[1][0], v[0][1], v[1][1]);
@@ -409,6 +488,8 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
   __syncthreads();
   const float4* kw = krad[warp];
   const float4* kp = kpair[warp];
+  // (k rho)^2 up to which a leaf's expansion is used (never without kg.moments)
+  const float bound2 = kg.moments ? MOMENT_X_TRI * MOMENT_X_TRI : -1.f;
   float kmax2 = 0.f;  // the warp's largest k^2
 #pragma unroll
   for (int i = 0; i < R; ++i) kmax2 = fmaxf(kmax2, kw[i].z);
@@ -421,6 +502,7 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
   // 2 FF_TILE and put their unit normals at tile[2 FF_TILE + e]);
   // tile[3 FF_TILE + e]: the low word of element e's centroid (centre).
   __shared__ float4 tile[4 * FF_TILE];
+  __shared__ float4 leaf[FF_TILE / PI_LEAF];
   // this CTA's elements [n0, n), whole chunks
   const int per = (od.n_elems + S * FF_CHUNK - 1) / (S * FF_CHUNK) * FF_CHUNK;
   const int n0 = min(od.n_elems, rank * per), n = min(od.n_elems, n0 + per);
@@ -428,17 +510,37 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
   if (od.type == PI_GEOM_TRIANGLE) {
     const float4* src = b.tri_pool + 3 * od.elem_off;
     const float4* lo = b.tri_lo + od.elem_off;
+    const float4* leaves = b.leaves + od.cl_off * (PI_CLUSTER / PI_LEAF);
     for (int base = n0; base < n; base += FF_TILE) {
       const int cnt = min(FF_TILE, n - base);
       __syncthreads();
       for (int t = threadIdx.x; t < 3 * cnt; t += FF_THREADS) tile[t] = src[3 * (int64_t)base + t];
       for (int t = threadIdx.x; t < cnt; t += FF_THREADS) tile[3 * FF_TILE + t] = lo[base + t];
+      for (int t = threadIdx.x; t * PI_LEAF < cnt; t += FF_THREADS) leaf[t] = leaves[base / PI_LEAF + t];
       __syncthreads();
-      if (active) {
+      if (busy) {  // every lane of a busy warp (the votes below); those without a direction write nothing
         // chunks of FF_CHUNK elements (tiles hold a multiple of FF_CHUNK)
         for (int e0 = 0; e0 < cnt; e0 += FF_CHUNK) {
         const int e1 = min(e0 + FF_CHUNK, cnt);
-        for (int e = e0; e < e1; ++e) {
+        for (int l0 = e0; l0 < e1; l0 += PI_LEAF) {
+        const int l1 = min(l0 + PI_LEAF, e1);
+        int from = skip;  // first radius of the block that the elements are summed at one by one
+        {
+          // radii ascend: those of the leading pairs lie within the expansion's reach of this leaf
+          const float4 lf = leaf[l0 / PI_LEAF];
+          const float reach2 = lf.w * lf.w;
+          int np = 0;
+#pragma unroll
+          for (int p = 0; p < R / 2; ++p) np += kp[2 * p + 1].y * reach2 <= bound2 ? 1 : 0;
+          // worth it for two pairs, or if nothing else is left (the moments
+          // cost about as much as one pair summed directly)
+          if (np == R / 2 || np >= skip / 2 + 2) {
+            leaf_sum<R>(tile, l0, l1, lf, dh, dl, inv_norm, ctab, kp, skip / 2, np, acc);
+            from = 2 * np;
+            if (from == R) continue;
+          }
+        }
+        for (int e = l0; e < l1; ++e) {
           const float4 q0 = tile[3 * e], q1 = tile[3 * e + 1], q2 = tile[3 * e + 2];
           const float3 m = make_float3(q0.x, q0.y, q0.z);  // centroid, object frame
           const float3 e1 = make_float3(q1.x, q1.y, q1.z);
@@ -451,16 +553,14 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
           const float slim = rcp_fast(kl * kl);  // the short series for k^2 < 1 / kl^2 (inf when kl = 0)
           const float s1 = fmaf(dh.x, e1.x, fmaf(dh.y, e1.y, dh.z * e1.z));
           const float s2 = fmaf(dh.x, e2.x, fmaf(dh.y, e2.y, dh.z * e2.z));
-          if (kmax2 < slim) {
+          if (__all_sync(0xffffffffu, kmax2 < slim)) {
             // every radius of this thread takes the short series (the same for
             // all lanes on a tensor grid: unit directions)
-            // two radii per packed FP32 instruction: the same operations,
-            // roundings and results as the scalar loop below
             const TriPolyShort tp = tri_series_coeffs_short(s1, s2, g);
             const float2 smh = make_float2(sm.hi, sm.hi), sml = make_float2(sm.lo, sm.lo);
 #pragma unroll
             for (int p = 0; p < R / 2; ++p) {
-              if (2 * p + 1 < skip) continue;
+              if (2 * p + 1 < from) continue;
               const float4 kx = ld_shared_f4(kp + 2 * p), ku = ld_shared_f4(kp + 2 * p + 1);
               const cf2 P = cis_tab_df2(ctab, make_float2(kx.x, kx.y), make_float2(kx.z, kx.w), smh, sml);
               const cf2 T = tri_series_eval_short2(tp, make_float2(ku.x, ku.y), make_float2(ku.z, ku.w));
@@ -469,35 +569,40 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
             }
             continue;
           }
-          const float sp = fmaxf(fmaxf(fabsf(s1), fabsf(s2)), fabsf(s2 - s1));
-          const float kthr2 = __fdividef(9.0f, sp * sp);  // the series for (k sp)^2 < 9 (inf when sp = 0)
-          const TriPoly tp = tri_series_coeffs(s1, s2, g);
-          // vertex phases relative to the centroid (a = m - (e1 + e2)/3, b = a + e1, c = a + e2)
-          const float da = -(s1 + s2) * (1.0f / 3.0f), db = da + s1, dc = da + s2;
+          const TriGaps tg = tri_gaps(s1, s2, sm);
+          const float ithr2 = 1.0f / 9.0f * tg.D * tg.D;  // the series for (k D)^2 < 9
+          const float gD = g * rcp_fast(tg.D);
+          // no series where every lane is wide at every radius left
+          TriPoly2 tp;
+          if (__any_sync(0xffffffffu, kw[from].z * ithr2 < 1.0f)) tp = tri_series_coeffs2(s1, s2, g);
+          // one radius per scalar instruction: packed pairs were tried and took
+          // more instructions (their constants and dot products need both halves
+          // of a register pair, moved there for every pair between the branches)
 #pragma unroll
           for (int i = 0; i < R; ++i) {
-            if (i < skip) continue;
+            if (i < from) continue;
             const float4 kr = ld_shared_f4(kw + i);
             const float2 kt = make_float2(kr.x, kr.y);
-            const cf P = cis_tab_df(ctab, kt, sm);  // centroid phase
-            cf T;
-            if (kr.z < slim) {  // the same for all lanes on a tensor grid (unit directions)
-              T = tri_series_eval_short(tp, kr.z, kr.w);
-            } else if (kr.z < kthr2) {
-              T = tri_series_eval(tp, kr.z, kr.w);  // centroid Taylor series, gamma folded in
+            const float kd2 = kr.z * ithr2;
+            cf P, T;  // the phase's phasor, and the rest with gamma folded in
+            if (__all_sync(0xffffffffu, kd2 < 1.0f)) {
+              P = cis_tab_df(ctab, kt, sm);
+              T = tri_series_eval(tp, kr.z, kr.w);  // centroid Taylor series
             } else {
-              // Large spread: e[pa, pb, pc] = e^{i k.m} e[k da, k db, k dc].  The
-              // relative phases are FP32 dot products times the double-float
-              // radius: their error |k d| 6e-8 rad multiplies a term of size
-              // ~1/|k d|^2 here.
-              const float k = kr.x * PI_TURN256;
-              const cf v = tri_generic(cis_tab_f(ctab, kt, da), cis_tab_f(ctab, kt, db), cis_tab_f(ctab, kt, dc),
-                                       k * s1, k * s2);
-              T = cf{g * v.re, g * v.im};
+              P = cis_tab_df(ctab, kt, tg.sv);
+              T = tri_wide(ctabm, kr.x, tg, gD * rcp_fast(kr.z));
+              // lanes of small spread, whose divided differences cancel
+              const bool narrow = kd2 < 1.0f / 9.0f;
+              if (__any_sync(0xffffffffu, narrow)) {
+                const cf Q = cis_tab_df(ctab, kt, sm), U = tri_series_eval(tp, kr.z, kr.w);
+                P = cf{narrow ? Q.re : P.re, narrow ? Q.im : P.im};
+                T = cf{narrow ? U.re : T.re, narrow ? U.im : T.im};
+              }
             }
             acc.re(i) = fmaf(P.re, T.re, fmaf(-P.im, T.im, acc.re(i)));
             acc.im(i) = fmaf(P.re, T.im, fmaf(P.im, T.re, acc.im(i)));
           }
+        }
         }
         if (e1 - e0 == FF_CHUNK) acc.flush();
         }
@@ -522,7 +627,7 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
         tile[3 * FF_TILE + t] = lo[base + t];
       }
       __syncthreads();
-      if (active) {
+      if (busy) {  // every lane of a busy warp (the votes below); those without a direction write nothing
         for (int e0 = 0; e0 < cnt; e0 += FF_CHUNK) {
         const int e1 = min(e0 + FF_CHUNK, cnt);
         for (int e = e0; e < e1; ++e) {
@@ -540,7 +645,7 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
           // two radii per packed FP32 phasor and accumulation (cis_tab_df2)
           const float2 sch = make_float2(sc.hi, sc.hi), scl = make_float2(sc.lo, sc.lo);
           if (disk) {
-            const float rr = q0.w * sqrt_fast(fmaxf(perp, 0.f)) * PI_TURN256;  // rho |k'_perp| / kmag, per 1/256 turn
+            const float rr = q0.w * sqrt_fast(fmaxf(perp, 0.f)) * PI_TURN64;  // rho |k'_perp| / kmag, per 1/64 turn
 #pragma unroll
             for (int p = 0; p < R / 2; ++p) {
               if (2 * p + 1 < skip) continue;
@@ -604,7 +709,7 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
       if (i >= skip && mine(i)) {
         const int64_t q = (int64_t)r * kg.M + j;
         cf v{acc.sre(i), acc.sim(i)};
-        if (kw[i].x * PI_TURN256 * dnorm < 1e-10f) v = cf{0.f, 0.f};  // A(0) = 0 (affine_dof.cpp:64-65)
+        if (kw[i].x * PI_TURN64 * dnorm < 1e-10f) v = cf{0.f, 0.f};  // A(0) = 0 (affine_dof.cpp:64-65)
         const float sw = kg.sqrtw[q];
         ev.dst[(int64_t)j * kg.L + r] = make_float2(v.re * sw, v.im * sw);
         m = fmaxf(m, fmaxf(fabsf(v.re * sw), fabsf(v.im * sw)));
@@ -630,9 +735,9 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
     const int r = rlo + i;
     if (i >= skip && mine(i)) {
       const int64_t q = (int64_t)r * kg.M + j;
-      const double kd = ((double)kw[i].x + (double)kw[i].y) * (6.283185307179586476925 / 256.0);
+      const double kd = ((double)kw[i].x + (double)kw[i].y) * (6.283185307179586476925 / 64.0);
       cf v = cmul(cis_f64(kd * so_d), cf{acc.sre(i), acc.sim(i)});
-      if (kw[i].x * PI_TURN256 * dnorm < 1e-10f) v = cf{0.f, 0.f};  // A(0) = 0 (affine_dof.cpp:64-65)
+      if (kw[i].x * PI_TURN64 * dnorm < 1e-10f) v = cf{0.f, 0.f};  // A(0) = 0 (affine_dof.cpp:64-65)
       if (jm >= 0) {  // the antipode: -conj (the origin phase included)
         const int64_t qm = (int64_t)r * kg.M + jm;
         const float s = scale_sqrt_w ? kg.sqrtw[qm] : 1.0f;
@@ -662,7 +767,7 @@ __global__ void to_double2_kernel(const float2* __restrict__ J, int64_t n, doubl
 namespace {
 
 template <int R>
-__global__ void __launch_bounds__(FF_THREADS, 5)
+__global__ void __launch_bounds__(FF_THREADS, FF_CTAS)
 ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, const EvalDev* __restrict__ evals,
           unsigned* __restrict__ row_amax) {
   ff_body<R, false>(kg, b, J, scale_sqrt_w, evals, row_amax);
@@ -673,7 +778,7 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
 constexpr int FF_SERVE_SPLIT = 4;
 
 template <int R>
-__global__ void __cluster_dims__(FF_SERVE_SPLIT, 1, 1) __launch_bounds__(FF_THREADS, 5)
+__global__ void __cluster_dims__(FF_SERVE_SPLIT, 1, 1) __launch_bounds__(FF_THREADS, FF_CTAS)
 ff_serve_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, const EvalDev* __restrict__ evals,
                 unsigned* __restrict__ row_amax) {
   ff_body<R, true>(kg, b, J, scale_sqrt_w, evals, row_amax);
@@ -708,7 +813,7 @@ int launch_prepare(pi_batch_impl* b, int only_index, cudaStream_t s) {
     dim3 grid((unsigned)((max_elems + PREP_THREADS - 1) / PREP_THREADS), (unsigned)nobj_launch);
     prepare_elems_kernel<<<grid, PREP_THREADS, 0, s>>>(d, b->d_objs, b->d_tri_pool, b->d_surf_pool, b->d_tri_lo,
                                                        b->d_surf_lo, b->d_surf_nref, b->d_perm, b->d_clusters,
-                                                       b->d_cl_rho, only_index);
+                                                       b->d_leaves, b->d_cl_rho, only_index);
     PI_LAUNCHED("prepare_elems_kernel");
   }
   // The host staging array `h` has been consumed by the copy above once the

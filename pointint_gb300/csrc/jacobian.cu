@@ -48,6 +48,8 @@ namespace {
 constexpr int JAC_THREADS = 128;
 constexpr int JAC_WARPS = JAC_THREADS / 32;
 constexpr int JAC_TILE = 128;
+// copies of the phasor table: the running sums leave no room for 16
+constexpr int JAC_COPIES = 4;
 
 enum { JAC_AFFINE_TRI = 0, JAC_AFFINE_SURF = 1, JAC_MESH_TRI = 2 };
 
@@ -82,7 +84,7 @@ struct JacThread {
   float3 dh, dl;
   float inv_norm, dnorm;
   df k;
-  float2 kt;  // |k| in 1/256 turns per unit length (double-float), for the table phasors
+  float2 kt;  // |k| in 1/64 turns per unit length (double-float), for the table phasors
 };
 
 __device__ __forceinline__ JacThread jac_thread(const KGridDev& kg) {
@@ -108,15 +110,15 @@ __device__ __forceinline__ JacThread jac_thread(const KGridDev& kg) {
     t.dnorm = l.w;
     const float2 km = kg.kmag[t.r];
     t.k = df{km.x, km.y};
-    t.kt = kg.kt256[t.r];
+    t.kt = kg.kt64[t.r];
   }
   return t;
 }
 
-// The 256-entry phasor table of cis_tab_df in shared memory; every thread of
-// the CTA calls this before its first use (it ends in __syncthreads).
+// The phasor table of cis_tab_df in shared memory; every thread of the CTA
+// calls this before its first use (it ends in __syncthreads).
 __device__ __forceinline__ void stage_cis_tab(const KGridDev& kg, float2* ctab) {
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) ctab[i] = kg.cis_tab[i];
+  stage_phasors<JAC_COPIES>(kg.cis_tab, ctab);
   __syncthreads();
 }
 
@@ -166,7 +168,7 @@ __device__ __forceinline__ TriNode tri_node(const JacThread& t, const float2* ct
   const float sp = fmaxf(fmaxf(fabsf(d1.hi), fabsf(d2.hi)), fabsf(d2.hi - d1.hi));
   const float al = t.k.hi * d1.hi, be = t.k.hi * d2.hi;
   if (t.k.hi * sp < 2.0f) {
-    const cf P = cis_tab_df(ctab, t.kt, sm);
+    const cf P = cis_tab_df<JAC_COPIES>(ctab, t.kt, sm);
     // the lanes of a warp share the radius and the element: a uniform branch
     if (t.k.hi * t.dnorm * ml.w < 1.0f)
       o.d = tri_series_der<8>(P, al, be);
@@ -175,7 +177,7 @@ __device__ __forceinline__ TriNode tri_node(const JacThread& t, const float2* ct
   } else {
     const df sa = df_add(sm, df_div3(df_add(d1, d2)) * -1.0f);
     const df sb = df_add(sa, d1), sc = df_add(sa, d2);
-    o.d = tri_generic_der(cis_tab_df(ctab, t.kt, sa), cis_tab_df(ctab, t.kt, sb), cis_tab_df(ctab, t.kt, sc), al, be);
+    o.d = tri_generic_der(cis_tab_df<JAC_COPIES>(ctab, t.kt, sa), cis_tab_df<JAC_COPIES>(ctab, t.kt, sb), cis_tab_df<JAC_COPIES>(ctab, t.kt, sc), al, be);
   }
   o.gam = (t.dh.x * S.x + t.dh.y * S.y + t.dh.z * S.z) * t.inv_norm;
   const float3 kh = make_float3(t.dh.x * t.inv_norm, t.dh.y * t.inv_norm, t.dh.z * t.inv_norm);
@@ -236,15 +238,16 @@ jac_affine_tri_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, 
     dnorm = l.w;
   }
   __shared__ float4 tile[7 * JAC_TILE];
-  __shared__ float2 ctab[256];
+  __shared__ float2 ctab_sm[PHASOR_ENTRIES * JAC_COPIES];
+  const float2* ctab = ctab_sm + (threadIdx.x % JAC_COPIES);
   __shared__ float4 krad[JAC_WARPS][R];  // (|k| hi, lo, |k| 256 / 2 pi hi, lo)
   __shared__ float run[2 * JAC_NSUM * R * JAC_THREADS];  // running sums, then compensations
-  for (int t = threadIdx.x; t < 256; t += JAC_THREADS) ctab[t] = kg.cis_tab[t];
+  stage_phasors<JAC_COPIES>(kg.cis_tab, ctab_sm);
   if (lane < R) {
     const int r = rb * R + lane;
     const bool ok = item < ndt * nrb && r < kg.L;
     const float2 km = ok ? kg.kmag[r] : make_float2(0.f, 0.f);
-    const float2 kt = ok ? kg.kt256[r] : make_float2(0.f, 0.f);
+    const float2 kt = ok ? kg.kt64[r] : make_float2(0.f, 0.f);
     krad[warp][lane] = make_float4(km.x, km.y, kt.x, kt.y);
   }
   for (int v = 0; v < 2 * JAC_NSUM * R; ++v) run[v * JAC_THREADS + threadIdx.x] = 0.f;
@@ -305,7 +308,7 @@ jac_affine_tri_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, 
         const float k = kr.x;
         cf F, Db, Dc;
         if (k < kthr) {
-          const cf P = cis_tab_df(ctab, make_float2(kr.z, kr.w), sm);
+          const cf P = cis_tab_df<JAC_COPIES>(ctab, make_float2(kr.z, kr.w), sm);
           const float u = k * k;
           float fre, fim, bre, bim, cre, cim;
           if (k < kshort) {
@@ -322,7 +325,7 @@ jac_affine_tri_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, 
           Dc = cmul(P, cf{k * cre, cim});
         } else {
           const df sa = df_add(sm, df_div3(df_add(d1, d2)) * -1.0f);
-          const TriDer d = tri_generic_der_at(ctab, make_float2(kr.z, kr.w), sa, df_add(sa, d1), df_add(sa, d2),
+          const TriDer d = tri_generic_der_at<JAC_COPIES>(ctab, make_float2(kr.z, kr.w), sa, df_add(sa, d1), df_add(sa, d2),
                                               k * d1.hi, k * d2.hi);
           F = d.F;
           Db = d.Db;
@@ -417,8 +420,9 @@ jac_affine_surf_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs,
   const JacThread t = jac_thread(kg);
   const bool disk = od.type == PI_GEOM_DISK;
   __shared__ float4 tile[6 * JAC_TILE];
-  __shared__ float2 ctab[256];
-  stage_cis_tab(kg, ctab);
+  __shared__ float2 ctab_sm[PHASOR_ENTRIES * JAC_COPIES];
+  const float2* ctab = ctab_sm + (threadIdx.x % JAC_COPIES);
+  stage_cis_tab(kg, ctab_sm);
   // v = A^T dir (k' = |k| v), qd = |v|^2
   const float* Af = od.A;
   const float3 v = make_float3(Af[0] * t.dh.x + Af[3] * t.dh.y + Af[6] * t.dh.z,
@@ -456,7 +460,7 @@ jac_affine_surf_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs,
                   cz = fmaf(v.x, nr.y, -v.y * nr.x);
       const float perp = fmaxf(fmaf(qd, nr.w, (1.0f - nr.w) * fmaf(cx, cx, fmaf(cy, cy, cz * cz))), 0.f);
       const float amp = sn * t.inv_norm;
-      const cf P = cis_tab_df(ctab, t.kt, sc);
+      const cf P = cis_tab_df<JAC_COPIES>(ctab, t.kt, sc);
       float S, Sr;
       if (disk) {
         const float x = k * q0.w * sqrt_fast(perp);
@@ -516,8 +520,9 @@ jac_mesh_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, const 
   const JacObj jo = jobs[blockIdx.y];
   const ObjDev od = b.objs[jo.obj];
   const JacThread t = jac_thread(kg);
-  __shared__ float2 ctab[256];
-  stage_cis_tab(kg, ctab);
+  __shared__ float2 ctab_sm[PHASOR_ENTRIES * JAC_COPIES];
+  const float2* ctab = ctab_sm + (threadIdx.x % JAC_COPIES);
+  stage_cis_tab(kg, ctab_sm);
   if (!t.active) return;
   const JacOut o = jac_out(kg, t.r, t.j, t.jm);
   const cf scl = jac_origin_phase(t, od);

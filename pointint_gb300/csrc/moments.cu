@@ -50,13 +50,14 @@ namespace {
 
 constexpr int FM_WARPS = 8, FM_THREADS = 32 * FM_WARPS;
 constexpr int FM_R = 8;                             // radii per warp and batch
+constexpr int FM_COPIES = 8;                        // of the phasor table: two CTAs per SM at 128 radii
 constexpr int FM_PAIRS = PI_CLUSTER / 2;            // staged element pairs per cluster
 constexpr int FM_PAIR_F4 = 6;                       // float4 per pair: 12 values of two elements
 static_assert(MOMENT_TERMS == 16, "coefficients are stored as four float4");
 
 // Shared memory, in float4: staged elements, coefficients, phasor table,
 // radius constants, then the running sums.
-constexpr int FM_F4_ELEM = FM_WARPS * FM_PAIRS * FM_PAIR_F4, FM_F4_MOM = FM_WARPS * 4 * 32, FM_F4_TAB = 128,
+constexpr int FM_F4_ELEM = FM_WARPS * FM_PAIRS * FM_PAIR_F4, FM_F4_MOM = FM_WARPS * 4 * 32, FM_F4_TAB = PHASOR_ENTRIES * FM_COPIES / 2,
               FM_F4_CTR = FM_WARPS * 16;            // cluster phases (hi, lo) per lane
 
 __host__ __device__ constexpr int fm_batches(int L) { return (L + FM_R - 1) / FM_R; }
@@ -71,22 +72,12 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 
-// Constants of the recurrences: the coefficient of (i k)^n is f[n] times the
-// n-th sum (with the triangles' -2 i^2 = 2 folded in), K[n] as above.
-template <int KIND>
-struct FmConst {
-  float f[MOMENT_TERMS], K[MOMENT_TERMS];
-  constexpr FmConst() : f(), K() {
-    double g = 1.0;  // 2/(n+2)!, lambda_n, 1/n!
-    for (int n = 0; n < MOMENT_TERMS; ++n) {
-      f[n] = (float)g;
-      K[n] = (float)(KIND == PI_GEOM_DISK ? n * (n + 2.0) / ((2.0 * n + 3.0) * (2.0 * n + 1.0)) : (double)n);
-      g *= KIND == PI_GEOM_TRIANGLE ? 1.0 / (n + 3.0)
-           : KIND == PI_GEOM_DISK   ? (2.0 * n + 3.0) / ((n + 1.0) * (n + 3.0))
-                                    : 1.0 / (n + 1.0);
-    }
-  }
-};
+// s += x with the compensation c (two sums at once).
+__device__ __forceinline__ void kahan2(float2& s, float2& c, float2 x) {
+  const float2 y = add2(x, neg2(c)), t = add2(s, y);
+  c = add2(add2(t, neg2(s)), neg2(y));
+  s = t;
+}
 
 struct FmDir {
   float3 dh, dl;
@@ -156,16 +147,8 @@ __device__ __forceinline__ void fm_moments(const float4* es, int pairs, const Fm
       const float2 a = s0;
       const float2 bb = fma2(dz, f2hi(q2), fma2(dy, f2lo(q2), mul2(dx, f2hi(q1))));
       const float2 c = fma2(dz, f2lo(q4), fma2(dy, f2hi(q3), mul2(dx, f2lo(q3))));
-      float2 an = fma2(dz, f2hi(q5), fma2(dy, f2lo(q5), mul2(dx, f2hi(q4))));  // gamma |d| (area vector . d)
-      float2 qn = an, hn = an;
-      mu[0] = add2(mu[0], hn);
-#pragma unroll
-      for (int n = 1; n < MOMENT_TERMS; ++n) {
-        an = mul2(an, a);
-        qn = fma2(bb, qn, an);
-        hn = fma2(c, hn, qn);
-        mu[n] = add2(mu[n], hn);
-      }
+      const float2 g = fma2(dz, f2hi(q5), fma2(dy, f2lo(q5), mul2(dx, f2hi(q4))));  // gamma |d| (area vector . d)
+      tri_moments(a, bb, c, g, mu);
     } else {
       const float2 amp = fma2(dz, f2hi(q2), fma2(dy, f2lo(q2), mul2(dx, f2hi(q1))));
       // |k'_perp|^2 / |k|^2 = qd (1 - |n|^2) + |n|^2 |v x n/|n||^2, as in ff_kernel
@@ -233,9 +216,10 @@ __device__ __forceinline__ void moment_body(const KGridDev& kg, const BatchDev& 
   const int nb = fm_batches(nr);
   float4* elem = sm;
   float4* mom = elem + FM_F4_ELEM;
-  float2* ctab = reinterpret_cast<float2*>(mom + FM_F4_MOM);
-  float2* csc = ctab + 256;                               // [cluster][lane]: d . c (hi, lo)
-  float4* kx = reinterpret_cast<float4*>(csc + 32 * FM_WARPS);  // radii (2p, 2p + 1) in 1/256 turns: (hi, hi', lo, lo')
+  float2* ctab_sm = reinterpret_cast<float2*>(mom + FM_F4_MOM);
+  const float2* ctab = ctab_sm + (threadIdx.x % FM_COPIES);
+  float2* csc = ctab_sm + PHASOR_ENTRIES * FM_COPIES;                      // [cluster][lane]: d . c (hi, lo)
+  float4* kx = reinterpret_cast<float4*>(csc + 32 * FM_WARPS);  // radii (2p, 2p + 1) in 1/64 turns: (hi, hi', lo, lo')
   float2* kk = reinterpret_cast<float2*>(kx + fm_batches(kg.L) * FM_R / 2);  // (k, k')
   float4* run = kx + fm_batches(kg.L) * FM_R;             // [radius][lane]: sums and compensations
   __shared__ float cscale_sm[FM_WARPS];
@@ -271,14 +255,14 @@ __device__ __forceinline__ void moment_body(const KGridDev& kg, const BatchDev& 
                     Am[2] * D.dh.x + Am[5] * D.dh.y + Am[8] * D.dh.z);
   D.qd = fmaf(D.v.x, D.v.x, fmaf(D.v.y, D.v.y, D.v.z * D.v.z));
 
-  for (int t = threadIdx.x; t < 256; t += FM_THREADS) ctab[t] = kg.cis_tab[t];
+  stage_phasors<FM_COPIES>(kg.cis_tab, ctab_sm);
   for (int t = threadIdx.x; t < nb * FM_R / 2; t += FM_THREADS) {
     float2 k[2], kt[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const bool ok = 2 * t + h < nr;
       k[h] = ok ? kg.kmag[2 * t + h] : make_float2(0.f, 0.f);
-      kt[h] = ok ? kg.kt256[2 * t + h] : make_float2(0.f, 0.f);
+      kt[h] = ok ? kg.kt64[2 * t + h] : make_float2(0.f, 0.f);
     }
     kx[t] = make_float4(kt[0].x, kt[1].x, kt[0].y, kt[1].y);
     kk[t] = make_float2(k[0].x, k[1].x);
@@ -318,9 +302,16 @@ __device__ __forceinline__ void moment_body(const KGridDev& kg, const BatchDev& 
     __syncthreads();
     const int nc = min(FM_WARPS, ncl - t0);
     for (int bt = warp; bt < nb; bt += FM_WARPS) {
-      float2 re[FM_R / 2], im[FM_R / 2];
+      // compensated running sums: a cluster's value is as large as all its
+      // elements' terms together, so plain partial sums would round coarsely
+      float2 re[FM_R / 2], im[FM_R / 2], cre[FM_R / 2], cim[FM_R / 2];
+      float4* rp = run + bt * FM_R * 32 + lane;
 #pragma unroll
-      for (int p = 0; p < FM_R / 2; ++p) re[p] = im[p] = make_float2(0.f, 0.f);
+      for (int p = 0; p < FM_R / 2; ++p) {
+        const float4 r0 = rp[64 * p], r1 = rp[64 * p + 32];
+        re[p] = make_float2(r0.x, r1.x); im[p] = make_float2(r0.y, r1.y);
+        cre[p] = make_float2(r0.z, r1.z); cim[p] = make_float2(r0.w, r1.w);
+      }
 #pragma unroll 1
       for (int c = 0; c < nc; ++c) {
         float a[8], bb[8];
@@ -333,25 +324,17 @@ __device__ __forceinline__ void moment_body(const KGridDev& kg, const BatchDev& 
 #pragma unroll
         for (int p = 0; p < FM_R / 2; ++p) {
           const float4 kt = kx[bt * (FM_R / 2) + p];
-          const cf2 P = cis_tab_df2(ctab, f2lo(kt), f2hi(kt), sh, sl);
+          const cf2 P = cis_tab_df2<FM_COPIES>(ctab, f2lo(kt), f2hi(kt), sh, sl);
           const float2 k = mul2(kk[bt * (FM_R / 2) + p], s2), u = mul2(k, k);
           const float2 x = horner8(a, u), y = mul2(k, horner8(bb, u));
-          re[p] = fma2(P.re, x, fma2(neg2(P.im), y, re[p]));
-          im[p] = fma2(P.re, y, fma2(P.im, x, im[p]));
+          kahan2(re[p], cre[p], fma2(P.re, x, neg2(mul2(P.im, y))));
+          kahan2(im[p], cim[p], fma2(P.re, y, mul2(P.im, x)));
         }
       }
 #pragma unroll
-      for (int i = 0; i < FM_R; ++i) {
-        float4* rp = run + (bt * FM_R + i) * 32 + lane;
-        float4 r = *rp;
-        float y = ((i & 1) ? re[i >> 1].y : re[i >> 1].x) - r.z, t = r.x + y;
-        r.z = (t - r.x) - y;
-        r.x = t;
-        y = ((i & 1) ? im[i >> 1].y : im[i >> 1].x) - r.w;
-        t = r.y + y;
-        r.w = (t - r.y) - y;
-        r.y = t;
-        *rp = r;
+      for (int p = 0; p < FM_R / 2; ++p) {
+        rp[64 * p] = make_float4(re[p].x, im[p].x, cre[p].x, cim[p].x);
+        rp[64 * p + 32] = make_float4(re[p].y, im[p].y, cre[p].y, cim[p].y);
       }
     }
   }
@@ -370,8 +353,8 @@ __device__ __forceinline__ void moment_body(const KGridDev& kg, const BatchDev& 
     cf v{re.hi + re.lo, im.hi + im.lo};
     const float2 km = kg.kmag[r];
     if (!SERVE) {
-      const float2 kt = kg.kt256[r];
-      v = cmul(cis_f64(((double)kt.x + (double)kt.y) * (6.283185307179586476925 / 256.0) * so), v);
+      const float2 kt = kg.kt64[r];
+      v = cmul(cis_f64(((double)kt.x + (double)kt.y) * (6.283185307179586476925 / 64.0) * so), v);
     }
     if (km.x * dnorm < 1e-10f) v = cf{0.f, 0.f};  // A(0) = 0 (affine_dof.cpp:64-65)
     const int64_t q = (int64_t)r * kg.M + j, qm = (int64_t)r * kg.M + jm;

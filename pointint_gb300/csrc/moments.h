@@ -34,6 +34,35 @@ __device__ __forceinline__ int moment_radii(const KGridDev& kg, int type, float 
   }
   return n;
 }
+// Constants of the recurrences: the coefficient of (i k)^n is f[n] times the
+// n-th sum (with the triangles' -2 i^2 = 2 folded in), K[n] as above.
+template <int KIND>
+struct FmConst {
+  float f[MOMENT_TERMS], K[MOMENT_TERMS];
+  constexpr FmConst() : f(), K() {
+    double g = 1.0;  // 2/(n+2)!, lambda_n, 1/n!
+    for (int n = 0; n < MOMENT_TERMS; ++n) {
+      f[n] = (float)g;
+      K[n] = (float)(KIND == PI_GEOM_DISK ? n * (n + 2.0) / ((2.0 * n + 3.0) * (2.0 * n + 1.0)) : (double)n);
+      g *= KIND == PI_GEOM_TRIANGLE ? 1.0 / (n + 3.0)
+           : KIND == PI_GEOM_DISK   ? (2.0 * n + 3.0) / ((n + 1.0) * (n + 3.0))
+                                    : 1.0 / (n + 1.0);
+    }
+  }
+};
+
+// Adds the moments of two triangles (in the halves) to mu: g h_n(a, b, c).
+__device__ __forceinline__ void tri_moments(float2 a, float2 b, float2 c, float2 g, float2 mu[MOMENT_TERMS]) {
+  float2 an = g, qn = g, hn = g;
+  mu[0] = __fadd2_rn(mu[0], hn);
+#pragma unroll
+  for (int n = 1; n < MOMENT_TERMS; ++n) {
+    an = __fmul2_rn(an, a);
+    qn = __ffma2_rn(b, qn, an);
+    hn = __ffma2_rn(c, hn, qn);
+    mu[n] = __fadd2_rn(mu[n], hn);
+  }
+}
 #endif
 
 // Form factors of the radii below moment_radii; ff_kernel evaluates the others.

@@ -52,8 +52,9 @@ struct KGridDev {
   const float* sqrtw;     // Q: sqrt(|w_q|)
   const float* sign;      // Q: sign(w_q), or nullptr when every weight is >= 0
   const float2* kturn;    // L: kmag / 2 pi (hi, lo)
-  const float2* kt256;    // L: kmag 256 / 2 pi (hi, lo): phases in units of 1/256 turn
-  const float2* cis_tab;  // 256: e^{2 pi i j / 256} (cos, sin), rounded once from FP64
+  const float2* kt64;     // L: kmag 64 / 2 pi (hi, lo): phases in units of 1/64 turn
+  const float2* cis_tab;  // 64: e^{2 pi i j / 64} (cos, sin), rounded once from FP64
+  const float2* cis_tabm; // 64: the same minus 1 (cos - 1, sin)
   // Evaluated directions: Me entries (j, j'), j' the direction antipodal to j
   // (d_j' = -d_j) or -1.  The form factor of a real solid satisfies
   // A(-k) = -conj A(k), so the kernels that produce per-node outputs evaluate
@@ -90,8 +91,8 @@ struct ObjDev {
   int64_t cl_off;         // its first cluster in BatchDev::clusters
 };
 
-// Elements per cluster: PI_CLUSTER consecutive pool entries of one object.
-constexpr int PI_CLUSTER = 64;
+// Elements per cluster, and per leaf: consecutive pool entries of one object.
+constexpr int PI_CLUSTER = 64, PI_LEAF = 4;
 
 // Pools in the kernels' layout, object-local frame, FP32:
 //   triangles: 3 x float4 per element  (m.xyz, S.x) (e1.xyz, S.y) (e2.xyz, S.z), m the centroid
@@ -103,7 +104,8 @@ constexpr int PI_CLUSTER = 64;
 // |k'_perp|^2 = |k'|^2 - (k'.n)^2 = |k'|^2 (1 - |n|^2) + |n|^2 |k' x n/|n||^2
 // without the cancellation of the difference form near the normal.
 // Pool entry p of an object holds its element perm[perm_off + p]: the host
-// orders elements so that PI_CLUSTER consecutive entries are compact in space.
+// orders elements so that PI_CLUSTER consecutive entries are compact in space,
+// and PI_LEAF within those.
 struct BatchDev {
   int n_obj;
   const ObjDev* objs;
@@ -115,6 +117,7 @@ struct BatchDev {
   const float4* surf_nref;
   const int32_t* perm;
   const float4* clusters;    // (centre, bounding radius) of each cluster, object frame
+  const float4* leaves;      // the same of each leaf (leaf PI_CLUSTER / PI_LEAF c + i belongs to cluster c)
   const unsigned* cl_rho;    // per object: FP32 bits of its largest cluster radius
 };
 
@@ -158,6 +161,7 @@ struct pi_batch_impl {
   float4* d_surf_nref = nullptr;
   int32_t* d_perm = nullptr;
   float4* d_clusters = nullptr;
+  float4* d_leaves = nullptr;
   unsigned* d_cl_rho = nullptr;
   ObjDev* d_objs = nullptr;
   int32_t* d_order = nullptr;
@@ -172,7 +176,7 @@ struct pi_batch_impl {
     BatchDev b;
     b.n_obj = n_obj; b.objs = d_objs; b.order = d_order; b.tri_pool = d_tri_pool; b.surf_pool = d_surf_pool;
     b.tri_lo = d_tri_lo; b.surf_lo = d_surf_lo; b.surf_nref = d_surf_nref;
-    b.perm = d_perm; b.clusters = d_clusters; b.cl_rho = d_cl_rho;
+    b.perm = d_perm; b.clusters = d_clusters; b.leaves = d_leaves; b.cl_rho = d_cl_rho;
     return b;
   }
 };
