@@ -27,6 +27,7 @@
 //    order FP64 block reduction per object) or TriangleMeshDoF vertex
 //    gradients (CSR gather per vertex, no atomics): results are bitwise
 //    reproducible.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
@@ -34,6 +35,7 @@
 #include "pi_internal.h"
 #include "dfmath.cuh"
 #include "bessel.cuh"
+#include "moments.h"
 #include "tri_adjoint.cuh"
 
 namespace pi {
@@ -59,114 +61,307 @@ struct kf {
   }
 };
 
-// B^[n][q] = sum_j W[n][j] J^[j][q]; grid (q blocks, n blocks of 16).
-__global__ void cotangent_kernel(const float2* __restrict__ Jw, const float* __restrict__ Cs, int n, int64_t Q,
-                                 float2* __restrict__ Bw) {
-  __shared__ float cs[16][64];
-  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int n0 = blockIdx.y * 16;
-  float2 acc[16];
+// The cotangent of every object, folded for the adjoint kernels: with
+// B_n = sum_j W_nj J^_j at the evaluated direction j and its antipode j'
+// (KGridDev::dpair),
+//   Bt[n][r][e] = s B_n(k_r d_j) e^{-ik.o} - conj(s' B_n(-k_r d_j) e^{ik.o}),
+// s = sign(w) sqrt|w| of the node, o the object's origin (zero at k = 0, where
+// A = 0 by definition).  A direction's antipode contributes
+// Re(conj(B') dA(-k)) with dA(-k) = -conj dA(k) for every real parameter,
+// which is Re(conj(-conj B') dA(k)), so it is never evaluated itself.
+// Grid (nodes of the evaluated directions, blocks of COT_N objects); one pass
+// over J per block.
+constexpr int COT_N = 16;
+__global__ void __launch_bounds__(256)
+cotangent_kernel(KGridDev kg, BatchDev b, const float2* __restrict__ Jw, const float* __restrict__ Cs,
+                 float2* __restrict__ Bt) {
+  __shared__ float cs[COT_N][64];
+  const int n = b.n_obj;
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool in = t < (int64_t)kg.Me * kg.L;
+  const int r = in ? (int)(t / kg.Me) : 0, e = in ? (int)(t - (int64_t)r * kg.Me) : 0;
+  const int2 jp = in ? kg.dpair[e] : make_int2(0, -1);
+  const int64_t q = (int64_t)r * kg.M + jp.x, qm = (int64_t)r * kg.M + max(jp.y, 0);
+  const int n0 = blockIdx.y * COT_N;
+  float2 acc[COT_N], accm[COT_N];
 #pragma unroll
-  for (int a = 0; a < 16; ++a) acc[a] = make_float2(0.f, 0.f);
+  for (int a = 0; a < COT_N; ++a) acc[a] = accm[a] = make_float2(0.f, 0.f);
   for (int j0 = 0; j0 < n; j0 += 64) {
     __syncthreads();
-    for (int t = threadIdx.x; t < 16 * 64; t += blockDim.x) {
-      const int a = t / 64, jj = t % 64;
+    for (int i = threadIdx.x; i < COT_N * 64; i += blockDim.x) {
+      const int a = i / 64, jj = i % 64;
       cs[a][jj] = (n0 + a < n && j0 + jj < n) ? Cs[(int64_t)(n0 + a) * n + j0 + jj] : 0.f;
     }
     __syncthreads();
-    if (q < Q) {
-      const int jn = min(64, n - j0);
-      for (int jj = 0; jj < jn; ++jj) {
-        const float2 v = Jw[(int64_t)(j0 + jj) * Q + q];
+    if (!in) continue;
+    const int jn = min(64, n - j0);
+    for (int jj = 0; jj < jn; ++jj) {
+      const float2 v = Jw[(int64_t)(j0 + jj) * kg.Q + q], vm = Jw[(int64_t)(j0 + jj) * kg.Q + qm];
 #pragma unroll
-        for (int a = 0; a < 16; ++a) {
-          acc[a].x = fmaf(cs[a][jj], v.x, acc[a].x);
-          acc[a].y = fmaf(cs[a][jj], v.y, acc[a].y);
-        }
+      for (int a = 0; a < COT_N; ++a) {
+        const float w = cs[a][jj];
+        acc[a].x = fmaf(w, v.x, acc[a].x);
+        acc[a].y = fmaf(w, v.y, acc[a].y);
+        accm[a].x = fmaf(w, vm.x, accm[a].x);
+        accm[a].y = fmaf(w, vm.y, accm[a].y);
       }
     }
   }
-  if (q < Q)
+  if (!in) return;
+  const float4 h = kg.dir_hi[jp.x], l = kg.dir_lo[jp.x];
+  const float2 km = kg.kmag[r];
+  const bool zero = !(km.x * l.w >= 1e-10f);
+  const float s = kg.sqrtw[q] * (kg.sign ? kg.sign[q] : 1.f);
+  const float sm = jp.y >= 0 ? kg.sqrtw[qm] * (kg.sign ? kg.sign[qm] : 1.f) : 0.f;
 #pragma unroll
-    for (int a = 0; a < 16; ++a)
-      if (n0 + a < n) Bw[(int64_t)(n0 + a) * Q + q] = acc[a];
+  for (int a = 0; a < COT_N; ++a) {
+    if (n0 + a >= n) break;
+    const double* o = b.objs[n0 + a].origin;
+    const double so = ((double)h.x + l.x) * o[0] + ((double)h.y + l.y) * o[1] + ((double)h.z + l.z) * o[2];
+    const cf p = cis_f64(((double)km.x + (double)km.y) * so);  // e^{ik.o}
+    const float2 u = acc[a], um = jp.y >= 0 ? accm[a] : make_float2(0.f, 0.f);
+    float2 v = make_float2(s * (u.x * p.re + u.y * p.im) - sm * (um.x * p.re - um.y * p.im),
+                           s * (u.y * p.re - u.x * p.im) + sm * (um.y * p.re + um.x * p.im));
+    if (zero) v = make_float2(0.f, 0.f);
+    Bt[((int64_t)(n0 + a) * kg.L + r) * kg.Me + e] = v;
+  }
 }
 
 struct AdjWork { int32_t obj, first; };
 
-// Shared staging of one direction tile: cotangent with sign(w) sqrt|w| and the
-// origin phase e^{-ik.o} folded in (zero at k = 0 nodes, where A = 0 by
-// definition), plus the directions.
+// A CTA's elements are ADJ_THREADS consecutive pool entries of one object:
+// whole clusters (moments.cu), whose radii [0, nr) with k rho below the bound
+// enter through the cluster's expansion.  The cotangent of a direction then
+// becomes, for each cluster (centre c, k in units of 1/s),
+//   beta_m = Re( i^m sum_r conj(Bt_r) e^{i k_r d.c} k_r^m ),   m < ADJ_TERMS,
+// 16 real numbers that all its elements share, and an element's contribution
+// and its derivatives are sums of beta_m times the moments of moments.cu and
+// their derivatives: ~150 FP32 operations per element and direction for all
+// those radii instead of ~70 for each.
+constexpr int ADJ_TERMS = MOMENT_TERMS;
+constexpr int ADJ_CL = ADJ_THREADS / PI_CLUSTER;  // clusters per CTA
+static_assert(ADJ_THREADS % PI_CLUSTER == 0 && PI_CLUSTER % 32 == 0, "a warp's elements share a cluster");
+// Bounds on k rho: the derivatives drop one (centres, vertices) or two (normals)
+// orders earlier than the values.  First dropped terms, relative to the
+// leading ones, of an element on the rim seen edge-on: 1.5e-7 (triangles'
+// vertex derivatives at 2.25), 9e-8 (surfels' normal derivatives at 1.9).
+constexpr float ADJ_X_TRI = 2.25f, ADJ_X_SURF = 1.9f;
+
+// Sums over the expansion of one element (scaled units).
+struct SurfSums { float F, Fs, Fp; };            // F, dF/dsigma, dF/dp^2
+struct TriSums { float F, Fb, Fc, Fsum; };       // t0, its derivatives by b, c and their sum with a's
+
+// Coefficients of the surfels' recurrences, nu = 1 (2 J1(x)/x), 2 (8 J2(x)/x^2)
+// or 0 (Gaussian): u_m = lambda_m w_m, w_{m+1} = sigma w_m + K_m q w_{m-1}.
+template <int NU>
+struct AdjConst {
+  float lambda[ADJ_TERMS], K[ADJ_TERMS];
+  constexpr AdjConst() : lambda(), K() {
+    double g = 1.0, prev = 1.0;
+    for (int m = 0; m < ADJ_TERMS; ++m) {
+      const double alpha = NU ? (2.0 * m + 2 * NU + 1) / ((m + 1.0) * (m + 2 * NU + 1)) : 1.0 / (m + 1.0);
+      const double beta = NU ? 1.0 / ((m + 1.0) * (m + 2 * NU + 1)) : 1.0 / (m + 1.0);
+      lambda[m] = (float)g;
+      K[m] = m == 0 ? 0.f : (float)(beta / (alpha * prev));
+      g *= alpha;
+      prev = alpha;
+    }
+  }
+};
+
+__device__ __forceinline__ SurfSums disk_adjoint(const float* be, float sg, float p2) {
+  constexpr AdjConst<1> C1{};
+  constexpr AdjConst<2> C2{};
+  const float q = fmaf(-sg, sg, p2);
+  SurfSums f{0.f, 0.f, 0.f};
+  float u0 = 0.f, u1 = 1.f, v0 = 0.f, v1 = 1.f;
+#pragma unroll
+  for (int m = 0; m < ADJ_TERMS; ++m) {
+    const float u = C1.lambda[m] * u1;
+    f.F = fmaf(be[m], u, f.F);
+    if (m + 1 < ADJ_TERMS) f.Fs = fmaf(be[m + 1], u, f.Fs);
+    if (m + 2 < ADJ_TERMS) f.Fp = fmaf(be[m + 2], (0.125f * C2.lambda[m]) * v1, f.Fp);
+    const float u2 = fmaf(sg, u1, (C1.K[m] * q) * u0), v2 = fmaf(sg, v1, (C2.K[m] * q) * v0);
+    u0 = u1; u1 = u2;
+    v0 = v1; v1 = v2;
+  }
+  return f;
+}
+
+__device__ __forceinline__ SurfSums gauss_adjoint(const float* be, float sg, float q) {
+  constexpr AdjConst<0> C{};
+  SurfSums f{0.f, 0.f, 0.f};
+  float u0 = 0.f, u1 = 1.f;
+#pragma unroll
+  for (int m = 0; m < ADJ_TERMS; ++m) {
+    const float u = C.lambda[m] * u1;
+    f.F = fmaf(be[m], u, f.F);
+    if (m + 1 < ADJ_TERMS) f.Fs = fmaf(be[m + 1], u, f.Fs);
+    if (m + 2 < ADJ_TERMS) f.Fp = fmaf(be[m + 2], 0.5f * u, f.Fp);
+    const float u2 = fmaf(sg, u1, (C.K[m] * q) * u0);
+    u0 = u1; u1 = u2;
+  }
+  return f;
+}
+
+__device__ __forceinline__ TriSums tri_adjoint(const float* be, float a, float b, float c) {
+  constexpr FmConst<PI_GEOM_TRIANGLE> C{};  // 2/(n+2)!
+  TriSums f{0.f, 0.f, 0.f, 0.f};
+  float an = 1.f, qn = 1.f, hn = 1.f, hb = 1.f, hc = 1.f;
+#pragma unroll
+  for (int n = 0; n < ADJ_TERMS; ++n) {
+    if (n > 0) {
+      an *= a;
+      qn = fmaf(b, qn, an);
+      hn = fmaf(c, hn, qn);
+    }
+    f.F = fmaf(be[n] * (-0.5f * C.f[n]), hn, f.F);
+    if (n + 1 < ADJ_TERMS) {
+      if (n > 0) {
+        hb = fmaf(b, hb, hn);
+        hc = fmaf(c, hc, hn);
+      }
+      const float w = be[n + 1] * (-0.5f * C.f[n + 1]);
+      f.Fb = fmaf(w, hb, f.Fb);
+      f.Fc = fmaf(w, hc, f.Fc);
+      f.Fsum = fmaf(w * (float)(n + 3), hn, f.Fsum);
+    }
+  }
+  return f;
+}
+
 struct AdjStage {
   float2 B[ADJ_DT * ADJ_LMAX];
   float4 dh[ADJ_DT], dl[ADJ_DT];
-  float4 va[ADJ_DT];  // v = A^T dir and qd = |v|^2 (disks/Gaussians: k' = |k| v)
-  double so[ADJ_DT];  // dir . origin
-  int2 jp[ADJ_DT];    // (direction, its antipode or -1); -1, -1 past the last direction
+  float4 va[ADJ_DT];                          // v = A^T dir and qd = |v|^2 (disks/Gaussians: k' = |k| v)
+  float beta[ADJ_DT][ADJ_CL][ADJ_TERMS];
+  float4 ctr[ADJ_CL];                         // cluster centre and scale s
+  float2 km[ADJ_LMAX], kt[ADJ_LMAX], ctab[PHASOR_ENTRIES * ADJ_COPIES];
+  int nr;
 };
 
-// Per-CTA copies of the radii (double-float |k|, and |k| in 1/64 turns per
-// unit length for the table phasors) and of the phasor table; the first
-// __syncthreads of the direction loop publishes them.
-__device__ __forceinline__ void stage_radii(const KGridDev& kg, float2* km, float2* kt, float2* ctab) {
+// Radii, phasor table and the clusters of this CTA's elements.
+__device__ __forceinline__ void adj_setup(AdjStage& st, const KGridDev& kg, const BatchDev& b, const ObjDev& od,
+                                          int first) {
   for (int r = threadIdx.x; r < kg.L; r += blockDim.x) {
-    km[r] = kg.kmag[r];
-    kt[r] = kg.kt64[r];
+    st.km[r] = kg.kmag[r];
+    st.kt[r] = kg.kt64[r];
   }
-  stage_phasors<ADJ_COPIES>(kg.cis_tab, ctab);
+  stage_phasors<ADJ_COPIES>(kg.cis_tab, st.ctab);
+  if (threadIdx.x < 32) {
+    float rho = 0.f;
+    for (int c = 0; c < ADJ_CL; ++c) {
+      if (first + c * PI_CLUSTER >= od.n_elems) continue;
+      const float4 cl = b.clusters[od.cl_off + first / PI_CLUSTER + c];
+      const int ex = cl.w > 0.f ? min(120, max(-100, ilogbf(cl.w) + 1)) : 0;
+      if (threadIdx.x == 0) st.ctr[c] = make_float4(cl.x, cl.y, cl.z, __int_as_float((127 + ex) << 23));
+      rho = cl.w > rho || !(cl.w == cl.w) ? cl.w : rho;
+    }
+    const float bound = od.type == PI_GEOM_TRIANGLE ? ADJ_X_TRI : ADJ_X_SURF;
+    int n = 0;
+    if (kg.moments)
+      for (int r0 = 0; r0 < kg.L; r0 += 32) {
+        const int r = r0 + (int)threadIdx.x;
+        n += __popc(__ballot_sync(0xffffffffu, r < kg.L && kg.kmag[r].x * rho <= bound));
+      }
+    if (threadIdx.x == 0) st.nr = n;
+  }
 }
 
-// The tile holds evaluated directions e0 .. e0 + ADJ_DT - 1 (KGridDev::dpair).
-// A direction's antipode contributes Re(conj(B') dA(-k)) with
-// dA(-k) = -conj dA(k) for every real parameter, which is
-// Re(conj(-conj B') dA(k)): the staged cotangent is B - conj(B') (each with
-// its own weight and origin phase) and the antipode is never evaluated.
-__device__ __forceinline__ void stage_tile(AdjStage& st, const KGridDev& kg, const ObjDev& od, const float2* Bw_obj,
-                                           const float2* km, int e0) {
-  const int tid = threadIdx.x;
+// Stages the cotangent and directions of the tile at e0, then the betas.
+__device__ __forceinline__ void stage_tile(AdjStage& st, const KGridDev& kg, const ObjDev& od, const float2* Bt_obj,
+                                           int n_cl, int e0) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int jn = min(ADJ_DT, kg.Me - e0);
   if (tid < ADJ_DT) {
-    const int e = e0 + tid;
     float4 h = make_float4(0.f, 0.f, 0.f, 0.f), l = h;
-    int2 jp = make_int2(-1, -1);
-    if (e < kg.Me) { jp = kg.dpair[e]; h = kg.dir_hi[jp.x]; l = kg.dir_lo[jp.x]; }
-    st.jp[tid] = jp;
+    if (tid < jn) { const int j = kg.dpair[e0 + tid].x; h = kg.dir_hi[j]; l = kg.dir_lo[j]; }
     st.dh[tid] = h;
     st.dl[tid] = l;
     const float* Am = od.A;
     const float vx = Am[0] * h.x + Am[3] * h.y + Am[6] * h.z, vy = Am[1] * h.x + Am[4] * h.y + Am[7] * h.z,
                 vz = Am[2] * h.x + Am[5] * h.y + Am[8] * h.z;
     st.va[tid] = make_float4(vx, vy, vz, fmaf(vx, vx, fmaf(vy, vy, vz * vz)));
-    const double so = ((double)h.x + l.x) * od.origin[0] + ((double)h.y + l.y) * od.origin[1] +
-                      ((double)h.z + l.z) * od.origin[2];
-    st.so[tid] = so;
+  }
+  for (int t = tid; t < ADJ_DT * kg.L; t += blockDim.x) {
+    const int r = t / ADJ_DT, jj = t % ADJ_DT;
+    if (jj < jn) st.B[jj * ADJ_LMAX + r] = Bt_obj[(int64_t)r * kg.Me + e0 + jj];
   }
   __syncthreads();
-  for (int t = tid; t < ADJ_DT * kg.L; t += blockDim.x) {
-    const int jj = t / kg.L, r = t % kg.L;
-    const int2 jp = st.jp[jj];
-    float2 v = make_float2(0.f, 0.f);
-    if (jp.x >= 0) {
-      const int64_t q = (int64_t)r * kg.M + jp.x;
-      const df k = df{km[r].x, km[r].y};
-      if (k.hi * st.dl[jj].w >= 1e-10f) {
-        const float2 b = Bw_obj[q];
-        const float s = kg.sqrtw[q] * (kg.sign ? kg.sign[q] : 1.f);
-        const cf e = cis_f64(((double)k.hi + (double)k.lo) * st.so[jj]);  // e^{ik.o}
-        // B e^{-ik.o} scaled: (b.x + i b.y)(e.re - i e.im)
-        v = make_float2(s * (b.x * e.re + b.y * e.im), s * (b.y * e.re - b.x * e.im));
-        if (jp.y >= 0) {  // minus conj of the antipode's B' e^{+ik.o}, scaled
-          const int64_t qm = (int64_t)r * kg.M + jp.y;
-          const float2 bm = Bw_obj[qm];
-          const float sm = kg.sqrtw[qm] * (kg.sign ? kg.sign[qm] : 1.f);
-          v.x -= sm * (bm.x * e.re - bm.y * e.im);
-          v.y += sm * (bm.y * e.re + bm.x * e.im);
+  const int nr = st.nr;
+  if (nr > 0) {
+    for (int w = warp; w < jn * n_cl; w += ADJ_THREADS / 32) {
+      const int jj = w / n_cl, c = w - jj * n_cl;
+      const float4 h = st.dh[jj], l = st.dl[jj], ct = st.ctr[c];
+      const df sc = cdot(make_float3(h.x, h.y, h.z), make_float3(l.x, l.y, l.z), make_float3(ct.x, ct.y, ct.z));
+      float p[ADJ_TERMS];  // sums over this lane's radii of Re, Im alternately of conj(B) e^{i k d.c} k^m
+#pragma unroll
+      for (int m = 0; m < ADJ_TERMS; ++m) p[m] = 0.f;
+      for (int r = lane; r < nr; r += 32) {
+        const float2 Bv = st.B[jj * ADJ_LMAX + r];
+        const cf P = cis_tab_df<ADJ_COPIES>(st.ctab, st.kt[r], sc);
+        const float k = st.km[r].x * ct.w, u = k * k;
+        float zr = fmaf(Bv.x, P.re, Bv.y * P.im), zi = k * fmaf(Bv.x, P.im, -Bv.y * P.re);
+#pragma unroll
+        for (int m = 0; m < ADJ_TERMS; m += 2) {
+          p[m] += zr;
+          p[m + 1] += zi;
+          zr *= u;
+          zi *= u;
         }
       }
+      // sum over the lanes, each step halving the values a lane carries: in
+      // the end lanes l and l ^ 1 hold value m = l / 2
+#pragma unroll
+      for (int w2 = 16, cnt = ADJ_TERMS; w2 >= 2; w2 >>= 1, cnt >>= 1) {
+        const bool up = (lane & w2) != 0;
+#pragma unroll
+        for (int i = 0; i < cnt / 2; ++i) {
+          const float give = up ? p[i] : p[i + cnt / 2], keep = up ? p[i + cnt / 2] : p[i];
+          p[i] = keep + __shfl_xor_sync(0xffffffffu, give, w2);
+        }
+      }
+      p[0] += __shfl_xor_sync(0xffffffffu, p[0], 1);
+      const int m = lane >> 1;
+      // Re(i^m z): z's real part for even m, minus its imaginary part for odd m, with the sign of i^(m - m mod 2)
+      if ((lane & 1) == 0) st.beta[jj][c][m] = ((m + 1) & 2) ? -p[0] : p[0];
     }
-    st.B[jj * ADJ_LMAX + r] = v;
+    __syncthreads();
   }
+}
+
+// The CTAs of a thread-block cluster (S along x) take the same elements and
+// split the tiles of directions; N sums per thread meet through distributed
+// shared memory (st.B is free by then), the first CTA writing them.
+template <int N>
+__device__ __forceinline__ bool adj_total(AdjStage& st, kf (&g)[N], float (&out)[N]) {
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+#pragma unroll
+  for (int i = 0; i < N; ++i) out[i] = g[i].s;
+  if (S == 1) return true;
+  float* sums = reinterpret_cast<float*>(st.B);
+  static_assert(2 * N * ADJ_THREADS * sizeof(float) <= sizeof(st.B), "sums fit the staged cotangent");
   __syncthreads();
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    sums[(2 * i) * ADJ_THREADS + threadIdx.x] = g[i].s;
+    sums[(2 * i + 1) * ADJ_THREADS + threadIdx.x] = g[i].c;
+  }
+  cluster.sync();
+  if (rank == 0)
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      kbsum t{0.f, 0.f};
+      for (int q = 0; q < S; ++q) {
+        const float* o = cluster.map_shared_rank(sums, q) + 2 * i * ADJ_THREADS + threadIdx.x;
+        t.add(o[0]);
+        t.lo -= o[ADJ_THREADS];
+      }
+      out[i] = t.hi + t.lo;
+    }
+  cluster.sync();  // no CTA leaves while its sums are read
+  return rank == 0;
 }
 
 // Per disk / Gaussian: 12 outputs dL/dc (3), dL/dn' (3), dL/dM (6, M = A A^T,
@@ -177,97 +372,140 @@ __device__ __forceinline__ void stage_tile(AdjStage& st, const KGridDev& kg, con
 //   dA/dM  = e^{ik.c} (k.n')/|k| (dS/dr)/(2r) k k^T
 // Disk S = area 2 J1(rho r)/(rho r), (dS/dr)/r = -2 area rho^2 J2(x)/x^2;
 // Gaussian S = w exp(-sigma^2 r^2/2), (dS/dr)/r = -sigma^2 S.
+// Expansion (p = rho |k'_perp| / |k|, sigma the projection from the cluster
+// centre): with F = Re sum_r conj(B) e^{ik(d.c + sigma)} S / area|w, i k f has
+// the coefficients of f shifted by one, and d(2 J1(x)/x)/d(x^2) = -Lambda_2(x)/8,
+// Lambda_2 = 8 J2(x)/x^2, so
+//   F = sum beta_m u_m,  dF/dsigma = sum beta_{m+1} u_m,
+//   dF/dp^2 = 1/8 sum beta_{m+2} v_m (disk), 1/2 sum beta_{m+2} u_m (Gaussian),
+// u_m, v_m the moments of 2 J1(x)/x and of Lambda_2:
+//   (m+1)(m+2 nu+1) u_{m+1} = (2m+2 nu+1) sigma u_m + (p^2 - sigma^2) u_{m-1}, nu = 1, 2.
 __global__ void __launch_bounds__(ADJ_THREADS)
-adj_surf_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const float2* __restrict__ Bw,
+adj_surf_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const float2* __restrict__ Bt,
                 float* __restrict__ out) {
   __shared__ AdjStage st;
-  __shared__ float2 km[ADJ_LMAX], kt[ADJ_LMAX], ctab_sm[PHASOR_ENTRIES * ADJ_COPIES];
-  const AdjWork wk = work[blockIdx.x];
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int S_cta = (int)cluster.num_blocks();
+  const AdjWork wk = work[blockIdx.x / S_cta];
   const ObjDev od = b.objs[wk.obj];
   const int e = wk.first + threadIdx.x;
   const bool valid = e < od.n_elems;
   const bool disk = od.type == PI_GEOM_DISK;
-  stage_radii(kg, km, kt, ctab_sm);
-  const float2* ctab = ctab_sm + (threadIdx.x % ADJ_COPIES);
-  float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0, ql = q0, nr = q0;
+  adj_setup(st, kg, b, od, wk.first);
+  __syncthreads();
+  const int nr = st.nr, n_cl = min(ADJ_CL, (od.n_elems - wk.first + PI_CLUSTER - 1) / PI_CLUSTER);
+  const int cl = threadIdx.x / PI_CLUSTER;
+  float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0, ql = q0, nr4 = q0;
   if (valid) {
     q0 = b.surf_pool[2 * (od.elem_off + e)];
     q1 = b.surf_pool[2 * (od.elem_off + e) + 1];
     ql = b.surf_lo[od.elem_off + e];
-    nr = b.surf_nref[od.elem_off + e];
+    nr4 = b.surf_nref[od.elem_off + e];
   }
+  const float4 ct = valid && nr > 0 ? st.ctr[cl] : make_float4(0.f, 0.f, 0.f, 1.f);
+  const float inv_s = 1.0f / ct.w;  // a power of two
+  const float3 rel = make_float3(((q0.x - ct.x) + ql.x) * inv_s, ((q0.y - ct.y) + ql.y) * inv_s,
+                                 ((q0.z - ct.z) + ql.z) * inv_s);
   const float3 c = make_float3(q0.x, q0.y, q0.z), nn = make_float3(q1.x, q1.y, q1.z);
-  const float3 cl = make_float3(ql.x, ql.y, ql.z);  // centre low word
-  const float p0 = q0.w, p1 = q1.w;
-  kf gc[3], gn[3], gm[6];
-  const float2* Bw_obj = Bw + (int64_t)wk.obj * kg.Q;
-  for (int j0 = 0; j0 < kg.Me; j0 += ADJ_DT) {
+  const float3 cl3 = make_float3(ql.x, ql.y, ql.z);  // centre low word
+  const float p0 = q0.w, p1 = q1.w, ps2 = (p0 * inv_s) * (p0 * inv_s);
+  kf g[12];
+  const float2* Bt_obj = Bt + (int64_t)wk.obj * kg.L * kg.Me;
+  for (int j0 = (int)cluster.block_rank() * ADJ_DT; j0 < kg.Me; j0 += S_cta * ADJ_DT) {
     __syncthreads();
-    stage_tile(st, kg, od, Bw_obj, km, j0);
+    stage_tile(st, kg, od, Bt_obj, n_cl, j0);
     if (!valid) continue;
     const int jn = min(ADJ_DT, kg.Me - j0);
+    float part[12];
+#pragma unroll
+    for (int i = 0; i < 12; ++i) part[i] = 0.f;
+#pragma unroll 1
     for (int jj = 0; jj < jn; ++jj) {
       const float4 h = st.dh[jj], l = st.dl[jj];
       const float3 dh = make_float3(h.x, h.y, h.z), dl = make_float3(l.x, l.y, l.z);
       const float inv_norm = h.w;
-      const df sc = cdot2(dh, dl, c, cl);
       const float sn = dh.x * nn.x + dh.y * nn.y + dh.z * nn.z;
       // |k'_perp|^2 / |k|^2 = qd (1 - |n|^2) + |n|^2 |v x n/|n||^2 (no cancellation near the normal)
       const float4 va = st.va[jj];
-      const float cx = fmaf(va.y, nr.z, -va.z * nr.y), cy = fmaf(va.z, nr.x, -va.x * nr.z),
-                  cz = fmaf(va.x, nr.y, -va.y * nr.x);
-      const float perp = fmaxf(fmaf(va.w, nr.w, (1.0f - nr.w) * fmaf(cx, cx, fmaf(cy, cy, cz * cz))), 0.f);
-      const float rr = p0 * sqrt_fast(perp);
+      const float cx = fmaf(va.y, nr4.z, -va.z * nr4.y), cy = fmaf(va.z, nr4.x, -va.x * nr4.z),
+                  cz = fmaf(va.x, nr4.y, -va.y * nr4.x);
+      const float perp = fmaxf(fmaf(va.w, nr4.w, (1.0f - nr4.w) * fmaf(cx, cx, fmaf(cy, cy, cz * cz))), 0.f);
       const float amp = sn * inv_norm;
       float s_c = 0.f, s_n = 0.f, s_m = 0.f;
-      const float2* Bj = st.B + jj * ADJ_LMAX;
-#pragma unroll 2
-      for (int r = 0; r < kg.L; ++r) {
-        const float2 Bv = Bj[r];
-        const df k = df{km[r].x, km[r].y};
-        const cf P = cis_tab_df<ADJ_COPIES>(ctab, kt[r], sc);
-        const float ure = Bv.x * P.re + Bv.y * P.im;  // Re(conj(B) P)
-        const float uim = Bv.x * P.im - Bv.y * P.re;  // Im(conj(B) P)
-        const float k2 = k.hi * k.hi;
-        float S, Sr;
-        if (disk) {
-          const float x = k.hi * rr;
-          S = p1 * ((x < 1e-10f) ? 1.0f : 2.0f * j1x(x));
-          Sr = -2.0f * p1 * p0 * p0 * j2x2(x);
-        } else {
-          S = p1 * __expf(-0.5f * p0 * p0 * k2 * perp);
-          Sr = -p0 * p0 * S;
-        }
-        s_c = fmaf(-k.hi * uim, S * amp, s_c);
-        s_n = fmaf(ure, fmaf(-k2 * sn * sn, Sr, S), s_n);
-        s_m = fmaf(k2 * ure, 0.5f * amp * Sr, s_m);
+      if (nr > 0) {
+        const float* be = st.beta[jj][cl];
+        const float sg = dh.x * rel.x + dh.y * rel.y + dh.z * rel.z;
+        const SurfSums f = disk ? disk_adjoint(be, sg, ps2 * perp) : gauss_adjoint(be, sg, ps2 * perp);
+        // dF/dperp = rho^2 (or sigma^2) dF/dp^2, in the scaled units s^2 dF/dp^2
+        const float fp = 2.0f * ps2 * f.Fp;  // = sum_r k^2 Re(..) Sr / (area|w)
+        s_c = inv_s * p1 * amp * f.Fs;
+        s_n = p1 * fmaf(-sn * sn, fp, f.F);
+        s_m = 0.5f * p1 * amp * fp;
       }
-      gc[0].add(dh.x * s_c); gc[1].add(dh.y * s_c); gc[2].add(dh.z * s_c);
+      const float2* Bj = st.B + jj * ADJ_LMAX;
+      if (nr < kg.L) {
+        const df sc = cdot2(dh, dl, c, cl3);
+        const float rr = p0 * sqrt_fast(perp);
+#pragma unroll 2
+        for (int r = nr; r < kg.L; ++r) {
+          const float2 Bv = Bj[r];
+          const float k = st.km[r].x;
+          const cf P = cis_tab_df<ADJ_COPIES>(st.ctab, st.kt[r], sc);
+          const float ure = Bv.x * P.re + Bv.y * P.im;  // Re(conj(B) P)
+          const float uim = Bv.x * P.im - Bv.y * P.re;  // Im(conj(B) P)
+          const float k2 = k * k;
+          float S, Sr;
+          if (disk) {
+            const float x = k * rr;
+            S = p1 * ((x < 1e-10f) ? 1.0f : 2.0f * j1x(x));
+            Sr = -2.0f * p1 * p0 * p0 * j2x2(x);
+          } else {
+            S = p1 * __expf(-0.5f * p0 * p0 * k2 * perp);
+            Sr = -p0 * p0 * S;
+          }
+          s_c = fmaf(-k * uim, S * amp, s_c);
+          s_n = fmaf(ure, fmaf(-k2 * sn * sn, Sr, S), s_n);
+          s_m = fmaf(k2 * ure, 0.5f * amp * Sr, s_m);
+        }
+      }
+      part[0] = fmaf(dh.x, s_c, part[0]); part[1] = fmaf(dh.y, s_c, part[1]); part[2] = fmaf(dh.z, s_c, part[2]);
       const float sn2 = s_n * inv_norm;
-      gn[0].add(dh.x * sn2); gn[1].add(dh.y * sn2); gn[2].add(dh.z * sn2);
-      gm[0].add(dh.x * dh.x * s_m); gm[1].add(dh.x * dh.y * s_m); gm[2].add(dh.x * dh.z * s_m);
-      gm[3].add(dh.y * dh.y * s_m); gm[4].add(dh.y * dh.z * s_m); gm[5].add(dh.z * dh.z * s_m);
+      part[3] = fmaf(dh.x, sn2, part[3]); part[4] = fmaf(dh.y, sn2, part[4]); part[5] = fmaf(dh.z, sn2, part[5]);
+      const float mx = dh.x * s_m, my = dh.y * s_m, mz = dh.z * s_m;
+      part[6] = fmaf(dh.x, mx, part[6]); part[7] = fmaf(dh.x, my, part[7]); part[8] = fmaf(dh.x, mz, part[8]);
+      part[9] = fmaf(dh.y, my, part[9]); part[10] = fmaf(dh.y, mz, part[10]); part[11] = fmaf(dh.z, mz, part[11]);
     }
+#pragma unroll
+    for (int i = 0; i < 12; ++i) g[i].add(part[i]);
   }
-  if (!valid) return;
+  float sum[12];
+  const bool mine = adj_total(st, g, sum);
+  if (!valid || !mine) return;
   float* o = out + 12 * (od.elem_off + e);
   const float sc8 = (float)INV8PI3;
-  for (int a = 0; a < 3; ++a) { o[a] = gc[a].s * sc8; o[3 + a] = gn[a].s * sc8; }
-  for (int a = 0; a < 6; ++a) o[6 + a] = gm[a].s * sc8;
+#pragma unroll
+  for (int i = 0; i < 12; ++i) o[i] = sum[i] * sc8;
 }
 
 // Per triangle: 9 outputs dL/dv0, dL/dv1, dL/dv2 (world-frame vertex positions).
+// Expansion: t0 = Re sum_r conj(B) e[..] = sum_n -beta_n/(n+2)! h_n(a, b, c) and
+// its derivatives by the projections, dh_{n+1}/db = h_n(a, b, b, c) by
+// h_n(a, b, b, c) = b h_{n-1}(a, b, b, c) + h_n(a, b, c), and their sum
+// (a + b + c derivatives of h_{n+1}) (n+3) h_n by translation.
 __global__ void __launch_bounds__(ADJ_THREADS, 4)
-adj_tri_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const float2* __restrict__ Bw,
+adj_tri_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const float2* __restrict__ Bt,
                float* __restrict__ out) {
   __shared__ AdjStage st;
-  __shared__ float2 km[ADJ_LMAX], kt[ADJ_LMAX], ctab_sm[PHASOR_ENTRIES * ADJ_COPIES];
-  const AdjWork wk = work[blockIdx.x];
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int S_cta = (int)cluster.num_blocks();
+  const AdjWork wk = work[blockIdx.x / S_cta];
   const ObjDev od = b.objs[wk.obj];
   const int e = wk.first + threadIdx.x;
   const bool valid = e < od.n_elems;
-  stage_radii(kg, km, kt, ctab_sm);
-  const float2* ctab = ctab_sm + (threadIdx.x % ADJ_COPIES);
+  adj_setup(st, kg, b, od, wk.first);
+  __syncthreads();
+  const int nr = st.nr, n_cl = min(ADJ_CL, (od.n_elems - wk.first + PI_CLUSTER - 1) / PI_CLUSTER);
+  const int cl = threadIdx.x / PI_CLUSTER;
   float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0, q2 = q0, ql = q0;
   if (valid) {
     q0 = b.tri_pool[3 * (od.elem_off + e)];
@@ -275,54 +513,73 @@ adj_tri_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const 
     q2 = b.tri_pool[3 * (od.elem_off + e) + 2];
     ql = b.tri_lo[od.elem_off + e];
   }
+  const float4 ct = valid && nr > 0 ? st.ctr[cl] : make_float4(0.f, 0.f, 0.f, 1.f);
+  const float inv_s = 1.0f / ct.w;  // a power of two
+  const float3 rel = make_float3((q0.x - ct.x) + ql.x, (q0.y - ct.y) + ql.y, (q0.z - ct.z) + ql.z);
   const float3 ml = make_float3(ql.x, ql.y, ql.z);  // centroid low word
   const float3 m = make_float3(q0.x, q0.y, q0.z), e1 = make_float3(q1.x, q1.y, q1.z),
                e2 = make_float3(q2.x, q2.y, q2.z), S = make_float3(q0.w, q1.w, q2.w);
   kf g[9];
-  const float2* Bw_obj = Bw + (int64_t)wk.obj * kg.Q;
-  for (int j0 = 0; j0 < kg.Me; j0 += ADJ_DT) {
+  const float2* Bt_obj = Bt + (int64_t)wk.obj * kg.L * kg.Me;
+  for (int j0 = (int)cluster.block_rank() * ADJ_DT; j0 < kg.Me; j0 += S_cta * ADJ_DT) {
     __syncthreads();
-    stage_tile(st, kg, od, Bw_obj, km, j0);
+    stage_tile(st, kg, od, Bt_obj, n_cl, j0);
     if (!valid) continue;
     const int jn = min(ADJ_DT, kg.Me - j0);
+    float part[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) part[i] = 0.f;
+#pragma unroll 1
     for (int jj = 0; jj < jn; ++jj) {
       const float4 h = st.dh[jj], l = st.dl[jj];
       const float3 dh = make_float3(h.x, h.y, h.z), dl = make_float3(l.x, l.y, l.z);
       const float inv_norm = h.w;
-      const df sm = cdot2(dh, dl, m, ml), d1 = cdot(dh, dl, e1), d2 = cdot(dh, dl, e2);
-      const df sa = df_add(sm, df_div3(df_add(d1, d2)) * -1.0f);
-      const df sb = df_add(sa, d1), sc = df_add(sa, d2);
-      const float sp = fmaxf(fmaxf(fabsf(d1.hi), fabsf(d2.hi)), fabsf(d2.hi - d1.hi));
-      const float kthr = __fdividef(2.0f, sp);  // the series for k sp < 2 (inf when sp = 0)
       const float gam = (dh.x * S.x + dh.y * S.y + dh.z * S.z) * inv_norm;
-      const TriDerPoly cp = tri_der_coeffs(d1.hi, d2.hi);
       float t0 = 0.f, ta = 0.f, tb = 0.f, tc = 0.f;
-      const float2* Bj = st.B + jj * ADJ_LMAX;
-      for (int r = 0; r < kg.L; ++r) {
-        const float2 Bv = Bj[r];
-        const df k = df{km[r].x, km[r].y};
-        if (k.hi < kthr) {
-          // F = P SF, D_v = P SV with the series as polynomials in k; with
-          // BP = conj(B) P, Re(conj(B) X) = Re(BP SX) and D_a = i F - D_b - D_c
-          const cf P = cis_tab_df<ADJ_COPIES>(ctab, kt[r], sm);
-          const float u = k.hi * k.hi, k3 = u * k.hi;
-          const float fre = poly_u(cp.fa, u), fim = k3 * poly_u(cp.fb, u);
-          const float bim = poly_u(cp.ba, u), bre = k.hi * poly_u(cp.bb, u);
-          const float cim = poly_u(cp.ca, u), cre = k.hi * poly_u(cp.cb, u);
-          const float pr = fmaf(Bv.x, P.re, Bv.y * P.im), pi = fmaf(Bv.x, P.im, -Bv.y * P.re);
-          const float f_re = fmaf(pr, fre, -pi * fim), f_im = fmaf(pr, fim, pi * fre);
-          const float b_re = fmaf(pr, bre, -pi * bim), c_re = fmaf(pr, cre, -pi * cim);
-          t0 += f_re;
-          ta = fmaf(k.hi, -f_im - b_re - c_re, ta);
-          tb = fmaf(k.hi, b_re, tb);
-          tc = fmaf(k.hi, c_re, tc);
-        } else {
-          const TriDer d = tri_generic_der_at<ADJ_COPIES>(ctab, kt[r], sa, sb, sc, k.hi * d1.hi, k.hi * d2.hi);
-          // Re(conj(B) X) = B.re X.re + B.im X.im
-          t0 = fmaf(Bv.x, d.F.re, fmaf(Bv.y, d.F.im, t0));
-          ta = fmaf(k.hi, fmaf(Bv.x, d.Da.re, Bv.y * d.Da.im), ta);
-          tb = fmaf(k.hi, fmaf(Bv.x, d.Db.re, Bv.y * d.Db.im), tb);
-          tc = fmaf(k.hi, fmaf(Bv.x, d.Dc.re, Bv.y * d.Dc.im), tc);
+      if (nr > 0) {
+        const float3 ds = make_float3(dh.x * inv_s, dh.y * inv_s, dh.z * inv_s);
+        const float s1 = ds.x * e1.x + ds.y * e1.y + ds.z * e1.z, s2 = ds.x * e2.x + ds.y * e2.y + ds.z * e2.z;
+        const float pa = fmaf(s1 + s2, -1.0f / 3.0f, ds.x * rel.x + ds.y * rel.y + ds.z * rel.z);
+        const TriSums f = tri_adjoint(st.beta[jj][cl], pa, pa + s1, pa + s2);
+        t0 = f.F;
+        tb = f.Fb * inv_s;
+        tc = f.Fc * inv_s;
+        ta = fmaf(f.Fsum, inv_s, -tb - tc);
+      }
+      if (nr < kg.L) {
+        const df sm = cdot2(dh, dl, m, ml), d1 = cdot(dh, dl, e1), d2 = cdot(dh, dl, e2);
+        const df sa = df_add(sm, df_div3(df_add(d1, d2)) * -1.0f);
+        const df sb = df_add(sa, d1), sc = df_add(sa, d2);
+        const float sp = fmaxf(fmaxf(fabsf(d1.hi), fabsf(d2.hi)), fabsf(d2.hi - d1.hi));
+        const float kthr = __fdividef(2.0f, sp);  // the series for k sp < 2 (inf when sp = 0)
+        const TriDerPoly cp = tri_der_coeffs(d1.hi, d2.hi);
+        const float2* Bj = st.B + jj * ADJ_LMAX;
+        for (int r = nr; r < kg.L; ++r) {
+          const float2 Bv = Bj[r];
+          const float k = st.km[r].x;
+          if (k < kthr) {
+            // F = P SF, D_v = P SV with the series as polynomials in k; with
+            // BP = conj(B) P, Re(conj(B) X) = Re(BP SX) and D_a = i F - D_b - D_c
+            const cf P = cis_tab_df<ADJ_COPIES>(st.ctab, st.kt[r], sm);
+            const float u = k * k, k3 = u * k;
+            const float fre = poly_u(cp.fa, u), fim = k3 * poly_u(cp.fb, u);
+            const float bim = poly_u(cp.ba, u), bre = k * poly_u(cp.bb, u);
+            const float cim = poly_u(cp.ca, u), cre = k * poly_u(cp.cb, u);
+            const float pr = fmaf(Bv.x, P.re, Bv.y * P.im), pi = fmaf(Bv.x, P.im, -Bv.y * P.re);
+            const float f_re = fmaf(pr, fre, -pi * fim), f_im = fmaf(pr, fim, pi * fre);
+            const float b_re = fmaf(pr, bre, -pi * bim), c_re = fmaf(pr, cre, -pi * cim);
+            t0 += f_re;
+            ta = fmaf(k, -f_im - b_re - c_re, ta);
+            tb = fmaf(k, b_re, tb);
+            tc = fmaf(k, c_re, tc);
+          } else {
+            const TriDer d = tri_generic_der_at<ADJ_COPIES>(st.ctab, st.kt[r], sa, sb, sc, k * d1.hi, k * d2.hi);
+            // Re(conj(B) X) = B.re X.re + B.im X.im
+            t0 = fmaf(Bv.x, d.F.re, fmaf(Bv.y, d.F.im, t0));
+            ta = fmaf(k, fmaf(Bv.x, d.Da.re, Bv.y * d.Da.im), ta);
+            tb = fmaf(k, fmaf(Bv.x, d.Db.re, Bv.y * d.Db.im), tb);
+            tc = fmaf(k, fmaf(Bv.x, d.Dc.re, Bv.y * d.Dc.im), tc);
+          }
         }
       }
       // khat x u / 2 terms for grad gamma
@@ -334,20 +591,22 @@ adj_tri_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const 
                                     -0.5f * (kh.x * e2.y - kh.y * e2.x));
       const float3 c2 = make_float3(0.5f * (kh.y * e1.z - kh.z * e1.y), 0.5f * (kh.z * e1.x - kh.x * e1.z),
                                     0.5f * (kh.x * e1.y - kh.y * e1.x));
-      // dL/dv = -2 (grad gamma t0 + gamma dir t_v)
-      g[0].add(-2.f * (c0.x * t0 + gam * dh.x * ta)); g[1].add(-2.f * (c0.y * t0 + gam * dh.y * ta));
-      g[2].add(-2.f * (c0.z * t0 + gam * dh.z * ta));
-      g[3].add(-2.f * (c1.x * t0 + gam * dh.x * tb)); g[4].add(-2.f * (c1.y * t0 + gam * dh.y * tb));
-      g[5].add(-2.f * (c1.z * t0 + gam * dh.z * tb));
-      g[6].add(-2.f * (c2.x * t0 + gam * dh.x * tc)); g[7].add(-2.f * (c2.y * t0 + gam * dh.y * tc));
-      g[8].add(-2.f * (c2.z * t0 + gam * dh.z * tc));
+      // dL/dv = -2 (grad gamma t0 + gamma dir t_v), the -2 applied at the end
+      const float ga = gam * ta, gb = gam * tb, gc = gam * tc;
+      part[0] += fmaf(dh.x, ga, c0.x * t0); part[1] += fmaf(dh.y, ga, c0.y * t0); part[2] += fmaf(dh.z, ga, c0.z * t0);
+      part[3] += fmaf(dh.x, gb, c1.x * t0); part[4] += fmaf(dh.y, gb, c1.y * t0); part[5] += fmaf(dh.z, gb, c1.z * t0);
+      part[6] += fmaf(dh.x, gc, c2.x * t0); part[7] += fmaf(dh.y, gc, c2.y * t0); part[8] += fmaf(dh.z, gc, c2.z * t0);
     }
-  }
-  if (!valid) return;
-  float* o = out + 9 * (od.elem_off + e);
-  const float sc8 = (float)INV8PI3;
 #pragma unroll
-  for (int a = 0; a < 9; ++a) o[a] = g[a].s * sc8;
+    for (int i = 0; i < 9; ++i) g[i].add(part[i]);
+  }
+  float sum[9];
+  const bool mine = adj_total(st, g, sum);
+  if (!valid || !mine) return;
+  float* o = out + 9 * (od.elem_off + e);
+  const float sc8 = -2.0f * (float)INV8PI3;
+#pragma unroll
+  for (int a = 0; a < 9; ++a) o[a] = sum[a] * sc8;
 }
 
 // ---- chain rule to DoF gradients ---------------------------------------------------
@@ -470,8 +729,8 @@ int launch_adjoint_elements(const pi_kgrid_impl* kg, const pi_batch_impl* b, con
   std::vector<float> cs((size_t)n * n);
   for (size_t t = 0; t < cs.size(); ++t) cs[t] = (float)W_host[t];
   PI_CUDA(cudaMemcpyAsync(Cs, cs.data(), cs.size() * sizeof(float), cudaMemcpyHostToDevice, s));
-  dim3 cg((unsigned)((kg->Q + 255) / 256), (unsigned)((n + 15) / 16));
-  cotangent_kernel<<<cg, 256, 0, s>>>(Jw, Cs, n, kg->Q, Bw);
+  dim3 cg((unsigned)(((int64_t)kg->Me * kg->L + 255) / 256), (unsigned)((n + COT_N - 1) / COT_N));
+  cotangent_kernel<<<cg, 256, 0, s>>>(kg->dev, b->dev(), Jw, Cs, Bw);
   PI_LAUNCHED("cotangent_kernel");
   std::vector<AdjWork> wt, ws2;
   for (int i = 0; i < n; ++i) {
@@ -486,12 +745,22 @@ int launch_adjoint_elements(const pi_kgrid_impl* kg, const pi_batch_impl* b, con
     std::vector<AdjWork> all(wt);
     all.insert(all.end(), ws2.begin(), ws2.end());
     PI_CUDA(cudaMemcpyAsync(dw, all.data(), nw * sizeof(AdjWork), cudaMemcpyHostToDevice, s));
+    // the directions split over a thread-block cluster until the launch has two
+    // waves of four CTAs per SM
+    const KGridDev K = kg->dev;
+    const BatchDev B = b->dev();
+    auto launch = [&](const void* fn, size_t items, const AdjWork* w, float* grad) {
+      int S = 1;
+      while (S < 16 && (int64_t)S * (int64_t)items < 8 * (int64_t)current_sm_count() && K.Me > 2 * S * ADJ_DT) S *= 2;
+      void* args[5] = {const_cast<KGridDev*>(&K), const_cast<BatchDev*>(&B), &w, &Bw, &grad};
+      return launch_split(fn, dim3((unsigned)(items * S)), ADJ_THREADS, 0, S, args, s);
+    };
     if (!wt.empty()) {
-      adj_tri_kernel<<<(unsigned)wt.size(), ADJ_THREADS, 0, s>>>(kg->dev, b->dev(), dw, Bw, tri_g);
+      if (int rc = launch(reinterpret_cast<const void*>(adj_tri_kernel), wt.size(), dw, tri_g)) return rc;
       PI_LAUNCHED("adj_tri_kernel");
     }
     if (!ws2.empty()) {
-      adj_surf_kernel<<<(unsigned)ws2.size(), ADJ_THREADS, 0, s>>>(kg->dev, b->dev(), dw + wt.size(), Bw, surf_g);
+      if (int rc = launch(reinterpret_cast<const void*>(adj_surf_kernel), ws2.size(), dw + wt.size(), surf_g)) return rc;
       PI_LAUNCHED("adj_surf_kernel");
     }
     PI_CUDA(cudaFreeAsync(dw, s));

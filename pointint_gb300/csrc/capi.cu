@@ -86,10 +86,9 @@ __global__ void jacobian_to_qd_kernel(const float2* __restrict__ G, int64_t Q, i
 }
 
 // Vertex -> (triangle, slot) adjacency of every TriangleMeshDoF object, for
-// the deterministic per-vertex gather of the adjoint.  Device-resident
-// elements are read back once.
-int build_vertex_csr(pi_batch_impl* b, const pi_object* objs, const std::vector<int32_t>& perm, int on_device,
-                     cudaStream_t s) {
+// the deterministic per-vertex gather of the adjoint.  Element orders (and
+// device-resident elements) are read back once.
+int build_vertex_csr(pi_batch_impl* b, const pi_object* objs, int on_device, cudaStream_t s) {
   int64_t nv = 0, goff = 0;
   std::vector<int64_t> voff(b->n_obj, -1), gofs(b->n_obj);
   for (int i = 0; i < b->n_obj; ++i) {
@@ -113,7 +112,13 @@ int build_vertex_csr(pi_batch_impl* b, const pi_object* objs, const std::vector<
     }
     const int64_t nvi = in.n_dofs / 3;
     std::vector<int32_t> pos(in.perm_off >= 0 ? in.n_elems : 0);  // pool entry of each element
-    for (int64_t p = 0; p < (int64_t)pos.size(); ++p) pos[perm[in.perm_off + p]] = (int32_t)p;
+    if (!pos.empty()) {
+      std::vector<int32_t> perm(in.n_elems);
+      PI_CUDA(cudaMemcpyAsync(perm.data(), b->d_perm + in.perm_off, perm.size() * sizeof(int32_t),
+                              cudaMemcpyDeviceToHost, s));
+      PI_CUDA(cudaStreamSynchronize(s));
+      for (int64_t p = 0; p < in.n_elems; ++p) pos[perm[p]] = (int32_t)p;
+    }
     for (int64_t f = 0; f < in.n_elems; ++f) {
       const int32_t v[3] = {T[f].vid0, T[f].vid1, T[f].vid2};
       if (v[0] < 0 || v[1] < 0 || v[2] < 0 || v[0] >= nvi || v[1] >= nvi || v[2] >= nvi) continue;
@@ -274,31 +279,31 @@ bool moment_grid(const std::vector<double>& dv, const std::vector<float2>& km, i
 
 // Order of an object's elements in which every PI_CLUSTER consecutive entries
 // are compact in space, and every PI_LEAF within them: recursive bisection of
-// the anchors (centroids of triangles, centres of surfels) at the widest
-// coordinate, the lower part taking whole clusters (leaves).  Coordinates that are not finite count as 0.
+// the anchors (centroids of triangles, centres of surfels, in the reference
+// frame) at the widest coordinate, the lower part taking whole clusters
+// (leaves).  Segments of up to ORDER_SEGMENT elements are bisected on the device
+// (order_kernel); a larger object is first cut into such segments here, by
+// several threads (its first levels move few, large runs).  Coordinates that
+// are not finite count as 0.
 struct OrderPoint { float x[3]; int32_t id; };
 
-// Large parts are handed to threads (200,000 elements: 17 -> 4 ms on 16 cores).
 void bisect_order(OrderPoint* p, int64_t n) {
   std::vector<std::future<void>> parts;
-  while (n > PI_LEAF) {
-    const int64_t unit = n > PI_CLUSTER ? PI_CLUSTER : PI_LEAF;
+  while (n > ORDER_SEGMENT) {
     float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
     for (int64_t t = 0; t < n; ++t)
       for (int c = 0; c < 3; ++c) { mn[c] = std::min(mn[c], p[t].x[c]); mx[c] = std::max(mx[c], p[t].x[c]); }
     int ax = 0;
     for (int c = 1; c < 3; ++c) if (mx[c] - mn[c] > mx[ax] - mn[ax]) ax = c;
-    const int64_t mid = ((n + unit - 1) / unit / 2) * unit;
+    const int64_t mid = order_mid(n);
     std::nth_element(p, p + mid, p + n, [ax](const OrderPoint& a, const OrderPoint& b) {
       return a.x[ax] < b.x[ax] || (a.x[ax] == b.x[ax] && a.id < b.id);
     });
     bool handed = false;
-    if (n > 16384) {
-      try {
-        parts.push_back(std::async(std::launch::async, bisect_order, p, mid));
-        handed = true;
-      } catch (const std::system_error&) {  // no thread to be had: this one does it
-      }
+    try {
+      parts.push_back(std::async(std::launch::async, bisect_order, p, mid));
+      handed = true;
+    } catch (const std::system_error&) {  // no thread to be had: this one does it
     }
     if (!handed) bisect_order(p, mid);
     p += mid;
@@ -307,14 +312,21 @@ void bisect_order(OrderPoint* p, int64_t n) {
   for (std::future<void>& f : parts) f.get();
 }
 
-// Element x node values from which a one-shot call orders an object's elements:
-// ordering takes ~0.1 us per element on the host, the direct sum of this many
-// values ~0.2 ms on the device.  (In the caller's order the cluster expansions
-// still apply where that order is compact.)
-constexpr double ORDER_MIN_VALUES = 2e8;
+// The segments that bisect_order leaves of n elements.
+void order_segments(int64_t at, int64_t n, const OrderSeg& proto, std::vector<OrderSeg>& segs) {
+  if (n > ORDER_SEGMENT) {
+    order_segments(at, order_mid(n), proto, segs);
+    order_segments(at + order_mid(n), n - order_mid(n), proto, segs);
+    return;
+  }
+  OrderSeg g = proto;
+  g.perm_off += at;
+  g.count = (int32_t)n;
+  segs.push_back(g);
+}
 
-// Appends the order of `o`'s elements to perm (host elements).
-void append_order(const pi_object& o, std::vector<int32_t>& perm) {
+// Cuts a large object's elements (on the host) into segments: perm[0, n).
+void order_large(const pi_object& o, int32_t* perm) {
   std::vector<OrderPoint> pts(o.n_elems);
   for (int64_t e = 0; e < o.n_elems; ++e) {
     double x[3];
@@ -332,9 +344,7 @@ void append_order(const pi_object& o, std::vector<int32_t>& perm) {
     pts[e].id = (int32_t)e;
   }
   bisect_order(pts.data(), o.n_elems);
-  const size_t at = perm.size();
-  perm.resize(at + (size_t)o.n_elems);
-  for (int64_t e = 0; e < o.n_elems; ++e) perm[at + e] = pts[e].id;
+  for (int64_t e = 0; e < o.n_elems; ++e) perm[e] = pts[e].id;
 }
 
 // Element gradients from pool order (width floats per element) to element order.
@@ -488,8 +498,7 @@ namespace {
 // source on the device (instances of one mesh under different DoFs upload
 // it once).  Only batches whose sources are never replaced share them: the
 // host entry points' temporary batches.
-// Q: the nodes of the one k-grid the batch is for, or 0 for a batch that is kept.
-int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t s, bool share_sources, int64_t Q,
+int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t s, bool share_sources,
                       pi_batch* out) {
   if (!out) return fail(PI_ERR_INVALID_ARGUMENT, "pi_batch_create: null output");
   *out = nullptr;
@@ -501,7 +510,8 @@ int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t 
   int64_t dof_count = 0;
   std::vector<char> owns_src(n, 1);  // whether object i's source is copied (first of its array)
   std::unordered_map<const void*, int> first_of;  // element array -> first object naming it
-  std::vector<int32_t> perm;  // element orders of the objects, one per distinct element array and DoF kind
+  int64_t n_perm = 0;         // entries of the element orders, one order per distinct element array and DoF kind
+  std::vector<int> ordered;   // the first object of each order
   std::unordered_map<const void*, int> order_of;  // element array -> first object ordered by it
   int64_t n_clusters = 0;
   for (int i = 0; i < n; ++i) {
@@ -538,19 +548,27 @@ int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t 
         if (T[f].vid0 >= nv || T[f].vid1 >= nv || T[f].vid2 >= nv)
           return fail(PI_ERR_INVALID_ARGUMENT, "TriangleMeshDoF vertex index beyond the DoF vector");
     }
-    // one cluster needs no order; elements that live on the device keep theirs
-    if (!on_device && in.n_elems > PI_CLUSTER && (Q == 0 || (double)in.n_elems * (double)Q >= ORDER_MIN_VALUES)) {
+    // one cluster needs no order; a large object that lives on the device keeps
+    // its caller's
+    if (in.n_elems > PI_CLUSTER && (!on_device || in.n_elems <= ORDER_SEGMENT)) {
       auto it = order_of.find(objs[i].elems);
       if (in.dof_type == PI_DOF_AFFINE && it != order_of.end() && b->info[it->second].n_elems == in.n_elems &&
           b->info[it->second].geom_type == in.geom_type) {
         in.perm_off = b->info[it->second].perm_off;
       } else {
-        in.perm_off = (int64_t)perm.size();
-        append_order(objs[i], perm);
+        in.perm_off = n_perm;
+        n_perm += in.n_elems;
+        ordered.push_back(i);
         if (in.dof_type == PI_DOF_AFFINE) order_of.emplace(objs[i].elems, i);
       }
     }
   }
+  std::vector<int32_t> perm;  // the host's part of the orders, uploaded before the device's
+  for (int i : ordered)
+    if (b->info[i].n_elems > ORDER_SEGMENT) {
+      perm.resize((size_t)n_perm);
+      order_large(objs[i], perm.data() + b->info[i].perm_off);
+    }
   b->order.resize(n);
   std::iota(b->order.begin(), b->order.end(), 0);
   std::stable_sort(b->order.begin(), b->order.end(),
@@ -568,7 +586,7 @@ int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t 
                            std::max<size_t>(b->n_surf * sizeof(float4), 16),
                            std::max<size_t>(n * sizeof(ObjDev), 16),
                            std::max<size_t>(n * sizeof(int32_t), 16),
-                           std::max<size_t>(perm.size() * sizeof(int32_t), 16),
+                           std::max<size_t>(n_perm * sizeof(int32_t), 16),
                            std::max<size_t>(n_clusters * sizeof(float4), 16),
                            std::max<size_t>(n * sizeof(unsigned), 16),
                            std::max<size_t>(n_clusters * (PI_CLUSTER / PI_LEAF) * sizeof(float4), 16)};
@@ -621,7 +639,21 @@ int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t 
   if (e == cudaSuccess && !perm.empty())
     e = cudaMemcpyAsync(b->d_perm, perm.data(), perm.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) { cleanup(); return cuda_fail(e, "pi_batch_create upload"); }
-  int rc0 = build_vertex_csr(b.get(), objs, perm, on_device, s);
+  std::vector<OrderSeg> segs;
+  for (int i : ordered) {
+    const HostObjInfo& in = b->info[i];
+    OrderSeg g{};
+    g.geom_type = in.geom_type;
+    g.dof_type = in.dof_type;
+    g.from_perm = in.n_elems > ORDER_SEGMENT;
+    g.perm_off = in.perm_off;
+    g.n_dofs = in.n_dofs;
+    g.src = static_cast<const unsigned char*>(b->d_src) + in.src_off;
+    g.dofs = b->d_dofs + in.dof_off;
+    order_segments(0, in.n_elems, g, segs);
+  }
+  int rc0 = launch_order(segs, b->d_perm, s);
+  if (rc0 == PI_OK) rc0 = build_vertex_csr(b.get(), objs, on_device, s);
   if (rc0) { cleanup(); return rc0; }
   int rc = launch_prepare(b.get(), -1, s);
   if (rc) { cleanup(); return rc; }
@@ -634,7 +666,7 @@ int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t 
 extern "C" {
 
 int pi_batch_create(const pi_object* objs, int n, int on_device, pi_stream stream, pi_batch* out) {
-  return batch_create_impl(objs, n, on_device, reinterpret_cast<cudaStream_t>(stream), false, 0, out);
+  return batch_create_impl(objs, n, on_device, reinterpret_cast<cudaStream_t>(stream), false, out);
 }
 
 int pi_batch_set_dofs(pi_batch b, int index, const double* d_dofs, pi_stream stream) {
@@ -814,7 +846,7 @@ int pi_volume_matrix_host(const pi_object* objs, int n, const double* dirs, cons
   int rc = pi_kgrid_create(dirs, kmag, w, Q, &kg.k);
   if (rc) return rc;
   BatchGuard b;
-  rc = batch_create_impl(objs, n, 0, s, true, Q, &b.b);
+  rc = batch_create_impl(objs, n, 0, s, true, &b.b);
   if (rc) return rc;
   size_t ws_bytes = 0;
   rc = pi_contract_workspace_size(kg.k, n, precision, &ws_bytes);
@@ -856,7 +888,7 @@ static int volume_and_grads_host(const pi_object* objs, int n, const double* dir
   int rc = pi_kgrid_create(dirs, kmag, w, Q, &kg.k);
   if (rc) return rc;
   BatchGuard b;
-  rc = batch_create_impl(objs, n, 0, s, true, Q, &b.b);
+  rc = batch_create_impl(objs, n, 0, s, true, &b.b);
   if (rc) return rc;
   size_t ws_c = 0, ws_a = 0;
   if ((rc = pi_contract_workspace_size(kg.k, n, PI_CONTRACT_FP32, &ws_c)) || (rc = pi_adjoint_workspace_size(kg.k, b.b, &ws_a)))
@@ -936,7 +968,7 @@ static int stacked_gram_host(const pi_object* objs, int n, const double* dirs, c
   int rc = pi_kgrid_create(dirs, kmag, w, Q, &kg.k);
   if (rc) return rc;
   BatchGuard b;
-  rc = batch_create_impl(objs, n, 0, s, true, Q, &b.b);
+  rc = batch_create_impl(objs, n, 0, s, true, &b.b);
   if (rc) return rc;
   const int64_t D = dof_gradient_size(b.b), m = n + D;
   if (m > INT32_MAX) return fail(PI_ERR_UNSUPPORTED, "too many DoFs for the Hessian");
@@ -1020,7 +1052,7 @@ int pi_compute_Ak(const pi_object* obj, const double* dirs, const double* kmag, 
   int rc = pi_kgrid_create(dirs, kmag, nullptr, Q, &kg.k);
   if (rc) return rc;
   BatchGuard b;
-  rc = batch_create_impl(obj, 1, 0, s, false, Q, &b.b);
+  rc = batch_create_impl(obj, 1, 0, s, false, &b.b);
   if (rc) return rc;
   DevBuf J;
   if ((rc = J.alloc((size_t)Q * sizeof(float2), s))) return rc;
@@ -1056,7 +1088,7 @@ int pi_compute_Ak_gradient(const pi_object* obj, const double* dirs, const doubl
   int rc = pi_kgrid_create(dirs, kmag, nullptr, Q, &kg.k);  // unit weights: G = dA/dtheta
   if (rc) return rc;
   BatchGuard b;
-  rc = batch_create_impl(obj, 1, 0, s, false, Q, &b.b);
+  rc = batch_create_impl(obj, 1, 0, s, false, &b.b);
   if (rc) return rc;
   const int64_t D = obj->n_dofs;
   DevBuf G;

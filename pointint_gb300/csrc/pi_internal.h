@@ -181,6 +181,28 @@ struct pi_batch_impl {
   }
 };
 
+// ---- element order (formfactor.cu) -----------------------------------------------
+// Recursive bisection of n > PI_LEAF elements: the lower part takes half the
+// clusters while there is more than one, then half the leaves.
+constexpr int ORDER_SEGMENT = 8192;
+template <class T>
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr T order_mid(T n) {
+  return n > PI_CLUSTER ? (n + PI_CLUSTER - 1) / PI_CLUSTER / 2 * PI_CLUSTER : (n + PI_LEAF - 1) / PI_LEAF / 2 * PI_LEAF;
+}
+
+// A run of at most ORDER_SEGMENT elements to be ordered on the device: the
+// object's elements perm[perm_off ..], or 0 .. count - 1 (from_perm = 0).
+struct OrderSeg {
+  int32_t geom_type, dof_type, count, from_perm;
+  int64_t perm_off, n_dofs;
+  const unsigned char* src;
+  const double* dofs;
+};
+int launch_order(const std::vector<OrderSeg>& segs, int32_t* d_perm, cudaStream_t s);
+
 // ---- launchers (formfactor.cu / contract.cu) ------------------------------------
 int launch_prepare(pi_batch_impl* b, int only_index, cudaStream_t s);
 // row_amax (optional, n_objects floats): each row's largest |Re|, |Im| of the
