@@ -741,7 +741,7 @@ int launch_adjoint_elements(const pi_kgrid_impl* kg, const pi_batch_impl* b, con
   AdjWork* dw = nullptr;
   const size_t nw = wt.size() + ws2.size();
   if (nw) {
-    PI_CUDA(cudaMallocAsync((void**)&dw, nw * sizeof(AdjWork), s));
+    PI_CUDA(pool_alloc((void**)&dw, nw * sizeof(AdjWork), s));
     std::vector<AdjWork> all(wt);
     all.insert(all.end(), ws2.begin(), ws2.end());
     PI_CUDA(cudaMemcpyAsync(dw, all.data(), nw * sizeof(AdjWork), cudaMemcpyHostToDevice, s));
@@ -788,7 +788,7 @@ int launch_dof_gradients(const pi_kgrid_impl* kg, pi_batch_impl* b, const float2
     any_mesh |= in.dof_type == PI_DOF_TRIANGLE_MESH;
   }
   ChainObj* dco = nullptr;
-  PI_CUDA(cudaMallocAsync((void**)&dco, n * sizeof(ChainObj), s));
+  PI_CUDA(pool_alloc((void**)&dco, n * sizeof(ChainObj), s));
   PI_CUDA(cudaMemcpyAsync(dco, co.data(), n * sizeof(ChainObj), cudaMemcpyHostToDevice, s));
   chain_affine_kernel<<<n, 128, 0, s>>>(dco, tri_g, surf_g, grad);
   PI_LAUNCHED("chain_affine_kernel");

@@ -112,30 +112,63 @@ __global__ void prepare_origin_kernel(const PrepObj* objs, ObjDev* out, unsigned
 }
 
 // Orders one segment of an object's elements (OrderSeg) per CTA by recursive
-// bisection of their anchors at the widest coordinate, level by level: every
-// part's axis from its bounding box, then one bitonic sort of the whole
-// segment by (part, coordinate, index).  The parts' sizes depend on the count
-// alone, so a thread finds the part of an entry by walking down from the root.
-// ~5 us per level for 8,192 elements (11 levels), against ~0.1 us per element
-// and call on the host.
-constexpr int ORDER_THREADS = 1024;
+// bisection of their anchors at the widest coordinate.  Parts of more than one
+// cluster: all parts of a level at once, each cut at its exact median, found
+// digit by digit (four 6-bit digits of the coordinate scaled to the part's
+// bounding box, ties by position) from histograms in shared memory, and moved
+// by a stable partition; parts are whole clusters, so a warp's 32 entries
+// share a part, and the parts' sizes depend on the count alone, so a warp
+// finds its part by walking down from the root.  Within a cluster a warp sorts
+// 64, 32, 16 and 8 entries by ranks counted through shuffles.  (Bitonic sorts
+// of the whole segment at every level took 185 us for 1,280 elements and 905
+// for 5,120; the host ~0.1 us per element.)
+constexpr int ORDER_SLOTS = ORDER_SEGMENT / PI_CLUSTER, ORDER_BLOCKS = ORDER_SEGMENT / 32;
+constexpr int ORDER_BITS = 6, ORDER_BINS = 1 << ORDER_BITS, ORDER_ROUNDS = 4;
 
-__host__ __device__ constexpr size_t order_smem(int n2) {  // keys, coordinates, indices, axes
-  return (size_t)n2 * (sizeof(unsigned long long) + 3 * sizeof(float) + sizeof(unsigned short) + 1);
+struct OrderShared {
+  unsigned mn[3][ORDER_SLOTS], mx[3][ORDER_SLOTS];  // bounding boxes as order-preserving integers
+  int axis[ORDER_SLOTS];
+  float base[ORDER_SLOTS], scale[ORDER_SLOTS];
+  unsigned prefix[ORDER_SLOTS], target[ORDER_SLOTS];
+  unsigned less[ORDER_BLOCKS], equal[ORDER_BLOCKS];  // per 32 entries, then their prefix sums
+  unsigned hist[ORDER_SLOTS][ORDER_BINS];
+};
+
+__host__ __device__ constexpr size_t order_smem(int n2) {
+  return sizeof(OrderShared) + (size_t)n2 * (3 * sizeof(float) + 2 * sizeof(unsigned short));
 }
 
-__global__ void __launch_bounds__(ORDER_THREADS)
+// The part of a level that holds entry i: [lo, lo + c).
+__device__ __forceinline__ void order_part(int n, int level, int i, int& lo, int& c) {
+  lo = 0;
+  c = n;
+  for (int d = 0; d < level && c > PI_CLUSTER; ++d) {
+    const int mid = order_mid(c);
+    if (i >= lo + mid) { lo += mid; c -= mid; } else c = mid;
+  }
+}
+
+__device__ __forceinline__ unsigned order_bits(float v) {
+  const unsigned u = __float_as_uint(v);
+  return (u >> 31) ? ~u : u | 0x80000000u;
+}
+
+__device__ __forceinline__ float order_float(unsigned u) {
+  return __uint_as_float((u >> 31) ? u & 0x7fffffffu : ~u);
+}
+
+__global__ void __launch_bounds__(1024)
 order_kernel(const OrderSeg* __restrict__ segs, int32_t* __restrict__ perm, int n2) {
-  extern __shared__ unsigned long long okey[];
-  float* ox = reinterpret_cast<float*>(okey + n2);  // x, y, z of the segment's elements
-  unsigned short* oidx = reinterpret_cast<unsigned short*>(ox + 3 * n2);
-  unsigned char* oax = reinterpret_cast<unsigned char*>(oidx + n2);  // axis of the part that starts there
+  extern __shared__ float4 osm[];
+  OrderShared& sh = *reinterpret_cast<OrderShared*>(osm);
+  float* ox = reinterpret_cast<float*>(&sh + 1);  // x, y, z of the segment's elements
+  unsigned short* ia = reinterpret_cast<unsigned short*>(ox + 3 * n2);  // entry -> element of the segment
+  unsigned short* ib = ia + n2;
   const OrderSeg g = segs[blockIdx.x];
-  const int n = g.count, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n = g.count, tid = threadIdx.x, T = blockDim.x, warp = tid >> 5, lane = tid & 31, nw = T >> 5;
+  const int nblk = (n + 31) / 32;
   int32_t* out = perm + g.perm_off;
-  int m2 = 1;  // the power of two that holds this segment
-  while (m2 < n) m2 <<= 1;
-  for (int i = tid; i < n; i += ORDER_THREADS) {
+  for (int i = tid; i < n; i += T) {
     const int64_t e = g.from_perm ? out[i] : i;
     double x[3] = {0.0, 0.0, 0.0};
     if (g.geom_type == PI_GEOM_TRIANGLE) {
@@ -152,85 +185,198 @@ order_kernel(const OrderSeg* __restrict__ segs, int32_t* __restrict__ perm, int 
       const SurfSrc& t = reinterpret_cast<const SurfSrc*>(g.src)[e];
       for (int c = 0; c < 3; ++c) x[c] = t.c[c];
     }
-    for (int c = 0; c < 3; ++c) ox[c * n2 + i] = isfinite((float)x[c]) ? (float)x[c] : 0.f;
-    oidx[i] = (unsigned short)i;
+    for (int c = 0; c < 3; ++c) ox[c * n2 + i] = isfinite((float)x[c]) ? (float)x[c] + 0.0f : 0.f;
+    ia[i] = (unsigned short)i;
   }
-  __syncthreads();
   for (int level = 0; level < 16; ++level) {
-    // the parts of this level, one per warp: bit b of the part's number (from
-    // the top) says which half is taken at depth b; paths that end early
-    // belong to the part whose remaining bits are zero
-    bool split = false;
-    for (int part = warp; part < (1 << level); part += ORDER_THREADS / 32) {
-      int lo = 0, c = n;
-      bool ok = true;
-      for (int b = level - 1; b >= 0 && ok; --b) {
-        if (c <= PI_LEAF) { ok = false; break; }
-        const int mid = order_mid((unsigned)c);
-        if ((part >> b) & 1) { lo += mid; c -= mid; } else c = mid;
+    for (int t = tid; t < 3 * ORDER_SLOTS; t += T) { (&sh.mn[0][0])[t] = ~0u; (&sh.mx[0][0])[t] = 0u; }
+    bool big = false;
+    __syncthreads();
+    for (int blk = warp; blk < nblk; blk += nw) {  // bounding boxes
+      int lo, c;
+      order_part(n, level, blk * 32, lo, c);
+      if (c <= PI_CLUSTER) continue;
+      big = true;
+      const int i = blk * 32 + lane;
+      for (int a = 0; a < 3; ++a) {
+        const unsigned u = i < n ? order_bits(ox[a * n2 + ia[i]]) : 0u;
+        const unsigned l = __reduce_min_sync(0xffffffffu, i < n ? u : ~0u), h = __reduce_max_sync(0xffffffffu, u);
+        if (lane == 0) { atomicMin(&sh.mn[a][lo / PI_CLUSTER], l); atomicMax(&sh.mx[a][lo / PI_CLUSTER], h); }
       }
-      if (!ok || c <= PI_LEAF) continue;
-      split = true;
-      float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
-      for (int i = lane; i < c; i += 32)
-        for (int a = 0; a < 3; ++a) {
-          const float v = ox[a * n2 + oidx[lo + i]];
-          mn[a] = fminf(mn[a], v);
-          mx[a] = fmaxf(mx[a], v);
-        }
-      for (int w = 16; w > 0; w >>= 1)
-        for (int a = 0; a < 3; ++a) {
-          mn[a] = fminf(mn[a], __shfl_xor_sync(0xffffffffu, mn[a], w));
-          mx[a] = fmaxf(mx[a], __shfl_xor_sync(0xffffffffu, mx[a], w));
-        }
+    }
+    if (!__syncthreads_or(big)) break;
+    for (int t = tid; t < ORDER_SLOTS && t * PI_CLUSTER < n; t += T) {  // one thread per part, at the slot it starts in
+      int lo, c;
+      order_part(n, level, t * PI_CLUSTER, lo, c);
+      if (lo != t * PI_CLUSTER || c <= PI_CLUSTER) continue;
       int ax = 0;
-      for (int a = 1; a < 3; ++a) if (mx[a] - mn[a] > mx[ax] - mn[ax]) ax = a;
-      if (lane == 0) oax[lo] = (unsigned char)ax;
-    }
-    if (!__syncthreads_or(split)) break;
-    for (int i = tid; i < m2; i += ORDER_THREADS) {
-      unsigned long long key = ~0ull;
-      if (i < n) {
-        int lo = 0, c = n;
-        for (int d = 0; d < level && c > PI_LEAF; ++d) {
-          const int mid = order_mid((unsigned)c);
-          if (i >= lo + mid) { lo += mid; c -= mid; } else c = mid;
-        }
-        const unsigned id = oidx[i];
-        unsigned v = 0;  // finished parts keep their order
-        if (c > PI_LEAF) {
-          const unsigned u = __float_as_uint(ox[oax[lo] * n2 + id] + 0.0f);
-          v = (u >> 31) ? ~u : u | 0x80000000u;
-        } else {
-          v = (unsigned)(i - lo);
-        }
-        key = ((unsigned long long)lo << 45) | ((unsigned long long)v << 13) | id;
+      float best = -1.f, base = 0.f;
+      for (int a = 0; a < 3; ++a) {
+        const float l = order_float(sh.mn[a][t]), h = order_float(sh.mx[a][t]);
+        if (h - l > best) { best = h - l; ax = a; base = l; }
       }
-      okey[i] = key;
+      sh.axis[t] = ax;
+      sh.base[t] = base;
+      sh.scale[t] = best > 0.f && isfinite(best) ? 16777215.0f / best : 0.f;
+      sh.prefix[t] = 0u;
+      sh.target[t] = (unsigned)order_mid(c);
+    }
+    // an entry's coordinate as 24 bits of its part's box
+    auto key_of = [&](int slot, int i) {
+      const float v = (ox[sh.axis[slot] * n2 + ia[i]] - sh.base[slot]) * sh.scale[slot];
+      return (unsigned)fminf(fmaxf(v, 0.f), 16777215.0f);
+    };
+    for (int round = 0; round < ORDER_ROUNDS; ++round) {
+      const int shift = ORDER_BITS * (ORDER_ROUNDS - 1 - round);
+      for (int t = tid; t < ORDER_SLOTS * ORDER_BINS; t += T) (&sh.hist[0][0])[t] = 0u;
+      __syncthreads();
+      for (int blk = warp; blk < nblk; blk += nw) {
+        int lo, c;
+        order_part(n, level, blk * 32, lo, c);
+        const int i = blk * 32 + lane, slot = lo / PI_CLUSTER;
+        if (c <= PI_CLUSTER || i >= n) continue;
+        const unsigned k = key_of(slot, i);
+        if ((k >> shift >> ORDER_BITS) == sh.prefix[slot]) atomicAdd(&sh.hist[slot][(k >> shift) & (ORDER_BINS - 1)], 1u);
+      }
+      __syncthreads();
+      for (int t = warp; t < ORDER_SLOTS && t * PI_CLUSTER < n; t += nw) {  // the digit of the median
+        int lo, c;
+        order_part(n, level, t * PI_CLUSTER, lo, c);
+        if (lo != t * PI_CLUSTER || c <= PI_CLUSTER) continue;
+        const unsigned h0 = sh.hist[t][2 * lane], h1 = sh.hist[t][2 * lane + 1], want = sh.target[t];
+        unsigned sum = h0 + h1;
+        for (int w = 1; w < 32; w <<= 1) {
+          const unsigned o = __shfl_up_sync(0xffffffffu, sum, w);
+          if (lane >= w) sum += o;
+        }
+        const unsigned b0 = sum - h0 - h1, b1 = b0 + h0;  // entries below bins 2 lane, 2 lane + 1
+        if (b0 <= want && want < b1) { sh.prefix[t] = (sh.prefix[t] << ORDER_BITS) | (2 * lane); sh.target[t] = want - b0; }
+        else if (b1 <= want && want < sum) { sh.prefix[t] = (sh.prefix[t] << ORDER_BITS) | (2 * lane + 1); sh.target[t] = want - b1; }
+      }
+      __syncthreads();
+    }
+    // stable partition: below the median, and the first `target` equal to it, to the left
+    for (int blk = warp; blk < nblk; blk += nw) {
+      int lo, c;
+      order_part(n, level, blk * 32, lo, c);
+      const int i = blk * 32 + lane, slot = lo / PI_CLUSTER;
+      const unsigned k = c > PI_CLUSTER && i < n ? key_of(slot, i) : ~0u, med = c > PI_CLUSTER ? sh.prefix[slot] : 0u;
+      const unsigned ml = __ballot_sync(0xffffffffu, k < med), me = __ballot_sync(0xffffffffu, k == med);
+      if (lane == 0) { sh.less[blk] = __popc(ml); sh.equal[blk] = __popc(me); }
     }
     __syncthreads();
-    for (int k = 2; k <= m2; k <<= 1)
-      for (int j = k >> 1; j > 0; j >>= 1) {
-        for (int t = tid; t < m2 / 2; t += ORDER_THREADS) {
-          const int i = 2 * t - (t & (j - 1)), p = i + j;
-          const unsigned long long x = okey[i], y = okey[p];
-          if ((x > y) == ((i & k) == 0)) { okey[i] = y; okey[p] = x; }
+    if (warp == 0) {  // exclusive prefix sums over the blocks
+      unsigned carry_l = 0, carry_e = 0;
+      for (int b0 = 0; b0 < nblk; b0 += 32) {
+        const int blk = b0 + lane;
+        const unsigned l = blk < nblk ? sh.less[blk] : 0u, e = blk < nblk ? sh.equal[blk] : 0u;
+        unsigned sl = l, se = e;
+        for (int w = 1; w < 32; w <<= 1) {
+          const unsigned ol = __shfl_up_sync(0xffffffffu, sl, w), oe = __shfl_up_sync(0xffffffffu, se, w);
+          if (lane >= w) { sl += ol; se += oe; }
         }
-        __syncthreads();
+        if (blk < nblk) { sh.less[blk] = carry_l + sl - l; sh.equal[blk] = carry_e + se - e; }
+        carry_l += __shfl_sync(0xffffffffu, sl, 31);
+        carry_e += __shfl_sync(0xffffffffu, se, 31);
       }
-    for (int i = tid; i < n; i += ORDER_THREADS) oidx[i] = (unsigned short)(okey[i] & 8191u);
+    }
     __syncthreads();
+    for (int blk = warp; blk < nblk; blk += nw) {
+      int lo, c;
+      order_part(n, level, blk * 32, lo, c);
+      const int i = blk * 32 + lane, slot = lo / PI_CLUSTER;
+      const bool in = c > PI_CLUSTER && i < n;
+      const unsigned k = in ? key_of(slot, i) : ~0u, med = c > PI_CLUSTER ? sh.prefix[slot] : 0u;
+      const unsigned ml = __ballot_sync(0xffffffffu, k < med), me = __ballot_sync(0xffffffffu, k == med);
+      if (i >= n) continue;
+      int dest = i;
+      if (in) {
+        const unsigned below = (1u << lane) - 1u;
+        const unsigned nl = sh.less[blk] - sh.less[lo / 32] + __popc(ml & below);
+        const unsigned ne = sh.equal[blk] - sh.equal[lo / 32] + __popc(me & below), rem = sh.target[slot];
+        const int left = (int)(nl + min(ne, rem));
+        const bool is_left = k < med || (k == med && ne < rem);
+        dest = is_left ? lo + left : lo + order_mid(c) + (i - lo - left);
+      }
+      ib[dest] = ia[i];
+    }
+    __syncthreads();
+    unsigned short* t = ia;
+    ia = ib;
+    ib = t;
   }
-  int32_t id[ORDER_SEGMENT / ORDER_THREADS];
+  // within each cluster: a warp's lanes hold entries lane and lane + 32
+  for (int q = warp; q * PI_CLUSTER < n; q += nw) {
+    const int p0 = q * PI_CLUSTER;
+    for (int grp = 64; grp >= 2 * PI_LEAF; grp >>= 1) {
+      int id[2];
+      float x[2][3], v[2];
 #pragma unroll
-  for (int t = 0; t < ORDER_SEGMENT / ORDER_THREADS; ++t) {
-    const int i = tid + t * ORDER_THREADS;
-    if (i < n) id[t] = g.from_perm ? out[oidx[i]] : oidx[i];
+      for (int h = 0; h < 2; ++h) {
+        const int i = p0 + lane + 32 * h;
+        id[h] = i < n ? ia[i] : -1;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) x[h][a] = i < n ? ox[a * n2 + ia[i]] : INFINITY;
+      }
+      // the widest coordinate of the entry's group (entries past the end do not count)
+      float mn[2][3], mx[2][3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) { mn[h][a] = x[h][a]; mx[h][a] = id[h] >= 0 ? x[h][a] : -INFINITY; }
+        if (grp == 64) {
+          mn[0][a] = mn[1][a] = fminf(mn[0][a], mn[1][a]);
+          mx[0][a] = mx[1][a] = fmaxf(mx[0][a], mx[1][a]);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          for (int w = 1; w < min(grp, 32); w <<= 1) {
+            mn[h][a] = fminf(mn[h][a], __shfl_xor_sync(0xffffffffu, mn[h][a], w));
+            mx[h][a] = fmaxf(mx[h][a], __shfl_xor_sync(0xffffffffu, mx[h][a], w));
+          }
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float dx = mx[h][0] - mn[h][0], dy = mx[h][1] - mn[h][1], dz = mx[h][2] - mn[h][2];
+        v[h] = dy > dx ? (dz > dy ? x[h][2] : x[h][1]) : (dz > dx ? x[h][2] : x[h][0]);
+      }
+      int rank[2] = {0, 0};
+      if (grp == 64) {
+        for (int t = 0; t < 32; ++t) {
+          const float u = __shfl_sync(0xffffffffu, v[0], t), w = __shfl_sync(0xffffffffu, v[1], t);
+          rank[0] += (u < v[0] || (u == v[0] && t < lane)) + (w < v[0]);
+          rank[1] += (u <= v[1]) + (w < v[1] || (w == v[1] && t < lane));
+        }
+      } else {
+        const int g0 = lane & ~(grp - 1);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          for (int t = 0; t < grp; ++t) {
+            const float u = __shfl_sync(0xffffffffu, v[h], g0 + t);
+            rank[h] += u < v[h] || (u == v[h] && g0 + t < lane);
+          }
+          rank[h] += 32 * h + g0;
+        }
+      }
+      __syncwarp();
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (id[h] >= 0) ia[p0 + rank[h]] = (unsigned short)id[h];
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  // the ids of all entries are read before any is written (from_perm)
+  int32_t id[ORDER_SEGMENT / 256];
+#pragma unroll
+  for (int t = 0; t < ORDER_SEGMENT / 256; ++t) {
+    const int i = tid + t * T;
+    if (i < n) id[t] = g.from_perm ? out[ia[i]] : ia[i];
   }
   __syncthreads();
 #pragma unroll
-  for (int t = 0; t < ORDER_SEGMENT / ORDER_THREADS; ++t) {
-    const int i = tid + t * ORDER_THREADS;
+  for (int t = 0; t < ORDER_SEGMENT / 256; ++t) {
+    const int i = tid + t * T;
     if (i < n) out[i] = id[t];
   }
 }
@@ -920,9 +1066,10 @@ int launch_order(const std::vector<OrderSeg>& segs, int32_t* d_perm, cudaStream_
   int rc = ensure_smem_limit(reinterpret_cast<const void*>(order_kernel), (int)order_smem(ORDER_SEGMENT), "order_kernel");
   if (rc) return rc;
   OrderSeg* d = nullptr;
-  PI_CUDA(cudaMallocAsync((void**)&d, segs.size() * sizeof(OrderSeg), s));
+  PI_CUDA(pool_alloc((void**)&d, segs.size() * sizeof(OrderSeg), s));
   PI_CUDA(cudaMemcpyAsync(d, segs.data(), segs.size() * sizeof(OrderSeg), cudaMemcpyHostToDevice, s));
-  order_kernel<<<(unsigned)segs.size(), ORDER_THREADS, order_smem(n2), s>>>(d, d_perm, n2);
+  // at most eight entries per thread, and a warp per part and block while there are few
+  order_kernel<<<(unsigned)segs.size(), n2 > 512 ? 1024 : 256, order_smem(n2), s>>>(d, d_perm, n2);
   PI_LAUNCHED("order_kernel");
   PI_CUDA(cudaFreeAsync(d, s));
   return PI_OK;
@@ -944,7 +1091,7 @@ int launch_prepare(pi_batch_impl* b, int only_index, cudaStream_t s) {
   }
   if (b->n_obj == 0) return PI_OK;
   PrepObj* d = nullptr;
-  PI_CUDA(cudaMallocAsync((void**)&d, sizeof(PrepObj) * h.size(), s));
+  PI_CUDA(pool_alloc((void**)&d, sizeof(PrepObj) * h.size(), s));
   PI_CUDA(cudaMemcpyAsync(d, h.data(), sizeof(PrepObj) * h.size(), cudaMemcpyHostToDevice, s));
   const int nobj_launch = only_index >= 0 ? 1 : b->n_obj;
   prepare_origin_kernel<<<nobj_launch, 256, 0, s>>>(d, b->d_objs, b->d_cl_rho, only_index);

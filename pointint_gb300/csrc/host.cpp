@@ -55,6 +55,34 @@ int ensure_smem_limit(const void* fn, int bytes, const char* what) {
   return it->second == cudaSuccess ? PI_OK : cuda_fail(it->second, what);
 }
 
+cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s) {
+  static std::mutex mu;
+  static std::map<int, cudaMemPool_t> pools;  // per device, for the life of the process
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  cudaMemPool_t pool = nullptr;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = pools.find(dev);
+    if (it == pools.end()) {
+      cudaMemPoolProps props{};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      if ((e = cudaMemPoolCreate(&pool, &props)) != cudaSuccess) return e;
+      uint64_t keep = POOL_KEEP;
+      if ((e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+        cudaMemPoolDestroy(pool);
+        return e;
+      }
+      it = pools.emplace(dev, pool).first;
+    }
+    pool = it->second;
+  }
+  return cudaMallocFromPoolAsync(p, bytes, pool, s);
+}
+
 int launch_split(const void* fn, dim3 grid, int threads, size_t smem, int split, void** args, cudaStream_t s) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;

@@ -591,7 +591,7 @@ int launch_jacobian(const pi_kgrid_impl* kg, const pi_batch_impl* b, float2* G, 
   all.insert(all.end(), surf.begin(), surf.end());
   all.insert(all.end(), mesh.begin(), mesh.end());
   JacObj* d = nullptr;
-  PI_CUDA(cudaMallocAsync((void**)&d, nj * sizeof(JacObj), s));
+  PI_CUDA(pool_alloc((void**)&d, nj * sizeof(JacObj), s));
   PI_CUDA(cudaMemcpyAsync(d, all.data(), nj * sizeof(JacObj), cudaMemcpyHostToDevice, s));
   const KGridDev K = kg->dev;
   const BatchDev B = b->dev();
