@@ -32,6 +32,7 @@
 // directions x JAC_R neighbouring radii); the others one radius per thread (a
 // warp owns 32 directions at one radius).  The origin phase e^{ik.o} and
 // sqrt|w| are applied once per output.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
@@ -39,6 +40,7 @@
 #include "pi_internal.h"
 #include "dfmath.cuh"
 #include "bessel.cuh"
+#include "moments.h"
 #include "tri_adjoint.cuh"
 
 namespace pi {
@@ -52,6 +54,14 @@ constexpr int JAC_TILE = 128;
 constexpr int JAC_COPIES = 4;
 
 enum { JAC_AFFINE_TRI = 0, JAC_AFFINE_SURF = 1, JAC_MESH_TRI = 2 };
+
+// Radii that the expansions cover (as moment_radii): the derivatives' first
+// dropped term is below 1.1e-7 of the leading one at k rho = 2.5 for an
+// element on the rim seen edge-on.
+constexpr float JAC_X_TRI = 2.5f;
+__device__ __forceinline__ int jac_moment_radii(const KGridDev& kg, float rho) {
+  return covered_radii(kg, rho, JAC_X_TRI);
+}
 
 struct JacObj {
   int32_t obj, kind;
@@ -77,6 +87,8 @@ struct kcf {
   }
   __device__ __forceinline__ cf value() const { return cf{sr, si}; }
 };
+
+constexpr int JAC_NSUM = 12;  // floats per radius of the affine triangles' sums: NF[3], W[3] (complex)
 
 struct JacThread {
   int j, jm, r;  // direction j evaluated, its antipode jm written from it (or -1)
@@ -193,6 +205,102 @@ __device__ __forceinline__ TriNode tri_node(const JacThread& t, const float2* ct
 
 __device__ __forceinline__ float comp(float3 v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : v.z); }
 
+// Writes the 12 derivatives of an affine triangle object at one node and its
+// antipode from the sums NF = sum_e F N0 (complex 3-vector) and
+// W = sum_e gamma (i F a0 + D_b E1 + D_c E2), both in the object frame:
+//   A = -2 sum gamma F = -khat . (cof(A) NF)     (S = cof(A) N0 / 2)
+//   dA/dt_r = i k d_r A
+//   dA/dA_rc = -2 (MF_rc + k d_r W_c),
+//   MF[r][c] = sum_e F_e sum_s grad_s(gamma)_r x0_s[c] = ((khat / 2) x (A (e_c x NF)))_r
+struct JacWriter {
+  float A[9], cofd[3];  // A row-major, cof(A)^T khat
+  float3 dh, kh;        // direction, khat / 2
+  double so_d;          // direction . origin
+  float dnorm;
+  int j, jm;
+  int64_t row0;
+  __device__ __forceinline__ JacWriter(const JacObj& jo, const ObjDev& od, float3 dh_, float3 dl, float inv_norm,
+                                       float dnorm_, int j_, int jm_)
+      : dh(dh_), dnorm(dnorm_), j(j_), jm(jm_), row0(jo.row0) {
+    const double* M = jo.dofs + 3;
+#pragma unroll
+    for (int a = 0; a < 9; ++a) A[a] = (float)M[a];
+    kh = make_float3(0.5f * dh.x * inv_norm, 0.5f * dh.y * inv_norm, 0.5f * dh.z * inv_norm);
+    const float k3[3] = {2.0f * kh.x, 2.0f * kh.y, 2.0f * kh.z};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const int c1 = (c + 1) % 3, c2 = (c + 2) % 3;
+      double v = 0.0;
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const int r1 = (r + 1) % 3, r2 = (r + 2) % 3;
+        v += (double)k3[r] * (M[3 * r1 + c1] * M[3 * r2 + c2] - M[3 * r1 + c2] * M[3 * r2 + c1]);
+      }
+      cofd[c] = (float)v;
+    }
+    so_d = ((double)dh.x + dl.x) * od.origin[0] + ((double)dh.y + dl.y) * od.origin[1] +
+           ((double)dh.z + dl.z) * od.origin[2];
+  }
+  __device__ __forceinline__ void put(const KGridDev& kg, float2* G, int r, float2 km, const float (&sv)[JAC_NSUM]) const {
+    const JacOut o = jac_out(kg, r, j, jm);
+    const float k = km.x;
+    // e^{ik.o} (0 at k = 0, where A = 0 by definition); sqrt|w| at the store
+    const cf eo = cis_f64(((double)km.x + (double)km.y) * so_d);
+    const cf sc = (k * dnorm < 1e-10f) ? cf{0.f, 0.f} : eo;
+    const cf Nt[3] = {cf{sv[0], sv[1]}, cf{sv[2], sv[3]}, cf{sv[4], sv[5]}};
+    const cf a = cmul(cf{-fmaf(cofd[0], Nt[0].re, fmaf(cofd[1], Nt[1].re, cofd[2] * Nt[2].re)),
+                         -fmaf(cofd[0], Nt[0].im, fmaf(cofd[1], Nt[1].im, cofd[2] * Nt[2].im))}, sc);
+    float2* out = G + row0 * kg.Q;
+#pragma unroll
+    for (int rr = 0; rr < 3; ++rr) {  // dA/dt_r = i k d_r A
+      const float kd = k * comp(dh, rr);
+      o.put(out + (int64_t)rr * kg.Q, cf{-kd * a.im, kd * a.re});
+    }
+    cf MF[9];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      cf v[3];  // e_c x NF
+      v[c] = cf{0.f, 0.f};
+      v[(c + 1) % 3] = cf{-Nt[(c + 2) % 3].re, -Nt[(c + 2) % 3].im};
+      v[(c + 2) % 3] = Nt[(c + 1) % 3];
+      cf mv[3];  // A v
+#pragma unroll
+      for (int a3 = 0; a3 < 3; ++a3) {
+        const float x0 = A[3 * a3], x1 = A[3 * a3 + 1], x2 = A[3 * a3 + 2];
+        mv[a3] = cf{fmaf(x0, v[0].re, fmaf(x1, v[1].re, x2 * v[2].re)), fmaf(x0, v[0].im, fmaf(x1, v[1].im, x2 * v[2].im))};
+      }
+      MF[c] = cf{kh.y * mv[2].re - kh.z * mv[1].re, kh.y * mv[2].im - kh.z * mv[1].im};
+      MF[3 + c] = cf{kh.z * mv[0].re - kh.x * mv[2].re, kh.z * mv[0].im - kh.x * mv[2].im};
+      MF[6 + c] = cf{kh.x * mv[1].re - kh.y * mv[0].re, kh.x * mv[1].im - kh.y * mv[0].im};
+    }
+#pragma unroll
+    for (int rr = 0; rr < 3; ++rr)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const cf mf = MF[3 * rr + c], w = cf{sv[6 + 2 * c], sv[7 + 2 * c]};
+        const float kd = k * comp(dh, rr);
+        const cf v = cmul(cf{-2.0f * (mf.re + kd * w.re), -2.0f * (mf.im + kd * w.im)}, sc);
+        o.put(out + (int64_t)(3 + 3 * rr + c) * kg.Q, v);
+      }
+  }
+};
+
+// Reference-frame values of one element: its first vertex a0, edges E1, E2 and
+// doubled area vector N0 = E1 x E2.
+struct TriRef { float a0[3], E1[3], E2[3], N0[3]; };
+
+__device__ __forceinline__ TriRef tri_ref(const TriSrcJ& s) {
+  TriRef t;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    t.a0[c] = (float)s.a[c];
+    t.E1[c] = (float)s.e1[c];
+    t.E2[c] = (float)s.e2[c];
+    t.N0[c] = (float)(s.e1[(c + 1) % 3] * s.e2[(c + 2) % 3] - s.e1[(c + 2) % 3] * s.e2[(c + 1) % 3]);
+  }
+  return t;
+}
+
 // ---- AffineDoF triangles -------------------------------------------------------------
 // A thread owns one direction and R neighbouring radii (the warp 32
 // directions, the CTA 4 neighbouring direction blocks of one radial block).
@@ -206,24 +314,29 @@ __device__ __forceinline__ float comp(float3 v, int i) { return i == 0 ? v.x : (
 // the same for the whole warp on a tensor grid) and three complex products.
 // Radial blocks run heavy-first and the CTA order is re-mapped so that every
 // object's heavy blocks start first, as in ff_kernel.  Per radius and node
-// seven complex sums, chunked in FP32 and Kahan-compensated in shared memory:
-//   A  += -2 gamma F                                   (translations: i k d A)
-//   NF += F N0,  N0 = E1 x E2 (reference edges)        (see MF below)
+// six complex sums, chunked in FP32 and Kahan-compensated in shared memory:
+//   NF += F N0,  N0 = E1 x E2 (reference edges)
 //   W  += gamma (i F a0 + D_b E1 + D_c E2)             (sum_s D_s x0_s, D_a + D_b + D_c = i F)
-constexpr int JAC_NSUM = 14;  // floats per radius: A, NF[3], W[3] (complex)
+// (JacWriter forms the 12 derivatives from them.)  The radii of the cluster
+// expansions (jac_moment_kernel) are left out; the CTAs of a thread-block
+// cluster split the elements, as in ff_kernel.
 
 template <int R>
 __global__ void __launch_bounds__(JAC_THREADS, 3)
 jac_affine_tri_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, float2* __restrict__ G) {
-  const unsigned lin = blockIdx.y * gridDim.x + blockIdx.x;
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const unsigned lin = (blockIdx.y * gridDim.x + blockIdx.x) / (unsigned)S;
   const int slot = (int)(lin % gridDim.y), cta = (int)(lin / gridDim.y);
   const JacObj jo = jobs[slot];
   const ObjDev od = b.objs[jo.obj];
-  const int nrb = (kg.L + R - 1) / R, ndt = (kg.Me + 31) / 32;
+  const int r_first = jac_moment_radii(kg, __uint_as_float(b.cl_rho[jo.obj]));
+  const int nrb = (kg.L - r_first + R - 1) / R, ndt = (kg.Me + 31) / 32;
+  if (cta * JAC_WARPS >= ndt * nrb) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int item = cta * JAC_WARPS + warp;
   const int ib = item / ndt, dt = item - ib * ndt;
-  const int rb = ib < nrb ? nrb - 1 - ib : 0;
+  const int rlo = kg.L - (ib + 1) * R, skip = max(0, r_first - rlo);  // radii rlo + i, i >= skip
   const int ei = dt * 32 + lane;
   const bool active = item < ndt * nrb && ei < kg.Me;
   int j = 0, jm = -1;  // direction evaluated, its antipode written from it (or -1)
@@ -244,8 +357,8 @@ jac_affine_tri_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, 
   __shared__ float run[2 * JAC_NSUM * R * JAC_THREADS];  // running sums, then compensations
   stage_phasors<JAC_COPIES>(kg.cis_tab, ctab_sm);
   if (lane < R) {
-    const int r = rb * R + lane;
-    const bool ok = item < ndt * nrb && r < kg.L;
+    const int r = rlo + lane;
+    const bool ok = item < ndt * nrb && lane >= skip;
     const float2 km = ok ? kg.kmag[r] : make_float2(0.f, 0.f);
     const float2 kt = ok ? kg.kt64[r] : make_float2(0.f, 0.f);
     krad[warp][lane] = make_float4(km.x, km.y, kt.x, kt.y);
@@ -273,21 +386,19 @@ jac_affine_tri_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, 
   const float4* pool = b.tri_pool + 3 * od.elem_off;
   const float4* pool_lo = b.tri_lo + od.elem_off;
   const TriSrcJ* src = reinterpret_cast<const TriSrcJ*>(jo.src);
-  for (int base = 0; base < od.n_elems; base += JAC_TILE) {
-    const int cnt = min(JAC_TILE, od.n_elems - base);
+  const int per = (od.n_elems + S * 16 - 1) / (S * 16) * 16;  // this CTA's elements, whole chunks
+  const int n0 = min(od.n_elems, rank * per), n1 = min(od.n_elems, n0 + per);
+  for (int base = n0; base < n1; base += JAC_TILE) {
+    const int cnt = min(JAC_TILE, n1 - base);
     __syncthreads();
     for (int e = threadIdx.x; e < cnt; e += JAC_THREADS) {
       tile[6 * e] = pool[3 * (int64_t)(base + e)];
       tile[6 * e + 1] = pool[3 * (int64_t)(base + e) + 1];
       tile[6 * e + 2] = pool[3 * (int64_t)(base + e) + 2];
-      // the reference vertex a0 and edges E1, E2; in .w the reference
-      // doubled area vector N0 = E1 x E2
-      const TriSrcJ& s = src[od.perm_off >= 0 ? b.perm[od.perm_off + base + e] : base + e];
-      const double n0x = s.e1[1] * s.e2[2] - s.e1[2] * s.e2[1], n0y = s.e1[2] * s.e2[0] - s.e1[0] * s.e2[2],
-                   n0z = s.e1[0] * s.e2[1] - s.e1[1] * s.e2[0];
-      tile[6 * e + 3] = make_float4((float)s.a[0], (float)s.a[1], (float)s.a[2], (float)n0x);
-      tile[6 * e + 4] = make_float4((float)s.e1[0], (float)s.e1[1], (float)s.e1[2], (float)n0y);
-      tile[6 * e + 5] = make_float4((float)s.e2[0], (float)s.e2[1], (float)s.e2[2], (float)n0z);
+      const TriRef t = tri_ref(src[od.perm_off >= 0 ? b.perm[od.perm_off + base + e] : base + e]);
+      tile[6 * e + 3] = make_float4(t.a0[0], t.a0[1], t.a0[2], t.N0[0]);
+      tile[6 * e + 4] = make_float4(t.E1[0], t.E1[1], t.E1[2], t.N0[1]);
+      tile[6 * e + 5] = make_float4(t.E2[0], t.E2[1], t.E2[2], t.N0[2]);
       tile[6 * JAC_TILE + e] = pool_lo[base + e];  // centroid low word, longest edge
     }
     __syncthreads();
@@ -304,6 +415,7 @@ jac_affine_tri_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, 
       const TriDerPoly cp = tri_der_coeffs(d1.hi, d2.hi);
 #pragma unroll
       for (int i = 0; i < R; ++i) {
+        if (i < skip) continue;
         const float4 kr = krad[warp][i];
         const float k = kr.x;
         cf F, Db, Dc;
@@ -332,84 +444,301 @@ jac_affine_tri_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, 
           Dc = d.Dc;
         }
         const float4 ta = tile[6 * e + 3], tb = tile[6 * e + 4], tc = tile[6 * e + 5];
-        const float g2 = -2.0f * gam;
-        acc[i][0] = fmaf(F.re, g2, acc[i][0]);
-        acc[i][1] = fmaf(F.im, g2, acc[i][1]);
-        acc[i][2] = fmaf(F.re, ta.w, acc[i][2]);
-        acc[i][3] = fmaf(F.im, ta.w, acc[i][3]);
-        acc[i][4] = fmaf(F.re, tb.w, acc[i][4]);
-        acc[i][5] = fmaf(F.im, tb.w, acc[i][5]);
-        acc[i][6] = fmaf(F.re, tc.w, acc[i][6]);
-        acc[i][7] = fmaf(F.im, tc.w, acc[i][7]);
+        acc[i][0] = fmaf(F.re, ta.w, acc[i][0]);
+        acc[i][1] = fmaf(F.im, ta.w, acc[i][1]);
+        acc[i][2] = fmaf(F.re, tb.w, acc[i][2]);
+        acc[i][3] = fmaf(F.im, tb.w, acc[i][3]);
+        acc[i][4] = fmaf(F.re, tc.w, acc[i][4]);
+        acc[i][5] = fmaf(F.im, tc.w, acc[i][5]);
         const cf gF = cscale(F, gam), gB = cscale(Db, gam), gC = cscale(Dc, gam);
         const float a0[3] = {ta.x, ta.y, ta.z}, E1[3] = {tb.x, tb.y, tb.z}, E2[3] = {tc.x, tc.y, tc.z};
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          acc[i][8 + 2 * c] = fmaf(-gF.im, a0[c], fmaf(gB.re, E1[c], fmaf(gC.re, E2[c], acc[i][8 + 2 * c])));
-          acc[i][9 + 2 * c] = fmaf(gF.re, a0[c], fmaf(gB.im, E1[c], fmaf(gC.im, E2[c], acc[i][9 + 2 * c])));
+          acc[i][6 + 2 * c] = fmaf(-gF.im, a0[c], fmaf(gB.re, E1[c], fmaf(gC.re, E2[c], acc[i][6 + 2 * c])));
+          acc[i][7 + 2 * c] = fmaf(gF.re, a0[c], fmaf(gB.im, E1[c], fmaf(gC.im, E2[c], acc[i][7 + 2 * c])));
         }
       }
       if ((e & 15) == 15) flush();
     }
     flush();
   }
-  if (!active) return;
-  // MF[r][c] = sum_e F_e sum_s grad_s(gamma)_r x0_s[c] = ((khat / 2) x (A (e_c x N~)))_r, N~ = sum_e F_e N0_e
-  const double* Am = jo.dofs + 3;  // A row-major
-  float Af[9];
+  const auto mine = [&](int i) { return (i & (S - 1)) == rank; };  // S is a power of two
+  if (S > 1) {
+    cluster.sync();
+    float tot[R][JAC_NSUM];
 #pragma unroll
-  for (int a = 0; a < 9; ++a) Af[a] = (float)Am[a];
-  const float3 kh = make_float3(0.5f * dh.x * inv_norm, 0.5f * dh.y * inv_norm, 0.5f * dh.z * inv_norm);
-  const double so_d = ((double)dh.x + dl.x) * od.origin[0] + ((double)dh.y + dl.y) * od.origin[1] +
-                      ((double)dh.z + dl.z) * od.origin[2];
+    for (int i = 0; i < R; ++i) {
+      if (!mine(i)) continue;
+#pragma unroll
+      for (int v = 0; v < JAC_NSUM; ++v) {
+        kbsum t{0.f, 0.f};
+        for (int q = 0; q < S; ++q) {
+          const float* o = cluster.map_shared_rank(run, q) + (i * JAC_NSUM + v) * JAC_THREADS + threadIdx.x;
+          t.add(o[0]);
+          t.lo -= o[JAC_NSUM * R * JAC_THREADS];
+        }
+        tot[i][v] = t.hi + t.lo;
+      }
+    }
+    cluster.sync();  // no CTA leaves, or overwrites them, while its sums are read
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+      if (mine(i))
+#pragma unroll
+        for (int v = 0; v < JAC_NSUM; ++v) run[(i * JAC_NSUM + v) * JAC_THREADS + threadIdx.x] = tot[i][v];
+  }
+  if (!active) return;
+  const JacWriter w(jo, od, dh, dl, inv_norm, dnorm, j, jm);
 #pragma unroll
   for (int i = 0; i < R; ++i) {
-    const int r = rb * R + i;
-    if (r >= kg.L) continue;
+    if (i < skip || !mine(i)) continue;
     const float4 kr = krad[warp][i];
-    const float k = kr.x;
-    const JacOut o = jac_out(kg, r, j, jm);
-    // e^{ik.o} (0 at k = 0, where A = 0 by definition); sqrt|w| at the store
-    const cf eo = cis_f64(((double)kr.x + (double)kr.y) * so_d);
-    const cf sc = (k * dnorm < 1e-10f) ? cf{0.f, 0.f} : eo;
     float sv[JAC_NSUM];
 #pragma unroll
     for (int v = 0; v < JAC_NSUM; ++v) sv[v] = run[(i * JAC_NSUM + v) * JAC_THREADS + threadIdx.x];
-    const cf a = cmul(cf{sv[0], sv[1]}, sc);
-    float2* out = G + jo.row0 * kg.Q;
+    w.put(kg, G, rlo + i, make_float2(kr.x, kr.y), sv);
+  }
+}
+
+// The sums NF and W at small k from cluster expansions (moments.cu): with the
+// vertices' projections a, b, c from the cluster's centre, F = e^{ik.c} sum_n
+// i^{n+2} k^n h_n(a, b, c)/(n+2)! and D_b = e^{ik.c} sum_n i^{n+3} k^n
+// h_n(a, b, b, c)/(n+3)!, so
+//   NF:  sum_n i^{n+2} k^n / (n+2)! sum_e N0 h_n
+//   W: i sum_n i^{n+2} k^n / (n+3)! sum_e gamma (a0 (n+3) h_n + E1 h_n(a,b,b,c) + E2 h_n(a,b,c,c)).
+// One CTA owns one object, 32 evaluated directions (one per lane) and up to
+// JM_RADII of the covered radii, and alternates between two phases over tiles
+// of four clusters: two warps per cluster form its 6 x 16 real moments (the
+// recurrences in both, NF and W_x in one, W_y and W_z in the other: ~190 FP32
+// operations per element, direction and warp for all radii, where the direct
+// sum takes ~190 for each), then each warp sums the tile over its own radii,
+// JM_R at a time.  The CTAs of a thread-block cluster split the tiles.
+constexpr int JM_WARPS = 8, JM_THREADS = 32 * JM_WARPS, JM_TILE = JM_WARPS / 2;
+constexpr int JM_SETS = JAC_NSUM / 2, JM_R = 3, JM_RADII = 2 * JM_R * JM_WARPS;
+constexpr int JM_ELEM_F4 = 6;  // staged floats of an element, as float4: vertices, S, N0, a0, E1, E2
+
+// float4 counts: staged elements, coefficients, running sums (and compensations)
+constexpr int JM_F4_ELEM = JM_TILE * PI_CLUSTER * JM_ELEM_F4, JM_F4_MOM = JM_TILE * JM_SETS * 4 * 32,
+              JM_F4_RUN = JM_RADII * JAC_NSUM * 2 * 32 / 4;
+constexpr int JM_SMEM = (JM_F4_ELEM + JM_F4_MOM + JM_F4_RUN) * (int)sizeof(float4);
+
+template <int HALF>
+__device__ __forceinline__ void jac_moments(const float4* es, int cnt, float3 d, float inv_norm, float4* mom) {
+  constexpr int NS = HALF == 0 ? 4 : 2;  // sets of this warp: NF, W_x / W_y, W_z
+  float mu[NS][MOMENT_TERMS];
 #pragma unroll
-    for (int rr = 0; rr < 3; ++rr) {  // dA/dt_r = i k d_r A
-      const float kd = k * comp(dh, rr);
-      o.put(out + (int64_t)rr * kg.Q, cf{-kd * a.im, kd * a.re});
-    }
-    const cf Nt[3] = {cf{sv[2], sv[3]}, cf{sv[4], sv[5]}, cf{sv[6], sv[7]}};
-    cf MF[9];
+  for (int v = 0; v < NS; ++v)
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      cf v[3];  // e_c x N~
-      v[c] = cf{0.f, 0.f};
-      v[(c + 1) % 3] = cf{-Nt[(c + 2) % 3].re, -Nt[(c + 2) % 3].im};
-      v[(c + 2) % 3] = Nt[(c + 1) % 3];
-      cf mv[3];  // A v
+    for (int n = 0; n < MOMENT_TERMS; ++n) mu[v][n] = 0.f;
+#pragma unroll 1
+  for (int i = 0; i < cnt; ++i) {
+    const float4 q0 = es[JM_ELEM_F4 * i], q1 = es[JM_ELEM_F4 * i + 1], q2 = es[JM_ELEM_F4 * i + 2],
+                 q3 = es[JM_ELEM_F4 * i + 3], q4 = es[JM_ELEM_F4 * i + 4], q5 = es[JM_ELEM_F4 * i + 5];
+    const float a = d.x * q0.x + d.y * q0.y + d.z * q0.z, bb = d.x * q0.w + d.y * q1.x + d.z * q1.y,
+                c = d.x * q1.z + d.y * q1.w + d.z * q2.x, g = (d.x * q2.y + d.y * q2.z + d.z * q2.w) * inv_norm;
+    const float N0[3] = {q3.x, q3.y, q3.z};
+    const float w0[2] = {g * (HALF == 0 ? q3.w : q4.x), g * q4.y};  // gamma a0
+    const float w1[2] = {g * (HALF == 0 ? q4.z : q4.w), g * q5.x};  // gamma E1
+    const float w2[2] = {g * (HALF == 0 ? q5.y : q5.z), g * q5.w};  // gamma E2
+    float an = 1.f, qn = 1.f, hn = 1.f, hb = 1.f, hc = 1.f;
 #pragma unroll
-      for (int a3 = 0; a3 < 3; ++a3) {
-        const float x0 = Af[3 * a3], x1 = Af[3 * a3 + 1], x2 = Af[3 * a3 + 2];
-        mv[a3] = cf{fmaf(x0, v[0].re, fmaf(x1, v[1].re, x2 * v[2].re)), fmaf(x0, v[0].im, fmaf(x1, v[1].im, x2 * v[2].im))};
+    for (int n = 0; n < MOMENT_TERMS; ++n) {
+      if (n > 0) {
+        an *= a;
+        qn = fmaf(bb, qn, an);
+        hn = fmaf(c, hn, qn);
+        hb = fmaf(bb, hb, hn);
+        hc = fmaf(c, hc, hn);
       }
-      MF[c] = cf{kh.y * mv[2].re - kh.z * mv[1].re, kh.y * mv[2].im - kh.z * mv[1].im};
-      MF[3 + c] = cf{kh.z * mv[0].re - kh.x * mv[2].re, kh.z * mv[0].im - kh.x * mv[2].im};
-      MF[6 + c] = cf{kh.x * mv[1].re - kh.y * mv[0].re, kh.x * mv[1].im - kh.y * mv[0].im};
+      const float hw = (float)(n + 3) * hn;
+      if (HALF == 0) {
+#pragma unroll
+        for (int v = 0; v < 3; ++v) mu[v][n] = fmaf(N0[v], hn, mu[v][n]);
+        mu[NS - 1][n] = fmaf(w0[0], hw, fmaf(w1[0], hb, fmaf(w2[0], hc, mu[NS - 1][n])));
+      } else {
+#pragma unroll
+        for (int v = 0; v < 2; ++v) mu[v][n] = fmaf(w0[v], hw, fmaf(w1[v], hb, fmaf(w2[v], hc, mu[v][n])));
+      }
+    }
+  }
+  constexpr FmConst<PI_GEOM_TRIANGLE> C{};  // 2/(n+2)!
+#pragma unroll
+  for (int v = 0; v < NS; ++v) {
+    const int set = HALF == 0 ? v : 4 + v;
+    float o[MOMENT_TERMS];
+#pragma unroll
+    for (int n = 0; n < MOMENT_TERMS; ++n) {  // i^{n+2}: real for even n, imaginary for odd n
+      const float f = (set < 3 ? 0.5f : 0.5f / (n + 3)) * C.f[n];
+      o[(n & 1) * (MOMENT_TERMS / 2) + n / 2] = mu[v][n] * ((n & 2) ? f : -f);
     }
 #pragma unroll
-    for (int rr = 0; rr < 3; ++rr)
+    for (int t = 0; t < 4; ++t) mom[(set * 4 + t) * 32] = make_float4(o[4 * t], o[4 * t + 1], o[4 * t + 2], o[4 * t + 3]);
+  }
+}
+
+__global__ void __launch_bounds__(JM_THREADS, 1)
+jac_moment_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, float2* __restrict__ G, int groups) {
+  extern __shared__ float4 jsm[];
+  float4* elem = jsm;
+  float4* mom = elem + JM_F4_ELEM;
+  float* run = reinterpret_cast<float*>(mom + JM_F4_MOM);  // [radius][sum or compensation][lane]
+  __shared__ float2 ctab_sm[PHASOR_ENTRIES * JAC_COPIES], csc[JM_TILE][32];
+  __shared__ float4 krad[JM_RADII];  // |k|, |k| 64 / 2 pi hi, lo
+  __shared__ float cscale[JM_TILE];
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const unsigned lin = (blockIdx.y * gridDim.x + blockIdx.x) / (unsigned)S;
+  const int slot = (int)(lin % gridDim.y), item = (int)(lin / gridDim.y);
+  const int dt = item / groups, r0 = (item - dt * groups) * JM_RADII;
+  const JacObj jo = jobs[slot];
+  const ObjDev od = b.objs[jo.obj];
+  const int nr = min(JM_RADII, jac_moment_radii(kg, __uint_as_float(b.cl_rho[jo.obj])) - r0);  // radii r0 .. r0 + nr - 1
+  if (nr <= 0) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ei = dt * 32 + lane;
+  const bool active = ei < kg.Me;
+  int j = 0, jm = -1;
+  float3 dh = make_float3(0.f, 0.f, 0.f), dl = dh;
+  float inv_norm = 0.f, dnorm = 0.f;
+  if (active) {
+    const int2 pr = kg.dpair[ei];
+    j = pr.x;
+    jm = pr.y;
+    const float4 h = kg.dir_hi[j], l = kg.dir_lo[j];
+    dh = make_float3(h.x, h.y, h.z);
+    dl = make_float3(l.x, l.y, l.z);
+    inv_norm = h.w;
+    dnorm = l.w;
+  }
+  stage_phasors<JAC_COPIES>(kg.cis_tab, ctab_sm);
+  const float2* ctab = ctab_sm + (threadIdx.x % JAC_COPIES);
+  for (int t = threadIdx.x; t < JM_RADII; t += JM_THREADS) {
+    const bool ok = t < nr;
+    const float2 km = ok ? kg.kmag[r0 + t] : make_float2(0.f, 0.f), kt = ok ? kg.kt64[r0 + t] : make_float2(0.f, 0.f);
+    krad[t] = make_float4(km.x, kt.x, kt.y, km.y);
+  }
+  for (int t = threadIdx.x; t < JM_F4_RUN; t += JM_THREADS) reinterpret_cast<float4*>(run)[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+  const TriSrcJ* src = reinterpret_cast<const TriSrcJ*>(jo.src);
+  const int ncl = (od.n_elems + PI_CLUSTER - 1) / PI_CLUSTER;
+  for (int t0 = rank * JM_TILE; t0 < ncl; t0 += S * JM_TILE) {
+    __syncthreads();  // the last tile's elements and coefficients have been read
+    // stage the tile's elements relative to their clusters' centres, in units of s
+    for (int t = threadIdx.x; t < JM_TILE * PI_CLUSTER; t += JM_THREADS) {
+      const int p = t0 * PI_CLUSTER + t;
+      if (p >= od.n_elems) continue;
+      const float4 ctr = b.clusters[od.cl_off + p / PI_CLUSTER];
+      const int ex = ctr.w > 0.f ? min(120, max(-100, ilogbf(ctr.w) + 1)) : 0;
+      const float inv_s = __int_as_float((127 - ex) << 23);
+      const int64_t e = od.elem_off + p;
+      const float4 q0 = b.tri_pool[3 * e], q1 = b.tri_pool[3 * e + 1], q2 = b.tri_pool[3 * e + 2], lo = b.tri_lo[e];
+      const float m[3] = {(q0.x - ctr.x) + lo.x, (q0.y - ctr.y) + lo.y, (q0.z - ctr.z) + lo.z};
+      const float e1[3] = {q1.x, q1.y, q1.z}, e2[3] = {q2.x, q2.y, q2.z};
+      float va[3], vb[3], vc[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const cf mf = MF[3 * rr + c], w = cf{sv[8 + 2 * c], sv[9 + 2 * c]};
-        const float kd = k * comp(dh, rr);
-        const cf v = cmul(cf{-2.0f * (mf.re + kd * w.re), -2.0f * (mf.im + kd * w.im)}, sc);
-        o.put(out + (int64_t)(3 + 3 * rr + c) * kg.Q, v);
+        const float a = m[c] - (e1[c] + e2[c]) * (1.0f / 3.0f);
+        va[c] = a * inv_s;
+        vb[c] = (a + e1[c]) * inv_s;
+        vc[c] = (a + e2[c]) * inv_s;
       }
+      const TriRef f = tri_ref(src[od.perm_off >= 0 ? b.perm[od.perm_off + p] : p]);
+      float4* d = elem + (size_t)t * JM_ELEM_F4;
+      d[0] = make_float4(va[0], va[1], va[2], vb[0]);
+      d[1] = make_float4(vb[1], vb[2], vc[0], vc[1]);
+      d[2] = make_float4(vc[2], q0.w, q1.w, q2.w);
+      d[3] = make_float4(f.N0[0], f.N0[1], f.N0[2], f.a0[0]);
+      d[4] = make_float4(f.a0[1], f.a0[2], f.E1[0], f.E1[1]);
+      d[5] = make_float4(f.E1[2], f.E2[0], f.E2[1], f.E2[2]);
+    }
+    __syncthreads();
+    const int c_own = warp >> 1, cl = t0 + c_own;
+    if (cl < ncl) {
+      const int cnt = min(PI_CLUSTER, od.n_elems - cl * PI_CLUSTER);
+      const float4* es = elem + (size_t)c_own * PI_CLUSTER * JM_ELEM_F4;
+      float4* mo = mom + c_own * JM_SETS * 4 * 32 + lane;
+      if (warp & 1) {
+        jac_moments<1>(es, cnt, dh, inv_norm, mo);
+        const float4 ctr = b.clusters[od.cl_off + cl];
+        const int ex = ctr.w > 0.f ? min(120, max(-100, ilogbf(ctr.w) + 1)) : 0;
+        const df sc = cdot(dh, dl, make_float3(ctr.x, ctr.y, ctr.z));
+        csc[c_own][lane] = make_float2(sc.hi, sc.lo);
+        if (lane == 0) cscale[c_own] = __int_as_float((127 + ex) << 23);
+      } else {
+        jac_moments<0>(es, cnt, dh, inv_norm, mo);
+      }
+    }
+    __syncthreads();
+    const int nc = min(JM_TILE, ncl - t0);
+    for (int rb = warp * JM_R; rb < nr; rb += JM_WARPS * JM_R) {
+      float acc[JM_R][JAC_NSUM];
+#pragma unroll
+      for (int i = 0; i < JM_R; ++i)
+#pragma unroll
+        for (int v = 0; v < JAC_NSUM; ++v) acc[i][v] = 0.f;
+#pragma unroll 1
+      for (int c = 0; c < nc; ++c) {
+        const float2 sc = csc[c][lane];
+        const float s = cscale[c];
+        cf P[JM_R];
+        float k[JM_R];
+#pragma unroll
+        for (int i = 0; i < JM_R; ++i) {
+          const float4 kr = krad[rb + i];
+          P[i] = cis_tab_df<JAC_COPIES>(ctab, make_float2(kr.y, kr.z), df{sc.x, sc.y});
+          k[i] = kr.x * s;
+        }
+#pragma unroll
+        for (int v = 0; v < JM_SETS; ++v) {
+          const float4* mo = mom + (c * JM_SETS + v) * 4 * 32 + lane;
+          const float4 m0 = mo[0], m1 = mo[32], m2 = mo[64], m3 = mo[96];
+#pragma unroll
+          for (int i = 0; i < JM_R; ++i) {
+            const float u = k[i] * k[i];
+            const float x = fmaf(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, m1.w, m1.z), m1.y), m1.x), m0.w), m0.z), m0.y), m0.x);
+            const float y = k[i] * fmaf(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, m3.w, m3.z), m3.y), m3.x), m2.w), m2.z), m2.y), m2.x);
+            acc[i][2 * v] = fmaf(P[i].re, x, fmaf(-P[i].im, y, acc[i][2 * v]));
+            acc[i][2 * v + 1] = fmaf(P[i].re, y, fmaf(P[i].im, x, acc[i][2 * v + 1]));
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < JM_R; ++i)
+#pragma unroll
+        for (int v = 0; v < JAC_NSUM; ++v) {
+          float* ps = run + ((rb + i) * 2 * JAC_NSUM + 2 * v) * 32 + lane;
+          const float sum = ps[0], y = acc[i][v] - ps[32], t = sum + y;
+          ps[32] = (t - sum) - y;
+          ps[0] = t;
+        }
+    }
   }
+  if (S > 1) cluster.sync();
+  else __syncthreads();
+  if (active) {
+    const JacWriter w(jo, od, dh, dl, inv_norm, dnorm, j, jm);
+    for (int r = warp * S + rank; r < nr; r += JM_WARPS * S) {
+      float sv[JAC_NSUM];
+#pragma unroll
+      for (int v = 0; v < JAC_NSUM; ++v) {
+        kbsum t{0.f, 0.f};
+        for (int q = 0; q < S; ++q) {
+          const float* o = (S > 1 ? cluster.map_shared_rank(run, q) : run) + (r * 2 * JAC_NSUM + 2 * v) * 32 + lane;
+          t.add(o[0]);
+          t.lo -= o[32];
+        }
+        sv[v] = t.hi + t.lo;
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {  // W = i times the sum
+        const float re = sv[6 + 2 * c];
+        sv[6 + 2 * c] = -sv[7 + 2 * c];
+        sv[7 + 2 * c] = re;
+      }
+      const float4 kr = krad[r];
+      w.put(kg, G, r0 + r, make_float2(kr.x, kr.w), sv);
+    }
+  }
+  if (S > 1) cluster.sync();  // no CTA leaves while its sums are read
 }
 
 // ---- AffineDoF disks / Gaussians --------------------------------------------------------
@@ -597,18 +926,38 @@ int launch_jacobian(const pi_kgrid_impl* kg, const pi_batch_impl* b, float2* G, 
   const BatchDev B = b->dev();
   const unsigned gx = (unsigned)(((int64_t)((K.Me + 31) / 32) * K.L + JAC_WARPS - 1) / JAC_WARPS);
   if (!tri.empty()) {
-    // the most radii per thread that still gives two waves of CTAs
     const int n_sm = current_sm_count();
+    int64_t n_max = 0, heavy = 0;
+    for (const JacObj& o : tri) n_max = std::max(n_max, b->info[o.obj].n_elems);
+    for (const JacObj& o : tri) heavy += 4 * b->info[o.obj].n_elems >= n_max;  // as in launch_form_factors
+    const int ndt = (K.Me + 31) / 32;
     auto ctas = [&](int R) {
-      return (int64_t)(((int64_t)((K.L + R - 1) / R) * ((K.Me + 31) / 32) + JAC_WARPS - 1) / JAC_WARPS);
+      return (int64_t)(((int64_t)((K.L + R - 1) / R) * ndt + JAC_WARPS - 1) / JAC_WARPS);
     };
-    const int64_t wave = (int64_t)n_sm * 3;
-    const int R = ctas(4) * (int64_t)tri.size() >= 2 * wave ? 4 : ctas(2) * (int64_t)tri.size() >= 2 * wave ? 2 : 1;
-    const dim3 grid((unsigned)ctas(R), (unsigned)tri.size());
-    if (R == 4) jac_affine_tri_kernel<4><<<grid, JAC_THREADS, 0, s>>>(K, B, d, G);
-    else if (R == 2) jac_affine_tri_kernel<2><<<grid, JAC_THREADS, 0, s>>>(K, B, d, G);
-    else jac_affine_tri_kernel<1><<<grid, JAC_THREADS, 0, s>>>(K, B, d, G);
+    auto busy = [&](int R) { return (K.moments ? (ctas(R) + 3) / 4 : ctas(R)) * heavy; };
+    // radii per thread and the split of the elements: two waves of three CTAs
+    // per SM, with four radii where sixteen splits give one
+    const int R = 16 * busy(4) >= 3 * (int64_t)n_sm ? 4 : 2;
+    int S = 1;
+    while (S < 16 && S * busy(R) < 6 * (int64_t)n_sm && n_max > 2 * S * 16) S *= 2;
+    void* args[4] = {const_cast<KGridDev*>(&K), const_cast<BatchDev*>(&B), &d, &G};
+    int rc = launch_split(R == 4 ? reinterpret_cast<const void*>(jac_affine_tri_kernel<4>)
+                                 : reinterpret_cast<const void*>(jac_affine_tri_kernel<2>),
+                          dim3((unsigned)(ctas(R) * S), (unsigned)tri.size()), JAC_THREADS, 0, S, args, s);
+    if (rc) return rc;
     PI_LAUNCHED("jac_affine_tri_kernel");
+    if (K.moments) {
+      const void* fn = reinterpret_cast<const void*>(jac_moment_kernel);
+      if ((rc = ensure_smem_limit(fn, JM_SMEM, "jac_moment_kernel"))) return rc;
+      int groups = (K.L + JM_RADII - 1) / JM_RADII;
+      int SM = 1;  // one CTA per SM
+      while (SM < 8 && (int64_t)SM * ndt * heavy < 2 * (int64_t)n_sm && n_max > SM * JM_TILE * PI_CLUSTER) SM *= 2;
+      void* margs[5] = {const_cast<KGridDev*>(&K), const_cast<BatchDev*>(&B), &d, &G, &groups};
+      rc = launch_split(fn, dim3((unsigned)(ndt * groups * SM), (unsigned)tri.size()), JM_THREADS, (size_t)JM_SMEM, SM,
+                        margs, s);
+      if (rc) return rc;
+      PI_LAUNCHED("jac_moment_kernel");
+    }
   }
   if (!surf.empty()) {
     jac_affine_surf_kernel<<<dim3(gx, (unsigned)surf.size()), JAC_THREADS, 0, s>>>(K, B, d + tri.size(), G);

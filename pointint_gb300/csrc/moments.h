@@ -22,17 +22,20 @@ constexpr float MOMENT_X_TRI = 3.0f, MOMENT_X_SURF = 2.25f;
 constexpr int MOMENT_MIN_L = 8, MOMENT_MAX_L = 288;
 
 #ifdef __CUDACC__
-// The radii [0, n) that the expansions of an object cover (radii ascend on a
-// grid with kg.moments); every lane of a warp calls this together.
-__device__ __forceinline__ int moment_radii(const KGridDev& kg, int type, float rho) {
+// The radii [0, n) with k rho <= bound (radii ascend on a grid with
+// kg.moments); every lane of a warp calls this together.
+__device__ __forceinline__ int covered_radii(const KGridDev& kg, float rho, float bound) {
   if (!kg.moments) return 0;
-  const float bound = type == PI_GEOM_TRIANGLE ? MOMENT_X_TRI : MOMENT_X_SURF;
   int n = 0;
   for (int r0 = 0; r0 < kg.L; r0 += 32) {
     const int r = r0 + (int)(threadIdx.x & 31);
     n += __popc(__ballot_sync(0xffffffffu, r < kg.L && kg.kmag[r].x * rho <= bound));
   }
   return n;
+}
+
+__device__ __forceinline__ int moment_radii(const KGridDev& kg, int type, float rho) {
+  return covered_radii(kg, rho, type == PI_GEOM_TRIANGLE ? MOMENT_X_TRI : MOMENT_X_SURF);
 }
 // Constants of the recurrences: the coefficient of (i k)^n is f[n] times the
 // n-th sum (with the triangles' -2 i^2 = 2 folded in), K[n] as above.
