@@ -288,6 +288,100 @@ __global__ void reduce_tiles_kernel(const float* __restrict__ partials, const Sy
   V[(int64_t)j * g.n + i] = s;
 }
 
+// Few rows (n <= SMALL_N): the 128 x 128 tile would be mostly padding (14 rows
+// on 76,928 nodes: 88 us for a read of 8.6 MB).  A warp owns a 4 x 4 block of
+// row pairs, its lanes 32 neighbouring columns read straight from global
+// memory (the rows come from L2, where the form factors were just written, and
+// L1 serves the blocks that share them): 8 loads per 32 multiply-adds, so L1
+// bounds it at ~16 cycles per step and block.  A lane sums SMALL_FOLD columns
+// into fresh FP32 registers, then into compensated sums, and the lanes are
+// added compensated; few blocks are repeated over column groups so that all
+// warps work.  partials[cta * cgs + group][i n + j].
+constexpr int SMALL_N = 64, SMALL_WARPS = 8, SMALL_FOLD = 16;
+
+__device__ __forceinline__ kbsum kb_merge(kbsum a, float hi, float lo) {
+  const df t = two_sum(a.hi, hi);
+  return {t.hi, a.lo + lo + t.lo};
+}
+
+__global__ void __launch_bounds__(32 * SMALL_WARPS)
+syrk_small_kernel(const float2* __restrict__ X, int n, int64_t Q, const float* __restrict__ sign, int tp, int cgs,
+                  float* __restrict__ partials) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t per = (Q + 32 * (int64_t)gridDim.x - 1) / (32 * (int64_t)gridDim.x) * 32;
+  const int64_t q0 = per * blockIdx.x, q1 = min(Q, q0 + per);
+  for (int unit = warp; unit < tp * cgs; unit += SMALL_WARPS) {
+    const int cg = unit / tp;
+    int bj = unit - cg * tp, bi = 0;  // block pair (bi, bj), bi <= bj, row-major over the upper triangle
+    for (int nb = (n + 3) / 4; bj >= nb - bi; ++bi) bj -= nb - bi;
+    bj += bi;
+    const float2 *a[4], *b[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      a[r] = X + (int64_t)min(4 * bi + r, n - 1) * Q;
+      b[r] = X + (int64_t)min(4 * bj + r, n - 1) * Q;
+    }
+    float acc[16], s[16], c[16];
+#pragma unroll
+    for (int v = 0; v < 16; ++v) acc[v] = s[v] = c[v] = 0.f;
+    int steps = 0;
+    auto fold = [&]() {
+#pragma unroll
+      for (int v = 0; v < 16; ++v) {
+        const float y = acc[v] - c[v], t = s[v] + y;
+        c[v] = (t - s[v]) - y;
+        s[v] = t;
+        acc[v] = 0.f;
+      }
+      steps = 0;
+    };
+    for (int64_t q = q0 + 32 * cg + lane; q < q1; q += 32 * cgs) {
+      float2 x[4], y[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) { x[r] = a[r][q]; y[r] = b[r][q]; }
+      if (sign) {
+        const float w = sign[q];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) { y[r].x *= w; y[r].y *= w; }
+      }
+#pragma unroll
+      for (int v = 0; v < 16; ++v)
+        acc[v] = fmaf(x[v >> 2].x, y[v & 3].x, fmaf(x[v >> 2].y, y[v & 3].y, acc[v]));
+      if (++steps == SMALL_FOLD) fold();
+    }
+    fold();
+    float* out = partials + ((int64_t)blockIdx.x * cgs + cg) * n * n;
+#pragma unroll
+    for (int v = 0; v < 16; ++v) {
+      kbsum t{s[v], -c[v]};
+#pragma unroll
+      for (int w = 16; w > 0; w >>= 1)
+        t = kb_merge(t, __shfl_xor_sync(0xffffffffu, t.hi, w), __shfl_xor_sync(0xffffffffu, t.lo, w));
+      const int i = 4 * bi + (v >> 2), j = 4 * bj + (v & 3);
+      if (lane == v && i <= j && j < n) out[i * n + j] = t.hi + t.lo;
+    }
+  }
+}
+
+// Fixed-order compensated sum of the partials, one warp per (i, j), i <= j.
+__global__ void reduce_small_kernel(const float* __restrict__ partials, int n, int count, double* __restrict__ V) {
+  const int t = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (t >= n * n) return;
+  const int i = t / n, j = t - i * n;
+  if (i > j) return;
+  kbsum acc{0.f, 0.f};
+#pragma unroll 8
+  for (int p = lane; p < count; p += 32) acc.add(__ldcs(partials + (int64_t)p * n * n + t));
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1)
+    acc = kb_merge(acc, __shfl_xor_sync(0xffffffffu, acc.hi, w), __shfl_xor_sync(0xffffffffu, acc.lo, w));
+  if (lane == 0) {
+    const double s = acc.value() * INV8PI3;
+    V[(int64_t)i * n + j] = s;
+    V[(int64_t)j * n + i] = s;
+  }
+}
+
 int sm_count() { return current_sm_count(); }
 
 // K ranges: a diagonal tile's 3 quadrants get 4/3 of an off-diagonal tile's
@@ -326,6 +420,20 @@ bool vector_loads_ok(const void* X, int64_t K) {
 }
 
 int launch_syrk(const float* X, const SyrkGeom& g, const float* sign, float* partials, double* V, cudaStream_t s) {
+  if (g.n <= SMALL_N) {
+    const int nb = (g.n + 3) / 4, tp = nb * (nb + 1) / 2, cgs = std::max(1, SMALL_WARPS / tp);
+    const int64_t Q = g.K / 2, blk = (int64_t)cgs * g.n * g.n;
+    // two CTAs per SM, at least one step per column group, and no more partials
+    // than the tiles' workspace holds
+    const int64_t cap = std::max<int64_t>(1, syrk_tiles(g) * TB * TB / blk);
+    const int64_t ctas = std::max<int64_t>(1, std::min({2 * (int64_t)sm_count(), (Q + 32 * cgs - 1) / (32 * cgs), cap}));
+    syrk_small_kernel<<<(unsigned)ctas, 32 * SMALL_WARPS, 0, s>>>(reinterpret_cast<const float2*>(X), g.n, Q, sign, tp,
+                                                                  cgs, partials);
+    PI_LAUNCHED("syrk_small_kernel");
+    reduce_small_kernel<<<(unsigned)((g.n * g.n + 7) / 8), 256, 0, s>>>(partials, g.n, (int)(ctas * cgs), V);
+    PI_LAUNCHED("reduce_small_kernel");
+    return PI_OK;
+  }
   const int attr = ensure_smem_limit(reinterpret_cast<const void*>(syrk_fp32_kernel), (int)SYRK_SMEM,
                                      "cudaFuncSetAttribute(syrk_fp32_kernel)");
   if (attr != PI_OK) return attr;

@@ -53,7 +53,8 @@ __device__ __forceinline__ void affine_apply(const double* d, const double* x, d
   }
 }
 
-// Anchor point of element e after the DoF transform (first vertex / centre).
+// Anchor point of element e before the DoF transform (first vertex / centre;
+// the moving vertex of a TriangleMeshDoF).
 __device__ __forceinline__ void anchor(const PrepObj& o, int64_t e, double* y) {
   if (o.geom_type == PI_GEOM_TRIANGLE) {
     const TriSrc& t = reinterpret_cast<const TriSrc*>(o.src)[e];
@@ -62,44 +63,63 @@ __device__ __forceinline__ void anchor(const PrepObj& o, int64_t e, double* y) {
       if (t.vid0 < 0 || t.vid0 >= nv) { y[0] = y[1] = y[2] = 0.0; return; }
       y[0] = o.dofs[3 * t.vid0]; y[1] = o.dofs[3 * t.vid0 + 1]; y[2] = o.dofs[3 * t.vid0 + 2];
     } else {
-      affine_apply(o.dofs, t.a, y, true);
+      y[0] = t.a[0]; y[1] = t.a[1]; y[2] = t.a[2];
     }
   } else {
     const SurfSrc& s = reinterpret_cast<const SurfSrc*>(o.src)[e];
-    affine_apply(o.dofs, s.c, y, true);
+    y[0] = s.c[0]; y[1] = s.c[1]; y[2] = s.c[2];
   }
 }
 
-// One CTA per object: fixed-order mean of the anchors (deterministic), plus
-// the object's A for the surfel k' = A^T k rule.
-__global__ void prepare_origin_kernel(const PrepObj* objs, ObjDev* out, unsigned* cl_rho, int only) {
-  const int oi = only >= 0 ? only : blockIdx.x;
+// Fixed-order mean of the anchors (deterministic), plus the object's A for the
+// surfel k' = A^T k rule.  FP64 adds run at ~2 per SM and clock, so the map is
+// applied to the mean (it is affine) and the S CTAs of a thread-block cluster
+// share an object's elements, their sums meeting in the first one (one CTA per
+// object and a transform per element: 230 us for 50,000 surfels).
+constexpr int ORIGIN_THREADS = 256, ORIGIN_SPLIT = 8;
+__global__ void __launch_bounds__(ORIGIN_THREADS)
+prepare_origin_kernel(const PrepObj* objs, ObjDev* out, unsigned* cl_rho, int only) {
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int oi = only >= 0 ? only : blockIdx.x / S;
   const PrepObj o = objs[oi];
-  __shared__ double red[3][256];
+  __shared__ double red[3][ORIGIN_THREADS / 32];
+  __shared__ double total[3];
   double s[3] = {0.0, 0.0, 0.0};
-  int64_t valid = 0;
-  for (int64_t e = threadIdx.x; e < o.n_elems; e += blockDim.x) {
+  for (int64_t e = rank * ORIGIN_THREADS + threadIdx.x; e < o.n_elems; e += S * ORIGIN_THREADS) {
     double y[3];
     anchor(o, e, y);
     s[0] += y[0]; s[1] += y[1]; s[2] += y[2];
-    ++valid;
   }
-  for (int c = 0; c < 3; ++c) red[c][threadIdx.x] = s[c];
+  for (int w = 16; w > 0; w >>= 1)
+    for (int c = 0; c < 3; ++c) s[c] += __shfl_xor_sync(0xffffffffu, s[c], w);
+  if ((threadIdx.x & 31) == 0)
+    for (int c = 0; c < 3; ++c) red[c][threadIdx.x >> 5] = s[c];
   __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w)
-      for (int c = 0; c < 3; ++c) red[c][threadIdx.x] += red[c][threadIdx.x + w];
-    __syncthreads();
+  if (threadIdx.x < 3) {
+    double t = 0.0;
+    for (int w = 0; w < ORIGIN_THREADS / 32; ++w) t += red[threadIdx.x][w];
+    total[threadIdx.x] = t;
   }
-  if (threadIdx.x == 0) {
+  if (S > 1) cluster.sync();
+  else __syncthreads();
+  if (rank == 0 && threadIdx.x == 0) {
+    double m[3] = {total[0], total[1], total[2]};
+    for (int q = 1; q < S; ++q) {
+      const double* t = cluster.map_shared_rank(total, q);
+      for (int c = 0; c < 3; ++c) m[c] += t[c];
+    }
     ObjDev d;
-    double inv = o.n_elems > 0 ? 1.0 / (double)o.n_elems : 0.0;
-    for (int c = 0; c < 3; ++c) d.origin[c] = red[c][0] * inv;
+    const double inv = o.n_elems > 0 ? 1.0 / (double)o.n_elems : 0.0;
+    for (int c = 0; c < 3; ++c) m[c] *= inv;
     if (o.dof_type == PI_DOF_AFFINE) {
       const double* A = o.dofs + 3;
       for (int i = 0; i < 9; ++i) d.A[i] = (float)A[i];
+      if (o.n_elems > 0) affine_apply(o.dofs, m, d.origin, true);
+      else d.origin[0] = d.origin[1] = d.origin[2] = 0.0;
     } else {
       for (int i = 0; i < 9; ++i) d.A[i] = (i % 4 == 0) ? 1.f : 0.f;
+      for (int c = 0; c < 3; ++c) d.origin[c] = m[c];
     }
     d.type = o.geom_type;
     d.n_elems = (int32_t)o.n_elems;
@@ -109,6 +129,7 @@ __global__ void prepare_origin_kernel(const PrepObj* objs, ObjDev* out, unsigned
     out[oi] = d;
     cl_rho[oi] = 0u;  // prepare_elems_kernel takes the maximum
   }
+  if (S > 1) cluster.sync();  // no CTA leaves while its sum is read
 }
 
 // Orders one segment of an object's elements (OrderSeg) per CTA by recursive
@@ -529,9 +550,7 @@ prepare_elems_kernel(const PrepObj* objs, const ObjDev* od, float4* tri_pool, fl
 
 constexpr int FF_THREADS = 128;
 constexpr int FF_WARPS = FF_THREADS / 32;
-#ifndef FF_CTAS
-#define FF_CTAS 4
-#endif
+constexpr int FF_CTAS = 4;  // per SM: 128 registers; at five, 96 registers spill and the kernel is 7% slower
 constexpr int FF_TILE = 256;  // elements staged per shared-memory tile (a multiple of FF_CHUNK)
 constexpr int FF_CHUNK = 32;  // elements summed in FP32 before the compensated outer sum
 static_assert(FF_TILE % FF_CHUNK == 0, "element chunks must not straddle tiles");
@@ -1094,7 +1113,11 @@ int launch_prepare(pi_batch_impl* b, int only_index, cudaStream_t s) {
   PI_CUDA(pool_alloc((void**)&d, sizeof(PrepObj) * h.size(), s));
   PI_CUDA(cudaMemcpyAsync(d, h.data(), sizeof(PrepObj) * h.size(), cudaMemcpyHostToDevice, s));
   const int nobj_launch = only_index >= 0 ? 1 : b->n_obj;
-  prepare_origin_kernel<<<nobj_launch, 256, 0, s>>>(d, b->d_objs, b->d_cl_rho, only_index);
+  const int S = max_elems > 4 * ORIGIN_THREADS ? ORIGIN_SPLIT : 1;
+  void* oargs[4] = {&d, &b->d_objs, &b->d_cl_rho, &only_index};
+  if (int rc = launch_split(reinterpret_cast<const void*>(prepare_origin_kernel), dim3((unsigned)(nobj_launch * S)),
+                            ORIGIN_THREADS, 0, S, oargs, s))
+    return rc;
   PI_LAUNCHED("prepare_origin_kernel");
   if (max_elems > 0) {
     dim3 grid((unsigned)((max_elems + PREP_THREADS - 1) / PREP_THREADS), (unsigned)nobj_launch);
@@ -1128,10 +1151,13 @@ int launch_form_factors(const pi_kgrid_impl* kg, const pi_batch_impl* b, int sca
   int64_t heavy = 0;
   for (int i = 0; i < b->n_obj; ++i) heavy += 4 * b->info[i].n_elems >= n_max;
   auto busy = [&](int r) { return (K.moments ? (ctas(r) + 4) / 5 : ctas(r)) * heavy; };
-  const int64_t full = 10 * (int64_t)current_sm_count();  // two waves of five CTAs per SM
-  if (R == 8 && 16 * busy(8) < full) R = 4;
+  const int64_t wave = FF_CTAS * (int64_t)current_sm_count();
+  // four radii per thread where 16 splits at eight give less than 7/4 waves
+  // (8 clouds of 50,000 disks: 7.1 ms at four, 8.2 at eight; a solid of 200,000
+  // triangles, just above: 36.2 and 30.0)
+  if (R == 8 && 4 * 16 * busy(8) < 7 * wave) R = 4;
   int S = 1;
-  while (S < 16 && S * busy(R) < full && n_max > 2 * S * FF_CHUNK) S *= 2;
+  while (S < 16 && S * busy(R) < 2 * wave && n_max > 2 * S * FF_CHUNK) S *= 2;
   const void* fn = R == 8   ? reinterpret_cast<const void*>(ff_kernel<8>)
                    : R == 4 ? reinterpret_cast<const void*>(ff_kernel<4>)
                             : reinterpret_cast<const void*>(ff_kernel<2>);
