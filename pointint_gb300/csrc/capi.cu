@@ -433,7 +433,8 @@ int kgrid_create_impl(const double* dirs, const double* kmag, const double* w, i
     for (int64_t j = 0; j < M && ok; ++j) ok = seen[j] == 1;
     if (!ok) return fail(PI_ERR_UNSUPPORTED, "pi_kgrid_create: bad direction pairing");
   }
-  const size_t total = align16(o_pair + Me * sizeof(int2));
+  const size_t o_eh = align16(o_pair + Me * sizeof(int2)), o_el = align16(o_eh + Me * sizeof(float4)),
+               total = align16(o_el + Me * sizeof(float4));
   std::vector<unsigned char> host(total, 0);
   std::memcpy(host.data() + o_dh, dh.data(), M * sizeof(float4));
   std::memcpy(host.data() + o_dl, dl.data(), M * sizeof(float4));
@@ -444,6 +445,10 @@ int kgrid_create_impl(const double* dirs, const double* kmag, const double* w, i
   std::memcpy(host.data() + o_k256, k256.data(), L * sizeof(float2));
   std::memcpy(host.data() + o_tab, tab.data(), tab.size() * sizeof(float2));
   std::memcpy(host.data() + o_pair, pairs.data(), Me * sizeof(int2));
+  for (int64_t e = 0; e < Me; ++e) {
+    std::memcpy(host.data() + o_eh + e * sizeof(float4), &dh[pairs[e].x], sizeof(float4));
+    std::memcpy(host.data() + o_el + e * sizeof(float4), &dl[pairs[e].x], sizeof(float4));
+  }
   kg->pooled = temporary;
   kg->pool_stream = s;
   PI_CUDA(temporary ? pool_alloc(&kg->d_mem, total, s) : cudaMalloc(&kg->d_mem, total));
@@ -467,6 +472,8 @@ int kgrid_create_impl(const double* dirs, const double* kmag, const double* w, i
   kg->dev.cis_tab = reinterpret_cast<const float2*>(base + o_tab);
   kg->dev.cis_tabm = kg->dev.cis_tab + PHASOR_ENTRIES;
   kg->dev.dpair = reinterpret_cast<const int2*>(base + o_pair);
+  kg->dev.edir_hi = reinterpret_cast<const float4*>(base + o_eh);
+  kg->dev.edir_lo = reinterpret_cast<const float4*>(base + o_el);
   kg->dev.Me = (int)Me;
   kg->Me = (int)Me;
   kg->dev.moments = moment_grid(dv, km, M, L, tensor) ? 1 : 0;

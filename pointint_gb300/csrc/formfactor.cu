@@ -999,14 +999,9 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
         const int64_t q = (int64_t)r * kg.M + j;
         cf v{acc.sre(i), acc.sim(i)};
         if (kw[i].x * PI_TURN64 * dnorm < 1e-10f) v = cf{0.f, 0.f};  // A(0) = 0 (affine_dof.cpp:64-65)
-        const float sw = kg.sqrtw[q];
-        ev.dst[(int64_t)j * kg.L + r] = make_float2(v.re * sw, v.im * sw);
+        const float sw = serve_scale(kg, q, jm >= 0 ? (int64_t)r * kg.M + jm : -1);
+        ev.dst[(int64_t)ei * kg.L + r] = make_float2(v.re * sw, v.im * sw);
         m = fmaxf(m, fmaxf(fabsf(v.re * sw), fabsf(v.im * sw)));
-        if (jm >= 0) {  // the antipode: -conj
-          const float swm = kg.sqrtw[(int64_t)r * kg.M + jm];
-          ev.dst[(int64_t)jm * kg.L + r] = make_float2(-v.re * swm, v.im * swm);
-          m = fmaxf(m, fmaxf(fabsf(v.re * swm), fabsf(v.im * swm)));
-        }
       }
     }
     atomicMax(reinterpret_cast<unsigned*>(ev.amax), __float_as_uint(m));

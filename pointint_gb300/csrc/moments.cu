@@ -358,18 +358,20 @@ __device__ __forceinline__ void moment_body(const KGridDev& kg, const BatchDev& 
     }
     if (km.x * dnorm < 1e-10f) v = cf{0.f, 0.f};  // A(0) = 0 (affine_dof.cpp:64-65)
     const int64_t q = (int64_t)r * kg.M + j, qm = (int64_t)r * kg.M + jm;
-    const bool scaled = SERVE || scale_sqrt_w;
-    const float sw = scaled ? kg.sqrtw[q] : 1.0f, swm = scaled && jm >= 0 ? kg.sqrtw[qm] : 1.0f;
-    const float2 o = make_float2(v.re * sw, v.im * sw), om = make_float2(-v.re * swm, v.im * swm);
-    m = fmaxf(m, fmaxf(fabsf(o.x), fabsf(o.y)));
-    if (jm >= 0) m = fmaxf(m, fmaxf(fabsf(om.x), fabsf(om.y)));
     if (SERVE) {
-      float2* dst = evals[slot].dst;
-      dst[(int64_t)j * kg.L + r] = o;
-      if (jm >= 0) dst[(int64_t)jm * kg.L + r] = om;  // the antipode: -conj
+      const float sw = serve_scale(kg, q, jm >= 0 ? qm : -1);
+      const float2 o = make_float2(v.re * sw, v.im * sw);
+      m = fmaxf(m, fmaxf(fabsf(o.x), fabsf(o.y)));
+      evals[slot].dst[(int64_t)ei * kg.L + r] = o;
     } else {
+      const float sw = scale_sqrt_w ? kg.sqrtw[q] : 1.0f, swm = scale_sqrt_w && jm >= 0 ? kg.sqrtw[qm] : 1.0f;
+      const float2 o = make_float2(v.re * sw, v.im * sw), om = make_float2(-v.re * swm, v.im * swm);
+      m = fmaxf(m, fmaxf(fabsf(o.x), fabsf(o.y)));
       J[(int64_t)oi * kg.Q + q] = o;
-      if (jm >= 0) J[(int64_t)oi * kg.Q + qm] = om;
+      if (jm >= 0) {  // the antipode: -conj
+        m = fmaxf(m, fmaxf(fabsf(om.x), fabsf(om.y)));
+        J[(int64_t)oi * kg.Q + qm] = om;
+      }
     }
   }
   if (S > 1) cluster.sync();  // no CTA leaves while its sums are read

@@ -34,6 +34,13 @@ __device__ __forceinline__ int covered_radii(const KGridDev& kg, float rho, floa
   return n;
 }
 
+// Scale of a serving row's column (EvalDev): the root of the weights of node q
+// and its antipode qm (-1: none).
+__device__ __forceinline__ float serve_scale(const KGridDev& kg, int64_t q, int64_t qm) {
+  const float sw = kg.sqrtw[q], swm = qm >= 0 ? kg.sqrtw[qm] : 0.f;
+  return sqrtf(fmaf(sw, sw, swm * swm));
+}
+
 __device__ __forceinline__ int moment_radii(const KGridDev& kg, int type, float rho) {
   return covered_radii(kg, rho, type == PI_GEOM_TRIANGLE ? MOMENT_X_TRI : MOMENT_X_SURF);
 }

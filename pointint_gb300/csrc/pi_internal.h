@@ -72,6 +72,8 @@ struct KGridDev {
   // a time into compact clusters of directions; otherwise (j, -1) in order.
   const int2* dpair;
   int Me;
+  const float4* edir_hi;  // dir_hi, dir_lo of the evaluated directions, in their order
+  const float4* edir_lo;
   // Whether the cluster expansions of moments.cu apply: a tensor grid of unit
   // directions whose radii ascend, so that "k rho <= bound" selects the first
   // radii (moment_radii).
@@ -134,8 +136,11 @@ struct BatchDev {
 
 // One form-factor evaluation of the serving path: library object `obj`,
 // optionally rotated (its form factors at k are the unrotated object's at
-// R^T k), written in the object-local frame (no origin phase), sqrt|w|-scaled
-// and direction-major (column j * L + r) to dst; the largest |Re|, |Im| goes
+// R^T k), written in the object-local frame (no origin phase) and
+// direction-major over the evaluated directions (column e * L + r) to dst,
+// scaled by the square root of the weight of the node and its antipode
+// together: Re(conj A_i A_j) is the same at k and -k, so half the grid's columns
+// give the whole volume; the largest |Re|, |Im| goes
 // to *amax (FP32 bits, atomicMax) for the FP16 operand scale.
 struct EvalDev {          // 104 bytes
   int32_t obj;

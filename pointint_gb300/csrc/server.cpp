@@ -96,10 +96,13 @@ struct Slot {
   float* d_part = nullptr;
   int* d_err = nullptr;
   GroupDev g{};
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  cudaGraphNode_t n_h2d = nullptr, n_ff = nullptr, n_fm = nullptr, n_d2h_out = nullptr;
-  bool ff_enabled = true;
+  // one graph for batches over resident rows alone, one for batches that also
+  // evaluate form factors
+  struct Graph {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    cudaGraphNode_t n_h2d = nullptr, n_ff = nullptr, n_fm = nullptr, n_d2h_out = nullptr;
+  } graphs[2];
   // current batch
   bool busy = false;
   uint64_t batch_id = 0;
@@ -218,52 +221,54 @@ Layout make_layout(const pi_server_config& c, int64_t max_out) {
   return L;
 }
 
-int build_graph(Server& S, Slot& sl) {
-  PI_CUDA(cudaGraphCreate(&sl.graph, 0));
+int build_graph(Server& S, Slot& sl, Slot::Graph& gr, bool evaluate) {
+  PI_CUDA(cudaGraphCreate(&gr.graph, 0));
   // descriptor upload (size set per launch)
   cudaGraphNode_t n_err = nullptr, n_con = nullptr, n_red = nullptr;
-  PI_CUDA(cudaGraphAddMemcpyNode1D(&sl.n_h2d, sl.graph, nullptr, 0, sl.d_io, sl.h_io, S.lay.rows,
+  PI_CUDA(cudaGraphAddMemcpyNode1D(&gr.n_h2d, gr.graph, nullptr, 0, sl.d_io, sl.h_io, S.lay.rows,
                                    cudaMemcpyHostToDevice));
   cudaMemsetParams ms{};
   ms.dst = sl.d_err; ms.value = 0; ms.elementSize = 4; ms.width = 1; ms.height = 1; ms.pitch = 4;
-  PI_CUDA(cudaGraphAddMemsetNode(&n_err, sl.graph, &sl.n_h2d, 1, &ms));
-  // form factors of the batch's new rows (grid set per launch)
-  KGridDev K = S.kg->dev;
-  BatchDev B = S.lib->dev();
-  float2* none = nullptr;
-  int one = 1;
-  EvalDev* evals = reinterpret_cast<EvalDev*>(sl.d_io + S.lay.evals);
-  unsigned* no_amax = nullptr;  // serving rows keep their maxima through EvalDev::amax
-  void* ff_args[6] = {&K, &B, &none, &one, &evals, &no_amax};
-  cudaKernelNodeParams kp{};
-  kp.func = const_cast<void*>(ff_serve_fn(S.kg));
-  kp.gridDim = dim3((unsigned)ff_serve_grid_x(S.kg), 1);
-  kp.blockDim = dim3((unsigned)ff_serve_threads());
-  kp.sharedMemBytes = 0;
-  kp.kernelParams = ff_args;
-  PI_CUDA(cudaGraphAddKernelNode(&sl.n_ff, sl.graph, &n_err, 1, &kp));
-  // beside it (other radii of the same rows) the cluster expansions
-  cudaGraphNode_t evaluated[2] = {sl.n_ff, nullptr};
-  if (K.moments) {
-    int rc = moment_setup();
-    if (rc) return rc;
-    kp.func = const_cast<void*>(moment_serve_fn());
-    kp.gridDim = dim3((unsigned)moment_serve_grid_x(S.kg), 1);
-    kp.blockDim = dim3((unsigned)moment_threads());
-    kp.sharedMemBytes = (unsigned)moment_smem_bytes(K.L);
-    PI_CUDA(cudaGraphAddKernelNode(&sl.n_fm, sl.graph, &n_err, 1, &kp));
-    evaluated[1] = sl.n_fm;
+  PI_CUDA(cudaGraphAddMemsetNode(&n_err, gr.graph, &gr.n_h2d, 1, &ms));
+  cudaGraphNode_t rows_ready = n_err;
+  if (evaluate) {
+    // form factors of the batch's new rows (grid set per launch)
+    KGridDev K = S.kg->dev;
+    BatchDev B = S.lib->dev();
+    float2* none = nullptr;
+    int one = 1;
+    EvalDev* evals = reinterpret_cast<EvalDev*>(sl.d_io + S.lay.evals);
+    unsigned* no_amax = nullptr;  // serving rows keep their maxima through EvalDev::amax
+    void* ff_args[6] = {&K, &B, &none, &one, &evals, &no_amax};
+    cudaKernelNodeParams kp{};
+    kp.func = const_cast<void*>(ff_serve_fn(S.kg));
+    kp.gridDim = dim3((unsigned)ff_serve_grid_x(S.kg), 1);
+    kp.blockDim = dim3((unsigned)ff_serve_threads());
+    kp.sharedMemBytes = 0;
+    kp.kernelParams = ff_args;
+    PI_CUDA(cudaGraphAddKernelNode(&gr.n_ff, gr.graph, &n_err, 1, &kp));
+    // beside it (other radii of the same rows) the cluster expansions
+    cudaGraphNode_t evaluated[2] = {gr.n_ff, nullptr};
+    if (K.moments) {
+      int rc = moment_setup();
+      if (rc) return rc;
+      kp.func = const_cast<void*>(moment_serve_fn());
+      kp.gridDim = dim3((unsigned)moment_serve_grid_x(S.kg), 1);
+      kp.blockDim = dim3((unsigned)moment_threads());
+      kp.sharedMemBytes = (unsigned)moment_smem_bytes(K.L);
+      PI_CUDA(cudaGraphAddKernelNode(&gr.n_fm, gr.graph, &n_err, 1, &kp));
+      evaluated[1] = gr.n_fm;
+    }
+    // row maxima of the new rows into the pool
+    const int32_t* n_evals = &reinterpret_cast<const GHeader*>(sl.d_io + S.lay.hdr)->n_evals;
+    void* cm_args[2] = {&evals, const_cast<int32_t**>(&n_evals)};
+    cudaKernelNodeParams cmp{};
+    cmp.func = const_cast<void*>(amax_commit_fn());
+    cmp.gridDim = dim3(1);
+    cmp.blockDim = dim3((unsigned)amax_commit_threads());
+    cmp.kernelParams = cm_args;
+    PI_CUDA(cudaGraphAddKernelNode(&rows_ready, gr.graph, evaluated, K.moments ? 2 : 1, &cmp));
   }
-  // row maxima of the new rows into the pool
-  const int32_t* n_evals = &reinterpret_cast<const GHeader*>(sl.d_io + S.lay.hdr)->n_evals;
-  void* cm_args[2] = {&evals, const_cast<int32_t**>(&n_evals)};
-  cudaKernelNodeParams cmp{};
-  cmp.func = const_cast<void*>(amax_commit_fn());
-  cmp.gridDim = dim3(1);
-  cmp.blockDim = dim3((unsigned)amax_commit_threads());
-  cmp.kernelParams = cm_args;
-  cudaGraphNode_t n_commit = nullptr;
-  PI_CUDA(cudaGraphAddKernelNode(&n_commit, sl.graph, evaluated, K.moments ? 2 : 1, &cmp));
   // contraction
   void* con_args[2] = {&sl.g, &S.pool_map};
   cudaKernelNodeParams cpar{};
@@ -272,7 +277,7 @@ int build_graph(Server& S, Slot& sl) {
   cpar.blockDim = dim3((unsigned)group_threads());
   cpar.sharedMemBytes = (unsigned)group_smem_bytes();
   cpar.kernelParams = con_args;
-  PI_CUDA(cudaGraphAddKernelNode(&n_con, sl.graph, &n_commit, 1, &cpar));
+  PI_CUDA(cudaGraphAddKernelNode(&n_con, gr.graph, &rows_ready, 1, &cpar));
   // reduction
   void* red_args[1] = {&sl.g};
   cudaKernelNodeParams rp{};
@@ -280,11 +285,11 @@ int build_graph(Server& S, Slot& sl) {
   rp.gridDim = dim3((unsigned)(4 * S.sms));
   rp.blockDim = dim3((unsigned)group_reduce_threads());
   rp.kernelParams = red_args;
-  PI_CUDA(cudaGraphAddKernelNode(&n_red, sl.graph, &n_con, 1, &rp));
+  PI_CUDA(cudaGraphAddKernelNode(&n_red, gr.graph, &n_con, 1, &rp));
   // error flag + results download (size set per launch)
-  PI_CUDA(cudaGraphAddMemcpyNode1D(&sl.n_d2h_out, sl.graph, &n_red, 1, sl.h_io + S.lay.err, sl.d_io + S.lay.err,
+  PI_CUDA(cudaGraphAddMemcpyNode1D(&gr.n_d2h_out, gr.graph, &n_red, 1, sl.h_io + S.lay.err, sl.d_io + S.lay.err,
                                    256 + sizeof(double), cudaMemcpyDeviceToHost));
-  PI_CUDA(cudaGraphInstantiate(&sl.exec, sl.graph, 0));
+  PI_CUDA(cudaGraphInstantiate(&gr.exec, gr.graph, 0));
   return PI_OK;
 }
 
@@ -309,17 +314,18 @@ int init_slot(Server& S, Slot& sl, int index) {
   g.phase = 1;
   g.tile_tma = 1;
   g.L = S.kg->L;
-  g.M = S.kg->M;
-  g.dir_hi = S.kg->dev.dir_hi;
-  g.dir_lo = S.kg->dev.dir_lo;
+  g.M = S.kg->Me;
+  g.dir_hi = S.kg->dev.edir_hi;
+  g.dir_lo = S.kg->dev.edir_lo;
   g.kturn = S.kg->dev.kturn;
   g.partials = sl.d_part;
   g.max_items = S.max_items;
   g.err = sl.d_err;
   g.out = reinterpret_cast<double*>(sl.d_io + S.lay.out);
   g.scale = INV_8PI3;
-  if (S.cfg.use_graphs) return build_graph(S, sl);
-  return PI_OK;
+  if (!S.cfg.use_graphs) return PI_OK;
+  const int rc = build_graph(S, sl, sl.graphs[0], false);
+  return rc ? rc : build_graph(S, sl, sl.graphs[1], true);
 }
 
 // ---------------------------------------------------------------------------
@@ -541,8 +547,9 @@ int launch_batch(Server& S, Slot& sl, const std::vector<cudaEvent_t>& waits) {
   const size_t h2d = S.lay.rows + (size_t)sl.n_rows * sizeof(GRow);
   const size_t out_bytes = 256 + (size_t)std::max<int64_t>(1, sl.n_out) * sizeof(double);  // flag + results
   if (S.cfg.use_graphs) {
-    PI_CUDA(cudaGraphExecMemcpyNodeSetParams1D(sl.exec, sl.n_h2d, sl.d_io, sl.h_io, h2d, cudaMemcpyHostToDevice));
     const bool ff = sl.n_evals > 0;
+    Slot::Graph& gr = sl.graphs[ff ? 1 : 0];
+    PI_CUDA(cudaGraphExecMemcpyNodeSetParams1D(gr.exec, gr.n_h2d, sl.d_io, sl.h_io, h2d, cudaMemcpyHostToDevice));
     if (ff) {
       KGridDev K = S.kg->dev;
       BatchDev B = S.lib->dev();
@@ -556,23 +563,18 @@ int launch_batch(Server& S, Slot& sl, const std::vector<cudaEvent_t>& waits) {
       kp.gridDim = dim3((unsigned)ff_serve_grid_x(S.kg), (unsigned)sl.n_evals);
       kp.blockDim = dim3((unsigned)ff_serve_threads());
       kp.kernelParams = ff_args;
-      PI_CUDA(cudaGraphExecKernelNodeSetParams(sl.exec, sl.n_ff, &kp));
+      PI_CUDA(cudaGraphExecKernelNodeSetParams(gr.exec, gr.n_ff, &kp));
       if (K.moments) {
         kp.func = const_cast<void*>(moment_serve_fn());
         kp.gridDim = dim3((unsigned)moment_serve_grid_x(S.kg), (unsigned)sl.n_evals);
         kp.blockDim = dim3((unsigned)moment_threads());
         kp.sharedMemBytes = (unsigned)moment_smem_bytes(K.L);
-        PI_CUDA(cudaGraphExecKernelNodeSetParams(sl.exec, sl.n_fm, &kp));
+        PI_CUDA(cudaGraphExecKernelNodeSetParams(gr.exec, gr.n_fm, &kp));
       }
     }
-    if (ff != sl.ff_enabled) {
-      PI_CUDA(cudaGraphNodeSetEnabled(sl.exec, sl.n_ff, ff ? 1u : 0u));
-      if (sl.n_fm) PI_CUDA(cudaGraphNodeSetEnabled(sl.exec, sl.n_fm, ff ? 1u : 0u));
-      sl.ff_enabled = ff;
-    }
-    PI_CUDA(cudaGraphExecMemcpyNodeSetParams1D(sl.exec, sl.n_d2h_out, sl.h_io + S.lay.err, sl.d_io + S.lay.err,
+    PI_CUDA(cudaGraphExecMemcpyNodeSetParams1D(gr.exec, gr.n_d2h_out, sl.h_io + S.lay.err, sl.d_io + S.lay.err,
                                                out_bytes, cudaMemcpyDeviceToHost));
-    PI_CUDA(cudaGraphLaunch(sl.exec, sl.stream));
+    PI_CUDA(cudaGraphLaunch(gr.exec, sl.stream));
     ++S.st.graph_launches;
   } else {
     PI_CUDA(cudaMemcpyAsync(sl.d_io, sl.h_io, h2d, cudaMemcpyHostToDevice, sl.stream));
@@ -718,7 +720,7 @@ int autotune(Server& S) {
   // synthetic rows (the pool is zeroed again afterwards)
   std::vector<float2> h((size_t)(S.Qpad));
   for (int64_t r = 0; r < rows; ++r) {
-    fill_rows_host(h, S.kg->Q, 1234567 + r);  // padding columns stay zero
+    fill_rows_host(h, (int64_t)S.kg->Me * S.kg->L, 1234567 + r);  // padding columns stay zero
     PI_CUDA(cudaMemcpy(S.d_pool + r * S.Qpad, h.data(), (size_t)S.Qpad * sizeof(float2), cudaMemcpyHostToDevice));
   }
   Slot& sl = S.slots[0];
@@ -788,8 +790,10 @@ void destroy_server(Server* S) {
   if (!S) return;
   for (int i = 0; i < MAX_SLOTS; ++i) {
     Slot& sl = S->slots[i];
-    if (sl.exec) cudaGraphExecDestroy(sl.exec);
-    if (sl.graph) cudaGraphDestroy(sl.graph);
+    for (Slot::Graph& gr : sl.graphs) {
+      if (gr.exec) cudaGraphExecDestroy(gr.exec);
+      if (gr.graph) cudaGraphDestroy(gr.graph);
+    }
     if (sl.stream) cudaStreamSynchronize(sl.stream);
     if (sl.done) cudaEventDestroy(sl.done);
     if (sl.stream) cudaStreamDestroy(sl.stream);
@@ -842,7 +846,7 @@ int pi_server_create(pi_kgrid kg, const pi_object* library, int n_library, const
   S->n_lib = n_library;
   PI_CUDA(cudaGetDevice(&S->device));
   PI_CUDA(cudaDeviceGetAttribute(&S->sms, cudaDevAttrMultiProcessorCount, S->device));
-  S->Qpad = (kg->Q + GROUP_CHUNK - 1) / GROUP_CHUNK * GROUP_CHUNK;
+  S->Qpad = ((int64_t)kg->Me * kg->L + GROUP_CHUNK - 1) / GROUP_CHUNK * GROUP_CHUNK;
   S->nch = S->Qpad / GROUP_CHUNK;
   // library: uploaded and prepared once
   int rc = pi_batch_create(library, n_library, 0, nullptr, &S->lib);
@@ -875,13 +879,15 @@ int pi_server_create(pi_kgrid kg, const pi_object* library, int n_library, const
   size_t free_b = 0, total_b = 0;
   PI_CUDA(cudaMemGetInfo(&free_b, &total_b));
   const int64_t budget = c.hbm_budget_bytes > 0 ? c.hbm_budget_bytes : (int64_t)(free_b / 4);
-  const int64_t row_bytes = S->Qpad * (int64_t)sizeof(float2);
+  // the number of rows is what the budget holds of whole-grid rows
+  const int64_t row_bytes = (kg->Q + GROUP_CHUNK - 1) / GROUP_CHUNK * GROUP_CHUNK * (int64_t)sizeof(float2);
   const int64_t pool_bytes = budget - (int64_t)slot_bytes * S->nslots;
   if (pool_bytes < row_bytes * 2)
     return fail(PI_ERR_OUT_OF_MEMORY, "pi_server_create: HBM budget leaves no room for resident rows");
   S->pool_rows = std::min<int64_t>(pool_bytes / row_bytes, 0x7fffffff);
-  PI_CUDA(cudaMalloc(reinterpret_cast<void**>(&S->d_pool), (size_t)(S->pool_rows * row_bytes)));
-  PI_CUDA(cudaMemset(S->d_pool, 0, (size_t)(S->pool_rows * row_bytes)));
+  const size_t pool_used = (size_t)S->pool_rows * (size_t)S->Qpad * sizeof(float2);
+  PI_CUDA(cudaMalloc(reinterpret_cast<void**>(&S->d_pool), pool_used));
+  PI_CUDA(cudaMemset(S->d_pool, 0, pool_used));
   S->row_obj.assign(S->pool_rows, -1);
   S->row_pin.assign(S->pool_rows, 0);
   rc = encode_row_map(&S->pool_map, S->d_pool, 2 * S->Qpad, S->pool_rows);
