@@ -83,6 +83,18 @@ cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s) {
   return cudaMallocFromPoolAsync(p, bytes, pool, s);
 }
 
+int allow_wide_clusters(const void* fn) {
+  static std::mutex mu;
+  static std::set<std::pair<const void*, int>> done;  // (function, device)
+  int dev = 0;
+  PI_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(mu);
+  if (done.count({fn, dev})) return PI_OK;
+  PI_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  done.insert({fn, dev});
+  return PI_OK;
+}
+
 int launch_split(const void* fn, dim3 grid, int threads, size_t smem, int split, void** args, cudaStream_t s) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
@@ -92,15 +104,8 @@ int launch_split(const void* fn, dim3 grid, int threads, size_t smem, int split,
   cudaLaunchAttribute at{};
   if (split > 1) {
     if (split > 8) {
-      static std::mutex mu;
-      static std::set<std::pair<const void*, int>> done;  // (function, device)
-      int dev = 0;
-      PI_CUDA(cudaGetDevice(&dev));
-      std::lock_guard<std::mutex> lock(mu);
-      if (!done.count({fn, dev})) {
-        PI_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        done.insert({fn, dev});
-      }
+      const int rc = allow_wide_clusters(fn);
+      if (rc) return rc;
     }
     at.id = cudaLaunchAttributeClusterDimension;
     at.val.clusterDim.x = (unsigned)split;

@@ -391,7 +391,7 @@ moment_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w,
 }
 
 // The split of a serving evaluation does not depend on its batch.
-constexpr int FM_SERVE_SPLIT = 2;
+constexpr int FM_SERVE_SPLIT = 8;
 
 __global__ void __cluster_dims__(FM_SERVE_SPLIT, 1, 1) __launch_bounds__(FM_THREADS, 2)
 moment_serve_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w,

@@ -30,6 +30,8 @@ int ensure_smem_limit(const void* fn, int bytes, const char* what);
 // synchronisation.  Safe with any number of threads and streams.
 constexpr uint64_t POOL_KEEP = uint64_t(64) << 20;
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s);
+// Allows fn thread-block clusters of more than 8 CTAs, once per (function, device).
+int allow_wide_clusters(const void* fn);
 // Launches fn with thread-block clusters of `split` CTAs along x (1: none;
 // above 8 the function's non-portable cluster size is allowed first).
 int launch_split(const void* fn, dim3 grid, int threads, size_t smem, int split, void** args, cudaStream_t s);
@@ -247,6 +249,7 @@ int launch_jacobian(const pi_kgrid_impl* kg, const pi_batch_impl* b, float2* G, 
 int ff_serve_grid_x(const pi_kgrid_impl* kg);
 int ff_serve_threads();
 const void* ff_serve_fn(const pi_kgrid_impl* kg);
+int ff_serve_setup(const pi_kgrid_impl* kg);  // before ff_serve_fn is launched or put into a graph
 int launch_form_factors_serve(const pi_kgrid_impl* kg, const pi_batch_impl* lib, const EvalDev* evals, int n_evals,
                               cudaStream_t s);
 // After the serving evaluations: *amax_keep = *amax for the first *n_evals evals

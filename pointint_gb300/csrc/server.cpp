@@ -240,6 +240,7 @@ int build_graph(Server& S, Slot& sl, Slot::Graph& gr, bool evaluate) {
     EvalDev* evals = reinterpret_cast<EvalDev*>(sl.d_io + S.lay.evals);
     unsigned* no_amax = nullptr;  // serving rows keep their maxima through EvalDev::amax
     void* ff_args[6] = {&K, &B, &none, &one, &evals, &no_amax};
+    if (int rc = ff_serve_setup(S.kg)) return rc;
     cudaKernelNodeParams kp{};
     kp.func = const_cast<void*>(ff_serve_fn(S.kg));
     kp.gridDim = dim3((unsigned)ff_serve_grid_x(S.kg), 1);
