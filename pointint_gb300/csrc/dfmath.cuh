@@ -248,14 +248,27 @@ __device__ __forceinline__ cf cis_tab_df(const float2* tab, float2 kt, df sm) {
 //   e^{i(a+b)} - 1 = ta + cm + i sn + ta (cm + i sn),  ta = e^{ia} - 1,
 // b = c f.  (Entry 0 is zero, so short phases come from cm and sn alone.)
 constexpr int PHASOR_M1_COPIES = 8;
-__device__ __forceinline__ cf cis_tab_m1(const float2* tabm, float kt, float d) {
-  const float t = fmaf(kt, d, PI_ROUND_SHIFT);
-  const float f = fmaf(kt, d, PI_ROUND_SHIFT - t);
+template <int C>
+__device__ __forceinline__ cf cis_tab_m1_frac(const float2* tabm, int idx, float f) {
   const float f2 = f * f;
   const float cm = f2 * fmaf(f2, PI_TURN64_C4, -PI_TURN64_C2);
   const float sn = f * fmaf(f2, -PI_TURN64_C3, PI_TURN64);
-  const float2 a = tabm[(__float_as_int(t) & (PHASOR_ENTRIES - 1)) * PHASOR_M1_COPIES];
+  const float2 a = tabm[(idx & (PHASOR_ENTRIES - 1)) * C];
   return {a.x + fmaf(a.x, cm, fmaf(-a.y, sn, cm)), a.y + fmaf(a.y, cm, fmaf(a.x, sn, sn))};
+}
+
+template <int C = PHASOR_M1_COPIES>
+__device__ __forceinline__ cf cis_tab_m1(const float2* tabm, float kt, float d) {
+  const float t = fmaf(kt, d, PI_ROUND_SHIFT);
+  return cis_tab_m1_frac<C>(tabm, __float_as_int(t), fmaf(kt, d, PI_ROUND_SHIFT - t));
+}
+
+// The same for a double-float radius and dot product.
+template <int C = PHASOR_M1_COPIES>
+__device__ __forceinline__ cf cis_tab_m1_df(const float2* tabm, float2 kt, df d) {
+  const float t = fmaf(kt.x, d.hi, PI_ROUND_SHIFT);
+  const float f = fmaf(kt.y, d.hi, fmaf(kt.x, d.lo, fmaf(kt.x, d.hi, PI_ROUND_SHIFT - t)));
+  return cis_tab_m1_frac<C>(tabm, __float_as_int(t), f);
 }
 
 // Two phasors at once with packed FP32 (sm_100 family): radii a, b in the

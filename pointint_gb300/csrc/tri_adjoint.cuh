@@ -201,4 +201,65 @@ static __device__ __noinline__ TriDer tri_generic_der_at(const float2* tab, floa
   return tri_generic_der(cis_tab_df<C>(tab, kt, sa), cis_tab_df<C>(tab, kt, sb), cis_tab_df<C>(tab, kt, sc), al, be);
 }
 
+// Large spread with the vertices sorted along the direction, u <= v <= w (as
+// TriGaps of the form factors, here with double-float gaps), the parts that do
+// not depend on the radius formed once per element and direction.  With
+// g1 = k G1 (w - v), g2 = k G2 (v - u), d = g1 + g2, M = e^{ig} - 1 and
+//   W(g) = f[0, g, g] = (i (1 + M) - M / g) / g,
+// all relative to e^{iv}:
+//   F   = (M1 / g1 + conj(M2) / g2) / d,
+//   D_w = (W(g1) - F) / d,  D_u = (F - conj(W(g2))) / d,  D_v = i F - D_u - D_w.
+// Three phasors and ~110 operations, where the form above takes its roles and
+// reciprocals at every radius (~220).
+struct TriSorted {
+  df sv, G1, G2;
+  float i1, i2, iD;  // 1 / G1, 1 / G2, 1 / D
+  int u, w;          // which vertex (0, 1, 2 = a, b, c) is u, w
+};
+
+__device__ __forceinline__ TriSorted tri_sorted(df sa, df d1, df d2) {
+  // phases relative to a: 0, d1, d2
+  const bool ab = d1.hi >= 0.f, ac = d2.hi >= 0.f, bc = d2.hi >= d1.hi;
+  TriSorted t;
+  t.u = ab ? (ac ? 0 : 2) : (bc ? 1 : 2);
+  t.w = ab ? (bc ? 2 : 1) : (ac ? 2 : 0);
+  if (t.u == t.w) t.w = t.u == 0 ? 1 : 0;  // only where comparisons with NaN disagree
+  const int v = 3 - t.u - t.w;
+  auto at = [&](int i) { return i == 0 ? df{0.f, 0.f} : (i == 1 ? d1 : d2); };
+  const df pu = at(t.u), pv = at(v), pw = at(t.w);
+  t.G1 = df_add(pw, pv * -1.0f);
+  t.G2 = df_add(pv, pu * -1.0f);
+  t.G1.hi = fmaxf(t.G1.hi, 1e-20f);  // M / g keeps its limit i at a closed gap
+  t.G2.hi = fmaxf(t.G2.hi, 1e-20f);
+  t.i1 = rcp_fast(t.G1.hi);
+  t.i2 = rcp_fast(t.G2.hi);
+  t.iD = rcp_fast(t.G1.hi + t.G2.hi);
+  t.sv = df_add(sa, pv);
+  return t;
+}
+
+// W(g) given M = e^{ig} - 1 and r = 1/g: the quotient from g = 1/2 on, below it
+// the series sum_m i^{m+2} (m+1) g^m / (m+2)! to m = 7 (truncation 1e-8).
+__device__ __forceinline__ cf tri_w(cf M, float g, float r) {
+  const float g2 = g * g;
+  const float re = fmaf(g2, fmaf(g2, fmaf(g2, 1.0f / 5760.0f, -1.0f / 144.0f), 1.0f / 8.0f), -0.5f);
+  const float im = g * fmaf(g2, fmaf(g2, fmaf(g2, 1.0f / 45360.0f, -1.0f / 840.0f), 1.0f / 30.0f), -1.0f / 3.0f);
+  const bool big = g >= 0.5f;
+  return {big ? -fmaf(M.re, r, M.im) * r : re, big ? fmaf(-M.im, r, M.re + 1.0f) * r : im};
+}
+
+struct TriWideDer { cf F, Du, Dw; };  // relative to e^{iv}
+
+template <int C>
+__device__ __forceinline__ TriWideDer tri_wide_der(const float2* tabm, float2 kt, float k, const TriSorted& t) {
+  const cf M1 = cis_tab_m1_df<C>(tabm, kt, t.G1), M2 = cis_tab_m1_df<C>(tabm, kt, t.G2);
+  const float ik = rcp_fast(k), r1 = t.i1 * ik, r2 = t.i2 * ik, id = t.iD * ik;
+  TriWideDer o;
+  o.F = cf{fmaf(M1.re, r1, M2.re * r2) * id, fmaf(M1.im, r1, -M2.im * r2) * id};
+  const cf W1 = tri_w(M1, k * t.G1.hi, r1), W2 = tri_w(M2, k * t.G2.hi, r2);
+  o.Dw = cf{(W1.re - o.F.re) * id, (W1.im - o.F.im) * id};
+  o.Du = cf{(o.F.re - W2.re) * id, (o.F.im + W2.im) * id};
+  return o;
+}
+
 }  // namespace pi
