@@ -716,11 +716,12 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
   const int ei = dt * 32 + lane;
   const bool busy = item < ndt * nrb, active = busy && ei < kg.Me;
   int j = 0, jm = -1;
-  if (active) { const int2 pr = kg.dpair[ei]; j = pr.x; jm = pr.y; }
+  // (lanes past the last direction repeat it, for the votes, and write nothing)
+  if (busy) { const int2 pr = kg.dpair[min(ei, kg.Me - 1)]; j = pr.x; jm = pr.y; }
 
   float3 dh = make_float3(0.f, 0.f, 0.f), dl = dh;
   float inv_norm = 0.f, dnorm = 0.f;
-  if (active) {
+  if (busy) {
     float4 h = kg.dir_hi[j], l = kg.dir_lo[j];
     dh = make_float3(h.x, h.y, h.z); dl = make_float3(l.x, l.y, l.z);
     inv_norm = h.w; dnorm = l.w;
@@ -779,9 +780,17 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
   const float4* kp = kpair[warp];
   // (k rho)^2 up to which a leaf's expansion is used (never without kg.moments)
   const float bound2 = kg.moments ? MOMENT_X_TRI * MOMENT_X_TRI : -1.f;
-  float kmax2 = 0.f;  // the warp's largest k^2
+  // the warp's largest k^2, and its smallest over all its radii and over the upper half
+  // of the block (a grid without kg.moments may hold its radii in any order)
+  constexpr int H = R / 2;
+  float kmax2 = 0.f, kmin2 = INFINITY, khalf2 = INFINITY;
 #pragma unroll
-  for (int i = 0; i < R; ++i) kmax2 = fmaxf(kmax2, kw[i].z);
+  for (int i = 0; i < R; ++i) {
+    const float k2 = kw[i].z;
+    kmax2 = fmaxf(kmax2, k2);
+    if (i >= skip) kmin2 = fminf(kmin2, k2);
+    if (i >= H) khalf2 = fminf(khalf2, k2);
+  }
   __shared__ float run_sm[4 * R * FF_THREADS];
   Acc<R> acc;
   acc.init(run_sm);
@@ -859,30 +868,53 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
             continue;
           }
           const TriGaps tg = tri_gaps(s1, s2, sm);
-          const float ithr2 = 1.0f / 9.0f * tg.D * tg.D;  // the series for (k D)^2 < 9
           const float gD = g * rcp_fast(tg.D);
+          // the warp's least and greatest spread (positive floats order as their bits):
+          // two reductions per element in place of two votes per radius
+          const unsigned Db = __float_as_uint(tg.D);
+          const float d_lo = __uint_as_float(__reduce_min_sync(0xffffffffu, Db)),
+                      d_hi = __uint_as_float(__reduce_max_sync(0xffffffffu, Db));
+          const float wide_lo = d_lo * d_lo, wide_hi = 1.0f / 9.0f * d_hi * d_hi;
           // no series where every lane is wide at every radius left
           TriPoly2 tp;
-          if (__any_sync(0xffffffffu, kw[from].z * ithr2 < 1.0f)) tp = tri_series_coeffs2(s1, s2, g);
+          if ((kg.moments ? kw[from].z : kmin2) * (1.0f / 9.0f) * wide_lo < 1.0f) tp = tri_series_coeffs2(s1, s2, g);
+          int to = R;  // radii [from, to) one by one, each with its own choice
+          {
+            // the upper half of the block, where all of it is wide for every lane
+            // (about every element of the block of the largest radii): R/2 radii
+            // without a branch, so that their chains overlap. 256 solids 15.37 ->
+            // 14.39 ms; two radii per packed instruction here took longer (14.83)
+            if (from <= H && khalf2 * wide_lo >= 1.0f && khalf2 * wide_hi >= 1.0f) {
+              to = H;
+#pragma unroll
+              for (int i = H; i < R; ++i) {
+                const float4 kr = ld_shared_f4(kw + i);
+                const cf P = cis_tab_df(ctab, make_float2(kr.x, kr.y), tg.sv);
+                const cf T = tri_wide(ctabm, kr.x, tg, gD * rcp_fast(kr.z));
+                acc.re(i) = fmaf(P.re, T.re, fmaf(-P.im, T.im, acc.re(i)));
+                acc.im(i) = fmaf(P.re, T.im, fmaf(P.im, T.re, acc.im(i)));
+              }
+              if (from == to) continue;
+            }
+          }
           // one radius per scalar instruction: packed pairs were tried and took
           // more instructions (their constants and dot products need both halves
           // of a register pair, moved there for every pair between the branches)
 #pragma unroll
           for (int i = 0; i < R; ++i) {
-            if (i < from) continue;
+            if (i < from || i >= to) continue;
             const float4 kr = ld_shared_f4(kw + i);
             const float2 kt = make_float2(kr.x, kr.y);
-            const float kd2 = kr.z * ithr2;
             cf P, T;  // the phase's phasor, and the rest with gamma folded in
-            if (__all_sync(0xffffffffu, kd2 < 1.0f)) {
+            if (kr.z * wide_hi < 1.0f) {
               P = cis_tab_df(ctab, kt, sm);
               T = tri_series_eval(tp, kr.z, kr.w);  // centroid Taylor series
             } else {
               P = cis_tab_df(ctab, kt, tg.sv);
               T = tri_wide(ctabm, kr.x, tg, gD * rcp_fast(kr.z));
               // lanes of small spread, whose divided differences cancel
-              const bool narrow = kd2 < 1.0f / 9.0f;
-              if (__any_sync(0xffffffffu, narrow)) {
+              if (kr.z * wide_lo < 1.0f) {
+                const bool narrow = kr.z * tg.D * tg.D < 1.0f;
                 const cf Q = cis_tab_df(ctab, kt, sm), U = tri_series_eval(tp, kr.z, kr.w);
                 P = cf{narrow ? Q.re : P.re, narrow ? Q.im : P.im};
                 T = cf{narrow ? U.re : T.re, narrow ? U.im : T.im};
