@@ -448,27 +448,46 @@ adj_surf_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const
       if (nr < kg.L) {
         const df sc = cdot2(dh, dl, c, cl3);
         const float rr = p0 * sqrt_fast(perp);
-#pragma unroll 2
-        for (int r = nr; r < kg.L; ++r) {
+        // with z = conj(B) P, S = C f(k) and (dS/dr)/r = -C p0^2 g(k) (disk: C = 2 p1,
+        // J1(x)/x and J2(x)/x^2; Gaussian: C = p1, f = g), sums of k Im(z) f, Re(z) f, k^2 Re(z) g
+        float a0 = 0.f, a1 = 0.f, a2 = 0.f;
+        const auto add = [&](int r, float k, float f, float gr) {
           const float2 Bv = Bj[r];
-          const float k = st.km[r].x;
           const cf P = cis_tab_df<ADJ_COPIES>(st.ctab, st.kt[r], sc);
-          const float ure = Bv.x * P.re + Bv.y * P.im;  // Re(conj(B) P)
-          const float uim = Bv.x * P.im - Bv.y * P.re;  // Im(conj(B) P)
-          const float k2 = k * k;
-          float S, Sr;
-          if (disk) {
-            const float x = k * rr;
-            S = p1 * ((x < 1e-10f) ? 1.0f : 2.0f * j1x(x));
-            Sr = -2.0f * p1 * p0 * p0 * j2x2(x);
-          } else {
-            S = p1 * __expf(-0.5f * p0 * p0 * k2 * perp);
-            Sr = -p0 * p0 * S;
+          const float ure = Bv.x * P.re + Bv.y * P.im, uim = Bv.x * P.im - Bv.y * P.re;
+          a0 = fmaf(k * uim, f, a0);
+          a1 = fmaf(ure, f, a1);
+          a2 = fmaf(k * k * ure, gr, a2);
+        };
+        if (disk) {
+          int r = nr;
+          // the radii up to the first with x >= 1, without a branch between them; then
+          // any (eight clouds of 50,000: 10.5 -> 8.7 ms with these sums)
+#pragma unroll 2
+          for (; r < kg.L; ++r) {
+            const float k = st.km[r].x, x = k * rr;
+            if (!(x < 1.0f)) break;
+            const J12 j = j12_series(0.25f * x * x);
+            add(r, k, j.j1, j.j2);
           }
-          s_c = fmaf(-k * uim, S * amp, s_c);
-          s_n = fmaf(ure, fmaf(-k2 * sn * sn, Sr, S), s_n);
-          s_m = fmaf(k2 * ure, 0.5f * amp * Sr, s_m);
+#pragma unroll 1
+          for (; r < kg.L; ++r) {
+            const float k = st.km[r].x;
+            const J12 j = j12(k * rr);
+            add(r, k, j.j1, j.j2);
+          }
+        } else {
+          const float hs = -0.5f * p0 * p0 * perp;
+#pragma unroll 2
+          for (int r = nr; r < kg.L; ++r) {
+            const float k = st.km[r].x, f = __expf(hs * k * k);
+            add(r, k, f, f);
+          }
         }
+        const float C = disk ? 2.0f * p1 : p1, Cp = C * p0 * p0;
+        s_c = fmaf(-C * amp, a0, s_c);
+        s_n += fmaf(sn * sn * Cp, a2, C * a1);
+        s_m = fmaf(-0.5f * amp * Cp, a2, s_m);
       }
       part[0] = fmaf(dh.x, s_c, part[0]); part[1] = fmaf(dh.y, s_c, part[1]); part[2] = fmaf(dh.z, s_c, part[2]);
       const float sn2 = s_n * inv_norm;

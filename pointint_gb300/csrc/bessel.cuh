@@ -91,4 +91,48 @@ __device__ __forceinline__ float j2x2(float x) {
   return hankel_scaled(x, P, Q, 3.9269907474517822f, 6.953546006e-08f) * rsqrtf(x) * ix * ix;
 }
 
+// j1x of two arguments, one test where both lie below 1.
+__device__ __forceinline__ float2 j1x_pair(float xa, float xb) {
+  if (fmaxf(xa, xb) < 1.0f) {
+    const float y[2] = {0.25f * xa * xa, 0.25f * xb * xb};
+    float v[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      v[h] = fmaf(y[h], fmaf(y[h], fmaf(y[h], fmaf(y[h], fmaf(y[h], -1.0f / 172800.0f, 1.0f / 5760.0f), -1.0f / 288.0f),
+                                        1.0f / 24.0f), -0.25f), 0.5f);
+    return make_float2(v[0], v[1]);
+  }
+  return make_float2(j1x(xa), j1x(xb));
+}
+
+// Both ratios at once, for the disks' gradients: one test per range, and from
+// x = 8 on one phasor for the two (chi_2 = chi_1 - pi/2).
+struct J12 { float j1, j2; };
+
+// The power series of x < 1, y = x^2 / 4.
+__device__ __forceinline__ J12 j12_series(float y) {
+  return {fmaf(y, fmaf(y, fmaf(y, fmaf(y, fmaf(y, -1.0f / 172800.0f, 1.0f / 5760.0f), -1.0f / 288.0f), 1.0f / 24.0f),
+                       -0.25f), 0.5f),
+          fmaf(y, fmaf(y, fmaf(y, fmaf(y, fmaf(y, -1.0f / 2419200.0f, 1.0f / 69120.0f), -1.0f / 2880.0f),
+                               1.0f / 192.0f), -1.0f / 24.0f), 0.125f)};
+}
+
+__device__ __forceinline__ J12 j12(float x) {
+  if (x < 1.0f) return j12_series(0.25f * x * x);
+  if (x < 8.0f) return {j1x(x), j2x2(x)};
+  const float P1[7] = {1.000000000e+00f, 1.831054571e-03f, -3.520296377e-05f, 2.574856353e-06f,
+                       -3.913895057e-07f, 7.990912110e-08f, -1.163217167e-08f};
+  const float Q1[7] = {4.687500000e-02f, -2.002715482e-04f, 8.470226021e-06f, -9.461746231e-07f,
+                       1.892280608e-07f, -4.536089548e-08f, 7.152803683e-09f};
+  const float P2[7] = {1.000000000e+00f, -1.281738281e-02f, 7.744745380e-05f, -4.293725397e-06f,
+                       5.753120718e-07f, -1.105211496e-07f, 1.565981123e-08f};
+  const float Q2[7] = {2.343750000e-01f, 6.008147611e-04f, -1.573086774e-05f, 1.463545800e-06f,
+                       -2.668556647e-07f, 6.115627116e-08f, -9.458235084e-09f};
+  const float ix = rcp_fast(x), s = 64.0f * ix * ix, ix8 = 8.0f * ix;
+  const cf e = cis(df_add(df{x, 0.f}, df{-2.356194496154785f, 5.962440319e-09f}));  // e^{i (x - 3 pi / 4)}
+  const float amp = 0.79788456080286536f * rsqrtf(x) * ix;                          // sqrt(2/pi) x^{-3/2}
+  return {amp * fmaf(horner7(P1, s), e.re, -horner7(Q1, s) * ix8 * e.im),
+          amp * ix * fmaf(horner7(P2, s), e.im, horner7(Q2, s) * ix8 * e.re)};
+}
+
 }  // namespace pi

@@ -966,16 +966,16 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
           // two radii per packed FP32 phasor and accumulation (cis_tab_df2)
           const float2 sch = make_float2(sc.hi, sc.hi), scl = make_float2(sc.lo, sc.lo);
           if (disk) {
+            const float amp2 = 2.0f * amp;
             const float rr = q0.w * sqrt_fast(fmaxf(perp, 0.f)) * PI_TURN64;  // rho |k'_perp| / kmag, per 1/64 turn
 #pragma unroll
             for (int p = 0; p < R / 2; ++p) {
               if (2 * p + 1 < skip) continue;
               const float4 kx = ld_shared_f4(kp + 2 * p);
               const float xa = kx.x * rr, xb = kx.y * rr;
-              const float Sa = (xa < 1e-10f) ? 1.0f : 2.0f * j1x(xa);
-              const float Sb = (xb < 1e-10f) ? 1.0f : 2.0f * j1x(xb);
+              const float2 S = j1x_pair(xa, xb);
               const cf2 P = cis_tab_df2(ctab, make_float2(kx.x, kx.y), make_float2(kx.z, kx.w), sch, scl);
-              const float2 m = make_float2(Sa * amp, Sb * amp);
+              const float2 m = make_float2(S.x * amp2, S.y * amp2);
               acc.re2[p] = __ffma2_rn(m, P.re, acc.re2[p]);
               acc.im2[p] = __ffma2_rn(m, P.im, acc.im2[p]);
             }
