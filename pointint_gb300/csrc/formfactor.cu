@@ -780,16 +780,12 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
   const float4* kp = kpair[warp];
   // (k rho)^2 up to which a leaf's expansion is used (never without kg.moments)
   const float bound2 = kg.moments ? MOMENT_X_TRI * MOMENT_X_TRI : -1.f;
-  // the warp's largest k^2, and its smallest over all its radii and over the upper half
-  // of the block (a grid without kg.moments may hold its radii in any order)
-  constexpr int H = R / 2;
-  float kmax2 = 0.f, kmin2 = INFINITY, khalf2 = INFINITY;
+  // the warp's largest k^2 and its smallest (a grid without kg.moments may hold its radii in any order)
+  float kmax2 = 0.f, kmin2 = INFINITY;
 #pragma unroll
   for (int i = 0; i < R; ++i) {
-    const float k2 = kw[i].z;
-    kmax2 = fmaxf(kmax2, k2);
-    if (i >= skip) kmin2 = fminf(kmin2, k2);
-    if (i >= H) khalf2 = fminf(khalf2, k2);
+    kmax2 = fmaxf(kmax2, kw[i].z);
+    if (i >= skip) kmin2 = fminf(kmin2, kw[i].z);
   }
   __shared__ float run_sm[4 * R * FF_THREADS];
   Acc<R> acc;
@@ -877,51 +873,51 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
           const float wide_lo = d_lo * d_lo, wide_hi = 1.0f / 9.0f * d_hi * d_hi;
           // no series where every lane is wide at every radius left
           TriPoly2 tp;
-          if ((kg.moments ? kw[from].z : kmin2) * (1.0f / 9.0f) * wide_lo < 1.0f) tp = tri_series_coeffs2(s1, s2, g);
-          int to = R;  // radii [from, to) one by one, each with its own choice
-          {
-            // the upper half of the block, where all of it is wide for every lane
-            // (about every element of the block of the largest radii): R/2 radii
-            // without a branch, so that their chains overlap. 256 solids 15.37 ->
-            // 14.39 ms; two radii per packed instruction here took longer (14.83)
-            if (from <= H && khalf2 * wide_lo >= 1.0f && khalf2 * wide_hi >= 1.0f) {
-              to = H;
-#pragma unroll
-              for (int i = H; i < R; ++i) {
-                const float4 kr = ld_shared_f4(kw + i);
-                const cf P = cis_tab_df(ctab, make_float2(kr.x, kr.y), tg.sv);
-                const cf T = tri_wide(ctabm, kr.x, tg, gD * rcp_fast(kr.z));
-                acc.re(i) = fmaf(P.re, T.re, fmaf(-P.im, T.im, acc.re(i)));
-                acc.im(i) = fmaf(P.re, T.im, fmaf(P.im, T.re, acc.im(i)));
-              }
-              if (from == to) continue;
-            }
-          }
-          // one radius per scalar instruction: packed pairs were tried and took
-          // more instructions (their constants and dot products need both halves
-          // of a register pair, moved there for every pair between the branches)
-#pragma unroll
-          for (int i = 0; i < R; ++i) {
-            if (i < from || i >= to) continue;
-            const float4 kr = ld_shared_f4(kw + i);
-            const float2 kt = make_float2(kr.x, kr.y);
-            cf P, T;  // the phase's phasor, and the rest with gamma folded in
-            if (kr.z * wide_hi < 1.0f) {
-              P = cis_tab_df(ctab, kt, sm);
-              T = tri_series_eval(tp, kr.z, kr.w);  // centroid Taylor series
-            } else {
-              P = cis_tab_df(ctab, kt, tg.sv);
-              T = tri_wide(ctabm, kr.x, tg, gD * rcp_fast(kr.z));
-              // lanes of small spread, whose divided differences cancel
-              if (kr.z * wide_lo < 1.0f) {
-                const bool narrow = kr.z * tg.D * tg.D < 1.0f;
-                const cf Q = cis_tab_df(ctab, kt, sm), U = tri_series_eval(tp, kr.z, kr.w);
-                P = cf{narrow ? Q.re : P.re, narrow ? Q.im : P.im};
-                T = cf{narrow ? U.re : T.re, narrow ? U.im : T.im};
-              }
-            }
+          if ((kg.moments ? kw[from].z : kmin2) * (1.0f / 9.0f * d_lo * d_lo) < 1.0f) tp = tri_series_coeffs2(s1, s2, g);
+          // a pair of radii at a time, without a branch between them where both are
+          // wide, or both narrow, for every lane: their chains overlap (256 solids
+          // 15.37 -> 14.19 ms; the two radii per packed instruction here took longer)
+          const auto add = [&](int i, cf P, cf T) {
             acc.re(i) = fmaf(P.re, T.re, fmaf(-P.im, T.im, acc.re(i)));
             acc.im(i) = fmaf(P.re, T.im, fmaf(P.im, T.re, acc.im(i)));
+          };
+#pragma unroll
+          for (int p = 0; p < R / 2; ++p) {
+            if (2 * p + 1 < from) continue;
+            const float4 ka = ld_shared_f4(kw + 2 * p), kb = ld_shared_f4(kw + 2 * p + 1);
+            const float klo = fminf(ka.z, kb.z), khi = fmaxf(ka.z, kb.z);
+            if (klo * wide_lo >= 1.0f && klo * wide_hi >= 1.0f) {
+              const cf P0 = cis_tab_df(ctab, make_float2(ka.x, ka.y), tg.sv), P1 = cis_tab_df(ctab, make_float2(kb.x, kb.y), tg.sv);
+              const cf T0 = tri_wide(ctabm, ka.x, tg, gD * rcp_fast(ka.z)), T1 = tri_wide(ctabm, kb.x, tg, gD * rcp_fast(kb.z));
+              add(2 * p, P0, T0);
+              add(2 * p + 1, P1, T1);
+            } else if (khi * wide_hi < 1.0f) {
+              const cf P0 = cis_tab_df(ctab, make_float2(ka.x, ka.y), sm), P1 = cis_tab_df(ctab, make_float2(kb.x, kb.y), sm);
+              add(2 * p, P0, tri_series_eval(tp, ka.z, ka.w));
+              add(2 * p + 1, P1, tri_series_eval(tp, kb.z, kb.w));
+            } else {
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const float4 kr = h ? kb : ka;
+                const float2 kt = make_float2(kr.x, kr.y);
+                cf P, T;  // the phase's phasor, and the rest with gamma folded in
+                if (kr.z * wide_hi < 1.0f) {
+                  P = cis_tab_df(ctab, kt, sm);
+                  T = tri_series_eval(tp, kr.z, kr.w);  // centroid Taylor series
+                } else {
+                  P = cis_tab_df(ctab, kt, tg.sv);
+                  T = tri_wide(ctabm, kr.x, tg, gD * rcp_fast(kr.z));
+                  if (kr.z * wide_lo < 1.0f) {
+                    // lanes of small spread, whose divided differences cancel
+                    const bool narrow = kr.z * tg.D * tg.D < 1.0f;
+                    const cf Q = cis_tab_df(ctab, kt, sm), U = tri_series_eval(tp, kr.z, kr.w);
+                    P = cf{narrow ? Q.re : P.re, narrow ? Q.im : P.im};
+                    T = cf{narrow ? U.re : T.re, narrow ? U.im : T.im};
+                  }
+                }
+                add(2 * p + h, P, T);
+              }
+            }
           }
         }
         }
