@@ -304,10 +304,11 @@ __device__ __forceinline__ TriRef tri_ref(const TriSrcJ& s) {
 // ---- AffineDoF triangles -------------------------------------------------------------
 // A thread owns one direction and R neighbouring radii (the warp 32
 // directions, the CTA 4 neighbouring direction blocks of one radial block).
-// R = 4 (three CTAs per SM: 168 registers, 74 KB of shared memory each)
-// where the launch has at least two waves of CTAs; fewer radii per thread
-// for small launches (one moving mesh of the alignment caller), which
-// would otherwise leave SMs idle.
+// R = 4 (three CTAs per SM: 168 registers, 70 KB of shared memory each)
+// where the launch has at least two waves of CTAs; two radii per thread for
+// small launches (one moving mesh of the alignment caller), which would
+// otherwise leave SMs idle, and then four CTAs per SM (128 registers without
+// spills; three took 1.40 ms an alignment step, four 1.33).
 // Per element and direction the small-spread series of F, D_b and D_c are
 // formed once as polynomials in k (tri_der_coeffs), so a radius costs a table
 // phasor, the Horner chains (cut after h_8 where k |e|max < 1, a test that is
@@ -322,7 +323,7 @@ __device__ __forceinline__ TriRef tri_ref(const TriSrcJ& s) {
 // cluster split the elements, as in ff_kernel.
 
 template <int R>
-__global__ void __launch_bounds__(JAC_THREADS, 3)
+__global__ void __launch_bounds__(JAC_THREADS, R == 2 ? 4 : 3)
 jac_affine_tri_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, float2* __restrict__ G) {
   const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
