@@ -516,49 +516,61 @@ jac_affine_tri_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, 
 // JM_R at a time.  The CTAs of a thread-block cluster split the tiles.
 constexpr int JM_WARPS = 8, JM_THREADS = 32 * JM_WARPS, JM_TILE = JM_WARPS / 2;
 constexpr int JM_SETS = JAC_NSUM / 2, JM_R = 3, JM_RADII = 2 * JM_R * JM_WARPS;
-constexpr int JM_ELEM_F4 = 6;  // staged floats of an element, as float4: vertices, S, N0, a0, E1, E2
+// staged element pairs, as float4: vertices, S, N0, a0, E1, E2 (24 values of
+// two elements, and one float4 that spreads the pairs over the banks)
+constexpr int JM_PAIR_F4 = 13;
 
 // float4 counts: staged elements, coefficients, running sums (and compensations)
-constexpr int JM_F4_ELEM = JM_TILE * PI_CLUSTER * JM_ELEM_F4, JM_F4_MOM = JM_TILE * JM_SETS * 4 * 32,
+constexpr int JM_F4_ELEM = JM_TILE * PI_CLUSTER / 2 * JM_PAIR_F4, JM_F4_MOM = JM_TILE * JM_SETS * 4 * 32,
               JM_F4_RUN = JM_RADII * JAC_NSUM * 2 * 32 / 4;
 constexpr int JM_SMEM = (JM_F4_ELEM + JM_F4_MOM + JM_F4_RUN) * (int)sizeof(float4);
 
 template <int HALF>
 __device__ __forceinline__ void jac_moments(const float4* es, int cnt, float3 d, float inv_norm, float4* mom) {
   constexpr int NS = HALF == 0 ? 4 : 2;  // sets of this warp: NF, W_x / W_y, W_z
-  float mu[NS][MOMENT_TERMS];
+  float2 mu[NS][MOMENT_TERMS];
 #pragma unroll
   for (int v = 0; v < NS; ++v)
 #pragma unroll
-    for (int n = 0; n < MOMENT_TERMS; ++n) mu[v][n] = 0.f;
+    for (int n = 0; n < MOMENT_TERMS; ++n) mu[v][n] = make_float2(0.f, 0.f);
+  const float2 dx = dup2(d.x), dy = dup2(d.y), dz = dup2(d.z), in2 = dup2(inv_norm);
 #pragma unroll 1
-  for (int i = 0; i < cnt; ++i) {
-    const float4 q0 = es[JM_ELEM_F4 * i], q1 = es[JM_ELEM_F4 * i + 1], q2 = es[JM_ELEM_F4 * i + 2],
-                 q3 = es[JM_ELEM_F4 * i + 3], q4 = es[JM_ELEM_F4 * i + 4], q5 = es[JM_ELEM_F4 * i + 5];
-    const float a = d.x * q0.x + d.y * q0.y + d.z * q0.z, bb = d.x * q0.w + d.y * q1.x + d.z * q1.y,
-                c = d.x * q1.z + d.y * q1.w + d.z * q2.x, g = (d.x * q2.y + d.y * q2.z + d.z * q2.w) * inv_norm;
-    const float N0[3] = {q3.x, q3.y, q3.z};
-    const float w0[2] = {g * (HALF == 0 ? q3.w : q4.x), g * q4.y};  // gamma a0
-    const float w1[2] = {g * (HALF == 0 ? q4.z : q4.w), g * q5.x};  // gamma E1
-    const float w2[2] = {g * (HALF == 0 ? q5.y : q5.z), g * q5.w};  // gamma E2
-    float an = 1.f, qn = 1.f, hn = 1.f, hb = 1.f, hc = 1.f;
+  for (int i = 0; i < cnt; i += 2, es += JM_PAIR_F4) {
+    // value c of the two elements
+    const auto val = [&](int c) {
+      const float4 q = es[c / 2];
+      return (c & 1) ? make_float2(q.z, q.w) : make_float2(q.x, q.y);
+    };
+    const auto dot = [&](int c) { return __ffma2_rn(dx, val(c), __ffma2_rn(dy, val(c + 1), __fmul2_rn(dz, val(c + 2)))); };
+    const float2 a = dot(0), bb = dot(3), c = dot(6), g = __fmul2_rn(dot(9), in2);
+    const float2 N0[3] = {val(12), val(13), val(14)};
+    float2 w0[2], w1[2], w2[2];  // gamma a0, gamma E1, gamma E2
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      const int x = HALF == 0 ? 0 : 1 + v;
+      w0[v] = __fmul2_rn(g, val(15 + x));
+      w1[v] = __fmul2_rn(g, val(18 + x));
+      w2[v] = __fmul2_rn(g, val(21 + x));
+    }
+    float2 an = dup2(1.f), qn = an, hn = an, hb = an, hc = an;
 #pragma unroll
     for (int n = 0; n < MOMENT_TERMS; ++n) {
       if (n > 0) {
-        an *= a;
-        qn = fmaf(bb, qn, an);
-        hn = fmaf(c, hn, qn);
-        hb = fmaf(bb, hb, hn);
-        hc = fmaf(c, hc, hn);
+        an = __fmul2_rn(an, a);
+        qn = __ffma2_rn(bb, qn, an);
+        hn = __ffma2_rn(c, hn, qn);
+        hb = __ffma2_rn(bb, hb, hn);
+        hc = __ffma2_rn(c, hc, hn);
       }
-      const float hw = (float)(n + 3) * hn;
+      const float2 hw = make_float2((float)(n + 3) * hn.x, (float)(n + 3) * hn.y);
       if (HALF == 0) {
 #pragma unroll
-        for (int v = 0; v < 3; ++v) mu[v][n] = fmaf(N0[v], hn, mu[v][n]);
-        mu[NS - 1][n] = fmaf(w0[0], hw, fmaf(w1[0], hb, fmaf(w2[0], hc, mu[NS - 1][n])));
+        for (int v = 0; v < 3; ++v) mu[v][n] = __ffma2_rn(N0[v], hn, mu[v][n]);
+        mu[NS - 1][n] = __ffma2_rn(w0[0], hw, __ffma2_rn(w1[0], hb, __ffma2_rn(w2[0], hc, mu[NS - 1][n])));
       } else {
 #pragma unroll
-        for (int v = 0; v < 2; ++v) mu[v][n] = fmaf(w0[v], hw, fmaf(w1[v], hb, fmaf(w2[v], hc, mu[v][n])));
+        for (int v = 0; v < 2; ++v)
+          mu[v][n] = __ffma2_rn(w0[v], hw, __ffma2_rn(w1[v], hb, __ffma2_rn(w2[v], hc, mu[v][n])));
       }
     }
   }
@@ -570,7 +582,7 @@ __device__ __forceinline__ void jac_moments(const float4* es, int cnt, float3 d,
 #pragma unroll
     for (int n = 0; n < MOMENT_TERMS; ++n) {  // i^{n+2}: real for even n, imaginary for odd n
       const float f = (set < 3 ? 0.5f : 0.5f / (n + 3)) * C.f[n];
-      o[(n & 1) * (MOMENT_TERMS / 2) + n / 2] = mu[v][n] * ((n & 2) ? f : -f);
+      o[(n & 1) * (MOMENT_TERMS / 2) + n / 2] = (mu[v][n].x + mu[v][n].y) * ((n & 2) ? f : -f);
     }
 #pragma unroll
     for (int t = 0; t < 4; ++t) mom[(set * 4 + t) * 32] = make_float4(o[4 * t], o[4 * t + 1], o[4 * t + 2], o[4 * t + 3]);
@@ -626,7 +638,12 @@ jac_moment_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, floa
     // stage the tile's elements relative to their clusters' centres, in units of s
     for (int t = threadIdx.x; t < JM_TILE * PI_CLUSTER; t += JM_THREADS) {
       const int p = t0 * PI_CLUSTER + t;
-      if (p >= od.n_elems) continue;
+      float2* d = reinterpret_cast<float2*>(elem + (size_t)(t / 2) * JM_PAIR_F4);
+      const auto put = [&](int c, float v) { reinterpret_cast<float*>(d + c)[t & 1] = v; };
+      if (p >= od.n_elems) {  // the missing half of the last pair
+        for (int c = 0; c < 24; ++c) put(c, 0.f);
+        continue;
+      }
       const float4 ctr = b.clusters[od.cl_off + p / PI_CLUSTER];
       const int ex = ctr.w > 0.f ? min(120, max(-100, ilogbf(ctr.w) + 1)) : 0;
       const float inv_s = __int_as_float((127 - ex) << 23);
@@ -634,28 +651,25 @@ jac_moment_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, floa
       const float4 q0 = b.tri_pool[3 * e], q1 = b.tri_pool[3 * e + 1], q2 = b.tri_pool[3 * e + 2], lo = b.tri_lo[e];
       const float m[3] = {(q0.x - ctr.x) + lo.x, (q0.y - ctr.y) + lo.y, (q0.z - ctr.z) + lo.z};
       const float e1[3] = {q1.x, q1.y, q1.z}, e2[3] = {q2.x, q2.y, q2.z};
-      float va[3], vb[3], vc[3];
+      const TriRef f = tri_ref(src[od.perm_off >= 0 ? b.perm[od.perm_off + p] : p]);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         const float a = m[c] - (e1[c] + e2[c]) * (1.0f / 3.0f);
-        va[c] = a * inv_s;
-        vb[c] = (a + e1[c]) * inv_s;
-        vc[c] = (a + e2[c]) * inv_s;
+        put(c, a * inv_s);
+        put(3 + c, (a + e1[c]) * inv_s);
+        put(6 + c, (a + e2[c]) * inv_s);
+        put(9 + c, c == 0 ? q0.w : (c == 1 ? q1.w : q2.w));
+        put(12 + c, f.N0[c]);
+        put(15 + c, f.a0[c]);
+        put(18 + c, f.E1[c]);
+        put(21 + c, f.E2[c]);
       }
-      const TriRef f = tri_ref(src[od.perm_off >= 0 ? b.perm[od.perm_off + p] : p]);
-      float4* d = elem + (size_t)t * JM_ELEM_F4;
-      d[0] = make_float4(va[0], va[1], va[2], vb[0]);
-      d[1] = make_float4(vb[1], vb[2], vc[0], vc[1]);
-      d[2] = make_float4(vc[2], q0.w, q1.w, q2.w);
-      d[3] = make_float4(f.N0[0], f.N0[1], f.N0[2], f.a0[0]);
-      d[4] = make_float4(f.a0[1], f.a0[2], f.E1[0], f.E1[1]);
-      d[5] = make_float4(f.E1[2], f.E2[0], f.E2[1], f.E2[2]);
     }
     __syncthreads();
     const int c_own = warp >> 1, cl = t0 + c_own;
     if (cl < ncl) {
       const int cnt = min(PI_CLUSTER, od.n_elems - cl * PI_CLUSTER);
-      const float4* es = elem + (size_t)c_own * PI_CLUSTER * JM_ELEM_F4;
+      const float4* es = elem + (size_t)c_own * (PI_CLUSTER / 2) * JM_PAIR_F4;
       float4* mo = mom + c_own * JM_SETS * 4 * 32 + lane;
       if (warp & 1) {
         jac_moments<1>(es, cnt, dh, inv_norm, mo);
