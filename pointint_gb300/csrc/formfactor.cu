@@ -1102,6 +1102,9 @@ ff_serve_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_
 }  // namespace
 
 static int radii_per_thread(int L) { return L >= 32 ? 8 : L >= 4 ? 4 : 2; }  // even: radii are paired
+// Serving evaluations: four, since the largest of a batch's few objects sets its
+// time (a burst with a fifth of its objects rotated: 12.5 ms at eight, 11.5 at four).
+static int serve_radii(int L) { return L >= 4 ? 4 : 2; }
 
 int launch_order(const std::vector<OrderSeg>& segs, int32_t* d_perm, cudaStream_t s) {
   if (segs.empty()) return PI_OK;
@@ -1199,14 +1202,13 @@ int ff_serve_threads() { return FF_THREADS; }
 int ff_serve_setup(const pi_kgrid_impl* kg) { return allow_wide_clusters(ff_serve_fn(kg)); }
 
 int ff_serve_grid_x(const pi_kgrid_impl* kg) {
-  const int R = radii_per_thread(kg->dev.L);
+  const int R = serve_radii(kg->dev.L);
   const int64_t items = (int64_t)((kg->dev.L + R - 1) / R) * ((kg->dev.Me + 31) / 32);
   return (int)((items + FF_WARPS - 1) / FF_WARPS) * FF_SERVE_SPLIT;
 }
 
 const void* ff_serve_fn(const pi_kgrid_impl* kg) {
-  switch (radii_per_thread(kg->dev.L)) {
-    case 8: return reinterpret_cast<const void*>(ff_serve_kernel<8>);
+  switch (serve_radii(kg->dev.L)) {
     case 4: return reinterpret_cast<const void*>(ff_serve_kernel<4>);
     default: return reinterpret_cast<const void*>(ff_serve_kernel<2>);
   }
