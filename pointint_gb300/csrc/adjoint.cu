@@ -143,10 +143,11 @@ constexpr int ADJ_TERMS = MOMENT_TERMS;
 constexpr int ADJ_CL = ADJ_THREADS / PI_CLUSTER;  // clusters per CTA
 static_assert(ADJ_THREADS % PI_CLUSTER == 0 && PI_CLUSTER % 32 == 0, "a warp's elements share a cluster");
 // Bounds on k rho: the derivatives drop one (centres, vertices) or two (normals)
-// orders earlier than the values.  First dropped terms, relative to the
-// leading ones, of an element on the rim seen edge-on: 1.5e-7 (triangles'
-// vertex derivatives at 2.25), 9e-8 (surfels' normal derivatives at 1.9).
-constexpr float ADJ_X_TRI = 2.25f, ADJ_X_SURF = 1.9f;
+// orders earlier than the values.  What is dropped, relative to the leading
+// term, of a small element on the rim seen along its offset (x^15 / 15!, x^14 /
+// 14! and the terms after them) stays below one FP32 rounding: 6.0e-8
+// (triangles' vertex derivatives at 2.1), 4.9e-8 (surfels' normal ones at 1.8).
+constexpr float ADJ_X_TRI = 2.1f, ADJ_X_SURF = 1.8f;
 
 // Sums over the expansion of one element (scaled units).
 struct SurfSums { float F, Fs, Fp; };            // F, dF/dsigma, dF/dp^2

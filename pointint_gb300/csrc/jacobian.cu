@@ -55,10 +55,9 @@ constexpr int JAC_COPIES = 4;
 
 enum { JAC_AFFINE_TRI = 0, JAC_AFFINE_SURF = 1, JAC_MESH_TRI = 2 };
 
-// Radii that the expansions cover (as moment_radii): the derivatives' first
-// dropped term is below 1.1e-7 of the leading one at k rho = 2.5 for an
-// element on the rim seen edge-on.
-constexpr float JAC_X_TRI = 2.5f;
+// Radii that the expansions cover (as moment_radii): the n-th term of the
+// derivatives' series is at most (k rho)^n / n! of the leading one, as the values'.
+constexpr float JAC_X_TRI = MOMENT_X_TRI;
 __device__ __forceinline__ int jac_moment_radii(const KGridDev& kg, float rho) {
   return covered_radii(kg, rho, JAC_X_TRI);
 }

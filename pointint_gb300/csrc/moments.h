@@ -8,13 +8,14 @@ namespace pi {
 
 // An element of a cluster lies within the cluster's bounding radius rho of its
 // centre, so its form factor is e^{i k.c} times a power series in k whose
-// n-th term is at most (k rho)^n / n! of the element's amplitude, and for a
-// triangle 2 / ((n + 1)(n + 2)) of that.  With the MOMENT_TERMS = 16 terms
-// kept, the first dropped one is below 1.4e-8 (triangles, k rho <= 3) and
-// 2.1e-8 (surfels, k rho <= 2.25) for an element on the rim seen edge-on, and
-// orders of magnitude below that for the others of its cluster.
+// n-th term is at most (k rho)^n / n! of the element's amplitude (reached by a
+// small element on the rim, seen along its offset from the centre).  With the
+// MOMENT_TERMS = 16 terms kept, all that is dropped stays below 5.7e-8 of the
+// element's amplitude (triangles, k rho <= 2.375) and 2.4e-8 (surfels, k rho
+// <= 2.25) there, less than one FP32 rounding (6.0e-8), and orders of
+// magnitude below that for the others of its cluster and the smaller radii.
 constexpr int MOMENT_TERMS = 16;
-constexpr float MOMENT_X_TRI = 3.0f, MOMENT_X_SURF = 2.25f;
+constexpr float MOMENT_X_TRI = 2.375f, MOMENT_X_SURF = 2.25f;
 
 // Radii a grid needs for the expansions to pay (an element's moments cost
 // about as much as two radii of the direct sum), and at most as many as the

@@ -40,3 +40,138 @@ def test_tensor_grid_with_radii_in_any_order(cuda, orc, order):
     rng = np.random.default_rng(1)
     objs = [shapes(k, rng) for k in ("cube", "ico3", "mesh_dof", "disks_affine", "gauss")]
     check_J(gpu_J(kg, objs), orc.form_factor_matrix(to_oracle(orc, objs), kg.dirs, kg.kmag))
+
+
+KINDS3 = ["tri", "disk", "gauss"]
+COUNTS = [1, 3, 4, 5, 15, 17, 63, 64, 65, 127, 129, 2047, 2048, 2049, 8192, 8193]
+
+
+def patch(kind, n, seed, shift=(0.0, 0.0, 0.0), affine=False):
+    """n elements scattered over a unit sphere in random order, each of the size
+    that n of them cover it with: an open surface, or one whose elements overlap."""
+    rng = np.random.default_rng(1000 * n + seed)
+    P = rng.normal(size=(n, 3))
+    N = P / np.linalg.norm(P, axis=1, keepdims=True)
+    size = 2.0 / np.sqrt(n)
+    if kind == "tri":
+        V = (N[:, None, :] + size * 0.5 * rng.normal(size=(n, 3, 3))).reshape(-1, 3)
+        geom = G.make_triangle_mesh(V, np.arange(3 * n).reshape(n, 3))
+    elif kind == "disk":
+        geom = G.make_point_cloud(N, N, size * rng.uniform(0.5, 1.0, n))
+    else:
+        geom = G.make_gaussian_splat(N, N, 0.5 * size * rng.uniform(0.5, 1.0, n), np.full(n, 4 * np.pi / n))
+    A = np.eye(3) + (0.2 * rng.normal(size=(3, 3)) if affine else 0.0)
+    return G.SceneObject(geom, pg.DOF_AFFINE, G.affine_dofs(A, shift))
+
+
+def check_J_weighted(kg, orc, objs):
+    """check_J on the sqrt|w|-weighted form factors, in which every radius counts
+    (an open surface's plain ones grow like 1/k towards k = 0)."""
+    Jo = orc.form_factor_matrix(to_oracle(orc, objs), kg.dirs, kg.kmag) * np.sqrt(np.abs(kg.w))[:, None]
+    check_J(gpu_J(kg, objs, True), Jo)
+
+
+@pytest.fixture(scope="module")
+def kg64():
+    return standard_kgrid(9, 64)  # 38 directions, 19 of them evaluated: a part of one warp
+
+
+@pytest.mark.parametrize("n", COUNTS)
+@pytest.mark.parametrize("kind", KINDS3)
+def test_form_factors_at_edge_element_counts(cuda, orc, kg64, kind, n):
+    check_J_weighted(kg64, orc, [patch(kind, n, 1, (0.3, -0.2, 0.5), affine=True)])
+
+
+@pytest.mark.parametrize("L", [7, 8, 9, 31, 32, 47, 48, 49, 288, 289])
+def test_radius_counts_around_the_expansions_limits(cuda, orc, L):
+    """Expansions from 8 to 288 radii; 32 radii a thread block of eight, 48 the
+    Jacobian's groups."""
+    kg = standard_kgrid(3, L)
+    check_J_weighted(kg, orc, [patch(k, 130, 2, (0.1, 0.2, 0.3), affine=True) for k in KINDS3])
+
+
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 129, 2049])
+@pytest.mark.parametrize("kind", KINDS3)
+def test_gradients_at_edge_element_counts(cuda, orc, kg64, kind, n):
+    """AffineDoF gradients of a pair (the adjoint's expansions, its clusters'
+    last one partly empty) and, for triangles, Gauss-Newton blocks (the
+    Jacobian's expansions, which surfels do not take)."""
+    o1, o2 = patch(kind, n, 3, (0.1, 0.0, -0.2), affine=True), patch("tri", 80, 4, (0.4, 0.1, 0.0))
+    got = core.pair_volume_hessian_host(kg64, o1, o2)
+    a, b = to_oracle(orc, [o1, o2])
+    ref = orc.pair_volume(a, b, (kg64.dirs, kg64.kmag, kg64.w), orc.VOLUME_ONLY | orc.GRADIENT | orc.HESSIAN)
+    assert_grad_close(got["grad_geom1"], ref["grad_geom1"], what=f"{kind} {n} grad1")
+    assert_grad_close(got["grad_geom2"], ref["grad_geom2"], what=f"{kind} {n} grad2")
+    if kind != "tri":
+        return
+    H11, H22 = ref["hessian_geom1"], ref["hessian_geom2"]
+    for key, Hi, Hj in (("hessian_geom1", H11, H11), ("hessian_geom2", H22, H22), ("hessian_cross", H11, H22)):
+        fro, _ = block_errors(got[key], ref[key], Hi, Hj)
+        assert fro <= 1e-5, (key, fro)
+
+
+def test_vertex_gradients_of_a_reordered_mesh(cuda, orc, kg64):
+    """2,420 triangles (reordered) with vertex DoFs: gradients stay with their vertices."""
+    V, F = G.geodesic_sphere(11)
+    assert len(F) > 2048
+    objs = [G.SceneObject(G.make_triangle_mesh(V, F), pg.DOF_TRIANGLE_MESH, V.reshape(-1)), patch("disk", 100, 5, (0.5, 0, 0))]
+    _, grad = core.volume_matrix_grad_host(kg64, objs)
+    _, ref, _ = orc.volume_matrix(to_oracle(orc, objs), (kg64.dirs, kg64.kmag, kg64.w), orc.VOLUME_ONLY | orc.GRADIENT)
+    assert_grad_close(grad[0][1], ref[0][1], what="vertices")
+
+
+@pytest.mark.parametrize("kind", ["disk", "gauss"])
+def test_surfel_gradients_of_a_reordered_cloud(cuda, orc, kg64, kind):
+    """2,049 surfels: the gradients come back in the caller's order."""
+    objs = [patch(kind, 2049, 6), patch(kind, 65, 7)]
+    scene = core.Scene(kg64, objs)
+    c, n = (t.requires_grad_(True) for t in scene.surfel_params())
+    scene.volume_matrix_of_surfels(c, n).sum().backward()
+    gp, gn = orc.surfel_param_grad(to_oracle(orc, objs), (kg64.dirs, kg64.kmag, kg64.w), np.ones((2, 2)))
+    assert_grad_close(c.grad.cpu().numpy(), gp, what="dL/dc")
+    assert_grad_close(n.grad.cpu().numpy(), gn, what="dL/dn")
+
+
+@pytest.mark.parametrize("n", [1, 2, 4, 5, 8, 9, 33, 63, 64, 65])
+@pytest.mark.parametrize("Q", [3, 1001])
+def test_few_row_contraction(cuda, n, Q):
+    """n <= 64 rows take the FP32 contraction of their own; weights of both signs,
+    a node count that is no multiple of anything."""
+    rng = np.random.default_rng(100 * n + Q)
+    dirs = rng.normal(size=(Q, 3))
+    dirs /= np.linalg.norm(dirs, axis=1, keepdims=True)
+    w = rng.uniform(0.5, 1.5, Q)
+    w[::5] *= -1.0
+    kg = KGrid(dirs, rng.uniform(0.1, 5.0, Q), w)
+    J = (rng.normal(size=(n, Q)) + 1j * rng.normal(size=(n, Q))).astype(np.complex64)
+    V = core.contract(kg, torch.from_numpy(J).cuda(), "fp32").cpu().numpy()
+    R = fp64_contract(J, w)
+    # conditioned by the sums of magnitudes: with weights of both signs the diagonal may cancel too
+    scale = fp64_contract(np.abs(J.real) + 1j * np.abs(J.imag), np.abs(w))
+    assert np.array_equal(V, V.T)
+    assert (np.abs(V - R) / scale).max() <= 1e-6
+
+
+@pytest.mark.parametrize("dirs_kept", ["every second", "one of each pair"])
+def test_serving_on_a_grid_with_unpaired_directions(cuda, orc, dirs_kept):
+    """Rows hold the evaluated directions only, weighted with their antipode where
+    the grid has it."""
+    from pointint_gb300.serving import Server
+    full = standard_kgrid(9, 16)
+    M = full.num_nodes // 16
+    keep = np.arange(0, M, 2) if dirs_kept == "every second" else full.direction_pairs()[:, 0]
+    sel = (np.arange(16)[:, None] * M + np.asarray(keep)[None, :]).reshape(-1)
+    kg = KGrid(full.dirs[sel], full.kmag[sel], full.w[sel])
+    rng = np.random.default_rng(3)
+    lib = [patch("tri", 300, 8), patch("disk", 200, 9), patch("gauss", 100, 10), shapes("ico3", rng)]
+    rots = np.array([np.eye(3), G.random_rotation(rng), G.random_rotation(rng), np.eye(3), G.random_rotation(rng)])
+    trans = rng.normal(0.0, 0.4, size=(5, 3))
+    ids = [0, 1, 2, 3, 3]
+    moved = []
+    for i, R, t in zip(ids, rots, trans):
+        d = lib[i].dofs
+        moved.append(G.SceneObject(lib[i].geom, pg.DOF_AFFINE, G.affine_dofs(R @ d[3:].reshape(3, 3), R @ d[:3] + t)))
+    ref, _, _ = orc.volume_matrix(to_oracle(orc, moved), (kg.dirs, kg.kmag, kg.w))
+    with Server(kg, lib, precision="fp16x3", autotune=False) as srv:
+        V = srv.query(ids, rots, trans)
+    assert cond_rel_err(V, ref).max() <= 1e-4
