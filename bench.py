@@ -324,34 +324,35 @@ def run_gb300(args):
     sfu_achieved = SFU_OPS_PER_EVAL * evals_kernel / ff_avg_s / 1e9
     sfu_peak = n_sm * SFU_PER_SM_PER_CLK * clk_max * 1e6 / 1e9
     # issue slots: 4 warp instructions per SM per clock; thread instructions per
-    # evaluation from the kernel's ncu capture on 32 of the 256 objects
+    # evaluation from the two kernels' ncu capture on 32 of the 256 objects
     issue_achieved = FF_THREAD_INSTR_PER_EVAL / 32.0 * evals_kernel / ff_avg_s / 1e9
     issue_peak = n_sm * 4 * clk_max * 1e6 / 1e9
-    roofline = {"kernel": "ff_kernel", "bound": "fp32-issue", "achieved": fp32_achieved, "peak": fp32_peak,
+    roofline = {"kernel": "ff_kernel + moment_kernel", "bound": "fp32-issue", "achieved": fp32_achieved, "peak": fp32_peak,
                 "unit": "TFLOP/s", "frac": fp32_achieved / fp32_peak, "traffic": FF_TRAFFIC_BYTES_PER_LAUNCH,
                 "kernel_ms": ff_avg_s * 1e3, "share_of_step": (ff_ms / total_ms) if world == 1 else None,
                 "algorithmic_unit": f"{FP32_FLOPS_PER_EVAL} FP32 flops (FMA = 2) per triangle x k evaluation, the "
-                                    f"reference algorithm's count, x {evals_kernel:.4e} evaluations the kernel "
-                                    f"performs: {n_eval_dirs} of the {n_dirs} directions, one of each antipodal pair "
+                                    f"reference algorithm's count, x {evals_kernel:.4e} triangle x k pairs "
+                                    f"of {n_eval_dirs} of the {n_dirs} directions, one of each antipodal pair "
                                     f"(A(-k) = -conj A(k) gives the other); the workload's {evals_step:.4e} "
-                                    "triangle x k pairs are all produced",
+                                    "triangle x k pairs are all produced. Most of the radii come from cluster "
+                                    "expansions shared by 64 elements, so the kernels do far fewer than the "
+                                    "reference's operations and the fraction may exceed 1",
                 "evaluated_directions": {"evaluated": n_eval_dirs, "of": n_dirs},
                 "peak_source": f"nominal FP32: {FP32_FLOPS_PER_SM_PER_CLK} flops/clk/SM x {n_sm} SMs x {clk_max} MHz "
                                "(MEASURED_PEAKS.json holds HBM and bf16 tensor peaks only)",
-                "binding": "FP32 issue and FMA pipe: no MUFU (SFU) instructions (sine/cosine are a phasor table "
-                           "and polynomials); the short-series loop runs two radii per packed FP32 instruction, which "
-                           "holds the FMA pipe two cycles, so the FMA pipe (math-pipe throttle, the second stall) and "
-                           "the issue slots bind together",
+                "binding": "issue slots: ff_kernel (87% of the time) sums the few largest radii element by element, "
+                           "three table phasors each, and waits at its tile barriers where the directions of a "
+                           "CTA's warps take different branches; sine/cosine are a phasor table and polynomials",
                 "pipes_from_capture": {"fma_pipe_active": FF_FMA_PIPE_ACTIVE, "issue_active": FF_ISSUE_ACTIVE,
-                                       "source": "ncu --set full of the same kernel on 32 of the 256 objects"},
+                                       "source": "ncu counters of ff_kernel on 32 of the 256 objects"},
                 "issue": {"thread_instructions_per_evaluation": FF_THREAD_INSTR_PER_EVAL,
                           "achieved": issue_achieved, "peak": issue_peak, "unit": "G warp-instructions/s",
                           "frac": issue_achieved / issue_peak,
                           "source": "instructions per evaluation from ncu (smsp__inst_executed.sum x 32 / "
-                                    "evaluations, 32-object capture); rate from this run's CUDA events"},
+                                    "evaluations of both kernels, 32-object capture); rate from this run's CUDA events"},
                 "sfu_count": {"achieved": sfu_achieved, "peak": sfu_peak, "unit": "Gop/s", "frac": sfu_achieved / sfu_peak,
                               "note": f"{SFU_OPS_PER_EVAL} SFU-class operations per evaluation in the reference "
-                                      "algorithm (accounting only: this kernel issues none)"}}
+                                      "algorithm (accounting only)"}}
 
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
@@ -360,9 +361,9 @@ def run_gb300(args):
             "vol_matrix_per_s": world * args.steps / (total_ms / 1e3),
             "contraction": contraction, "clocks": clocks, "gpu_launches": launches, "roofline": roofline,
             "work_note": (f"value counts the workload's {evals_step:.4e} triangle x k pairs per step, all of them "
-                          f"produced in J; the form-factor kernel evaluates {evals_kernel:.4e} of them (one direction "
-                          f"of each antipodal pair, {n_eval_dirs} of {n_dirs}) and writes the rest as "
-                          "A(-k) = -conj A(k)")}
+                          f"produced in J; the kernels evaluate {evals_kernel:.4e} of them (one direction "
+                          f"of each antipodal pair, {n_eval_dirs} of {n_dirs}), most radii through expansions of "
+                          "64-element clusters, and write the rest as A(-k) = -conj A(k)")}
 
     if rank == 0 and not args.no_e2e:
         line["e2e"] = e2e_host(kg, objs, precision, args.steps, evals_step, world)
@@ -386,26 +387,22 @@ def run_gb300(args):
         dist.destroy_process_group()
 
 
-# DRAM bytes (read + write) of one full-size ff_kernel launch.  Reads: captured
-# with ncu on 32 of the 256 objects (82,112 triangles: 5.70 MB with the
-# centroid low words) and scaled by the triangle count (656,896 / 82,112),
-# since element reads grow with the elements.  Writes: that capture's J
-# (19.7 MB) stayed in L2, but the full J (256 x 76,928 complex64 = 157.5 MB)
-# exceeds the 129 MB L2 and is counted as written once.
-FF_TRAFFIC_BYTES_PER_LAUNCH = 5.70e6 * 656896 / 82112 + 256 * 76928 * 8
-# Thread instructions per evaluation the kernel performs (one direction of
-# each antipodal pair), from its ncu capture on 32 of the 256 objects
-# (smsp__inst_executed.sum 4.481e9 x 32 / 3.158e9 evaluations; packed FP32
-# instructions count once).
-FF_THREAD_INSTR_PER_EVAL = 45.4
-# The same capture's FMA-pipe busy share (sm__pipe_fma_cycles_active, 51.0%
-# of active cycles, packed FP32 instructions holding the pipe two cycles) and
-# issue-slot share (smsp__issue_active, 59.0%).  The 32-object launch is 1.6
-# waves of CTAs and ends on a tail (2.8 warps per scheduler on average), so
-# both read lower than in the 256-object launch, whose issue share the line's
-# `issue.frac` gives from its own time.
-FF_FMA_PIPE_ACTIVE = 0.510
-FF_ISSUE_ACTIVE = 0.590
+# DRAM bytes (read + write) of one full-size launch of ff_kernel and
+# moment_kernel.  Reads: captured with ncu on 32 of the 256 objects (82,112
+# triangles: 5.94 and 7.46 MB) and scaled by the triangle count (656,896 /
+# 82,112), since element reads grow with the elements.  Writes: that capture's
+# J (19.7 MB) stayed in L2, but the full J (256 x 76,928 complex64 = 157.5 MB)
+# exceeds the 129 MB L2 and is counted as written once, every node by one of
+# the two kernels.
+FF_TRAFFIC_BYTES_PER_LAUNCH = (5.94e6 + 7.46e6) * 656896 / 82112 + 256 * 76928 * 8
+# Thread instructions per triangle x k pair of the evaluated directions, from
+# the two kernels' ncu capture on 32 of the 256 objects (smsp__inst_executed.sum
+# (1.391e9 + 0.135e9) x 32 / 3.158e9 pairs; packed FP32 instructions count once).
+FF_THREAD_INSTR_PER_EVAL = 15.5
+# The same capture's FMA-pipe busy share of ff_kernel (sm__pipe_fma_cycles_active,
+# 48.2% of active cycles) and its issue-slot share (smsp__issue_active, 63.2%).
+FF_FMA_PIPE_ACTIVE = 0.482
+FF_ISSUE_ACTIVE = 0.632
 
 
 def _pcts(ms):

@@ -434,7 +434,7 @@ int kgrid_create_impl(const double* dirs, const double* kmag, const double* w, i
     if (!ok) return fail(PI_ERR_UNSUPPORTED, "pi_kgrid_create: bad direction pairing");
   }
   const size_t o_eh = align16(o_pair + Me * sizeof(int2)), o_el = align16(o_eh + Me * sizeof(float4)),
-               total = align16(o_el + Me * sizeof(float4));
+               o_col = align16(o_el + Me * sizeof(float4)), total = align16(o_col + Me * sizeof(int32_t));
   std::vector<unsigned char> host(total, 0);
   std::memcpy(host.data() + o_dh, dh.data(), M * sizeof(float4));
   std::memcpy(host.data() + o_dl, dl.data(), M * sizeof(float4));
@@ -445,9 +445,18 @@ int kgrid_create_impl(const double* dirs, const double* kmag, const double* w, i
   std::memcpy(host.data() + o_k256, k256.data(), L * sizeof(float2));
   std::memcpy(host.data() + o_tab, tab.data(), tab.size() * sizeof(float2));
   std::memcpy(host.data() + o_pair, pairs.data(), Me * sizeof(int2));
-  for (int64_t e = 0; e < Me; ++e) {
-    std::memcpy(host.data() + o_eh + e * sizeof(float4), &dh[pairs[e].x], sizeof(float4));
-    std::memcpy(host.data() + o_el + e * sizeof(float4), &dl[pairs[e].x], sizeof(float4));
+  {
+    // columns of the serving rows: the evaluated directions in the grid's order
+    std::vector<int32_t> col_of(M, -1), col(Me);
+    for (int64_t e = 0; e < Me; ++e) col_of[pairs[e].x] = 0;
+    int32_t c = 0;
+    for (int64_t j = 0; j < M; ++j) if (col_of[j] >= 0) col_of[j] = c++;
+    for (int64_t e = 0; e < Me; ++e) {
+      col[e] = col_of[pairs[e].x];
+      std::memcpy(host.data() + o_eh + col[e] * sizeof(float4), &dh[pairs[e].x], sizeof(float4));
+      std::memcpy(host.data() + o_el + col[e] * sizeof(float4), &dl[pairs[e].x], sizeof(float4));
+    }
+    std::memcpy(host.data() + o_col, col.data(), Me * sizeof(int32_t));
   }
   kg->pooled = temporary;
   kg->pool_stream = s;
@@ -474,6 +483,7 @@ int kgrid_create_impl(const double* dirs, const double* kmag, const double* w, i
   kg->dev.dpair = reinterpret_cast<const int2*>(base + o_pair);
   kg->dev.edir_hi = reinterpret_cast<const float4*>(base + o_eh);
   kg->dev.edir_lo = reinterpret_cast<const float4*>(base + o_el);
+  kg->dev.ecol = reinterpret_cast<const int*>(base + o_col);
   kg->dev.Me = (int)Me;
   kg->Me = (int)Me;
   kg->dev.moments = moment_grid(dv, km, M, L, tensor) ? 1 : 0;

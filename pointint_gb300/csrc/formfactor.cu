@@ -1028,7 +1028,7 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
         cf v{acc.sre(i), acc.sim(i)};
         if (kw[i].x * PI_TURN64 * dnorm < 1e-10f) v = cf{0.f, 0.f};  // A(0) = 0 (affine_dof.cpp:64-65)
         const float sw = serve_scale(kg, q, jm >= 0 ? (int64_t)r * kg.M + jm : -1);
-        ev.dst[(int64_t)ei * kg.L + r] = make_float2(v.re * sw, v.im * sw);
+        ev.dst[(int64_t)kg.ecol[ei] * kg.L + r] = make_float2(v.re * sw, v.im * sw);
         m = fmaxf(m, fmaxf(fabsf(v.re * sw), fabsf(v.im * sw)));
       }
     }

@@ -362,7 +362,7 @@ __device__ __forceinline__ void moment_body(const KGridDev& kg, const BatchDev& 
       const float sw = serve_scale(kg, q, jm >= 0 ? qm : -1);
       const float2 o = make_float2(v.re * sw, v.im * sw);
       m = fmaxf(m, fmaxf(fabsf(o.x), fabsf(o.y)));
-      evals[slot].dst[(int64_t)ei * kg.L + r] = o;
+      evals[slot].dst[(int64_t)kg.ecol[ei] * kg.L + r] = o;
     } else {
       const float sw = scale_sqrt_w ? kg.sqrtw[q] : 1.0f, swm = scale_sqrt_w && jm >= 0 ? kg.sqrtw[qm] : 1.0f;
       const float2 o = make_float2(v.re * sw, v.im * sw), om = make_float2(-v.re * swm, v.im * swm);

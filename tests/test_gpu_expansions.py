@@ -175,3 +175,29 @@ def test_serving_on_a_grid_with_unpaired_directions(cuda, orc, dirs_kept):
     with Server(kg, lib, precision="fp16x3", autotune=False) as srv:
         V = srv.query(ids, rots, trans)
     assert cond_rel_err(V, ref).max() <= 1e-4
+
+
+def test_serving_precision_of_disjoint_objects(cuda):
+    """Serving rows keep the grid's direction order: small volumes of disjoint
+    objects, conditioned at 1e-3 sqrt(V_ii V_jj), within 3e-5 of an FP64
+    contraction in the mean over scenes (2e-5 is the plain path's own level with
+    the FP16 split; rows in compact groups of directions measured 5.3e-5)."""
+    from pointint_gb300.serving import Server
+    kg = standard_kgrid(59, 64)
+    V3, F3 = G.icosphere(3)
+    worst = []
+    for seed in range(4):
+        rng = np.random.default_rng(seed)
+        objs = []
+        for i in range(40):
+            A = G.random_rotation(rng) @ np.diag(rng.uniform(0.5, 1.5, 3))
+            V, F = (V3, F3) if i % 2 else G.box_mesh(rng.uniform(0.5, 2.0, 3))
+            objs.append(G.SceneObject(G.make_triangle_mesh(V, F), pg.DOF_AFFINE, G.affine_dofs(A, rng.uniform(0, 3, 3))))
+        tr = rng.normal(0.0, 0.5, (40, 3))
+        with Server(kg, objs, precision="fp16x3", autotune=False) as srv:
+            V = srv.query(np.arange(40), None, tr)
+        moved = [G.SceneObject(o.geom, o.dof_type, np.concatenate([o.dofs[:3] + t, o.dofs[3:]])) for o, t in zip(objs, tr)]
+        X = torch.view_as_real(core.form_factors(kg, core.ObjectBatch(moved), True)).reshape(40, -1).double()
+        worst.append(cond_rel_err(V, ((X @ X.T) / (8 * np.pi ** 3)).cpu().numpy()).max())
+    print(f"\nserved disjoint objects: {worst}")
+    assert np.mean(worst) <= 3e-5
