@@ -301,6 +301,22 @@ __device__ __forceinline__ cf2 cis_tab_df2(const float2* tab, float2 kth, float2
   return cis_tab_frac2<C>(tab, t, __ffma2_rn(ktl, smh, f));
 }
 
+// cis_tab_m1_df on both halves.
+template <int C>
+__device__ __forceinline__ cf2 cis_tab_m1_df2(const float2* tabm, float2 kth, float2 ktl, float2 dh, float2 dl) {
+  const float2 t = __ffma2_rn(kth, dh, dup2(PI_ROUND_SHIFT));
+  float2 f = __ffma2_rn(kth, dh, __ffma2_rn(t, dup2(-1.0f), dup2(PI_ROUND_SHIFT)));
+  f = __ffma2_rn(ktl, dh, __ffma2_rn(kth, dl, f));
+  const float2 f2 = __fmul2_rn(f, f);
+  const float2 cm = __fmul2_rn(f2, __ffma2_rn(f2, dup2(PI_TURN64_C4), dup2(-PI_TURN64_C2)));
+  const float2 sn = __fmul2_rn(f, __ffma2_rn(f2, dup2(-PI_TURN64_C3), dup2(PI_TURN64)));
+  const float2* ta = tabm + (__float_as_int(t.x) & (PHASOR_ENTRIES - 1)) * C;
+  const float2* tb = tabm + (__float_as_int(t.y) & (PHASOR_ENTRIES - 1)) * C;
+  const float2 ax = make_float2(ta->x, tb->x), ay = make_float2(ta->y, tb->y);
+  return {__fadd2_rn(ax, __ffma2_rn(ax, cm, __ffma2_rn(neg2(ay), sn, cm))),
+          __fadd2_rn(ay, __ffma2_rn(ay, cm, __ffma2_rn(ax, sn, sn)))};
+}
+
 __device__ __forceinline__ cf cmul(cf a, cf b) { return {a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re}; }
 __device__ __forceinline__ cf csub(cf a, cf b) { return {a.re - b.re, a.im - b.im}; }
 __device__ __forceinline__ cf cscale(cf a, float s) { return {a.re * s, a.im * s}; }

@@ -813,11 +813,13 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
       for (int t = threadIdx.x; t * PI_LEAF < cnt; t += FF_THREADS) leaf[t] = leaves[base / PI_LEAF + t];
       __syncthreads();
       if (busy) {  // every lane of a busy warp (the votes below); those without a direction write nothing
-        // chunks of FF_CHUNK elements (tiles hold a multiple of FF_CHUNK)
-        for (int e0 = 0; e0 < cnt; e0 += FF_CHUNK) {
-        const int e1 = min(e0 + FF_CHUNK, cnt);
-        for (int l0 = e0; l0 < e1; l0 += PI_LEAF) {
-        const int l1 = min(l0 + PI_LEAF, e1);
+        // chunks of FF_CHUNK elements: leaves from all over the tile, since the
+        // elements of a compact patch add up in phase and their FP32 partial sum
+        // would round coarser
+        const int nch = (cnt + FF_CHUNK - 1) / FF_CHUNK;
+        for (int ch = 0; ch < nch; ++ch) {
+        for (int l0 = ch * PI_LEAF; l0 < cnt; l0 += nch * PI_LEAF) {
+        const int l1 = min(l0 + PI_LEAF, cnt);
         int from = skip;  // first radius of the block that the elements are summed at one by one
         {
           // radii ascend: those of the leading pairs lie within the expansion's reach of this leaf
@@ -921,7 +923,7 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
           }
         }
         }
-        if (e1 - e0 == FF_CHUNK) acc.flush();
+        acc.flush();
         }
       }
     }
@@ -945,9 +947,9 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
       }
       __syncthreads();
       if (busy) {  // every lane of a busy warp (the votes below); those without a direction write nothing
-        for (int e0 = 0; e0 < cnt; e0 += FF_CHUNK) {
-        const int e1 = min(e0 + FF_CHUNK, cnt);
-        for (int e = e0; e < e1; ++e) {
+        const int nch = (cnt + FF_CHUNK - 1) / FF_CHUNK;  // as above
+        for (int ch = 0; ch < nch; ++ch) {
+        for (int e = ch; e < cnt; e += nch) {
           const float4 q0 = tile[2 * e], q1 = tile[2 * e + 1], nr = tile[2 * FF_TILE + e];
           const float4 cl = tile[3 * FF_TILE + e];
           const df sc = cdot2_un(dh, dl, make_float3(q0.x, q0.y, q0.z), make_float3(cl.x, cl.y, cl.z));
@@ -988,7 +990,7 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
             }
           }
         }
-        if (e1 - e0 == FF_CHUNK) acc.flush();
+        acc.flush();
         }
       }
     }

@@ -63,7 +63,7 @@ constexpr int FM_F4_ELEM = FM_WARPS * FM_PAIRS * FM_PAIR_F4, FM_F4_MOM = FM_WARP
 __host__ __device__ constexpr int fm_batches(int L) { return (L + FM_R - 1) / FM_R; }
 __host__ __device__ constexpr int fm_smem_f4(int L) {
   return FM_F4_ELEM + FM_F4_MOM + FM_F4_TAB + FM_F4_CTR + fm_batches(L) * FM_R /* kx, kk */ +
-         fm_batches(L) * FM_R * 32 /* running sums: (re, im, compensations) */;
+         (fm_batches(L) * FM_R + 1) * 32 /* running sums: (re, im, compensations), and of the zeroth moments */;
 }
 
 __device__ __forceinline__ float2 f2lo(float4 v) { return make_float2(v.x, v.y); }
@@ -131,10 +131,11 @@ __device__ __forceinline__ void fm_stage(const BatchDev& b, const ObjDev& od, in
 }
 
 // Sums the moments of the staged elements; mu in the even entries' and odd
-// entries' halves.
+// entries' halves.  Returns the zeroth, compensated (hi, lo).
 template <int KIND>
-__device__ __forceinline__ void fm_moments(const float4* es, int pairs, const FmDir& D, float2 mu[MOMENT_TERMS]) {
+__device__ __forceinline__ float2 fm_moments(const float4* es, int pairs, const FmDir& D, float2 mu[MOMENT_TERMS]) {
   constexpr FmConst<KIND> C{};
+  float2 z = make_float2(0.f, 0.f), cz0 = z;
 #pragma unroll
   for (int n = 0; n < MOMENT_TERMS; ++n) mu[n] = make_float2(0.f, 0.f);
   const float2 dx = dup2(D.dh.x), dy = dup2(D.dh.y), dz = dup2(D.dh.z);
@@ -149,6 +150,7 @@ __device__ __forceinline__ void fm_moments(const float4* es, int pairs, const Fm
       const float2 c = fma2(dz, f2lo(q4), fma2(dy, f2hi(q3), mul2(dx, f2lo(q3))));
       const float2 g = fma2(dz, f2hi(q5), fma2(dy, f2lo(q5), mul2(dx, f2hi(q4))));  // gamma |d| (area vector . d)
       tri_moments(a, bb, c, g, mu);
+      kahan2(z, cz0, g);
     } else {
       const float2 amp = fma2(dz, f2hi(q2), fma2(dy, f2lo(q2), mul2(dx, f2hi(q1))));
       // |k'_perp|^2 / |k|^2 = qd (1 - |n|^2) + |n|^2 |v x n/|n||^2, as in ff_kernel
@@ -162,7 +164,7 @@ __device__ __forceinline__ void fm_moments(const float4* es, int pairs, const Fm
       // disk: q = p^2 - s^2; Gaussian: q = sigma^2 |k'_perp|^2 / |k|^2 (= 2 q' of e^{-q' k^2})
       const float2 q = disk ? fma2(p2, perp, neg2(mul2(s0, s0))) : mul2(p2, perp);
       float2 w0 = amp, w1 = mul2(s0, amp);
-      mu[0] = add2(mu[0], w0);
+      kahan2(z, cz0, w0);
       mu[1] = add2(mu[1], w1);
 #pragma unroll
       for (int n = 1; n < MOMENT_TERMS - 1; ++n) {
@@ -173,6 +175,9 @@ __device__ __forceinline__ void fm_moments(const float4* es, int pairs, const Fm
       }
     }
   }
+  mu[0] = z;
+  const df s = two_sum(z.x, z.y);
+  return make_float2(s.hi, s.lo - (cz0.x + cz0.y));
 }
 
 // e^{ik.c} sum_n (i k)^n .. of the cluster: coefficients as Re = sum_j a_j u^j,
@@ -186,6 +191,14 @@ __device__ __forceinline__ void fm_store(const float2 mu[MOMENT_TERMS], float no
     c[(n & 1) * (MOMENT_TERMS / 2) + n / 2] = (mu[n].x + mu[n].y) * (((n & 2) ? -C.f[n] : C.f[n]) * norm);
 #pragma unroll
   for (int t = 0; t < 4; ++t) mom[32 * t] = make_float4(c[4 * t], c[4 * t + 1], c[4 * t + 2], c[4 * t + 3]);
+}
+
+// c[1] u + c[2] u^2 + ... + c[7] u^7
+__device__ __forceinline__ float2 horner_rest(const float (&c)[8], float2 u) {
+  float2 r = dup2(c[7]);
+#pragma unroll
+  for (int i = 6; i >= 1; --i) r = fma2(r, u, dup2(c[i]));
+  return mul2(r, u);
 }
 
 __device__ __forceinline__ float2 horner8(const float (&c)[8], float2 u) {
@@ -222,6 +235,7 @@ __device__ __forceinline__ void moment_body(const KGridDev& kg, const BatchDev& 
   float4* kx = reinterpret_cast<float4*>(csc + 32 * FM_WARPS);  // radii (2p, 2p + 1) in 1/64 turns: (hi, hi', lo, lo')
   float2* kk = reinterpret_cast<float2*>(kx + fm_batches(kg.L) * FM_R / 2);  // (k, k')
   float4* run = kx + fm_batches(kg.L) * FM_R;             // [radius][lane]: sums and compensations
+  float4* run0 = run + nb * FM_R * 32;                    // the zeroth moments', in the first and third
   __shared__ float cscale_sm[FM_WARPS];
 
   const int ei = dt * 32 + lane;
@@ -255,7 +269,7 @@ __device__ __forceinline__ void moment_body(const KGridDev& kg, const BatchDev& 
                     Am[2] * D.dh.x + Am[5] * D.dh.y + Am[8] * D.dh.z);
   D.qd = fmaf(D.v.x, D.v.x, fmaf(D.v.y, D.v.y, D.v.z * D.v.z));
 
-  stage_phasors<FM_COPIES>(kg.cis_tab, ctab_sm);
+  stage_phasors<FM_COPIES>(kg.cis_tabm, ctab_sm);
   for (int t = threadIdx.x; t < nb * FM_R / 2; t += FM_THREADS) {
     float2 k[2], kt[2];
 #pragma unroll
@@ -267,7 +281,7 @@ __device__ __forceinline__ void moment_body(const KGridDev& kg, const BatchDev& 
     kx[t] = make_float4(kt[0].x, kt[1].x, kt[0].y, kt[1].y);
     kk[t] = make_float2(k[0].x, k[1].x);
   }
-  for (int t = threadIdx.x; t < nb * FM_R * 32; t += FM_THREADS) run[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int t = threadIdx.x; t < (nb * FM_R + 1) * 32; t += FM_THREADS) run[t] = make_float4(0.f, 0.f, 0.f, 0.f);
 
   const int ncl = (od.n_elems + PI_CLUSTER - 1) / PI_CLUSTER;
   for (int t0 = rank * FM_WARPS; t0 < ncl; t0 += S * FM_WARPS) {
@@ -280,27 +294,44 @@ __device__ __forceinline__ void moment_body(const KGridDev& kg, const BatchDev& 
       const float s = __int_as_float((127 + ex) << 23), inv_s = __int_as_float((127 - ex) << 23);
       const int first = cl * PI_CLUSTER, cnt = min(PI_CLUSTER, od.n_elems - first), pairs = (cnt + 1) / 2;
       float4* es = elem + warp * FM_PAIRS * FM_PAIR_F4;
-      float2 mu[MOMENT_TERMS];
+      float2 mu[MOMENT_TERMS], m0;
       float4* mo = mom + warp * 4 * 32 + lane;
       if (od.type == PI_GEOM_TRIANGLE) {
         fm_stage<PI_GEOM_TRIANGLE>(b, od, first, cnt, ctr, inv_s, reinterpret_cast<float*>(es));
-        fm_moments<PI_GEOM_TRIANGLE>(es, pairs, D, mu);
+        m0 = fm_moments<PI_GEOM_TRIANGLE>(es, pairs, D, mu);
         fm_store<PI_GEOM_TRIANGLE>(mu, D.inv_norm, mo);
       } else if (od.type == PI_GEOM_DISK) {
         fm_stage<PI_GEOM_DISK>(b, od, first, cnt, ctr, inv_s, reinterpret_cast<float*>(es));
-        fm_moments<PI_GEOM_DISK>(es, pairs, D, mu);
+        m0 = fm_moments<PI_GEOM_DISK>(es, pairs, D, mu);
         fm_store<PI_GEOM_DISK>(mu, D.inv_norm, mo);
       } else {
         fm_stage<PI_GEOM_GAUSSIAN>(b, od, first, cnt, ctr, inv_s, reinterpret_cast<float*>(es));
-        fm_moments<PI_GEOM_GAUSSIAN>(es, pairs, D, mu);
+        m0 = fm_moments<PI_GEOM_GAUSSIAN>(es, pairs, D, mu);
         fm_store<PI_GEOM_GAUSSIAN>(mu, D.inv_norm, mo);
       }
       const df sc = cdot(D.dh, D.dl, make_float3(ctr.x, ctr.y, ctr.z));
       csc[warp * 32 + lane] = make_float2(sc.hi, sc.lo);
+      __syncwarp();  // the cluster's elements have been read: their place takes its zeroth moment
+      reinterpret_cast<float2*>(es)[lane] = m0;
       if (lane == 0) cscale_sm[warp] = s;
     }
     __syncthreads();
     const int nc = min(FM_WARPS, ncl - t0);
+    if (warp == FM_WARPS - 1) {
+      const float4 z = run0[lane];
+      kbsum s{z.x, z.z};
+      for (int c = 0; c < nc; ++c) {
+        const float2 v = reinterpret_cast<const float2*>(elem + c * FM_PAIRS * FM_PAIR_F4)[lane];
+        s.add(v.x);
+        s.lo += v.y;
+      }
+      run0[lane] = make_float4(s.hi, 0.f, s.lo, 0.f);
+    }
+    // Every cluster's value is its zeroth moment, the same at all radii and
+    // summed above, and the rest, which vanishes with k: e^{ik.c} enters less 1.
+    // A closed surface's form factor at small k is what the zeroth moments leave
+    // of each other, ~k of their size, and rounding each cluster's value (all
+    // its elements in phase) would leave ten times the error of rounding elements.
     for (int bt = warp; bt < nb; bt += FM_WARPS) {
       // compensated running sums: a cluster's value is as large as all its
       // elements' terms together, so plain partial sums would round coarsely
@@ -324,11 +355,11 @@ __device__ __forceinline__ void moment_body(const KGridDev& kg, const BatchDev& 
 #pragma unroll
         for (int p = 0; p < FM_R / 2; ++p) {
           const float4 kt = kx[bt * (FM_R / 2) + p];
-          const cf2 P = cis_tab_df2<FM_COPIES>(ctab, f2lo(kt), f2hi(kt), sh, sl);
+          const cf2 M = cis_tab_m1_df2<FM_COPIES>(ctab, f2lo(kt), f2hi(kt), sh, sl);
           const float2 k = mul2(kk[bt * (FM_R / 2) + p], s2), u = mul2(k, k);
-          const float2 x = horner8(a, u), y = mul2(k, horner8(bb, u));
-          kahan2(re[p], cre[p], fma2(P.re, x, neg2(mul2(P.im, y))));
-          kahan2(im[p], cim[p], fma2(P.re, y, mul2(P.im, x)));
+          const float2 xr = horner_rest(a, u), x = add2(xr, dup2(a[0])), y = mul2(k, horner8(bb, u));
+          kahan2(re[p], cre[p], fma2(M.re, x, fma2(neg2(M.im), y, xr)));
+          kahan2(im[p], cim[p], fma2(M.re, y, fma2(M.im, x, y)));
         }
       }
 #pragma unroll
@@ -343,6 +374,15 @@ __device__ __forceinline__ void moment_body(const KGridDev& kg, const BatchDev& 
   float m = 0.f;
   const double so = ((double)D.dh.x + (double)D.dl.x) * od.origin[0] + ((double)D.dh.y + (double)D.dl.y) * od.origin[1] +
                     ((double)D.dh.z + (double)D.dl.z) * od.origin[2];
+  kbsum zero{0.f, 0.f};  // the zeroth moments' sum, its product with 1/|d| split as well
+  for (int q = 0; q < S; ++q) {
+    const float4 v4 = (S > 1 ? cluster.map_shared_rank(run0, q) : run0)[lane];
+    zero.add(v4.x); zero.lo += v4.z;
+  }
+  {
+    const float p = zero.hi * D.inv_norm;
+    zero = kbsum{p, fmaf(zero.hi, D.inv_norm, -p) + zero.lo * D.inv_norm};
+  }
   for (int r = warp * S + rank; r < nr && active; r += FM_WARPS * S) {
     kbsum re{0.f, 0.f}, im{0.f, 0.f};  // over the cluster, in the order of the ranks
     for (int q = 0; q < S; ++q) {
@@ -350,6 +390,7 @@ __device__ __forceinline__ void moment_body(const KGridDev& kg, const BatchDev& 
       re.add(v4.x); im.add(v4.y);
       re.lo -= v4.z; im.lo -= v4.w;
     }
+    re.add(zero.hi); re.lo += zero.lo;
     cf v{re.hi + re.lo, im.hi + im.lo};
     const float2 km = kg.kmag[r];
     if (!SERVE) {

@@ -201,3 +201,28 @@ def test_serving_precision_of_disjoint_objects(cuda):
         worst.append(cond_rel_err(V, ((X @ X.T) / (8 * np.pi ** 3)).cpu().numpy()).max())
     print(f"\nserved disjoint objects: {worst}")
     assert np.mean(worst) <= 3e-5
+
+
+@pytest.mark.parametrize("kind", ["ico4", "cube", "cloud", "splat"])
+def test_each_small_radius_on_its_own(cuda, orc, kg64, kind):
+    """The form factors at every radius below k = 1, each against its own norm
+    (closed surfaces: A(k) ~ k, the elements' zeroth moments cancelling): the
+    2e-6 norm contract radius by radius, plus what the rounding of the
+    elements' own area vectors leaves (two FP32 roundings each, independent)."""
+    if kind == "ico4":
+        obj = G.SceneObject(G.make_triangle_mesh(*G.icosphere(4)), pg.DOF_AFFINE, G.affine_dofs(np.eye(3), [0.3, -0.2, 0.5]))
+    elif kind == "cube":
+        obj = shapes("cube", np.random.default_rng(0))
+    elif kind == "cloud":
+        obj = G.SceneObject(G.make_point_cloud(*G.create_sphere_pointcloud(3000)))
+    else:
+        obj = G.SceneObject(G.make_gaussian_splat(*G.create_sphere_gaussians(3000)))
+    L = 64
+    Jo = orc.form_factor_matrix(to_oracle(orc, [obj]), kg64.dirs, kg64.kmag)[:, 0].reshape(L, -1)
+    Jg = gpu_J(kg64, [obj])[0].reshape(L, -1)
+    k = kg64.kmag.reshape(L, -1)[:, 0]
+    n = obj.geom.num_elements()
+    inputs = 2.0 ** -23 * 4 * np.pi / np.sqrt(n) * np.sqrt(Jo.shape[1])  # sqrt(sum area^2) over the directions
+    err, tol = np.linalg.norm(Jg - Jo, axis=1), 2e-6 * np.linalg.norm(Jo, axis=1) + inputs
+    print(f"\n{kind}: worst radius {(err / tol)[k < 1].max():.2f} of the tolerance")
+    assert (err <= tol)[k < 1].all()
