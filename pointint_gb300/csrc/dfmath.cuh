@@ -280,6 +280,13 @@ struct cf2 { float2 re, im; };
 __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
 __device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
 
+// s += x with the compensation c (two sums at once).
+__device__ __forceinline__ void kahan2(float2& s, float2& c, float2 x) {
+  const float2 y = __fadd2_rn(x, neg2(c)), t = __fadd2_rn(s, y);
+  c = __fadd2_rn(__fadd2_rn(t, neg2(s)), neg2(y));
+  s = t;
+}
+
 // cis_tab_frac on both halves, the indices in the low bits of t.
 template <int C>
 __device__ __forceinline__ cf2 cis_tab_frac2(const float2* tab, float2 t, float2 f) {

@@ -525,13 +525,17 @@ constexpr int JM_F4_ELEM = JM_TILE * PI_CLUSTER / 2 * JM_PAIR_F4, JM_F4_MOM = JM
 constexpr int JM_SMEM = (JM_F4_ELEM + JM_F4_MOM + JM_F4_RUN) * (int)sizeof(float4);
 
 template <int HALF>
-__device__ __forceinline__ void jac_moments(const float4* es, int cnt, float3 d, float inv_norm, float4* mom) {
+__device__ __forceinline__ void jac_moments(const float4* es, int cnt, float3 d, float inv_norm, float4* mom,
+                                            kbsum (&zero)[4]) {
   constexpr int NS = HALF == 0 ? 4 : 2;  // sets of this warp: NF, W_x / W_y, W_z
   float2 mu[NS][MOMENT_TERMS];
 #pragma unroll
   for (int v = 0; v < NS; ++v)
 #pragma unroll
     for (int n = 0; n < MOMENT_TERMS; ++n) mu[v][n] = make_float2(0.f, 0.f);
+  float2 zc[NS];  // compensations of the zeroth moments
+#pragma unroll
+  for (int v = 0; v < NS; ++v) zc[v] = make_float2(0.f, 0.f);
   const float2 dx = dup2(d.x), dy = dup2(d.y), dz = dup2(d.z), in2 = dup2(inv_norm);
 #pragma unroll 1
   for (int i = 0; i < cnt; i += 2, es += JM_PAIR_F4) {
@@ -562,7 +566,14 @@ __device__ __forceinline__ void jac_moments(const float4* es, int cnt, float3 d,
         hc = __ffma2_rn(c, hc, hn);
       }
       const float2 hw = make_float2((float)(n + 3) * hn.x, (float)(n + 3) * hn.y);
-      if (HALF == 0) {
+      if (n == 0) {  // h's are 1
+#pragma unroll
+        for (int v = 0; v < NS; ++v) {
+          const int x = HALF == 0 ? 0 : v;
+          const float2 w3 = make_float2(3.f * w0[x].x, 3.f * w0[x].y);
+          kahan2(mu[v][0], zc[v], HALF == 0 && v < 3 ? N0[v] : __fadd2_rn(w3, __fadd2_rn(w1[x], w2[x])));
+        }
+      } else if (HALF == 0) {
 #pragma unroll
         for (int v = 0; v < 3; ++v) mu[v][n] = __ffma2_rn(N0[v], hn, mu[v][n]);
         mu[NS - 1][n] = __ffma2_rn(w0[0], hw, __ffma2_rn(w1[0], hb, __ffma2_rn(w2[0], hc, mu[NS - 1][n])));
@@ -572,6 +583,12 @@ __device__ __forceinline__ void jac_moments(const float4* es, int cnt, float3 d,
           mu[v][n] = __ffma2_rn(w0[v], hw, __ffma2_rn(w1[v], hb, __ffma2_rn(w2[v], hc, mu[v][n])));
       }
     }
+  }
+#pragma unroll
+  for (int v = 0; v < NS; ++v) {
+    zero[v].add(mu[v][0].x);
+    zero[v].add(mu[v][0].y);
+    zero[v].lo -= zc[v].x + zc[v].y;
   }
   constexpr FmConst<PI_GEOM_TRIANGLE> C{};  // 2/(n+2)!
 #pragma unroll
@@ -622,8 +639,12 @@ jac_moment_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, floa
     inv_norm = h.w;
     dnorm = l.w;
   }
-  stage_phasors<JAC_COPIES>(kg.cis_tab, ctab_sm);
+  stage_phasors<JAC_COPIES>(kg.cis_tabm, ctab_sm);
   const float2* ctab = ctab_sm + (threadIdx.x % JAC_COPIES);
+  // this warp's clusters' zeroth moments: they are the same at every radius, and
+  // what they leave of each other is a closed surface's value at small k
+  // (moments.cu), so they are summed apart and e^{ik.c} enters less 1
+  kbsum zero[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
   for (int t = threadIdx.x; t < JM_RADII; t += JM_THREADS) {
     const bool ok = t < nr;
     const float2 km = ok ? kg.kmag[r0 + t] : make_float2(0.f, 0.f), kt = ok ? kg.kt64[r0 + t] : make_float2(0.f, 0.f);
@@ -671,14 +692,14 @@ jac_moment_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, floa
       const float4* es = elem + (size_t)c_own * (PI_CLUSTER / 2) * JM_PAIR_F4;
       float4* mo = mom + c_own * JM_SETS * 4 * 32 + lane;
       if (warp & 1) {
-        jac_moments<1>(es, cnt, dh, inv_norm, mo);
+        jac_moments<1>(es, cnt, dh, inv_norm, mo, zero);
         const float4 ctr = b.clusters[od.cl_off + cl];
         const int ex = ctr.w > 0.f ? min(120, max(-100, ilogbf(ctr.w) + 1)) : 0;
         const df sc = cdot(dh, dl, make_float3(ctr.x, ctr.y, ctr.z));
         csc[c_own][lane] = make_float2(sc.hi, sc.lo);
         if (lane == 0) cscale[c_own] = __int_as_float((127 + ex) << 23);
       } else {
-        jac_moments<0>(es, cnt, dh, inv_norm, mo);
+        jac_moments<0>(es, cnt, dh, inv_norm, mo, zero);
       }
     }
     __syncthreads();
@@ -693,12 +714,12 @@ jac_moment_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, floa
       for (int c = 0; c < nc; ++c) {
         const float2 sc = csc[c][lane];
         const float s = cscale[c];
-        cf P[JM_R];
+        cf M[JM_R];
         float k[JM_R];
 #pragma unroll
         for (int i = 0; i < JM_R; ++i) {
           const float4 kr = krad[rb + i];
-          P[i] = cis_tab_df<JAC_COPIES>(ctab, make_float2(kr.y, kr.z), df{sc.x, sc.y});
+          M[i] = cis_tab_m1_df<JAC_COPIES>(ctab, make_float2(kr.y, kr.z), df{sc.x, sc.y});
           k[i] = kr.x * s;
         }
 #pragma unroll
@@ -708,10 +729,11 @@ jac_moment_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, floa
 #pragma unroll
           for (int i = 0; i < JM_R; ++i) {
             const float u = k[i] * k[i];
-            const float x = fmaf(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, m1.w, m1.z), m1.y), m1.x), m0.w), m0.z), m0.y), m0.x);
+            const float xr = u * fmaf(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, m1.w, m1.z), m1.y), m1.x), m0.w), m0.z), m0.y);
+            const float x = xr + m0.x;
             const float y = k[i] * fmaf(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, fmaf(u, m3.w, m3.z), m3.y), m3.x), m2.w), m2.z), m2.y), m2.x);
-            acc[i][2 * v] = fmaf(P[i].re, x, fmaf(-P[i].im, y, acc[i][2 * v]));
-            acc[i][2 * v + 1] = fmaf(P[i].re, y, fmaf(P[i].im, x, acc[i][2 * v + 1]));
+            acc[i][2 * v] += fmaf(M[i].re, x, fmaf(-M[i].im, y, xr));
+            acc[i][2 * v + 1] += fmaf(M[i].re, y, fmaf(M[i].im, x, y));
           }
         }
       }
@@ -726,10 +748,29 @@ jac_moment_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, floa
         }
     }
   }
+  __syncthreads();  // the last tile's elements have been read: their place takes the zeroth moments
+  float2* zs = reinterpret_cast<float2*>(elem);  // [cluster of the tile][set][lane]
+#pragma unroll
+  for (int v = 0; v < 4; ++v)
+    if ((warp & 1) == 0 || v < 2)
+      zs[((warp >> 1) * JM_SETS + 4 * (warp & 1) + v) * 32 + lane] = make_float2(zero[v].hi, zero[v].lo);
   if (S > 1) cluster.sync();
   else __syncthreads();
   if (active) {
     const JacWriter w(jo, od, dh, dl, inv_norm, dnorm, j, jm);
+    kbsum zt[JM_SETS];
+#pragma unroll
+    for (int v = 0; v < JM_SETS; ++v) {
+      zt[v] = kbsum{0.f, 0.f};
+      for (int q = 0; q < S * JM_TILE; ++q) {
+        const float2* o = S > 1 ? cluster.map_shared_rank(zs, q / JM_TILE) : zs;
+        const float2 z = o[((q % JM_TILE) * JM_SETS + v) * 32 + lane];
+        zt[v].add(z.x);
+        zt[v].lo += z.y;
+      }
+      const float f = v < 3 ? -0.5f : -1.0f / 6.0f, p = zt[v].hi * f;  // i^2 / 2!, i^2 / 3!
+      zt[v] = kbsum{p, fmaf(zt[v].hi, f, -p) + zt[v].lo * f};
+    }
     for (int r = warp * S + rank; r < nr; r += JM_WARPS * S) {
       float sv[JAC_NSUM];
 #pragma unroll
@@ -739,6 +780,10 @@ jac_moment_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, floa
           const float* o = (S > 1 ? cluster.map_shared_rank(run, q) : run) + (r * 2 * JAC_NSUM + 2 * v) * 32 + lane;
           t.add(o[0]);
           t.lo -= o[32];
+        }
+        if ((v & 1) == 0) {
+          t.add(zt[v / 2].hi);
+          t.lo += zt[v / 2].lo;
         }
         sv[v] = t.hi + t.lo;
       }

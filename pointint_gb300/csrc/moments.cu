@@ -72,13 +72,6 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 
-// s += x with the compensation c (two sums at once).
-__device__ __forceinline__ void kahan2(float2& s, float2& c, float2 x) {
-  const float2 y = add2(x, neg2(c)), t = add2(s, y);
-  c = add2(add2(t, neg2(s)), neg2(y));
-  s = t;
-}
-
 struct FmDir {
   float3 dh, dl;
   float inv_norm;

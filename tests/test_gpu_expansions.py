@@ -226,3 +226,18 @@ def test_each_small_radius_on_its_own(cuda, orc, kg64, kind):
     err, tol = np.linalg.norm(Jg - Jo, axis=1), 2e-6 * np.linalg.norm(Jo, axis=1) + inputs
     print(f"\n{kind}: worst radius {(err / tol)[k < 1].max():.2f} of the tolerance")
     assert (err <= tol)[k < 1].all()
+
+
+def test_jacobian_translation_rows_at_each_small_radius(cuda, orc, kg64):
+    """dA/dt = i k A radius by radius below k = 1, to the tolerance of the form
+    factors above times k."""
+    obj = G.SceneObject(G.make_triangle_mesh(*G.icosphere(4)), pg.DOF_AFFINE,
+                        G.affine_dofs(np.diag([1.4, 0.9, 0.6]), [0.3, -0.2, 0.5]))
+    L = 64
+    got = core.dof_jacobian(kg64, core.ObjectBatch([obj])).cpu().numpy()[:3] / np.sqrt(kg64.w)
+    Jo = orc.form_factor_matrix(to_oracle(orc, [obj]), kg64.dirs, kg64.kmag)[:, 0]
+    ref = 1j * (kg64.dirs * kg64.kmag[:, None]).T * Jo
+    k = kg64.kmag.reshape(L, -1)[:, 0]
+    norm = lambda x: np.linalg.norm(x.reshape(3, L, -1), axis=(0, 2))
+    inputs = 2.0 ** -23 * 4 * np.pi * 1.4 * 0.9 / np.sqrt(5120) * np.sqrt(Jo.size / L) * k
+    assert (norm(got - ref) <= 2e-6 * norm(ref) + inputs)[k < 1].all()
