@@ -418,7 +418,9 @@ __device__ __forceinline__ cf tri_series_eval(const TriPoly2& t, float u, float 
   return {a.x, k3 * a.y};
 }
 
-// The coefficients that tri_series_eval_short reads (a[0..3], b[0..2]) alone.
+// The series cut after a[3] and b[2], for k |e|max < 1 (|e|max the longest
+// edge, so k sp < 1): the dropped terms stay below 6.2e-9 of |a[0]| (FP64
+// evaluation over icosphere and box triangles at the bound).
 struct TriPolyShort { float a[4], b[3]; };
 
 __device__ __forceinline__ TriPolyShort tri_series_coeffs_short(float s1, float s2, float g) {
@@ -441,20 +443,10 @@ __device__ __forceinline__ TriPolyShort tri_series_coeffs_short(float s1, float 
   return t;
 }
 
-// tri_series_eval_short for two radii (u = k^2, k3 = k^3 per half) with packed FP32.
+// It for two radii (u = k^2, k3 = k^3 per half) with packed FP32.
 __device__ __forceinline__ cf2 tri_series_eval_short2(const TriPolyShort& t, float2 u, float2 k3) {
   const float2 re = __ffma2_rn(u, __ffma2_rn(u, __ffma2_rn(u, dup2(t.a[3]), dup2(t.a[2])), dup2(t.a[1])), dup2(t.a[0]));
   const float2 im = __fmul2_rn(k3, __ffma2_rn(u, __ffma2_rn(u, dup2(t.b[2]), dup2(t.b[1])), dup2(t.b[0])));
-  return {re, im};
-}
-
-// The same series cut after a[3] and b[2], for k |e|max < 1 (|e|max the longest
-// edge, so k sp < 1): the dropped terms stay below 6.2e-9 of |a[0]| (FP64
-// evaluation over icosphere and box triangles at the bound).
-template <class Poly>
-__device__ __forceinline__ cf tri_series_eval_short(const Poly& t, float u, float k3) {
-  const float re = fmaf(u, fmaf(u, fmaf(u, t.a[3], t.a[2]), t.a[1]), t.a[0]);
-  const float im = k3 * fmaf(u, fmaf(u, t.b[2], t.b[1]), t.b[0]);
   return {re, im};
 }
 
@@ -518,8 +510,7 @@ __device__ __forceinline__ cf tri_wide(const float2* tabm, float kt, const TriGa
   return {gik * fmaf(M1.re, t.i1, M2.re * t.i2), gik * fmaf(M1.im, t.i1, -M2.im * t.i2)};
 }
 
-// tri_generic: spread D >= 2 (the form-factor kernel takes it for D >= 3,
-// the adjoint's tri_generic_der for D >= 2).
+// tri_generic: spread D >= 2 (the Jacobian's tri_generic_der).
 // e[u, v, w] = (f[v, w] - f[u, v]) / (w - u) with (u, v) the pair of
 // vertices with the smallest gap.  The two gaps to w
 // are then the middle one and D, both at least D / 2 >= 1, so f[v, w] takes

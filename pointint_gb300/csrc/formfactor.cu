@@ -9,11 +9,17 @@
 //    its AffineDoF / TriangleMeshDoF into an FP32 object-local frame (origin =
 //    centroid of the transformed anchors), centroids (centres) as FP32 hi + lo;
 //    the origin phase e^{ik.o} is formed and reduced in FP64 per output.
-//  * ff_kernel: one CTA = one object x 4 warps; a warp owns 32 directions
+//  * ff_kernel: the radii that the cluster expansions (moments.cu) leave, about
+//    the six largest of 64 (all of them on grids the expansions do not take).
+//    One CTA = one object x 4 warps; a warp owns 32 directions
 //    (one per lane) x R neighbouring radial nodes of the factored k-grid, so
 //    each element's direction dot products and series coefficients are
 //    formed once and reused for R radii; where all R radii take the short
-//    series, two radii share each packed FP32 instruction.  On a centrally
+//    series, two radii share each packed FP32 instruction; leaves of four
+//    triangles have expansions of their own.  The CTAs of a thread-block
+//    cluster split the elements where few objects would leave SMs idle.
+//    Bound by instruction issue (63-70% active; 256 solids of 5,120 and 12
+//    triangles at N_k = 76,928: 38.8 ms for all radii, 12.2 now).  On a centrally
 //    symmetric direction set a lane evaluates one direction of an antipodal
 //    pair and writes both (A(-k) = -conj A(k) for a real solid: half the
 //    evaluations), and a warp's 32 directions form a compact cluster.  Radial
@@ -560,8 +566,8 @@ static_assert(FF_TILE % FF_CHUNK == 0, "element chunks must not straddle tiles")
 // sum, so rounding does not grow with the element count (a plain FP32 sum over
 // 1,280 triangles measured ~1e-6 of max|A| per node).  The partials live in
 // registers; the running sums and compensations live in shared memory, where
-// they are touched once per FF_CHUNK elements, which leaves the registers for
-// five CTAs per SM.
+// they are touched once per FF_CHUNK elements, which leaves the registers to
+// the element loop.
 // A float4 from shared memory, loaded where it is written in the source: the
 // element loop reads its radius constants each time instead of keeping them
 // in registers across the loop.

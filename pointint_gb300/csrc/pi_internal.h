@@ -145,7 +145,7 @@ struct BatchDev {
 // One form-factor evaluation of the serving path: library object `obj`,
 // optionally rotated (its form factors at k are the unrotated object's at
 // R^T k), written in the object-local frame (no origin phase) and
-// direction-major over the evaluated directions (column e * L + r) to dst,
+// direction-major over the evaluated directions (column ecol[e] * L + r) to dst,
 // scaled by the square root of the weight of the node and its antipode
 // together: Re(conj A_i A_j) is the same at k and -k, so half the grid's columns
 // give the whole volume; the largest |Re|, |Im| goes

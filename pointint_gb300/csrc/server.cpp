@@ -7,8 +7,9 @@
 //
 //  * the library (elements + DoFs of every object a query may name) is
 //    uploaded and prepared once, in each object's local frame;
-//  * a pool of rows in HBM holds local-frame, direction-major, sqrt|w|-scaled
-//    form factors: canonical rows (the object unrotated) stay resident under
+//  * a pool of rows in HBM holds local-frame, direction-major form factors of
+//    one direction of each antipodal pair, scaled by the root of the pair's
+//    weights: canonical rows (the object unrotated) stay resident under
 //    an LRU policy within the HBM budget; a rotated object gets a row owned by
 //    its batch (its form factors at R^T k);
 //  * a translation never touches form factors: the contraction applies
@@ -20,8 +21,9 @@
 //  * each batch is one graph launch on its slot's stream: descriptor upload,
 //    form factors of the batch's new rows, the persistent tensor-core
 //    contraction over every query of the batch, the split-K reduction, download
-//    of results and row maxima.  Only the copy sizes, the form-factor grid and
-//    whether that node runs change between launches of a slot's graph.
+//    of results and row maxima.  A slot has two graphs, with and without
+//    form-factor nodes; only the copy sizes and those nodes' grids change
+//    between their launches.
 //
 // A query's work items, k-chunk assignment and reduction order depend only on
 // the query itself (its size and the autotuned items-per-SM of its size

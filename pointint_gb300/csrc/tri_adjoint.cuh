@@ -194,7 +194,7 @@ __device__ __forceinline__ TriDer tri_generic_der(cf Pa, cf Pb, cf Pc, float al,
 // series outgrows the instruction cache (the loop then stalls on instruction
 // fetch), while the call costs little on the few nodes that take it.
 // The vertex phasors come from the phasor table (cis_tab_df): tab is the
-// 256-entry table, kt the radius in 1/64 turns per unit length.
+// phasor table, kt the radius in 1/64 turns per unit length.
 template <int C>
 static __device__ __noinline__ TriDer tri_generic_der_at(const float2* tab, float2 kt, df sa, df sb, df sc, float al,
                                                          float be) {
