@@ -131,17 +131,24 @@ cotangent_kernel(KGridDev kg, BatchDev b, const float2* __restrict__ Jw, const f
 struct AdjWork { int32_t obj, first; };
 
 // A CTA's elements are ADJ_THREADS consecutive pool entries of one object:
-// whole clusters (moments.cu), whose radii [0, nr) with k rho below the bound
-// enter through the cluster's expansion.  The cotangent of a direction then
-// becomes, for each cluster (centre c, k in units of 1/s),
+// whole patches, whose radii [0, nr) with k rho below the bound enter through
+// the patch's expansion (moments.cu).  The cotangent of a direction then
+// becomes, for each patch (centre c, k in units of 1/s),
 //   beta_m = Re( i^m sum_r conj(Bt_r) e^{i k_r d.c} k_r^m ),   m < ADJ_TERMS,
 // 16 real numbers that all its elements share, and an element's contribution
 // and its derivatives are sums of beta_m times the moments of moments.cu and
 // their derivatives: ~150 FP32 operations per element and direction for all
-// those radii instead of ~70 for each.
+// those radii instead of ~70 for each.  (24 bodies, N_k = 76,928: adj_tri_kernel
+// 13.7 -> 3.94 ms; eight clouds of 50,000 disks: adj_surf_kernel 43.8 -> 8.25.)
 constexpr int ADJ_TERMS = MOMENT_TERMS;
-constexpr int ADJ_CL = ADJ_THREADS / PI_CLUSTER;  // clusters per CTA
-static_assert(ADJ_THREADS % PI_CLUSTER == 0 && PI_CLUSTER % 32 == 0, "a warp's elements share a cluster");
+// Patches of half a cluster (a warp's elements): the expansions reach 1.4 times
+// the k.  A quarter reaches twice the k but its betas, every covered radius for
+// every patch and direction, cost more than the radii they save (eight clouds
+// 10.2 ms, 24 bodies 4.21).
+constexpr int ADJ_PATCH = PI_CLUSTER / 2;
+constexpr int ADJ_CL = ADJ_THREADS / ADJ_PATCH;  // patches per CTA
+static_assert(ADJ_PATCH % PI_LEAF == 0 && 4 * ADJ_CL * ADJ_DT == ADJ_THREADS, "four threads per patch and direction");
+static_assert(ADJ_TERMS == 16, "eight orders per thread");
 // Bounds on k rho: the derivatives drop one (centres, vertices) or two (normals)
 // orders earlier than the values.  What is dropped, relative to the leading
 // term, of a small element on the rim seen along its offset (x^15 / 15!, x^14 /
@@ -237,7 +244,8 @@ struct AdjStage {
   float4 dh[ADJ_DT], dl[ADJ_DT];
   float4 va[ADJ_DT];                          // v = A^T dir and qd = |v|^2 (disks/Gaussians: k' = |k| v)
   float beta[ADJ_DT][ADJ_CL][ADJ_TERMS];
-  float4 ctr[ADJ_CL];                         // cluster centre and scale s
+  float4 ctr[ADJ_CL];                         // patch centre and scale s (one for the CTA)
+  float4 pw[2 * ADJ_LMAX];                    // (k s)^0, ^2, .. ^14 of each covered radius
   float2 km[ADJ_LMAX], kt[ADJ_LMAX], ctab[PHASOR_ENTRIES * ADJ_COPIES], ctabm[PHASOR_ENTRIES * ADJ_COPIES];
   int nr;
 };
@@ -252,29 +260,44 @@ __device__ __forceinline__ void adj_setup(AdjStage& st, const KGridDev& kg, cons
   stage_phasors<ADJ_COPIES>(kg.cis_tab, st.ctab);
   stage_phasors<ADJ_COPIES>(kg.cis_tabm, st.ctabm);
   if (threadIdx.x < 32) {
-    float rho = 0.f;
-    for (int c = 0; c < ADJ_CL; ++c) {
-      if (first + c * PI_CLUSTER >= od.n_elems) continue;
-      const float4 cl = b.clusters[od.cl_off + first / PI_CLUSTER + c];
-      const int ex = cl.w > 0.f ? min(120, max(-100, ilogbf(cl.w) + 1)) : 0;
-      if (threadIdx.x == 0) st.ctr[c] = make_float4(cl.x, cl.y, cl.z, __int_as_float((127 + ex) << 23));
-      rho = cl.w > rho || !(cl.w == cl.w) ? cl.w : rho;
-    }
-    const float bound = od.type == PI_GEOM_TRIANGLE ? ADJ_X_TRI : ADJ_X_SURF;
-    int n = 0;
-    if (kg.moments)
-      for (int r0 = 0; r0 < kg.L; r0 += 32) {
-        const int r = r0 + (int)threadIdx.x;
-        n += __popc(__ballot_sync(0xffffffffu, r < kg.L && kg.kmag[r].x * rho <= bound));
+    // a patch's sphere from its leaves'
+    const int lane = threadIdx.x, p0 = first + lane * ADJ_PATCH;
+    float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (lane < ADJ_CL && p0 < od.n_elems) {
+      const float4* leaf = b.leaves + od.cl_off * (PI_CLUSTER / PI_LEAF) + p0 / PI_LEAF;
+      const int nl = min(ADJ_PATCH, od.n_elems - p0 + PI_LEAF - 1) / PI_LEAF;
+      for (int l = 0; l < nl; ++l) { c.x += leaf[l].x; c.y += leaf[l].y; c.z += leaf[l].z; }
+      const float inv = 1.0f / nl;
+      c = make_float4(c.x * inv, c.y * inv, c.z * inv, 0.f);
+      for (int l = 0; l < nl; ++l) {
+        const float dx = leaf[l].x - c.x, dy = leaf[l].y - c.y, dz = leaf[l].z - c.z;
+        const float reach = sqrtf(dx * dx + dy * dy + dz * dz) * 1.000001f + leaf[l].w;
+        c.w = reach > c.w || !(reach == reach) ? reach : c.w;
       }
-    if (threadIdx.x == 0) st.nr = n;
+    }
+    float rho = c.w;  // of all patches; NaN stays
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+      const float o = __shfl_xor_sync(0xffffffffu, rho, w);
+      rho = o > rho || !(o == o) ? o : rho;
+    }
+    const int ex = rho > 0.f ? min(120, max(-100, ilogbf(rho) + 1)) : 0;
+    if (lane < ADJ_CL) st.ctr[lane] = make_float4(c.x, c.y, c.z, __int_as_float((127 + ex) << 23));
+    const int n = covered_radii(kg, rho, od.type == PI_GEOM_TRIANGLE ? ADJ_X_TRI : ADJ_X_SURF);
+    if (lane == 0) st.nr = n;
+  }
+  __syncthreads();
+  for (int r = threadIdx.x; r < st.nr; r += blockDim.x) {
+    const float k = st.km[r].x * st.ctr[0].w, u = k * k, u2 = u * u, u4 = u2 * u2;
+    st.pw[2 * r] = make_float4(1.f, u, u2, u2 * u);
+    st.pw[2 * r + 1] = make_float4(u4, u4 * u, u4 * u2, u4 * u2 * u);
   }
 }
 
 // Stages the cotangent and directions of the tile at e0, then the betas.
 __device__ __forceinline__ void stage_tile(AdjStage& st, const KGridDev& kg, const ObjDev& od, const float2* Bt_obj,
                                            int n_cl, int e0) {
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
   const int jn = min(ADJ_DT, kg.Me - e0);
   if (tid < ADJ_DT) {
     float4 h = make_float4(0.f, 0.f, 0.f, 0.f), l = h;
@@ -293,41 +316,38 @@ __device__ __forceinline__ void stage_tile(AdjStage& st, const KGridDev& kg, con
   __syncthreads();
   const int nr = st.nr;
   if (nr > 0) {
-    for (int w = warp; w < jn * n_cl; w += ADJ_THREADS / 32) {
-      const int jj = w / n_cl, c = w - jj * n_cl;
+    // four threads per patch and direction: the even and the odd orders, of every
+    // other pair of radii; the two of a pair each form one radius's term and hand
+    // the other its half
+    const int jj = tid / (4 * ADJ_CL), c = tid / 4 % ADJ_CL, odd = tid & 1;
+    if (jj < jn && c < n_cl) {
+      const unsigned quad = 15u << (lane & ~3);
       const float4 h = st.dh[jj], l = st.dl[jj], ct = st.ctr[c];
       const df sc = cdot(make_float3(h.x, h.y, h.z), make_float3(l.x, l.y, l.z), make_float3(ct.x, ct.y, ct.z));
-      float p[ADJ_TERMS];  // sums over this lane's radii of Re, Im alternately of conj(B) e^{i k d.c} k^m
+      const float2* Bj = st.B + jj * ADJ_LMAX;
+      float p[ADJ_TERMS / 2];
 #pragma unroll
-      for (int m = 0; m < ADJ_TERMS; ++m) p[m] = 0.f;
-      for (int r = lane; r < nr; r += 32) {
-        const float2 Bv = st.B[jj * ADJ_LMAX + r];
+      for (int m = 0; m < ADJ_TERMS / 2; ++m) p[m] = 0.f;
+      for (int s0 = 0; s0 < nr; s0 += 4) {
+        const int ra = s0 + (tid & 2), r0 = min(ra, nr - 1), r = min(ra + odd, nr - 1), r1 = min(ra + 1, nr - 1);
+        const float2 Bv = Bj[r];
         const cf P = cis_tab_df<ADJ_COPIES>(st.ctab, st.kt[r], sc);
-        const float k = st.km[r].x * ct.w, u = k * k;
-        float zr = fmaf(Bv.x, P.re, Bv.y * P.im), zi = k * fmaf(Bv.x, P.im, -Bv.y * P.re);
-#pragma unroll
-        for (int m = 0; m < ADJ_TERMS; m += 2) {
-          p[m] += zr;
-          p[m + 1] += zi;
-          zr *= u;
-          zi *= u;
-        }
+        const float keep = ra + odd < nr ? 1.f : 0.f;
+        const float zr = keep * fmaf(Bv.x, P.re, Bv.y * P.im), zi = keep * (st.km[r].x * ct.w) * fmaf(Bv.x, P.im, -Bv.y * P.re);
+        const float got = __shfl_xor_sync(quad, odd ? zr : zi, 1);
+        const float za = odd ? got : zr, zb = odd ? zi : got;  // of radii r0 and r1
+        const float4 a0 = st.pw[2 * r0], a1 = st.pw[2 * r0 + 1], b0 = st.pw[2 * r1], b1 = st.pw[2 * r1 + 1];
+        p[0] = fmaf(za, a0.x, fmaf(zb, b0.x, p[0])); p[1] = fmaf(za, a0.y, fmaf(zb, b0.y, p[1]));
+        p[2] = fmaf(za, a0.z, fmaf(zb, b0.z, p[2])); p[3] = fmaf(za, a0.w, fmaf(zb, b0.w, p[3]));
+        p[4] = fmaf(za, a1.x, fmaf(zb, b1.x, p[4])); p[5] = fmaf(za, a1.y, fmaf(zb, b1.y, p[5]));
+        p[6] = fmaf(za, a1.z, fmaf(zb, b1.z, p[6])); p[7] = fmaf(za, a1.w, fmaf(zb, b1.w, p[7]));
       }
-      // sum over the lanes, each step halving the values a lane carries: in
-      // the end lanes l and l ^ 1 hold value m = l / 2
-#pragma unroll
-      for (int w2 = 16, cnt = ADJ_TERMS; w2 >= 2; w2 >>= 1, cnt >>= 1) {
-        const bool up = (lane & w2) != 0;
-#pragma unroll
-        for (int i = 0; i < cnt / 2; ++i) {
-          const float give = up ? p[i] : p[i + cnt / 2], keep = up ? p[i + cnt / 2] : p[i];
-          p[i] = keep + __shfl_xor_sync(0xffffffffu, give, w2);
-        }
-      }
-      p[0] += __shfl_xor_sync(0xffffffffu, p[0], 1);
-      const int m = lane >> 1;
       // Re(i^m z): z's real part for even m, minus its imaginary part for odd m, with the sign of i^(m - m mod 2)
-      if ((lane & 1) == 0) st.beta[jj][c][m] = ((m + 1) & 2) ? -p[0] : p[0];
+#pragma unroll
+      for (int j = 0; j < ADJ_TERMS / 2; ++j) {
+        p[j] += __shfl_xor_sync(quad, p[j], 2);
+        if ((tid & 2) == 0) st.beta[jj][c][2 * j + odd] = ((2 * j + odd + 1) & 2) ? -p[j] : p[j];
+      }
     }
     __syncthreads();
   }
@@ -396,8 +416,8 @@ adj_surf_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const
   const bool disk = od.type == PI_GEOM_DISK;
   adj_setup(st, kg, b, od, wk.first);
   __syncthreads();
-  const int nr = st.nr, n_cl = min(ADJ_CL, (od.n_elems - wk.first + PI_CLUSTER - 1) / PI_CLUSTER);
-  const int cl = threadIdx.x / PI_CLUSTER;
+  const int nr = st.nr, n_cl = min(ADJ_CL, (od.n_elems - wk.first + ADJ_PATCH - 1) / ADJ_PATCH);
+  const int cl = threadIdx.x / ADJ_PATCH;
   float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0, ql = q0, nr4 = q0;
   if (valid) {
     q0 = b.surf_pool[2 * (od.elem_off + e)];
@@ -526,8 +546,8 @@ adj_tri_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const 
   const bool valid = e < od.n_elems;
   adj_setup(st, kg, b, od, wk.first);
   __syncthreads();
-  const int nr = st.nr, n_cl = min(ADJ_CL, (od.n_elems - wk.first + PI_CLUSTER - 1) / PI_CLUSTER);
-  const int cl = threadIdx.x / PI_CLUSTER;
+  const int nr = st.nr, n_cl = min(ADJ_CL, (od.n_elems - wk.first + ADJ_PATCH - 1) / ADJ_PATCH);
+  const int cl = threadIdx.x / ADJ_PATCH;
   float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0, q2 = q0, ql = q0;
   if (valid) {
     q0 = b.tri_pool[3 * (od.elem_off + e)];
