@@ -299,8 +299,10 @@ void bisect_order(OrderPoint* p, int64_t n) {
     std::nth_element(p, p + mid, p + n, [ax](const OrderPoint& a, const OrderPoint& b) {
       return a.x[ax] < b.x[ax] || (a.x[ax] == b.x[ax] && a.id < b.id);
     });
+    // (a thread for every part down to one segment cost more to start than it
+    // saved: a batch of one solid of 200,000 triangles 18 ms, 12 with this bound)
     bool handed = false;
-    try {
+    if (mid > 4 * ORDER_SEGMENT) try {
       parts.push_back(std::async(std::launch::async, bisect_order, p, mid));
       handed = true;
     } catch (const std::system_error&) {  // no thread to be had: this one does it
@@ -603,11 +605,29 @@ int batch_create_impl(const pi_object* objs, int n, int on_device, cudaStream_t 
     }
   }
   std::vector<int32_t> perm;  // the host's part of the orders, uploaded before the device's
-  for (int i : ordered)
-    if (b->info[i].n_elems > ORDER_SEGMENT) {
-      perm.resize((size_t)n_perm);
-      order_large(objs[i], perm.data() + b->info[i].perm_off);
+  try {
+    std::vector<int> large;
+    for (int i : ordered) if (b->info[i].n_elems > ORDER_SEGMENT) large.push_back(i);
+    if (!large.empty()) perm.resize((size_t)n_perm);
+    // a few objects at a time (their own cuts take threads too); eight clouds of
+    // 50,000 points added 12 ms one after another
+    for (size_t at = 0; at < large.size(); at += 8) {
+      std::vector<std::future<void>> jobs;
+      for (size_t t = at; t < std::min(large.size(), at + 8); ++t) {
+        const int i = large[t];
+        int32_t* dst = perm.data() + b->info[i].perm_off;
+        const pi_object* obj = objs + i;
+        try {
+          jobs.push_back(std::async(std::launch::async, [obj, dst] { order_large(*obj, dst); }));
+        } catch (const std::system_error&) {  // no thread to be had: this one does it
+          order_large(*obj, dst);
+        }
+      }
+      for (std::future<void>& f : jobs) f.get();
     }
+  } catch (const std::bad_alloc&) {
+    return fail(PI_ERR_OUT_OF_MEMORY, "pi_batch_create: no host memory for the element order");
+  }
   b->order.resize(n);
   std::iota(b->order.begin(), b->order.end(), 0);
   std::stable_sort(b->order.begin(), b->order.end(),
