@@ -58,8 +58,15 @@ enum { JAC_AFFINE_TRI = 0, JAC_AFFINE_SURF = 1, JAC_MESH_TRI = 2 };
 // Radii that the expansions cover (as moment_radii): the n-th term of the
 // derivatives' series is at most (k rho)^n / n! of the leading one, as the values'.
 constexpr float JAC_X_TRI = MOMENT_X_TRI;
-__device__ __forceinline__ int jac_moment_radii(const KGridDev& kg, float rho) {
-  return covered_radii(kg, rho, JAC_X_TRI);
+constexpr int JM_RADII = 48;  // radii of a CTA of jac_moment_kernel: its running sums fill shared memory
+// Few radii over a multiple of that go to the direct kernel where its threads own
+// four radii: they cost it less than another group of CTAs that forms all moments
+// again (256 solids 70.2 -> 65.7 ms).  At two radii per thread they cost more (one
+// mesh 0.98 -> 1.06 ms).
+constexpr int JM_SPARE = 4;
+__device__ __forceinline__ int jac_moment_radii(const KGridDev& kg, float rho, int spare) {
+  const int n = covered_radii(kg, rho, JAC_X_TRI), over = n % JM_RADII;
+  return n > JM_RADII && over <= spare ? n - over : n;
 }
 
 struct JacObj {
@@ -330,7 +337,7 @@ jac_affine_tri_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, 
   const int slot = (int)(lin % gridDim.y), cta = (int)(lin / gridDim.y);
   const JacObj jo = jobs[slot];
   const ObjDev od = b.objs[jo.obj];
-  const int r_first = jac_moment_radii(kg, __uint_as_float(b.cl_rho[jo.obj]));
+  const int r_first = jac_moment_radii(kg, __uint_as_float(b.cl_rho[jo.obj]), R == 4 ? JM_SPARE : 0);
   const int nrb = (kg.L - r_first + R - 1) / R, ndt = (kg.Me + 31) / 32;
   if (cta * JAC_WARPS >= ndt * nrb) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -514,7 +521,8 @@ jac_affine_tri_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, 
 // sum takes ~190 for each), then each warp sums the tile over its own radii,
 // JM_R at a time.  The CTAs of a thread-block cluster split the tiles.
 constexpr int JM_WARPS = 8, JM_THREADS = 32 * JM_WARPS, JM_TILE = JM_WARPS / 2;
-constexpr int JM_SETS = JAC_NSUM / 2, JM_R = 3, JM_RADII = 2 * JM_R * JM_WARPS;
+constexpr int JM_SETS = JAC_NSUM / 2, JM_R = 3;
+static_assert(JM_RADII == 2 * JM_R * JM_WARPS, "two batches of radii per warp");
 // staged element pairs, as float4: vertices, S, N0, a0, E1, E2 (24 values of
 // two elements, and one float4 that spreads the pairs over the banks)
 constexpr int JM_PAIR_F4 = 13;
@@ -606,7 +614,8 @@ __device__ __forceinline__ void jac_moments(const float4* es, int cnt, float3 d,
 }
 
 __global__ void __launch_bounds__(JM_THREADS, 1)
-jac_moment_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, float2* __restrict__ G, int groups) {
+jac_moment_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, float2* __restrict__ G, int groups,
+                  int spare) {
   extern __shared__ float4 jsm[];
   float4* elem = jsm;
   float4* mom = elem + JM_F4_ELEM;
@@ -621,7 +630,7 @@ jac_moment_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, floa
   const int dt = item / groups, r0 = (item - dt * groups) * JM_RADII;
   const JacObj jo = jobs[slot];
   const ObjDev od = b.objs[jo.obj];
-  const int nr = min(JM_RADII, jac_moment_radii(kg, __uint_as_float(b.cl_rho[jo.obj])) - r0);  // radii r0 .. r0 + nr - 1
+  const int nr = min(JM_RADII, jac_moment_radii(kg, __uint_as_float(b.cl_rho[jo.obj]), spare) - r0);  // radii r0 .. r0 + nr - 1
   if (nr <= 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ei = dt * 32 + lane;
@@ -1011,7 +1020,8 @@ int launch_jacobian(const pi_kgrid_impl* kg, const pi_batch_impl* b, float2* G, 
       int groups = (K.L + JM_RADII - 1) / JM_RADII;
       int SM = 1;  // one CTA per SM
       while (SM < 8 && (int64_t)SM * ndt * heavy < 2 * (int64_t)n_sm && n_max > SM * JM_TILE * PI_CLUSTER) SM *= 2;
-      void* margs[5] = {const_cast<KGridDev*>(&K), const_cast<BatchDev*>(&B), &d, &G, &groups};
+      int spare = R == 4 ? JM_SPARE : 0;  // as the direct kernel
+      void* margs[6] = {const_cast<KGridDev*>(&K), const_cast<BatchDev*>(&B), &d, &G, &groups, &spare};
       rc = launch_split(fn, dim3((unsigned)(ndt * groups * SM), (unsigned)tri.size()), JM_THREADS, (size_t)JM_SMEM, SM,
                         margs, s);
       if (rc) return rc;
