@@ -47,7 +47,7 @@ constexpr int ADJ_DT = 8;        // directions staged per shared-memory tile
 constexpr int ADJ_LMAX = 256;    // radii per direction held in shared memory
 // one copy of the phasor table: the lanes of a warp hold neighbouring elements
 // at one direction and radius, whose phases mostly share an entry (a broadcast);
-// eight copies, one a lane group, took 7% longer (4.43 against 4.13 ms for 24 spheres)
+// eight copies, one a lane group, took 7% longer (4.43 against 4.13 ms for 24 bodies)
 constexpr int ADJ_COPIES = 1;
 constexpr double INV8PI3 = 1.0 / (8.0 * 3.14159265358979323846 * 3.14159265358979323846 * 3.14159265358979323846);
 

@@ -1190,8 +1190,8 @@ int launch_form_factors(const pi_kgrid_impl* kg, const pi_batch_impl* b, int sca
   auto busy = [&](int r) { return (K.moments ? (ctas(r) + 4) / 5 : ctas(r)) * heavy; };
   const int64_t wave = FF_CTAS * (int64_t)current_sm_count();
   // four radii per thread where 16 splits at eight give less than 7/4 waves
-  // (8 clouds of 50,000 disks: 7.1 ms at four, 8.2 at eight; a solid of 200,000
-  // triangles, just above: 36.2 and 30.0)
+  // (8 clouds of 50,000 disks: 6.7 ms at four, 6.8 at eight; a solid of 200,000
+  // triangles, just above: 38.2 and 29.7)
   if (R == 8 && 4 * 16 * busy(8) < 7 * wave) R = 4;
   int S = 1;
   while (S < 16 && S * busy(R) < 2 * wave && n_max > 2 * S * FF_CHUNK) S *= 2;
