@@ -241,3 +241,23 @@ def test_jacobian_translation_rows_at_each_small_radius(cuda, orc, kg64):
     norm = lambda x: np.linalg.norm(x.reshape(3, L, -1), axis=(0, 2))
     inputs = 2.0 ** -23 * 4 * np.pi * 1.4 * 0.9 / np.sqrt(5120) * np.sqrt(Jo.size / L) * k
     assert (norm(got - ref) <= 2e-6 * norm(ref) + inputs)[k < 1].all()
+
+
+def test_one_shot_calls_from_several_threads(cuda, kg64):
+    """Host entry points take their device memory from a shared pool: concurrent
+    calls give the serial calls' results, bit for bit."""
+    import threading
+    scenes = [[patch("tri", 200 + 50 * i, i), patch("disk", 300, 20 + i)] for i in range(4)]
+    serial = [core.volume_matrix_host(kg64, s) for s in scenes]
+    got = [[None] * 3 for _ in scenes]
+
+    def work(i):
+        for r in range(3):
+            got[i][r] = core.volume_matrix_host(kg64, scenes[i])
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert all(g is not None and np.array_equal(g, serial[i]) for i in range(4) for g in got[i])
