@@ -158,8 +158,10 @@ __device__ __forceinline__ float2 fm_moments(const float4* es, int pairs, const 
       const float2 cx = fma2(vy, rz, neg2(mul2(vz, ry))), cy = fma2(vz, rx, neg2(mul2(vx, rz))),
                    cz = fma2(vx, ry, neg2(mul2(vy, rx)));
       const float2 cc = fma2(cx, cx, fma2(cy, cy, mul2(cz, cz)));
-      const float2 perp = fma2(dup2(D.qd), nw, mul2(add2(dup2(1.0f), neg2(nw)), cc));
+      float2 perp = fma2(dup2(D.qd), nw, mul2(add2(dup2(1.0f), neg2(nw)), cc));
       const bool disk = KIND == PI_GEOM_DISK;
+      // a disk's is at least 0 (normals longer than 1 make it negative near them), a Gaussian's is not clamped
+      if (disk) perp = make_float2(fmaxf(perp.x, 0.f), fmaxf(perp.y, 0.f));
       // disk: q = p^2 - s^2; Gaussian: q = sigma^2 |k'_perp|^2 / |k|^2 (= 2 q' of e^{-q' k^2})
       const float2 q = disk ? fma2(p2, perp, neg2(mul2(s0, s0))) : mul2(p2, perp);
       float2 w0 = amp, w1 = mul2(s0, amp);
