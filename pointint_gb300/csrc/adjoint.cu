@@ -557,7 +557,12 @@ adj_tri_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const 
   }
   const float4 ct = valid && nr > 0 ? st.ctr[cl] : make_float4(0.f, 0.f, 0.f, 1.f);
   const float inv_s = 1.0f / ct.w;  // a power of two
-  const float3 rel = make_float3((q0.x - ct.x) + ql.x, (q0.y - ct.y) + ql.y, (q0.z - ct.z) + ql.z);
+  // A triangle without edges has no gradient wherever it lies.  One with unset vertex
+  // ids is stored so at the object's origin, outside its patch's sphere (that of the
+  // others): the powers of its projection would overflow, and 0 inf is not 0.
+  const bool edges = q1.x != 0.f || q1.y != 0.f || q1.z != 0.f || q2.x != 0.f || q2.y != 0.f || q2.z != 0.f;
+  const float3 rel = edges ? make_float3((q0.x - ct.x) + ql.x, (q0.y - ct.y) + ql.y, (q0.z - ct.z) + ql.z)
+                           : make_float3(0.f, 0.f, 0.f);
   const float3 ml = make_float3(ql.x, ql.y, ql.z);  // centroid low word
   const float3 m = make_float3(q0.x, q0.y, q0.z), e1 = make_float3(q1.x, q1.y, q1.z),
                e2 = make_float3(q2.x, q2.y, q2.z), S = make_float3(q0.w, q1.w, q2.w);
