@@ -243,8 +243,8 @@ __device__ __forceinline__ cf cis_tab_df(const float2* tab, float2 kt, df sm) {
   return cis_tab_frac<C>(tab, __float_as_int(t), f);
 }
 
-// e^{2 pi i kt d / 64} - 1 for FP32 kt and d, to a relative 1e-7 or so however
-// small the phase: tabm holds (cos - 1, sin), rounded once from FP64, and
+// e^{2 pi i kt d / 64} - 1 for an FP32 d and a double-float kt, to a relative 1e-7 or so
+// however small the phase: tabm holds (cos - 1, sin), rounded once from FP64, and
 //   e^{i(a+b)} - 1 = ta + cm + i sn + ta (cm + i sn),  ta = e^{ia} - 1,
 // b = c f.  (Entry 0 is zero, so short phases come from cm and sn alone.)
 constexpr int PHASOR_M1_COPIES = 8;
@@ -258,9 +258,9 @@ __device__ __forceinline__ cf cis_tab_m1_frac(const float2* tabm, int idx, float
 }
 
 template <int C = PHASOR_M1_COPIES>
-__device__ __forceinline__ cf cis_tab_m1(const float2* tabm, float kt, float d) {
-  const float t = fmaf(kt, d, PI_ROUND_SHIFT);
-  return cis_tab_m1_frac<C>(tabm, __float_as_int(t), fmaf(kt, d, PI_ROUND_SHIFT - t));
+__device__ __forceinline__ cf cis_tab_m1(const float2* tabm, float2 kt, float d) {
+  const float t = fmaf(kt.x, d, PI_ROUND_SHIFT);
+  return cis_tab_m1_frac<C>(tabm, __float_as_int(t), fmaf(kt.y, d, fmaf(kt.x, d, PI_ROUND_SHIFT - t)));
 }
 
 // The same for a double-float radius and dot product.
@@ -478,8 +478,7 @@ __device__ __forceinline__ cf dd1(cf Pu, cf Pv, float g) {
 // takes four phasors with the centroid's, and at every radius selects its
 // near pair and one of two forms of its divided difference).  The triangle is
 // consistent by construction (the outer vertices are v plus the gaps), so
-// the rounding of the FP32 gaps, and of the FP32 radius in their phases,
-// changes its size by 6e-8.
+// the rounding of the FP32 gaps changes its size by 6e-8.
 struct TriGaps {
   df sv;           // middle vertex
   float G1, G2;    // at least 1e-20, so that M / G has its limit i k at a closed gap
@@ -505,7 +504,7 @@ __device__ __forceinline__ TriGaps tri_gaps(float s1, float s2, df sm) {
 
 // g e[u, v, w] without the factor e^{iv}; tabm: the table of cis_tab_m1, kt
 // the radius in 1/64 turns, gik = g/(D k^2).
-__device__ __forceinline__ cf tri_wide(const float2* tabm, float kt, const TriGaps& t, float gik) {
+__device__ __forceinline__ cf tri_wide(const float2* tabm, float2 kt, const TriGaps& t, float gik) {
   const cf M1 = cis_tab_m1(tabm, kt, t.G1), M2 = cis_tab_m1(tabm, kt, t.G2);
   return {gik * fmaf(M1.re, t.i1, M2.re * t.i2), gik * fmaf(M1.im, t.i1, -M2.im * t.i2)};
 }

@@ -895,8 +895,9 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
             const float4 ka = ld_shared_f4(kw + 2 * p), kb = ld_shared_f4(kw + 2 * p + 1);
             const float klo = fminf(ka.z, kb.z), khi = fmaxf(ka.z, kb.z);
             if (klo * wide_lo >= 1.0f && klo * wide_hi >= 1.0f) {
-              const cf P0 = cis_tab_df(ctab, make_float2(ka.x, ka.y), tg.sv), P1 = cis_tab_df(ctab, make_float2(kb.x, kb.y), tg.sv);
-              const cf T0 = tri_wide(ctabm, ka.x, tg, gD * rcp_fast(ka.z)), T1 = tri_wide(ctabm, kb.x, tg, gD * rcp_fast(kb.z));
+              const float2 kta = make_float2(ka.x, ka.y), ktb = make_float2(kb.x, kb.y);
+              const cf P0 = cis_tab_df(ctab, kta, tg.sv), P1 = cis_tab_df(ctab, ktb, tg.sv);
+              const cf T0 = tri_wide(ctabm, kta, tg, gD * rcp_fast(ka.z)), T1 = tri_wide(ctabm, ktb, tg, gD * rcp_fast(kb.z));
               add(2 * p, P0, T0);
               add(2 * p + 1, P1, T1);
             } else if (khi * wide_hi < 1.0f) {
@@ -914,7 +915,7 @@ __device__ __forceinline__ void ff_body(const KGridDev& kg, const BatchDev& b, f
                   T = tri_series_eval(tp, kr.z, kr.w);  // centroid Taylor series
                 } else {
                   P = cis_tab_df(ctab, kt, tg.sv);
-                  T = tri_wide(ctabm, kr.x, tg, gD * rcp_fast(kr.z));
+                  T = tri_wide(ctabm, kt, tg, gD * rcp_fast(kr.z));
                   if (kr.z * wide_lo < 1.0f) {
                     // lanes of small spread, whose divided differences cancel
                     const bool narrow = kr.z * tg.D * tg.D < 1.0f;
