@@ -439,9 +439,6 @@ adj_surf_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const
     stage_tile(st, kg, od, Bt_obj, n_cl, j0);
     if (!valid) continue;
     const int jn = min(ADJ_DT, kg.Me - j0);
-    float part[12];
-#pragma unroll
-    for (int i = 0; i < 12; ++i) part[i] = 0.f;
 #pragma unroll 1
     for (int jj = 0; jj < jn; ++jj) {
       const float4 h = st.dh[jj], l = st.dl[jj];
@@ -510,15 +507,13 @@ adj_surf_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const
         s_n += fmaf(sn * sn * Cp, a2, C * a1);
         s_m = fmaf(-0.5f * amp * Cp, a2, s_m);
       }
-      part[0] = fmaf(dh.x, s_c, part[0]); part[1] = fmaf(dh.y, s_c, part[1]); part[2] = fmaf(dh.z, s_c, part[2]);
+      g[0].add(dh.x * s_c); g[1].add(dh.y * s_c); g[2].add(dh.z * s_c);
       const float sn2 = s_n * inv_norm;
-      part[3] = fmaf(dh.x, sn2, part[3]); part[4] = fmaf(dh.y, sn2, part[4]); part[5] = fmaf(dh.z, sn2, part[5]);
+      g[3].add(dh.x * sn2); g[4].add(dh.y * sn2); g[5].add(dh.z * sn2);
       const float mx = dh.x * s_m, my = dh.y * s_m, mz = dh.z * s_m;
-      part[6] = fmaf(dh.x, mx, part[6]); part[7] = fmaf(dh.x, my, part[7]); part[8] = fmaf(dh.x, mz, part[8]);
-      part[9] = fmaf(dh.y, my, part[9]); part[10] = fmaf(dh.y, mz, part[10]); part[11] = fmaf(dh.z, mz, part[11]);
+      g[6].add(dh.x * mx); g[7].add(dh.x * my); g[8].add(dh.x * mz);
+      g[9].add(dh.y * my); g[10].add(dh.y * mz); g[11].add(dh.z * mz);
     }
-#pragma unroll
-    for (int i = 0; i < 12; ++i) g[i].add(part[i]);
   }
   float sum[12];
   const bool mine = adj_total(st, g, sum);
@@ -573,9 +568,6 @@ adj_tri_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const 
     stage_tile(st, kg, od, Bt_obj, n_cl, j0);
     if (!valid) continue;
     const int jn = min(ADJ_DT, kg.Me - j0);
-    float part[9];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) part[i] = 0.f;
 #pragma unroll 1
     for (int jj = 0; jj < jn; ++jj) {
       const float4 h = st.dh[jj], l = st.dl[jj];
@@ -646,12 +638,10 @@ adj_tri_kernel(KGridDev kg, BatchDev b, const AdjWork* __restrict__ work, const 
                                     0.5f * (kh.x * e1.y - kh.y * e1.x));
       // dL/dv = -2 (grad gamma t0 + gamma dir t_v), the -2 applied at the end
       const float ga = gam * ta, gb = gam * tb, gc = gam * tc;
-      part[0] += fmaf(dh.x, ga, c0.x * t0); part[1] += fmaf(dh.y, ga, c0.y * t0); part[2] += fmaf(dh.z, ga, c0.z * t0);
-      part[3] += fmaf(dh.x, gb, c1.x * t0); part[4] += fmaf(dh.y, gb, c1.y * t0); part[5] += fmaf(dh.z, gb, c1.z * t0);
-      part[6] += fmaf(dh.x, gc, c2.x * t0); part[7] += fmaf(dh.y, gc, c2.y * t0); part[8] += fmaf(dh.z, gc, c2.z * t0);
+      g[0].add(fmaf(dh.x, ga, c0.x * t0)); g[1].add(fmaf(dh.y, ga, c0.y * t0)); g[2].add(fmaf(dh.z, ga, c0.z * t0));
+      g[3].add(fmaf(dh.x, gb, c1.x * t0)); g[4].add(fmaf(dh.y, gb, c1.y * t0)); g[5].add(fmaf(dh.z, gb, c1.z * t0));
+      g[6].add(fmaf(dh.x, gc, c2.x * t0)); g[7].add(fmaf(dh.y, gc, c2.y * t0)); g[8].add(fmaf(dh.z, gc, c2.z * t0));
     }
-#pragma unroll
-    for (int i = 0; i < 9; ++i) g[i].add(part[i]);
   }
   float sum[9];
   const bool mine = adj_total(st, g, sum);
