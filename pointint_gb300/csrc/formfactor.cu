@@ -1094,18 +1094,14 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
   ff_body<R, false>(kg, b, J, scale_sqrt_w, evals, row_amax);
 }
 
-// Serving evaluations always split their elements over FF_SERVE_SPLIT CTAs: a
-// row's value must not depend on the batch it is evaluated in.  Batches hold a
-// few to a few tens of objects of very different sizes, and the largest sets
-// the batch's time: at a split of 4, one mesh of 50,000 triangles took 10 ms
-// beside others that were done in 2.
-constexpr int FF_SERVE_SPLIT = 16;
+// CTAs per serving evaluation of each class (SERVE_CLASSES).
+constexpr int FF_SERVE_SPLIT[SERVE_CLASSES] = {16, 4, 1};
 
 template <int R>
-__global__ void __cluster_dims__(FF_SERVE_SPLIT, 1, 1) __launch_bounds__(FF_THREADS, FF_CTAS)
-ff_serve_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, const EvalDev* __restrict__ evals,
-                unsigned* __restrict__ row_amax) {
-  ff_body<R, true>(kg, b, J, scale_sqrt_w, evals, row_amax);
+__global__ void __launch_bounds__(FF_THREADS, FF_CTAS)
+ff_serve_kernel(KGridDev kg, BatchDev b, const EvalDev* __restrict__ evals, int n_evals) {
+  if (n_evals == 0) return;  // a class that the batch has no evaluation of
+  ff_body<R, true>(kg, b, nullptr, 1, evals, nullptr);
 }
 
 }  // namespace
@@ -1206,44 +1202,33 @@ int launch_form_factors(const pi_kgrid_impl* kg, const pi_batch_impl* b, int sca
   return launch_moments(kg, b, scale_sqrt_w, J, s, row_amax);
 }
 
-int ff_serve_threads() { return FF_THREADS; }
-
-int ff_serve_setup(const pi_kgrid_impl* kg) { return allow_wide_clusters(ff_serve_fn(kg)); }
-
-int ff_serve_grid_x(const pi_kgrid_impl* kg) {
-  const int R = serve_radii(kg->dev.L);
+ServeKernel ff_serve(const pi_kgrid_impl* kg, int cls) {
+  const int R = serve_radii(kg->dev.L), S = FF_SERVE_SPLIT[cls];
   const int64_t items = (int64_t)((kg->dev.L + R - 1) / R) * ((kg->dev.Me + 31) / 32);
-  return (int)((items + FF_WARPS - 1) / FF_WARPS) * FF_SERVE_SPLIT;
+  return {R == 4 ? reinterpret_cast<const void*>(ff_serve_kernel<4>) : reinterpret_cast<const void*>(ff_serve_kernel<2>),
+          (unsigned)((items + FF_WARPS - 1) / FF_WARPS * S), FF_THREADS, S, 0};
 }
 
-const void* ff_serve_fn(const pi_kgrid_impl* kg) {
-  switch (serve_radii(kg->dev.L)) {
-    case 4: return reinterpret_cast<const void*>(ff_serve_kernel<4>);
-    default: return reinterpret_cast<const void*>(ff_serve_kernel<2>);
-  }
-}
+int ff_serve_setup(const pi_kgrid_impl* kg) { return allow_wide_clusters(ff_serve(kg, 0).fn); }
 
-int launch_form_factors_serve(const pi_kgrid_impl* kg, const pi_batch_impl* lib, const EvalDev* evals, int n_evals,
-                              cudaStream_t s) {
-  if (n_evals <= 0) return PI_OK;
-  if (n_evals > 65535) return fail(PI_ERR_UNSUPPORTED, "more than 65535 evaluations in one launch");
-  if (int rc = ff_serve_setup(kg)) return rc;
+int launch_form_factors_serve(const pi_kgrid_impl* kg, const pi_batch_impl* lib, const EvalDev* evals,
+                              const int (&n_class)[SERVE_CLASSES], cudaStream_t s) {
   KGridDev K = kg->dev;
   BatchDev B = lib->dev();
-  float2* none = nullptr;
-  int scale = 1;
-  unsigned* no_amax = nullptr;
-  void* args[6] = {&K, &B, &none, &scale, const_cast<EvalDev**>(&evals), &no_amax};
-  PI_CUDA(cudaLaunchKernel(ff_serve_fn(kg), dim3((unsigned)ff_serve_grid_x(kg), (unsigned)n_evals), dim3(FF_THREADS),
-                           args, 0, s));
-  count_launch();
-  if (!K.moments) return PI_OK;
-  int rc = moment_setup();
-  if (rc) return rc;
-  PI_CUDA(cudaLaunchKernel(moment_serve_fn(), dim3((unsigned)moment_serve_grid_x(kg), (unsigned)n_evals),
-                           dim3((unsigned)moment_threads()), args, (size_t)moment_smem_bytes(K.L), s));
-  count_launch();
-  return PI_OK;
+  int rc = ff_serve_setup(kg);
+  if (rc == PI_OK && K.moments) rc = moment_setup();
+  for (int c = 0; c < SERVE_CLASSES && rc == PI_OK; evals += n_class[c++]) {
+    if (n_class[c] <= 0) continue;
+    if (n_class[c] > 65535) return fail(PI_ERR_UNSUPPORTED, "more than 65535 evaluations in one launch");
+    int n = n_class[c];
+    void* args[4] = {&K, &B, const_cast<EvalDev**>(&evals), &n};
+    const ServeKernel k[2] = {ff_serve(kg, c), moment_serve(kg, c)};
+    for (int i = 0; i < (K.moments ? 2 : 1) && rc == PI_OK; ++i) {
+      rc = launch_split(k[i].fn, dim3(k[i].grid_x, (unsigned)n_class[c]), k[i].threads, k[i].smem, k[i].split, args, s);
+      if (rc == PI_OK) count_launch();
+    }
+  }
+  return rc;
 }
 
 namespace {

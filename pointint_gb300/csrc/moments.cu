@@ -432,27 +432,31 @@ moment_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w,
   moment_body<false>(kg, b, J, scale_sqrt_w, evals, row_amax);
 }
 
-// The split of a serving evaluation does not depend on its batch.
-constexpr int FM_SERVE_SPLIT = 8;
+// CTAs per serving evaluation of each class (SERVE_CLASSES).
+constexpr int FM_SERVE_SPLIT[SERVE_CLASSES] = {8, 2, 1};
 
-__global__ void __cluster_dims__(FM_SERVE_SPLIT, 1, 1) __launch_bounds__(FM_THREADS, 2)
-moment_serve_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w,
-                    const EvalDev* __restrict__ evals, unsigned* __restrict__ row_amax) {
-  moment_body<true>(kg, b, J, scale_sqrt_w, evals, row_amax);
+__global__ void __launch_bounds__(FM_THREADS, 2)
+moment_serve_kernel(KGridDev kg, BatchDev b, const EvalDev* __restrict__ evals, int n_evals) {
+  if (n_evals == 0) return;  // a class that the batch has no evaluation of
+  moment_body<true>(kg, b, nullptr, 1, evals, nullptr);
 }
 
 }  // namespace
 
-int moment_threads() { return FM_THREADS; }
-int moment_smem_bytes(int L) { return fm_smem_f4(L) * (int)sizeof(float4); }
-int moment_serve_grid_x(const pi_kgrid_impl* kg) { return (kg->dev.Me + 31) / 32 * FM_SERVE_SPLIT; }
-const void* moment_serve_fn() { return reinterpret_cast<const void*>(moment_serve_kernel); }
+static int moment_smem_bytes(int L) { return fm_smem_f4(L) * (int)sizeof(float4); }
+
+ServeKernel moment_serve(const pi_kgrid_impl* kg, int cls) {
+  const int S = FM_SERVE_SPLIT[cls];
+  return {reinterpret_cast<const void*>(moment_serve_kernel), (unsigned)((kg->dev.Me + 31) / 32 * S), FM_THREADS, S,
+          (size_t)moment_smem_bytes(kg->dev.L)};
+}
 
 int moment_setup() {
   int rc = ensure_smem_limit(reinterpret_cast<const void*>(moment_kernel), moment_smem_bytes(MOMENT_MAX_L),
                              "moment_kernel");
   if (rc == PI_OK)
-    rc = ensure_smem_limit(moment_serve_fn(), moment_smem_bytes(MOMENT_MAX_L), "moment_kernel");
+    rc = ensure_smem_limit(reinterpret_cast<const void*>(moment_serve_kernel), moment_smem_bytes(MOMENT_MAX_L),
+                           "moment_kernel");
   return rc;
 }
 

@@ -79,12 +79,8 @@ __device__ __forceinline__ void tri_moments(float2 a, float2 b, float2 c, float2
 // Form factors of the radii below moment_radii; ff_kernel evaluates the others.
 int launch_moments(const pi_kgrid_impl* kg, const pi_batch_impl* b, int scale_sqrt_w, float2* J, cudaStream_t s,
                    float* row_amax);
-// Serving evaluations: a node with this function, block and shared memory, the
-// arguments of ff_serve_fn's, grid (moment_serve_grid_x, n_evals).
-const void* moment_serve_fn();
-int moment_threads();
-int moment_serve_grid_x(const pi_kgrid_impl* kg);
-int moment_smem_bytes(int L);
+// The same of a class of serving evaluations, with the arguments of ff_serve's kernels.
+ServeKernel moment_serve(const pi_kgrid_impl* kg, int cls);
 int moment_setup();
 
 }  // namespace pi

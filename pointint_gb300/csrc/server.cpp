@@ -103,7 +103,8 @@ struct Slot {
   struct Graph {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    cudaGraphNode_t n_h2d = nullptr, n_ff = nullptr, n_fm = nullptr, n_d2h_out = nullptr;
+    cudaGraphNode_t n_h2d = nullptr, n_d2h_out = nullptr;
+    cudaGraphNode_t n_eval[SERVE_CLASSES][2] = {};  // form factors of each class: direct sum, expansions
   } graphs[2];
   // current batch
   bool busy = false;
@@ -113,6 +114,7 @@ struct Slot {
   std::vector<int> temps;        // pool rows owned by this batch
   std::vector<int> produced;     // canonical rows evaluated by this batch
   int n_rows = 0, n_queries = 0, n_evals = 0;
+  int n_class[SERVE_CLASSES] = {};  // evaluations of each class
   int64_t n_items = 0, n_out = 0;
 };
 
@@ -223,6 +225,18 @@ Layout make_layout(const pi_server_config& c, int64_t max_out) {
   return L;
 }
 
+// (a class without evaluations launches one cluster, which returns at once: a node
+// whose cluster size is an attribute cannot be disabled)
+cudaKernelNodeParams eval_params(const ServeKernel& k, int n, void** args) {
+  cudaKernelNodeParams kp{};
+  kp.func = const_cast<void*>(k.fn);
+  kp.gridDim = n ? dim3(k.grid_x, (unsigned)n) : dim3((unsigned)k.split);
+  kp.blockDim = dim3((unsigned)k.threads);
+  kp.sharedMemBytes = (unsigned)k.smem;
+  kp.kernelParams = args;
+  return kp;
+}
+
 int build_graph(Server& S, Slot& sl, Slot::Graph& gr, bool evaluate) {
   PI_CUDA(cudaGraphCreate(&gr.graph, 0));
   // descriptor upload (size set per launch)
@@ -234,34 +248,30 @@ int build_graph(Server& S, Slot& sl, Slot::Graph& gr, bool evaluate) {
   PI_CUDA(cudaGraphAddMemsetNode(&n_err, gr.graph, &gr.n_h2d, 1, &ms));
   cudaGraphNode_t rows_ready = n_err;
   if (evaluate) {
-    // form factors of the batch's new rows (grid set per launch)
+    // form factors of the batch's new rows, side by side: a node for the direct
+    // sum and one for the cluster expansions (other radii of the same rows) of
+    // each class of objects (grids set per launch)
     KGridDev K = S.kg->dev;
     BatchDev B = S.lib->dev();
-    float2* none = nullptr;
-    int one = 1;
     EvalDev* evals = reinterpret_cast<EvalDev*>(sl.d_io + S.lay.evals);
-    unsigned* no_amax = nullptr;  // serving rows keep their maxima through EvalDev::amax
-    void* ff_args[6] = {&K, &B, &none, &one, &evals, &no_amax};
-    if (int rc = ff_serve_setup(S.kg)) return rc;
-    cudaKernelNodeParams kp{};
-    kp.func = const_cast<void*>(ff_serve_fn(S.kg));
-    kp.gridDim = dim3((unsigned)ff_serve_grid_x(S.kg), 1);
-    kp.blockDim = dim3((unsigned)ff_serve_threads());
-    kp.sharedMemBytes = 0;
-    kp.kernelParams = ff_args;
-    PI_CUDA(cudaGraphAddKernelNode(&gr.n_ff, gr.graph, &n_err, 1, &kp));
-    // beside it (other radii of the same rows) the cluster expansions
-    cudaGraphNode_t evaluated[2] = {gr.n_ff, nullptr};
-    if (K.moments) {
-      int rc = moment_setup();
-      if (rc) return rc;
-      kp.func = const_cast<void*>(moment_serve_fn());
-      kp.gridDim = dim3((unsigned)moment_serve_grid_x(S.kg), 1);
-      kp.blockDim = dim3((unsigned)moment_threads());
-      kp.sharedMemBytes = (unsigned)moment_smem_bytes(K.L);
-      PI_CUDA(cudaGraphAddKernelNode(&gr.n_fm, gr.graph, &n_err, 1, &kp));
-      evaluated[1] = gr.n_fm;
-    }
+    int n_class = 0;
+    void* ff_args[4] = {&K, &B, &evals, &n_class};
+    int rc = ff_serve_setup(S.kg);
+    if (rc == PI_OK && K.moments) rc = moment_setup();
+    if (rc) return rc;
+    std::vector<cudaGraphNode_t> evaluated;
+    for (int c = 0; c < SERVE_CLASSES; ++c)
+      for (int i = 0; i < (K.moments ? 2 : 1); ++i) {
+        const ServeKernel k = i ? moment_serve(S.kg, c) : ff_serve(S.kg, c);
+        cudaKernelNodeParams kp = eval_params(k, n_class, ff_args);
+        PI_CUDA(cudaGraphAddKernelNode(&gr.n_eval[c][i], gr.graph, &n_err, 1, &kp));
+        cudaLaunchAttributeValue dim{};
+        dim.clusterDim.x = (unsigned)k.split;
+        dim.clusterDim.y = dim.clusterDim.z = 1;
+        if (k.split > 1)
+          PI_CUDA(cudaGraphKernelNodeSetAttribute(gr.n_eval[c][i], cudaLaunchAttributeClusterDimension, &dim));
+        evaluated.push_back(gr.n_eval[c][i]);
+      }
     // row maxima of the new rows into the pool
     const int32_t* n_evals = &reinterpret_cast<const GHeader*>(sl.d_io + S.lay.hdr)->n_evals;
     void* cm_args[2] = {&evals, const_cast<int32_t**>(&n_evals)};
@@ -270,7 +280,7 @@ int build_graph(Server& S, Slot& sl, Slot::Graph& gr, bool evaluate) {
     cmp.gridDim = dim3(1);
     cmp.blockDim = dim3((unsigned)amax_commit_threads());
     cmp.kernelParams = cm_args;
-    PI_CUDA(cudaGraphAddKernelNode(&rows_ready, gr.graph, evaluated, K.moments ? 2 : 1, &cmp));
+    PI_CUDA(cudaGraphAddKernelNode(&rows_ready, gr.graph, evaluated.data(), evaluated.size(), &cmp));
   }
   // contraction
   void* con_args[2] = {&sl.g, &S.pool_map};
@@ -528,12 +538,15 @@ int build_batch(Server& S, Slot& sl, std::vector<cudaEvent_t>* waits) {
     n_elems += out;
   }
   if (sl.n_queries == 0) return 0;
-  // Largest objects first: the evaluation grid's CTAs start in this order, so
+  // Largest objects first: the classes one after another, and within each the
+  // evaluation grid's CTAs start in this order, so
   // a large object's CTAs do not start last and leave the SMs idle at the end
   // (each evaluation carries its own destination row and row-maximum slots).
   std::stable_sort(evals, evals + sl.n_evals, [&](const EvalDev& x, const EvalDev& y) {
     return S.lib->info[x.obj].n_elems > S.lib->info[y.obj].n_elems;
   });
+  for (int& n : sl.n_class) n = 0;
+  for (int k = 0; k < sl.n_evals; ++k) ++sl.n_class[serve_class(S.lib->info[evals[k].obj].n_elems)];
   hdr->n_items = (int32_t)sl.n_items;
   hdr->n_queries = sl.n_queries;
   hdr->n_elems = n_elems;
@@ -556,24 +569,13 @@ int launch_batch(Server& S, Slot& sl, const std::vector<cudaEvent_t>& waits) {
     if (ff) {
       KGridDev K = S.kg->dev;
       BatchDev B = S.lib->dev();
-      float2* none = nullptr;
-      int one = 1;
       EvalDev* evals = reinterpret_cast<EvalDev*>(sl.d_io + S.lay.evals);
-      unsigned* no_amax = nullptr;
-      void* ff_args[6] = {&K, &B, &none, &one, &evals, &no_amax};
-      cudaKernelNodeParams kp{};
-      kp.func = const_cast<void*>(ff_serve_fn(S.kg));
-      kp.gridDim = dim3((unsigned)ff_serve_grid_x(S.kg), (unsigned)sl.n_evals);
-      kp.blockDim = dim3((unsigned)ff_serve_threads());
-      kp.kernelParams = ff_args;
-      PI_CUDA(cudaGraphExecKernelNodeSetParams(gr.exec, gr.n_ff, &kp));
-      if (K.moments) {
-        kp.func = const_cast<void*>(moment_serve_fn());
-        kp.gridDim = dim3((unsigned)moment_serve_grid_x(S.kg), (unsigned)sl.n_evals);
-        kp.blockDim = dim3((unsigned)moment_threads());
-        kp.sharedMemBytes = (unsigned)moment_smem_bytes(K.L);
-        PI_CUDA(cudaGraphExecKernelNodeSetParams(gr.exec, gr.n_fm, &kp));
-      }
+      for (int c = 0; c < SERVE_CLASSES; evals += sl.n_class[c++])
+        for (int i = 0; i < (K.moments ? 2 : 1); ++i) {
+          void* ff_args[4] = {&K, &B, &evals, &sl.n_class[c]};
+          cudaKernelNodeParams kp = eval_params(i ? moment_serve(S.kg, c) : ff_serve(S.kg, c), sl.n_class[c], ff_args);
+          PI_CUDA(cudaGraphExecKernelNodeSetParams(gr.exec, gr.n_eval[c][i], &kp));
+        }
     }
     PI_CUDA(cudaGraphExecMemcpyNodeSetParams1D(gr.exec, gr.n_d2h_out, sl.h_io + S.lay.err, sl.d_io + S.lay.err,
                                                out_bytes, cudaMemcpyDeviceToHost));
@@ -582,7 +584,7 @@ int launch_batch(Server& S, Slot& sl, const std::vector<cudaEvent_t>& waits) {
   } else {
     PI_CUDA(cudaMemcpyAsync(sl.d_io, sl.h_io, h2d, cudaMemcpyHostToDevice, sl.stream));
     PI_CUDA(cudaMemsetAsync(sl.d_err, 0, sizeof(int), sl.stream));
-    int rc = launch_form_factors_serve(S.kg, S.lib, reinterpret_cast<EvalDev*>(sl.d_io + S.lay.evals), sl.n_evals,
+    int rc = launch_form_factors_serve(S.kg, S.lib, reinterpret_cast<EvalDev*>(sl.d_io + S.lay.evals), sl.n_class,
                                        sl.stream);
     if (rc) return rc;
     rc = launch_amax_commit(reinterpret_cast<EvalDev*>(sl.d_io + S.lay.evals),
