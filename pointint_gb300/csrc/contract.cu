@@ -288,7 +288,7 @@ __global__ void reduce_tiles_kernel(const float* __restrict__ partials, const Sy
   V[(int64_t)j * g.n + i] = s;
 }
 
-// Few rows (n <= SMALL_N): the 128 x 128 tile would be mostly padding (14 rows
+// Few rows (small_rows): the 128 x 128 tile would be mostly padding (14 rows
 // on 76,928 nodes: 88 us for a read of 8.6 MB).  A warp owns a 4 x 4 block of
 // row pairs, its lanes 32 neighbouring columns read straight from global
 // memory (the rows come from L2, where the form factors were just written, and
@@ -297,7 +297,15 @@ __global__ void reduce_tiles_kernel(const float* __restrict__ partials, const Sy
 // into fresh FP32 registers, then into compensated sums, and the lanes are
 // added compensated; few blocks are repeated over column groups so that all
 // warps work.  partials[cta * cgs + group][i n + j].
-constexpr int SMALL_N = 64, SMALL_WARPS = 8, SMALL_FOLD = 16;
+// Its time grows with the block pairs p, 20 us + p (0.21 us + what their columns
+// take), the tile's with the nodes alone: on 743,680 nodes 557 us at 48 rows (p =
+// 78), 756 at 56 (105), 850 at 60 and 963 at 64, against 850 .. 865; on 2,432 nodes
+// 24 us at 24 rows (21), 27.8 at 32 (36) and 44 at 56, against 27; on 19,328 nodes
+// 44 at 40 (55) and 50 at 44 (66), against 48.  The two cross at about p = 24 + Q / 600.
+constexpr int SMALL_N = 56;
+constexpr int small_pairs(int n) { return (n + 3) / 4 * ((n + 3) / 4 + 1) / 2; }
+constexpr bool small_rows(int n, int64_t Q) { return n <= SMALL_N && small_pairs(n) <= 24 + Q / 600; }
+constexpr int SMALL_WARPS = 8, SMALL_FOLD = 16;
 
 __device__ __forceinline__ kbsum kb_merge(kbsum a, float hi, float lo) {
   const df t = two_sum(a.hi, hi);
@@ -420,9 +428,10 @@ bool vector_loads_ok(const void* X, int64_t K) {
 }
 
 int launch_syrk(const float* X, const SyrkGeom& g, const float* sign, float* partials, double* V, cudaStream_t s) {
-  if (g.n <= SMALL_N) {
-    const int nb = (g.n + 3) / 4, tp = nb * (nb + 1) / 2, cgs = std::max(1, SMALL_WARPS / tp);
-    const int64_t Q = g.K / 2, blk = (int64_t)cgs * g.n * g.n;
+  const int64_t Q = g.K / 2;
+  if (small_rows(g.n, Q)) {
+    const int tp = small_pairs(g.n), cgs = std::max(1, SMALL_WARPS / tp);
+    const int64_t blk = (int64_t)cgs * g.n * g.n;
     // two CTAs per SM, at least one step per column group, and no more partials
     // than the tiles' workspace holds
     const int64_t cap = std::max<int64_t>(1, syrk_tiles(g) * TB * TB / blk);
