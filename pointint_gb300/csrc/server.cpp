@@ -884,13 +884,12 @@ int pi_server_create(pi_kgrid kg, const pi_object* library, int n_library, const
   size_t free_b = 0, total_b = 0;
   PI_CUDA(cudaMemGetInfo(&free_b, &total_b));
   const int64_t budget = c.hbm_budget_bytes > 0 ? c.hbm_budget_bytes : (int64_t)(free_b / 4);
-  // the number of rows is what the budget holds of whole-grid rows
-  const int64_t row_bytes = (kg->Q + GROUP_CHUNK - 1) / GROUP_CHUNK * GROUP_CHUNK * (int64_t)sizeof(float2);
+  const int64_t row_bytes = S->Qpad * (int64_t)sizeof(float2);
   const int64_t pool_bytes = budget - (int64_t)slot_bytes * S->nslots;
   if (pool_bytes < row_bytes * 2)
     return fail(PI_ERR_OUT_OF_MEMORY, "pi_server_create: HBM budget leaves no room for resident rows");
   S->pool_rows = std::min<int64_t>(pool_bytes / row_bytes, 0x7fffffff);
-  const size_t pool_used = (size_t)S->pool_rows * (size_t)S->Qpad * sizeof(float2);
+  const size_t pool_used = (size_t)(S->pool_rows * row_bytes);
   PI_CUDA(cudaMalloc(reinterpret_cast<void**>(&S->d_pool), pool_used));
   PI_CUDA(cudaMemset(S->d_pool, 0, pool_used));
   S->row_obj.assign(S->pool_rows, -1);
