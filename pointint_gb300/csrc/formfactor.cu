@@ -150,6 +150,7 @@ prepare_origin_kernel(const PrepObj* objs, ObjDev* out, unsigned* cl_rho, int on
 // of the whole segment at every level took 185 us for 1,280 elements and 905
 // for 5,120; the host ~0.1 us per element.)
 constexpr int ORDER_SLOTS = ORDER_SEGMENT / PI_CLUSTER, ORDER_BLOCKS = ORDER_SEGMENT / 32;
+constexpr int ORDER_THREADS = 1024;  // segments have 2,048 to ORDER_SEGMENT elements: at most eight entries per thread
 constexpr int ORDER_BITS = 6, ORDER_BINS = 1 << ORDER_BITS, ORDER_ROUNDS = 4;
 
 struct OrderShared {
@@ -184,7 +185,7 @@ __device__ __forceinline__ float order_float(unsigned u) {
   return __uint_as_float((u >> 31) ? u & 0x7fffffffu : ~u);
 }
 
-__global__ void __launch_bounds__(1024)
+__global__ void __launch_bounds__(ORDER_THREADS)
 order_kernel(const OrderSeg* __restrict__ segs, int32_t* __restrict__ perm, int n2) {
   extern __shared__ float4 osm[];
   OrderShared& sh = *reinterpret_cast<OrderShared*>(osm);
@@ -192,7 +193,8 @@ order_kernel(const OrderSeg* __restrict__ segs, int32_t* __restrict__ perm, int 
   unsigned short* ia = reinterpret_cast<unsigned short*>(ox + 3 * n2);  // entry -> element of the segment
   unsigned short* ib = ia + n2;
   const OrderSeg g = segs[blockIdx.x];
-  const int n = g.count, tid = threadIdx.x, T = blockDim.x, warp = tid >> 5, lane = tid & 31, nw = T >> 5;
+  constexpr int T = ORDER_THREADS;
+  const int n = g.count, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = T >> 5;
   const int nblk = (n + 31) / 32;
   int32_t* out = perm + g.perm_off;
   for (int i = tid; i < n; i += T) {
@@ -394,15 +396,15 @@ order_kernel(const OrderSeg* __restrict__ segs, int32_t* __restrict__ perm, int 
   }
   __syncthreads();
   // the ids of all entries are read before any is written (from_perm)
-  int32_t id[ORDER_SEGMENT / 256];
+  int32_t id[ORDER_SEGMENT / T];
 #pragma unroll
-  for (int t = 0; t < ORDER_SEGMENT / 256; ++t) {
+  for (int t = 0; t < ORDER_SEGMENT / T; ++t) {
     const int i = tid + t * T;
     if (i < n) id[t] = g.from_perm ? out[ia[i]] : ia[i];
   }
   __syncthreads();
 #pragma unroll
-  for (int t = 0; t < ORDER_SEGMENT / 256; ++t) {
+  for (int t = 0; t < ORDER_SEGMENT / T; ++t) {
     const int i = tid + t * T;
     if (i < n) out[i] = id[t];
   }
@@ -1121,8 +1123,7 @@ int launch_order(const std::vector<OrderSeg>& segs, int32_t* d_perm, cudaStream_
   OrderSeg* d = nullptr;
   PI_CUDA(pool_alloc((void**)&d, segs.size() * sizeof(OrderSeg), s));
   PI_CUDA(cudaMemcpyAsync(d, segs.data(), segs.size() * sizeof(OrderSeg), cudaMemcpyHostToDevice, s));
-  // at most eight entries per thread, and a warp per part and block while there are few
-  order_kernel<<<(unsigned)segs.size(), n2 > 512 ? 1024 : 256, order_smem(n2), s>>>(d, d_perm, n2);
+  order_kernel<<<(unsigned)segs.size(), ORDER_THREADS, order_smem(n2), s>>>(d, d_perm, n2);
   PI_LAUNCHED("order_kernel");
   PI_CUDA(cudaFreeAsync(d, s));
   return PI_OK;
