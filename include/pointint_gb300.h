@@ -139,8 +139,12 @@ int pi_kgrid_direction_pairs(const double* dirs, const double* kmag, int64_t Q, 
 /* ---- device-resident object batch ------------------------------------------- */
 /* A set of objects transformed by their DoFs into the kernels' FP32 local-frame
  * layout.  `on_device` says whether elems/dofs in `objs` are device (1) or host
- * (0) pointers; the batch keeps its own copies.  Replaces the per-object,
- * per-call uploads of the reference's registry wrappers. */
+ * (0) pointers; the batch keeps its own copies.  Objects of 2,048 elements and more
+ * are ordered in space inside the batch, which the expansions at small k need to
+ * reach far (results stay in the caller's order), except device-resident ones
+ * above 8,192 elements: those keep the caller's order, so a compact one (a mesh's
+ * own, a space-filling curve's) pays there.  Replaces the per-object, per-call
+ * uploads of the reference's registry wrappers. */
 typedef struct pi_batch_s* pi_batch;
 int pi_batch_create(const pi_object* objs, int n_objects, int on_device, pi_stream stream, pi_batch* out);
 /* Replace the DoF vector of object `index` (device pointer, same length) and
@@ -218,7 +222,8 @@ int pi_batch_layout(pi_batch b, int index, int64_t* pool_offset, int64_t* n_elem
  *  cpp/src/compute_intersection_volume.cu:60-101; cpp/src/compute_intersection_volume_multi_object.cu:124-176)
  * without materialising dA/dtheta per k-node. */
 int pi_adjoint_workspace_size(pi_kgrid kg, pi_batch b, size_t* bytes);
-/* Per-element gradients (device float outputs in pool order, either may be NULL):
+/* Per-element gradients (device float outputs in the caller's element order, the
+ * objects of each pool one after another (pi_batch_layout); either may be NULL):
  *   triangles: 9 per element = dL/dv0, dL/dv1, dL/dv2 (world-frame vertex positions);
  *   disks / Gaussians: 12 per element = dL/dc (3), dL/dn' (3, n' = A n), dL/dM (6: xx xy xz yy yz zz, M = A A^T). */
 int pi_element_gradients(pi_kgrid kg, pi_batch b, const void* d_Jw, const double* W, float* d_tri_grad,

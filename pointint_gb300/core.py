@@ -194,7 +194,7 @@ def element_gradients(kgrid: KGrid, batch: ObjectBatch, Jw: torch.Tensor, W, wor
                       stream=None):
     """Per-element gradients for cotangents B_i = sum_j W_ij A_j (W = C + C^T for
     L = sum C_ij V_ij).  Returns (tri [n_tri, 9], surf [n_surf, 12]) float32
-    tensors in pool (object) order: triangles dL/dv0,dv1,dv2; surfels dL/dc,
+    tensors in the caller's element order, object after object: triangles dL/dv0,dv1,dv2; surfels dL/dc,
     dL/dn', dL/dM(6)."""
     n = len(batch)
     W = _w64(W, n)

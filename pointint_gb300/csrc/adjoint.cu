@@ -14,15 +14,16 @@
 // ~9.5 GB for an icosphere-4 at N_k = 76,928) and reduced it with FP64
 // atomics.  Here nothing of size Q x (parameters) exists:
 //
-//  * cotangent_kernel: B^ = W J^ on the sqrt|w|-scaled J (one pass over J);
+//  * cotangent_kernel: forms B^ = W J^ on the sqrt|w|-scaled J (one pass over J)
+//    and folds each direction's antipode into it, with the object's origin phase and
+//    the quadrature weights, so that one direction of a pair is evaluated;
 //  * adj_surf_kernel / adj_tri_kernel: one thread per element; the CTA's
 //    elements share one object, so the cotangent of a tile of directions is
-//    staged once in shared memory (with the object's origin phase and the
-//    quadrature weight folded in) and read as broadcasts, while every thread
-//    recomputes its element's form factor and derivatives at each k-node and
-//    accumulates the element's parameter gradient in registers; of two
-//    antipodal directions only one is evaluated, the other's cotangent folded
-//    into it (stage_tile);
+//    staged once in shared memory and read as broadcasts.  The small radii enter
+//    through sums that a patch of 32 elements shares (beta, below); at the others every
+//    thread recomputes its element's form factor and derivatives.  The element's
+//    parameter gradient is accumulated in registers, every direction's contribution
+//    compensated;
 //  * chain kernels turn element gradients into AffineDoF gradients (fixed
 //    order FP64 block reduction per object) or TriangleMeshDoF vertex
 //    gradients (CSR gather per vertex, no atomics): results are bitwise
@@ -139,7 +140,7 @@ struct AdjWork { int32_t obj, first; };
 // and its derivatives are sums of beta_m times the moments of moments.cu and
 // their derivatives: ~150 FP32 operations per element and direction for all
 // those radii instead of ~70 for each.  (24 bodies, N_k = 76,928: adj_tri_kernel
-// 13.7 -> 3.94 ms; eight clouds of 50,000 disks: adj_surf_kernel 43.8 -> 8.25.)
+// 13.7 -> 3.80 ms; eight clouds of 50,000 disks: adj_surf_kernel 43.8 -> 8.46.)
 constexpr int ADJ_TERMS = MOMENT_TERMS;
 // Patches of half a cluster (a warp's elements): the expansions reach 1.4 times
 // the k.  A quarter reaches twice the k but its betas, every covered radius for

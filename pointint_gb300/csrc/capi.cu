@@ -381,7 +381,7 @@ int kgrid_create_impl(const double* dirs, const double* kmag, const double* w, i
   const bool tensor = grid_layout(dirs, kmag, Q, &M);
   const int64_t L = tensor ? Q / M : 1;
   std::vector<float4> dh(M), dl(M);
-  std::vector<float2> km(L), kt(L), k256(L), tab(2 * PHASOR_ENTRIES);
+  std::vector<float2> km(L), kt(L), k64(L), tab(2 * PHASOR_ENTRIES);
   const std::vector<double> dv = direction_vectors(dirs, kmag, M, tensor);
   for (int64_t j = 0; j < M; ++j) {
     double d[3];
@@ -401,7 +401,7 @@ int kgrid_create_impl(const double* dirs, const double* kmag, const double* w, i
     kt[r] = make_float2(uh, (float)(u - (double)uh));
     const double v = u * 64.0;
     const float vh = (float)v;
-    k256[r] = make_float2(vh, (float)(v - (double)vh));
+    k64[r] = make_float2(vh, (float)(v - (double)vh));
   }
   for (int j = 0; j < PHASOR_ENTRIES; ++j) {
     const double a = 2.0 * 3.14159265358979323846 * j / PHASOR_ENTRIES;
@@ -420,8 +420,8 @@ int kgrid_create_impl(const double* dirs, const double* kmag, const double* w, i
   }
   const size_t o_dh = 0, o_dl = align16(o_dh + M * sizeof(float4)), o_km = align16(o_dl + M * sizeof(float4)),
                o_sw = align16(o_km + L * sizeof(float2)), o_sg = align16(o_sw + Q * sizeof(float)),
-               o_kt = align16(o_sg + Q * sizeof(float)), o_k256 = align16(o_kt + L * sizeof(float2)),
-               o_tab = align16(o_k256 + L * sizeof(float2)), o_pair = align16(o_tab + 2 * PHASOR_ENTRIES * sizeof(float2));
+               o_kt = align16(o_sg + Q * sizeof(float)), o_k64 = align16(o_kt + L * sizeof(float2)),
+               o_tab = align16(o_k64 + L * sizeof(float2)), o_pair = align16(o_tab + 2 * PHASOR_ENTRIES * sizeof(float2));
   const std::vector<int2> pairs = direction_pairs(dv, M, tensor);
   const int64_t Me = (int64_t)pairs.size();
   {  // every direction is written exactly once, as evaluated or as a mirror
@@ -444,7 +444,7 @@ int kgrid_create_impl(const double* dirs, const double* kmag, const double* w, i
   std::memcpy(host.data() + o_sw, sw.data(), Q * sizeof(float));
   std::memcpy(host.data() + o_sg, sg.data(), Q * sizeof(float));
   std::memcpy(host.data() + o_kt, kt.data(), L * sizeof(float2));
-  std::memcpy(host.data() + o_k256, k256.data(), L * sizeof(float2));
+  std::memcpy(host.data() + o_k64, k64.data(), L * sizeof(float2));
   std::memcpy(host.data() + o_tab, tab.data(), tab.size() * sizeof(float2));
   std::memcpy(host.data() + o_pair, pairs.data(), Me * sizeof(int2));
   {
@@ -479,7 +479,7 @@ int kgrid_create_impl(const double* dirs, const double* kmag, const double* w, i
   kg->dev.sqrtw = reinterpret_cast<const float*>(base + o_sw);
   kg->dev.sign = reinterpret_cast<const float*>(base + o_sg);
   kg->dev.kturn = reinterpret_cast<const float2*>(base + o_kt);
-  kg->dev.kt64 = reinterpret_cast<const float2*>(base + o_k256);
+  kg->dev.kt64 = reinterpret_cast<const float2*>(base + o_k64);
   kg->dev.cis_tab = reinterpret_cast<const float2*>(base + o_tab);
   kg->dev.cis_tabm = kg->dev.cis_tab + PHASOR_ENTRIES;
   kg->dev.dpair = reinterpret_cast<const int2*>(base + o_pair);

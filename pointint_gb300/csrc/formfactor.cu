@@ -9,8 +9,9 @@
 //    its AffineDoF / TriangleMeshDoF into an FP32 object-local frame (origin =
 //    centroid of the transformed anchors), centroids (centres) as FP32 hi + lo;
 //    the origin phase e^{ik.o} is formed and reduced in FP64 per output.
-//  * ff_kernel: the radii that the cluster expansions (moments.cu) leave, about
-//    the six largest of 64 (all of them on grids the expansions do not take).
+//  * ff_kernel: the radii that the cluster expansions (moments.cu) leave: 13 to
+//    17 of 64 for bodies of 5,120 triangles, whose leaves' expansions cover eight of
+//    them (all radii on grids the expansions do not take).
 //    One CTA = one object x 4 warps; a warp owns 32 directions
 //    (one per lane) x R neighbouring radial nodes of the factored k-grid, so
 //    each element's direction dot products and series coefficients are
@@ -19,7 +20,7 @@
 //    triangles have expansions of their own.  The CTAs of a thread-block
 //    cluster split the elements where few objects would leave SMs idle.
 //    Bound by instruction issue (63-70% active; 256 solids of 5,120 and 12
-//    triangles at N_k = 76,928: 38.8 ms for all radii, 12.2 now).  On a centrally
+//    triangles at N_k = 76,928: 38.8 ms for all radii, 12.4 now).  On a centrally
 //    symmetric direction set a lane evaluates one direction of an antipodal
 //    pair and writes both (A(-k) = -conj A(k) for a real solid: half the
 //    evaluations), and a warp's 32 directions form a compact cluster.  Radial
@@ -417,7 +418,8 @@ static_assert(PREP_THREADS % PI_CLUSTER == 0 && PI_CLUSTER == 64, "a cluster is 
 // pools and the bounding sphere of every cluster and leaf: its centre (that of the
 // bounding box, an FP32 point) and its radius, which for a surfel includes the
 // reach of its own expansion, rho |A| for a disk and 2.5 sigma |A| for a
-// Gaussian (the n-th root of E|Z|^n at n = 16 is 2.48).
+// Gaussian (the n-th root of E|Z|^n at n = 16 is 2.48), |A| bounded by the root of
+// its squared entries' sum.
 __global__ void __launch_bounds__(PREP_THREADS)
 prepare_elems_kernel(const PrepObj* objs, const ObjDev* od, float4* tri_pool, float4* surf_pool, float4* tri_lo,
                      float4* surf_lo, float4* surf_nref, const int32_t* perm, float4* clusters, float4* leaves,
@@ -1187,9 +1189,13 @@ int launch_form_factors(const pi_kgrid_impl* kg, const pi_batch_impl* b, int sca
   for (int i = 0; i < b->n_obj; ++i) heavy += 4 * b->info[i].n_elems >= n_max;
   auto busy = [&](int r) { return (K.moments ? (ctas(r) + 4) / 5 : ctas(r)) * heavy; };
   const int64_t wave = FF_CTAS * (int64_t)current_sm_count();
-  // four radii per thread where 16 splits at eight give less than 7/4 waves
-  // (8 clouds of 50,000 disks: 6.7 ms at four, 6.8 at eight; a solid of 200,000
-  // triangles, just above: 38.2 and 29.7)
+  // Four radii per thread where 16 splits at eight give less than 7/4 waves.  Both
+  // sides over 14 grids (L = 32 .. 128) and 16 batches: below 0.6 waves four takes 4 to
+  // 36% less, above five eight up to 16% less, and between them either may win,
+  // triangles and surfels alike: any line from 1 to 4.5 waves loses 1.1 to 1.4% in the
+  // mean.  A solid of 200,000 triangles on 5,810 directions,
+  // at four and at eight: 17.4 and 19.5 ms at 64 radii (0.97 waves), 23.1 and 24.7 at
+  // 112 (1.68), 25.8 and 25.4 at 128 (1.92).
   if (R == 8 && 4 * 16 * busy(8) < 7 * wave) R = 4;
   int S = 1;
   while (S < 16 && S * busy(R) < 2 * wave && n_max > 2 * S * FF_CHUNK) S *= 2;

@@ -360,7 +360,7 @@ jac_affine_tri_kernel(KGridDev kg, BatchDev b, const JacObj* __restrict__ jobs, 
   __shared__ float4 tile[7 * JAC_TILE];
   __shared__ float2 ctab_sm[PHASOR_ENTRIES * JAC_COPIES];
   const float2* ctab = ctab_sm + (threadIdx.x % JAC_COPIES);
-  __shared__ float4 krad[JAC_WARPS][R];  // (|k| hi, lo, |k| 256 / 2 pi hi, lo)
+  __shared__ float4 krad[JAC_WARPS][R];  // (|k| hi, lo, |k| 64 / 2 pi hi, lo)
   __shared__ float run[2 * JAC_NSUM * R * JAC_THREADS];  // running sums, then compensations
   stage_phasors<JAC_COPIES>(kg.cis_tab, ctab_sm);
   if (lane < R) {

@@ -39,9 +39,9 @@
 //
 // Bound by the FP32 pipe (58% busy, its packed instructions holding it two
 // cycles) and the waits between the two phases.  256 solids of 5,120 and 12
-// triangles, N_k = 76,928: 1.9 ms for about 58 of the 64 radii, which took 27 of
-// the 38.8 ms of the direct sum; one solid of 200,000 triangles on 743,680
-// nodes: 4.2 ms.
+// triangles, N_k = 76,928: 1.9 ms for 47 to 51 of the 64 radii (42 of a box), where
+// the direct sum of all radii took 38.8; one solid of 200,000 triangles on
+// 743,680 nodes: 4.4 ms for 115 of its 128.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <algorithm>
