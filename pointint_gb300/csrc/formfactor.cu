@@ -1099,7 +1099,7 @@ ff_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w, con
 }
 
 // CTAs per serving evaluation of each class (SERVE_CLASSES).
-constexpr int FF_SERVE_SPLIT[SERVE_CLASSES] = {16, 4, 1};
+constexpr int FF_SERVE_SPLIT[SERVE_CLASSES] = {16, 8, 4, 1};
 
 template <int R>
 __global__ void __launch_bounds__(FF_THREADS, FF_CTAS)

@@ -433,7 +433,7 @@ moment_kernel(KGridDev kg, BatchDev b, float2* __restrict__ J, int scale_sqrt_w,
 }
 
 // CTAs per serving evaluation of each class (SERVE_CLASSES).
-constexpr int FM_SERVE_SPLIT[SERVE_CLASSES] = {8, 2, 1};
+constexpr int FM_SERVE_SPLIT[SERVE_CLASSES] = {8, 4, 2, 1};
 
 __global__ void __launch_bounds__(FM_THREADS, 2)
 moment_serve_kernel(KGridDev kg, BatchDev b, const EvalDev* __restrict__ evals, int n_evals) {

@@ -253,18 +253,23 @@ int launch_to_double2(const float2* J, int64_t n, double* out, cudaStream_t s);
 int launch_jacobian(const pi_kgrid_impl* kg, const pi_batch_impl* b, float2* G, cudaStream_t s);
 // Serving evaluations.  The CTAs that share an object's elements (a thread-block
 // cluster) depend on its element count alone, so that a row's value does not
-// depend on the batch it is evaluated in: three classes, the largest objects
+// depend on the batch it is evaluated in: four classes, the largest objects
 // first, each a launch of its own over the class's evaluations.  At 16 CTAs for
 // every object 200 rotated boxes took 5,150 us, 15 of each 16 CTAs staging their
-// tables for no elements; at one 580.  Large ones need them: one mesh of 50,000
+// tables for no elements; at one 590.  Large ones need them: one mesh of 50,000
 // triangles 2.1 ms at 16 CTAs, 7.1 at 4, 26.8 at one.  The lines lie where bursts
 // of one to 200 objects cross: 80 triangles 177 .. 1,154 us at one CTA and 179 ..
 // 1,811 at 4, 720 triangles 474 .. 5,538 and 251 .. 6,125; 2,880 triangles 553 ..
-// 15,050 at 4 and 402 .. 19,705 at 16, 5,120 triangles 843 .. 5,239 (40 objects)
-// and 403 .. 6,476.
-constexpr int SERVE_CLASSES = 3;
-constexpr int64_t SERVE_LARGE = 4096, SERVE_SMALL = 256;  // above the first: class 0; up to the second: class 2
-constexpr int serve_class(int64_t n_elems) { return n_elems > SERVE_LARGE ? 0 : n_elems > SERVE_SMALL ? 1 : 2; }
+// 15,050 at 4, 410 .. 16,830 at 8 and 402 .. 19,705 at 16; 5,120 triangles 843 ..
+// 5,239 (40 objects) at 4 and 403 .. 6,476 at 16.  (The class at 8 is for single
+// meshes: a stream of scenes at 45 a second, p50 4.95 ms without it, 4.55 with.)
+constexpr int SERVE_CLASSES = 4;
+constexpr int64_t SERVE_MAX[SERVE_CLASSES - 1] = {4096, 1024, 256};  // elements of the classes 1, 2, 3
+constexpr int serve_class(int64_t n_elems) {
+  int c = 0;
+  while (c < SERVE_CLASSES - 1 && n_elems <= SERVE_MAX[c]) ++c;
+  return c;
+}
 // A class's kernel: arguments (KGridDev, BatchDev, const EvalDev*, int n, the class's
 // evaluations), grid (grid_x, n), `split` CTAs along x per cluster; with n = 0 it does nothing.
 struct ServeKernel {
@@ -275,7 +280,7 @@ struct ServeKernel {
 };
 ServeKernel ff_serve(const pi_kgrid_impl* kg, int cls);
 int ff_serve_setup(const pi_kgrid_impl* kg);  // before ff_serve's kernels are launched or put into a graph
-// evals: those of class 0, then 1, then 2, n_class[c] of each.
+// evals: those of class 0, then 1 and so on, n_class[c] of each.
 int launch_form_factors_serve(const pi_kgrid_impl* kg, const pi_batch_impl* lib, const EvalDev* evals,
                               const int (&n_class)[SERVE_CLASSES], cudaStream_t s);
 // After the serving evaluations: *amax_keep = *amax for the first *n_evals evals

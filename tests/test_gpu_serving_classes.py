@@ -1,4 +1,4 @@
-"""Serving evaluations by size of object: up to 256 elements, up to 4,096, more.
+"""Serving evaluations by size of object: up to 256 elements, up to 1,024, up to 4,096, more.
 
 A row is the same whatever evaluations share its batch (bit for bit, with and
 without graphs), and small objects do not pay for the large ones' split.
@@ -18,7 +18,7 @@ from test_gpu_parity import cond_rel_err
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [1, 12, 255, 256, 257, 1000, 4095, 4096, 4097, 6000]
+SIZES = [1, 12, 255, 256, 257, 1023, 1024, 1025, 4095, 4096, 4097, 6000]
 
 
 def moved(o, R, t):
