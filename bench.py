@@ -340,8 +340,8 @@ def run_gb300(args):
                 "evaluated_directions": {"evaluated": n_eval_dirs, "of": n_dirs},
                 "peak_source": f"nominal FP32: {FP32_FLOPS_PER_SM_PER_CLK} flops/clk/SM x {n_sm} SMs x {clk_max} MHz "
                                "(MEASURED_PEAKS.json holds HBM and bf16 tensor peaks only)",
-                "binding": "issue slots: ff_kernel (87% of the time) sums the few largest radii element by element, "
-                           "three table phasors each, and waits at its tile barriers where the directions of a "
+                "binding": "issue slots: ff_kernel (87% of the time) sums the largest radii element by element (13 to 17 "
+                           "of 64, the lower half of them through leaves of four), three table phasors each, and waits at its tile barriers where the directions of a "
                            "CTA's warps take different branches; sine/cosine are a phasor table and polynomials",
                 "pipes_from_capture": {"fma_pipe_active": FF_FMA_PIPE_ACTIVE, "issue_active": FF_ISSUE_ACTIVE,
                                        "source": "ncu counters of ff_kernel on 32 of the 256 objects"},
@@ -389,20 +389,20 @@ def run_gb300(args):
 
 # DRAM bytes (read + write) of one full-size launch of ff_kernel and
 # moment_kernel.  Reads: captured with ncu on 32 of the 256 objects (82,112
-# triangles: 5.94 and 7.46 MB) and scaled by the triangle count (656,896 /
+# triangles: 5.95 and 7.39 MB) and scaled by the triangle count (656,896 /
 # 82,112), since element reads grow with the elements.  Writes: that capture's
 # J (19.7 MB) stayed in L2, but the full J (256 x 76,928 complex64 = 157.5 MB)
 # exceeds the 129 MB L2 and is counted as written once, every node by one of
 # the two kernels.
-FF_TRAFFIC_BYTES_PER_LAUNCH = (5.94e6 + 7.46e6) * 656896 / 82112 + 256 * 76928 * 8
+FF_TRAFFIC_BYTES_PER_LAUNCH = (5.95e6 + 7.39e6) * 656896 / 82112 + 256 * 76928 * 8
 # Thread instructions per triangle x k pair of the evaluated directions, from
 # the two kernels' ncu capture on 32 of the 256 objects (smsp__inst_executed.sum
-# (1.391e9 + 0.135e9) x 32 / 3.158e9 pairs; packed FP32 instructions count once).
-FF_THREAD_INSTR_PER_EVAL = 15.5
+# (1.395e9 + 0.144e9) x 32 / 3.158e9 pairs; packed FP32 instructions count once).
+FF_THREAD_INSTR_PER_EVAL = 15.6
 # The same capture's FMA-pipe busy share of ff_kernel (sm__pipe_fma_cycles_active,
-# 48.2% of active cycles) and its issue-slot share (smsp__issue_active, 63.2%).
+# 48.2% of active cycles) and its issue-slot share (smsp__issue_active, 62.6%).
 FF_FMA_PIPE_ACTIVE = 0.482
-FF_ISSUE_ACTIVE = 0.632
+FF_ISSUE_ACTIVE = 0.626
 
 
 def _pcts(ms):
